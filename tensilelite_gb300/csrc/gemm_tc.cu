@@ -222,6 +222,10 @@ size_t tc_smem_bytes(int bm, int stages)
     return static_cast<size_t>(stages) * (kTcTileN * kTcRowBytes + bm * kTcRowBytes) + kTcEpiStageBytes + 1024 + 512;
 }
 
+// Staging buffers per epilogue warp: two where they fit beside the ring (every tile at up to six
+// 32 KB stages), else one.
+static int epi_buffers(size_t smem_one) { return smem_one + kTcEpiStageBytes <= kTcMaxSmem ? 2 : 1; }
+
 int tc_workers(int in_dtype, int out_dtype, int cl, int bm, int stages, int sm_count)
 {
     const int cta_group = cl >= 2 ? 2 : 1;
@@ -366,7 +370,9 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.num_kb = static_cast<int>((L.K + W - 1) / W);
     kp.kb_elems = W;
     kp.promote_kb = L.promote_k > 0 ? static_cast<int>((L.promote_k + W - 1) / W) : 0;
-    const size_t smem = tc_smem_bytes(L.bm / cta_group, L.stages);
+    size_t smem = tc_smem_bytes(L.bm / cta_group, L.stages);
+    kp.epi_bufs = epi_buffers(smem);
+    smem += static_cast<size_t>(kp.epi_bufs - 1) * kTcEpiStageBytes;
     const int64_t tiles = static_cast<int64_t>(kp.tiles_m) * kp.tiles_n * L.batch;
     kp.bal_kb = 0;
     kp.bal_workers = 0;
@@ -510,7 +516,9 @@ tl_status tc_grouped_launch(const TcGroupLaunch& G, cudaStream_t stream, int64_t
     kp.out_trunc = G.out_trunc;
     kp.err = G.err;
     kp.timeout_ns = G.timeout_ns;
-    const size_t smem = tc_smem_bytes(G.bm / cta_group, G.stages);
+    size_t smem = tc_smem_bytes(G.bm / cta_group, G.stages);
+    kp.epi_bufs = epi_buffers(smem);
+    smem += static_cast<size_t>(kp.epi_bufs - 1) * kTcEpiStageBytes;
     tl_status st = dispatch(G.in_dtype, G.out_dtype, cg, kp, G.ctas, G.sm_count, G.total_tiles, smem, stream, 0);
     if (st == TL_SUCCESS && launches) ++*launches;
     return st;

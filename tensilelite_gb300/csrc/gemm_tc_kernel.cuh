@@ -23,6 +23,7 @@ struct TcKernelParams {
     CUtensorMap tmN[3], tmM[3];   // split-precision pieces 0..2 (piece 0 = the operand itself)
     CUtensorMap tmD;              // the output, boxes of 128 bytes x 32 rows (tma_store)
     int tma_store;                // whole tiles leave through shared memory and TMA stores
+    int epi_bufs;                 // staging buffers of 4 KB per epilogue warp (1 or 2)
     int direct_last;              // a CTA's last tile (beta == 0) leaves through direct stores
     // fused epilogue (kernels instantiated with EPI): D = act(alpha*acc + beta*C + bias[m]), and
     // max |D| into *epi_amax
@@ -877,9 +878,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
     const uint32_t bmc = static_cast<uint32_t>(p.bm) / CG;            // m-side rows staged by this CTA
     const uint32_t tileN_bytes = kTcTileN * kTcRowBytes;
     const uint32_t stage_bytes = tileN_bytes + bmc * kTcRowBytes;
-    // output staging for TMA stores: 4 epilogue warps x 32 rows x 128 bytes, 1024-byte aligned
+    // output staging for TMA stores: 4 epilogue warps x epi_bufs x 32 rows x 128 bytes, 1024-byte aligned
     uint8_t* epi_stage = smem + static_cast<size_t>(p.stages) * stage_bytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + kTcEpiStageBytes);
+    uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + static_cast<size_t>(p.epi_bufs) * kTcEpiStageBytes);
     uint64_t* empty = full + kTcMaxStages;
     uint64_t* tfull = empty + kTcMaxStages;     // main accumulator buffers (per tile, or per chain)
     uint64_t* tempty = tfull + 2;
@@ -888,6 +889,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(sempty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     volatile int* last_flag = abort_flag + 1;
+
+    const uint32_t ring_a = ptx::smem_u32(smem), full_a = ptx::smem_u32(full), empty_a = ptx::smem_u32(empty);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -953,122 +956,176 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (each CTA)
-        // One flat loop over (k-block, product) per tile, run by the whole warp in step: its waits
-        // (single PTX blocks, voted across the warp) and bookkeeping are warp-uniform, and one
-        // elected lane issues the copies.
+        // One flat loop over (k-block, product) per tile, run by one lane: a wait on a completed barrier
+        // costs it 36 clocks (130 when 32 lanes ask), and everything that does not change from one
+        // k-block to the next (shared-memory and barrier addresses, the peer's barrier, the tensor
+        // maps of a single product) is formed outside the loop.  With the warp in step, a k-block
+        // cost this loop 465-570 clocks and the MMA issuer's 455-525 whatever the tile, more than the
+        // 256 clocks of a 128-column k-block's MMAs.
+        if (ptx::elect_one())
         {
-            uint32_t stage = 0, phase = 0;
+            uint32_t phase = 0;
             constexpr int W = kTcRowBytes / (KIND == 0 ? 2 : 1);   // elements per 128-byte row
-            const int n_mn = p.n_mn_major, m_mn = p.m_mn_major;
-            const int nstages = p.stages;
+            constexpr uint32_t kChunk = W * kTcRowBytes;           // bytes of one MN-major box
+            const bool skip = p.debug_skip_loads != 0;
+            // the barrier that counts this CTA's bytes: its own, or the pair leader's
+            const uint32_t full_off = (CG == 2) ? ptx::mapa_shared(full_a, pair_base) - empty_a : full_a - empty_a;
+            const int nchunk = static_cast<int>(bmc) / W;          // MN-major m-side boxes
+            const uint32_t bar_end = empty_a + 8u * static_cast<uint32_t>(p.stages);
+            uint32_t bar = empty_a;                // empty barrier and slot of the current stage
+            uint32_t sN = ring_a;
             bool ok = true;
-            int4 u_next = load_unit(p, unit0);
-            for (int64_t w = unit0; w < p.total_work && ok; w += units) {
-                const int4 u = u_next;
-                u_next = load_unit(p, w + units);      // in flight during this tile
-                TileJob j;
-                get_job(p, w, u, j);
-                const int n0 = j.n0 + static_cast<int>(rank) * kTcTileN;
-                const int m0 = j.m0 + static_cast<int>(pair_rank * bmc);
-                const int total = (j.kb1 - j.kb0) * nvirt;
-                int kb = j.kb0, v = 0;
-                // timeline stamps stay outside the k-block loops (a branch there slows the issue)
-                if (w == unit0 && lane == 0) trace_mark(p, TL_TRACE_LOAD_FIRST);
-                for (int i = 0; i < total; ++i) {
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty[stage], phase ^ 1u, tlim))) {
-                        if (lane == 0) record_error(p, abort_flag, 1);
-                        ok = false;
-                        break;
-                    }
-                    // the timeout-path test issues nothing: the full barriers never complete, the
-                    // MMA and epilogue waits run out, and no copy is left in flight
-                    if (!p.debug_skip_loads && ptx::elect_one()) {
-                        uint8_t* sN = smem + static_cast<size_t>(stage) * stage_bytes;
-                        uint8_t* sM = sN + tileN_bytes;
-                        // split-precision products, smallest first (term table set by the host)
-                        const void* mapN = p.group ? j.tmN : static_cast<const void*>(&p.tmN[p.term_n[v]]);
-                        const void* mapM = p.group ? j.tmM : static_cast<const void*>(&p.tmM[p.term_m[v]]);
-                        const int k0 = kb * W;
-                        if constexpr (CG == 2) {
-                            // the leader arms its full barrier with both CTAs' bytes; the peer's loads
-                            // only complete transactions on it (they cannot run a phase ahead: the
-                            // peer refills a slot only after the leader's MMAs released it)
-                            const uint32_t fb = ptx::mapa_shared(ptx::smem_u32(&full[stage]), pair_base);
-                            if (leader) ptx::mbar_arrive_expect_tx(&full[stage], 2u * stage_bytes);
-                            if (!n_mn) {
-                                ptx::tma_load_3d_pair(sN, mapN, fb, k0, n0, j.b);
-                            } else {
-#pragma unroll
-                                for (int c = 0; c < kTcTileN / W; ++c)
-                                    ptx::tma_load_3d_pair(sN + c * W * kTcRowBytes, mapN, fb, n0 + c * W, k0, j.b);
-                            }
-                            if constexpr (MC == 2) {
-                                // this CTA's half of the m rows shared with CTA pair_rank of the other
-                                // pair; the copy lands in both and is counted on each pair's leader
-                                const int half = static_cast<int>(rank >> 1);
-                                const uint16_t mask = static_cast<uint16_t>((1u << pair_rank) | (1u << (pair_rank + 2)));
-                                if (!m_mn)
-                                    ptx::tma_load_3d_pair_mc(sM + half * (bmc / 2) * kTcRowBytes, mapM, fb, mask, k0,
-                                                             m0 + half * static_cast<int>(bmc / 2), j.b);
-                                else
-                                    ptx::tma_load_3d_pair_mc(sM + half * W * kTcRowBytes, mapM, fb, mask,
-                                                             m0 + half * W, k0, j.b);
-                            } else if (!m_mn) {
-                                ptx::tma_load_3d_pair(sM, mapM, fb, k0, m0, j.b);
-                            } else {
-#pragma unroll
-                                for (int c = 0; c < 4; ++c)      // bmc / W <= 4 chunks
-                                    if (c * W < static_cast<int>(bmc))
-                                        ptx::tma_load_3d_pair(sM + c * W * kTcRowBytes, mapM, fb, m0 + c * W, k0, j.b);
-                            }
+            // one stage: wait for its slot, arm its full barrier, issue its copies
+            auto fill = [&](auto n_mn, auto m_mn, const void* mapN, const void* mapM, int k0, int n0, int m0, int b) {
+                if (!ptx::mbar_wait(bar, phase ^ 1u, tlim)) {
+                    record_error(p, abort_flag, 1);
+                    return false;
+                }
+                // the timeout-path test issues nothing: the full barriers never complete, the
+                // MMA and epilogue waits run out, and no copy is left in flight
+                if (!skip) {
+                    const uint32_t sM = sN + tileN_bytes;
+                    const uint32_t fb = bar + full_off;
+                    if constexpr (CG == 2) {
+                        // the leader arms its full barrier with both CTAs' bytes; the peer's loads
+                        // only complete transactions on it (they cannot run a phase ahead: the
+                        // peer refills a slot only after the leader's MMAs released it)
+                        if (leader) ptx::mbar_arrive_expect_tx(bar + (full_a - empty_a), 2u * stage_bytes);
+                        if constexpr (!decltype(n_mn)::value) {
+                            ptx::tma_load_3d_pair(sN, mapN, fb, k0, n0, b);
                         } else {
-                            ptx::mbar_arrive_expect_tx(&full[stage], stage_bytes);
-                            if (!n_mn) {
-                                ptx::tma_load_3d(sN, mapN, &full[stage], k0, n0, j.b);
-                            } else {
 #pragma unroll
-                                for (int c = 0; c < kTcTileN / W; ++c)
-                                    ptx::tma_load_3d(sN + c * W * kTcRowBytes, mapN, &full[stage], n0 + c * W, k0, j.b);
-                            }
-                            if (!m_mn) {
-                                ptx::tma_load_3d(sM, mapM, &full[stage], k0, m0, j.b);
-                            } else {
+                            for (int c = 0; c < kTcTileN / W; ++c)
+                                ptx::tma_load_3d_pair(sN + c * kChunk, mapN, fb, n0 + c * W, k0, b);
+                        }
+                        if constexpr (MC == 2) {
+                            // this CTA's half of the m rows shared with CTA pair_rank of the other
+                            // pair; the copy lands in both and is counted on each pair's leader
+                            const int half = static_cast<int>(rank >> 1);
+                            const uint16_t mask = static_cast<uint16_t>((1u << pair_rank) | (1u << (pair_rank + 2)));
+                            if constexpr (!decltype(m_mn)::value)
+                                ptx::tma_load_3d_pair_mc(sM + half * (bmc / 2) * kTcRowBytes, mapM, fb, mask, k0,
+                                                         m0 + half * static_cast<int>(bmc / 2), b);
+                            else
+                                ptx::tma_load_3d_pair_mc(sM + half * kChunk, mapM, fb, mask, m0 + half * W, k0, b);
+                        } else if constexpr (!decltype(m_mn)::value) {
+                            ptx::tma_load_3d_pair(sM, mapM, fb, k0, m0, b);
+                        } else {
 #pragma unroll
-                                for (int c = 0; c < 4; ++c)      // bmc / W <= 4 chunks
-                                    if (c * W < static_cast<int>(bmc))
-                                        ptx::tma_load_3d(sM + c * W * kTcRowBytes, mapM, &full[stage], m0 + c * W, k0, j.b);
-                            }
+                            for (int c = 0; c < 2; ++c)      // 64 or 128 m rows per CTA: at most two boxes
+                                if (c < nchunk) ptx::tma_load_3d_pair(sM + c * kChunk, mapM, fb, m0 + c * W, k0, b);
+                        }
+                    } else {
+                        ptx::mbar_arrive_expect_tx(fb, stage_bytes);
+                        if constexpr (!decltype(n_mn)::value) {
+                            ptx::tma_load_3d(sN, mapN, fb, k0, n0, b);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < kTcTileN / W; ++c)
+                                ptx::tma_load_3d(sN + c * kChunk, mapN, fb, n0 + c * W, k0, b);
+                        }
+                        if constexpr (!decltype(m_mn)::value) {
+                            ptx::tma_load_3d(sM, mapM, fb, k0, m0, b);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 4; ++c)      // at most four boxes
+                                if (c < nchunk) ptx::tma_load_3d(sM + c * kChunk, mapM, fb, m0 + c * W, k0, b);
                         }
                     }
-                    __syncwarp();
-                    if (++stage == static_cast<uint32_t>(nstages)) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
-                    if (++v == nvirt) {
-                        v = 0;
-                        ++kb;
-                    }
                 }
-                if (w == unit0 && lane == 0) trace_mark(p, TL_TRACE_LOAD_LAST);
+                bar += 8u;
+                sN += stage_bytes;
+                if (bar == bar_end) {
+                    bar = empty_a;
+                    sN = ring_a;
+                    phase ^= 1u;
+                }
+                return true;
+            };
+            auto produce = [&](auto n_mn, auto m_mn) {
+                int4 u_next = load_unit(p, unit0);
+                for (int64_t w = unit0; w < p.total_work && ok; w += units) {
+                    const int4 u = u_next;
+                    u_next = load_unit(p, w + units);      // in flight during this tile
+                    TileJob j;
+                    get_job(p, w, u, j);
+                    const int n0 = j.n0 + static_cast<int>(rank) * kTcTileN;
+                    const int m0 = j.m0 + static_cast<int>(pair_rank * bmc);
+                    // timeline stamps stay outside the k-block loops (a branch there slows the issue)
+                    if (w == unit0) trace_mark(p, TL_TRACE_LOAD_FIRST);
+                    int k0 = j.kb0 * W;
+                    if (nvirt == 1) {
+                        const void* mapN = j.tmN;
+                        const void* mapM = j.tmM;
+                        for (int i = j.kb1 - j.kb0; i > 0; --i) {
+                            if (!(ok = fill(n_mn, m_mn, mapN, mapM, k0, n0, m0, j.b))) break;
+                            k0 += W;
+                        }
+                    } else {
+                        // split-precision products, smallest first (term table set by the host)
+                        for (int i = j.kb1 - j.kb0; i > 0 && ok; --i) {
+                            for (int v = 0; v < nvirt; ++v)
+                                if (!(ok = fill(n_mn, m_mn, &p.tmN[p.term_n[v]], &p.tmM[p.term_m[v]], k0, n0, m0, j.b)))
+                                    break;
+                            k0 += W;
+                        }
+                    }
+                    if (w == unit0) trace_mark(p, TL_TRACE_LOAD_LAST);
+                }
+            };
+            using Yes = std::true_type;
+            using No = std::false_type;
+            if (p.n_mn_major) {
+                if (p.m_mn_major) produce(Yes{}, Yes{});
+                else produce(Yes{}, No{});
+            } else {
+                if (p.m_mn_major) produce(No{}, Yes{});
+                else produce(No{}, No{});
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader CTA)
         // Without promotion a tile's whole k range accumulates in one TMEM buffer (two buffers
         // alternate between tiles).  With promotion the A0*B0 product restarts its accumulation
         // every promote_kb k-blocks in the alternate buffer (the epilogue drains each chain into
         // fp32 registers), and the small split-precision products accumulate for the whole tile in
-        // a separate pair of buffers.  One flat loop per tile over (k-block, product), run by the
-        // whole warp in step (uniform waits and bookkeeping); one elected lane issues the MMAs and
-        // their commits.
-        if (leader) {
-            uint32_t stage = 0, phase = 0, mbuf = 0, mph = 0, sbuf = 0, sph = 0;
+        // a separate pair of buffers.  One flat loop per tile over (k-block, product), run by one
+        // lane (see the producer).
+        if (leader && ptx::elect_one()) {
+            uint32_t phase = 0, mbuf = 0, mph = 0, sbuf = 0, sph = 0;
             const uint16_t pair_mask = static_cast<uint16_t>(0x3u << pair_base);
             const uint32_t idesc = p.idesc;
-            const uint32_t n_kstep = p.n_kstep, m_kstep = p.m_kstep, n_lbo = p.n_lbo, m_lbo = p.m_lbo;
+            const uint32_t n_kstep = p.n_kstep >> 4, m_kstep = p.m_kstep >> 4;
             const uint32_t bmu = static_cast<uint32_t>(p.bm);
-            const int nstages = p.stages;
+            // the current slot: its full barrier and the low word of its n-side descriptor (the m-side
+            // word is a constant further, the high word a constant)
+            constexpr uint32_t dhi = ptx::sdesc_hi(1024);
+            const uint32_t dN0 = ptx::sdesc_lo(ring_a, p.n_lbo);
+            const uint32_t dNM = ptx::sdesc_lo(ring_a + tileN_bytes, p.m_lbo) - dN0;
+            const uint32_t dstep = stage_bytes >> 4;
+            const uint32_t bar_end = full_a + 8u * static_cast<uint32_t>(p.stages);
+            uint32_t dN = dN0, bar = full_a;
+            // one stage into `d_tmem`: wait for its bytes, issue its MMAs, release its slot when they complete
+            auto consume = [&](uint32_t d_tmem, uint32_t accumulate) {
+                if (!ptx::mbar_wait(bar, phase, tlim)) {
+                    record_error(p, abort_flag, 4);
+                    return false;
+                }
+                ptx::tc_fence_after();
+                ptx::mma_kblock<KIND, CG>(d_tmem, dN, dN + dNM, dhi, idesc, accumulate, n_kstep, m_kstep);
+                // both pairs' ring slots are released (MC == 2: every CTA of the cluster)
+                if constexpr (CG == 2) ptx::mma_commit_pair(bar + (empty_a - full_a), MC == 2 ? 0xF : 0x3);
+                else ptx::mma_commit(bar + (empty_a - full_a));
+                bar += 8u;
+                dN += dstep;
+                if (bar == bar_end) {
+                    bar = full_a;
+                    dN = dN0;
+                    phase ^= 1u;
+                }
+                return true;
+            };
             bool ok = true;
             int4 u_next = load_unit(p, unit0);
             for (int64_t w = unit0; w < p.total_work && ok; w += units) {
@@ -1078,114 +1135,78 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                 get_job(p, w, u, j);
                 const int nkb = j.kb1 - j.kb0;
                 if (nkb <= 0) continue;                 // an empty unit of a balanced split
-                const int chunk = promo ? p.promote_kb : nkb;
                 if (sep_small) {
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&sempty[sbuf], sph ^ 1u, tlim))) {
-                        if (lane == 0) record_error(p, abort_flag, 2);
+                    if (!ptx::mbar_wait(&sempty[sbuf], sph ^ 1u, tlim)) {
+                        record_error(p, abort_flag, 2);
                         break;
                     }
                     ptx::tc_fence_after();
                 }
-                if (nkb > 0) {
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim))) {
-                        if (lane == 0) record_error(p, abort_flag, 2);
-                        break;
-                    }
-                    ptx::tc_fence_after();
+                if (!ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
+                    record_error(p, abort_flag, 2);
+                    break;
                 }
-                bool main_started = false, small_started = false;
-                const int total = nkb * nvirt;
-                int v = 0, kb_in_chain = 0;
-                if (p.trace != nullptr && w == unit0 && total > 0) {
+                ptx::tc_fence_after();
+                if (p.trace != nullptr && w == unit0) {
                     // timeline: the first stage's arrival, waited for here (the loop's own wait on
                     // it then passes at once) so that the k-block loop carries no stamp
-                    ptx::mbar_wait(&full[stage], phase, tlim);
-                    if (lane == 0) trace_mark(p, TL_TRACE_MMA_FIRST);
-                    __syncwarp();
+                    ptx::mbar_wait(bar, phase, tlim);
+                    trace_mark(p, TL_TRACE_MMA_FIRST);
                 }
-                for (int i = 0; i < total; ++i) {
-                    if (!__all_sync(0xffffffffu, ptx::mbar_wait(&full[stage], phase, tlim))) {
-                        if (lane == 0) record_error(p, abort_flag, 4);
-                        ok = false;
-                        break;
+                if (!promo) {
+                    // every product of the tile into one accumulator
+                    const uint32_t d_tmem = tmem_base + mbuf * bmu;
+                    uint32_t accumulate = 0;
+                    for (int i = nkb * nvirt; i > 0; --i) {
+                        if (!(ok = consume(d_tmem, accumulate))) break;
+                        accumulate = 1;
                     }
-                    ptx::tc_fence_after();
-                    const bool is_main = !sep_small || v == nvirt - 1;
-                    const uint32_t d_tmem = tmem_base + (is_main ? mbuf * bmu : (2u + sbuf) * bmu);
-                    const bool started = is_main ? main_started : small_started;
-                    const uint32_t sN = ptx::smem_u32(smem + static_cast<size_t>(stage) * stage_bytes);
-                    const uint32_t sM = sN + tileN_bytes;
-                    if (ptx::elect_one()) {
-#pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            const uint64_t adesc = ptx::sdesc_sw128(sN + ks * n_kstep, n_lbo, 1024);
-                            const uint64_t bdesc = ptx::sdesc_sw128(sM + ks * m_kstep, m_lbo, 1024);
-                            const uint32_t accumulate = (started || ks > 0) ? 1u : 0u;
-                            if constexpr (CG == 2) {
-                                if (KIND == 0) ptx::mma_f16_pair(d_tmem, adesc, bdesc, idesc, accumulate);
-                                else ptx::mma_f8_pair(d_tmem, adesc, bdesc, idesc, accumulate);
-                            } else {
-                                if (KIND == 0) ptx::mma_f16(d_tmem, adesc, bdesc, idesc, accumulate);
-                                else ptx::mma_f8(d_tmem, adesc, bdesc, idesc, accumulate);
-                            }
-                        }
-                        // both pairs' ring slots are released (MC == 2: every CTA of the cluster)
-                        if constexpr (CG == 2) ptx::mma_commit_pair(&empty[stage], MC == 2 ? 0xF : 0x3);
-                        else ptx::mma_commit(&empty[stage]);
-                    }
-                    __syncwarp();
-                    main_started = main_started || is_main;
-                    small_started = small_started || !is_main;
-                    if (++stage == static_cast<uint32_t>(nstages)) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
-                    if (++v == nvirt) {
-                        v = 0;
-                        // end of a chain of the main product: hand it to the epilogue, continue in
-                        // the other buffer (a tile's last chain is handed over after the loop)
-                        if (++kb_in_chain == chunk && i + 1 < total) {
-                            if (ptx::elect_one()) {
-                                if constexpr (CG == 2) ptx::mma_commit_pair(&tfull[mbuf], pair_mask);
-                                else ptx::mma_commit(&tfull[mbuf]);
-                            }
-                            __syncwarp();
+                } else {
+                    uint32_t main_acc = 0, small_acc = 0;
+                    int in_chain = 0;
+                    for (int kb = 0; kb < nkb && ok; ++kb) {
+                        if (in_chain == p.promote_kb) {
+                            // end of a chain of the main product: hand it to the epilogue, continue in
+                            // the other buffer (a tile's last chain is handed over after the loop)
+                            if constexpr (CG == 2) ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
+                            else ptx::mma_commit(ptx::smem_u32(&tfull[mbuf]));
                             mbuf ^= 1u;
                             if (mbuf == 0) mph ^= 1u;
-                            kb_in_chain = 0;
-                            main_started = false;
-                            if (!__all_sync(0xffffffffu, ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim))) {
-                                if (lane == 0) record_error(p, abort_flag, 2);
+                            in_chain = 0;
+                            main_acc = 0;
+                            if (!ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
+                                record_error(p, abort_flag, 2);
                                 ok = false;
                                 break;
                             }
                             ptx::tc_fence_after();
                         }
+                        for (int v = 0; v < nvirt - 1 && ok; ++v) {
+                            ok = consume(tmem_base + (2u + sbuf) * bmu, small_acc);
+                            small_acc = 1;
+                        }
+                        if (ok) ok = consume(tmem_base + mbuf * bmu, main_acc);
+                        main_acc = 1;
+                        ++in_chain;
                     }
                 }
                 if (!ok) break;
-                if (ptx::elect_one()) {
-                    if (nkb > 0) {
-                        if constexpr (CG == 2) ptx::mma_commit_pair(&tfull[mbuf], pair_mask);
-                        else ptx::mma_commit(&tfull[mbuf]);
-                    }
-                    if (sep_small) {
-                        if constexpr (CG == 2) ptx::mma_commit_pair(&sfull[sbuf], pair_mask);
-                        else ptx::mma_commit(&sfull[sbuf]);
-                    }
+                if constexpr (CG == 2) ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
+                else ptx::mma_commit(ptx::smem_u32(&tfull[mbuf]));
+                if (sep_small) {
+                    if constexpr (CG == 2) ptx::mma_commit_pair(ptx::smem_u32(&sfull[sbuf]), pair_mask);
+                    else ptx::mma_commit(ptx::smem_u32(&sfull[sbuf]));
                 }
-                __syncwarp();
-                if (w == unit0 && lane == 0) trace_mark(p, TL_TRACE_MMA_LAST);
-                if (nkb > 0) {
-                    mbuf ^= 1u;
-                    if (mbuf == 0) mph ^= 1u;
-                }
+                if (w == unit0) trace_mark(p, TL_TRACE_MMA_LAST);
+                mbuf ^= 1u;
+                if (mbuf == 0) mph ^= 1u;
                 if (sep_small) {
                     sbuf ^= 1u;
                     if (sbuf == 0) sph ^= 1u;
                 }
             }
         }
+        __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue (4 warps, each CTA)
         // All four warps run the same loop and, in split-k mode, the same named barriers: after a
@@ -1194,6 +1215,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
         const int quarter = warp & 3;             // TMEM lanes 32*quarter .. +31
         const int row = quarter * 32 + lane;      // tile row = problem n offset within this CTA
         const int et = threadIdx.x - 64;          // 0..127
+        uint8_t* const my_stage = epi_stage + static_cast<size_t>(quarter) * p.epi_bufs * 4096u;   // this warp's staging
+        const uint32_t my_stage_a = ptx::smem_u32(my_stage);
+        uint32_t stage_off = 0;                   // buffer the next staged store fills
         const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
         uint32_t mbuf = 0, mph = 0, sbuf = 0, sph = 0;
         const int chunks = p.bm / 32;
@@ -1248,7 +1272,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                 const int nkb = j.kb1 - j.kb0;
                 const int nchain = (nkb + p.promote_kb - 1) / p.promote_kb;
                 for (int c = 0; c < nchain; ++c) {
-                    bool got = ok && ptx::mbar_wait(&tfull[mbuf], mph, tlim, abort_flag);
+                    bool got = ok && ptx::mbar_wait(&tfull[mbuf], mph, tlim);
                     got = __all_sync(0xffffffffu, got);
                     if (ok && !got) {
                         if (lane == 0) record_error(p, abort_flag, 8);
@@ -1271,7 +1295,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                     if (mbuf == 0) mph ^= 1u;
                 }
                 if (sep_small) {
-                    bool got = ok && ptx::mbar_wait(&sfull[sbuf], sph, tlim, abort_flag);
+                    bool got = ok && ptx::mbar_wait(&sfull[sbuf], sph, tlim);
                     got = __all_sync(0xffffffffu, got);
                     if (ok && !got) {
                         if (lane == 0) record_error(p, abort_flag, 8);
@@ -1329,8 +1353,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
             // output staging buffer (free in this mode: no TMA store is in flight from it) while the
             // tile accumulates.
             bool c_staged = false;
-            const uint32_t c_row = ptx::smem_u32(epi_stage) + static_cast<uint32_t>(quarter) * 4096u +
-                                   static_cast<uint32_t>(lane) * 128u;
+            const uint32_t c_row = my_stage_a + static_cast<uint32_t>(lane) * 128u;
             if constexpr (sizeof(TD) >= 2) {
                 const int mc = j.m0 + j.split * 32;
                 if (p.par_reduce && !j.out_t && j.nsplit > 1 && j.beta != 0.0f && j.C != nullptr && j.split * 32 < p.bm) {
@@ -1347,7 +1370,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                     ptx::cp_async_commit();
                 }
             }
-            bool got = ok && ptx::mbar_wait(&tfull[mbuf], mph, tlim, abort_flag);
+            // (D may be C itself: a chunk's C is read before any of its columns is stored)
+            uint32_t cw[32];
+            if (row_ok && j.nsplit == 1 && !j.out_t && j.tmD != nullptr) load_c_chunk<TD>(j, base_c, j.m0, cw);
+            bool got = ok && ptx::mbar_wait(&tfull[mbuf], mph, tlim);
             got = __all_sync(0xffffffffu, got);
             if (ok && !got) {
                 if (lane == 0) record_error(p, abort_flag, 8);
@@ -1365,23 +1391,24 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                 if (j.out_t && j.nsplit == 1 && j.tmD != nullptr) {
                     // transposed output: a warp's 32 rows are 32 consecutive elements of D's columns,
                     // so each 32-column chunk is one 32 x 32 box of D, staged [column][row] (two boxes
-                    // per 4 KB buffer for 16-bit outputs, one for fp32) and written by one TMA store;
-                    // a box's buffer is refilled once the store two (16-bit) or one (fp32) back has
-                    // read it.  With beta, lane L first brings column L of the chunk's C (contiguous
+                    // per 4 KB buffer for 16-bit outputs, one for fp32) and written by one TMA store.
+                    // The boxes are filled in turn, one per committed store; a box is refilled once
+                    // the store that last used it has read it.  With beta, lane L first brings column L of the chunk's C (contiguous
                     // in memory) into the box, and every lane then replaces its row of C by D.
                     constexpr int CB = 32 * 32 * static_cast<int>(sizeof(TD));   // bytes per box
-                    constexpr int NB = 4096 / CB;
+                    const uint32_t stage_bytes_all = static_cast<uint32_t>(p.epi_bufs) * 4096u;
                     constexpr int COLB = CB / 32;                                  // bytes per box column
                     const int nrow0 = j.n0 + quarter * 32;
                     const bool use_c = j.beta != 0.0f && j.C != nullptr;
                     for (int c = 0; c < chunks && ok; ++c) {
                         const int m = j.m0 + c * 32;
                         if (lane == 0) {
-                            if constexpr (NB == 2) ptx::bulk_wait_read1();
+                            if (stage_bytes_all == 4 * CB) ptx::bulk_wait_read3();
+                            else if (stage_bytes_all == 2 * CB) ptx::bulk_wait_read1();
                             else ptx::bulk_wait_read0();
                         }
                         __syncwarp();
-                        uint8_t* box = epi_stage + quarter * 4096 + (c % NB) * CB;
+                        uint8_t* box = my_stage + stage_off;
                         const uint32_t ba = ptx::smem_u32(box);
                         if (use_c) {
                             const int ccol = m + lane;
@@ -1442,9 +1469,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                         }
                         ptx::fence_proxy_async_smem();
                         __syncwarp();
-                        if (lane == 0 && m < j.M && nrow0 < j.N) {
-                            ptx::tma_store_3d(j.tmD, box, nrow0, m, j.b);
-                            ptx::bulk_commit();
+                        if (m < j.M && nrow0 < j.N) {
+                            if (lane == 0) {
+                                ptx::tma_store_3d(j.tmD, box, nrow0, m, j.b);
+                                ptx::bulk_commit();
+                            }
+                            stage_off += CB;
+                            if (stage_off == stage_bytes_all) stage_off = 0;
                         }
                     }
                     if (tr) trace_mark(p, TL_TRACE_STORED);
@@ -1456,25 +1487,28 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
             if (j.nsplit == 1 && j.tmD != nullptr && !direct) {
                 // each warp stages its 32 rows x 128 bytes of output (128-byte swizzle: 16-byte unit
                 // u of row r sits at u ^ (r & 7)) and writes them with one TMA store; the tensor
-                // map clips the ragged edges.  One staging buffer per warp: before refilling it the
-                // issuing lane waits until the previous store has read it.
+                // map clips the ragged edges.  With two buffers per warp a store is read out of one
+                // while the other fills (the issuing lane waits until the store before the last has
+                // been read); with one, every 128 bytes of columns wait ~1 us for the store before.
+                // C of the next 32 columns is in flight while the current ones are finished.
                 constexpr int CPS = static_cast<int>(4 / sizeof(TD));    // 32-column chunks per 128 bytes
-                const uint32_t stg = ptx::smem_u32(epi_stage) + static_cast<uint32_t>(quarter) * 4096u;
                 const int nrow0 = j.n0 + quarter * 32;
                 for (int c0 = 0; c0 < chunks && ok; c0 += CPS) {
                     const int m = j.m0 + c0 * 32;
-                    if (lane == 0) ptx::bulk_wait_read0();
+                    if (lane == 0) {
+                        if (p.epi_bufs == 2) ptx::bulk_wait_read1();
+                        else ptx::bulk_wait_read0();
+                    }
                     __syncwarp();
-                    const uint32_t rowaddr = stg + static_cast<uint32_t>(lane) * 128u;
+                    const uint32_t rowaddr = my_stage_a + stage_off + static_cast<uint32_t>(lane) * 128u;
 #pragma unroll
                     for (int q = 0; q < CPS; ++q) {
-                        uint32_t cw[32];
-                        if (row_ok) load_c_chunk<TD>(j, base_c, m + 32 * q, cw);
                         uint32_t r[32];
                         __syncwarp();
                         ptx::tmem_ld32(tbase + (c0 + q) * 32, r);
                         uint32_t w[32 / CPS];
                         finish_pack<TD, EPI>(p, amax, j, m + 32 * q, row_ok, r, cw, p.out_trunc, w);
+                        if (row_ok && c0 + q + 1 < chunks) load_c_chunk<TD>(j, base_c, m + 32 * (q + 1), cw);
 #pragma unroll
                         for (int uu = 0; uu < 8 / CPS; ++uu) {
                             const int u = q * (8 / CPS) + uu;
@@ -1485,9 +1519,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                     if (c0 + CPS >= chunks) release_tmem<CG>(&tempty[mbuf], lane);
                     ptx::fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0 && m < j.M && nrow0 < j.N) {
-                        ptx::tma_store_3d(j.tmD, epi_stage + quarter * 4096, m, nrow0, j.b);
-                        ptx::bulk_commit();
+                    if (m < j.M && nrow0 < j.N) {
+                        if (lane == 0) {
+                            ptx::tma_store_3d(j.tmD, my_stage + stage_off, m, nrow0, j.b);
+                            ptx::bulk_commit();
+                        }
+                        // the buffers alternate with the committed stores, which the wait counts
+                        if (p.epi_bufs == 2) stage_off ^= 4096u;
                     }
                 }
                 if (tr) trace_mark(p, TL_TRACE_STORED);
@@ -1571,7 +1609,7 @@ tl_status launch_kernel(const TcKernelParams& kp, int grid, size_t smem, cudaStr
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [&] {
-        attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        attr_err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTcMaxSmem));
     });
     if (attr_err != cudaSuccess) return cuda_fail(attr_err, "cudaFuncSetAttribute(tc_gemm_kernel)");
     cudaLaunchConfig_t cfg;
@@ -1616,7 +1654,7 @@ int max_clusters(size_t smem)
     auto it = cache.find(smem);
     if (it != cache.end()) return it->second;
     auto kern = tc_gemm_kernel<KIND, TD, CL, false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTcMaxSmem));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(CL, 1, 1);

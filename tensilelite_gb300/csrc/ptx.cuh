@@ -61,10 +61,9 @@ __device__ __forceinline__ void fence_proxy_async_smem()
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes)
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes)
 {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
@@ -72,7 +71,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar)
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 {
     uint32_t ok;
     asm volatile(
@@ -80,41 +79,44 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
 }
 
-// Bounded wait on the phase with the given parity: spins on mbarrier.try_wait until the phase has
-// completed (true) or `limit_ns` of %globaltimer time has passed (false; the caller records the
-// timeout and leaves its loop).  The whole spin is one PTX block, so a single-lane issue loop that
-// calls it carries no data-dependent inner loop of its own (which measurably slowed tcgen05.mma
-// issue from such a loop).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns,
-                                          const volatile int* /*abort*/ = nullptr)
+// Bounded wait on the phase with the given parity: true once the phase has completed, false when
+// `limit_ns` of %globaltimer time has passed (the caller records the timeout and leaves its loop).
+// `bar` is a shared-memory address.  A phase that has completed, or completes while the hardware holds
+// the first try_wait, costs one instruction and a predicate; the spin (one PTX block, so an issue loop that
+// calls it carries no data-dependent inner loop of its own) is off that path.  Called by one lane it
+// costs 36 clocks on a completed phase; by 32 lanes 130.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns)
 {
+    if (mbar_try_wait(bar, parity)) return true;
     uint32_t ok;
     asm volatile(
         "{\n\t"
         ".reg .pred p, q;\n\t"
         ".reg .u64 t0, t1;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra.uni TL_WAIT_DONE;\n\t"
         "mov.u64 t0, %%globaltimer;\n\t"
         "TL_WAIT_LOOP:\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "@p bra.uni TL_WAIT_DONE;\n\t"
+        "@p bra TL_WAIT_DONE;\n\t"
         "mov.u64 t1, %%globaltimer;\n\t"
         "sub.u64 t1, t1, t0;\n\t"
         "setp.lt.u64 q, t1, %3;\n\t"
-        "@q bra.uni TL_WAIT_LOOP;\n\t"
+        "@q bra TL_WAIT_LOOP;\n\t"
         "TL_WAIT_DONE:\n\t"
         "selp.u32 %0, 1, 0, p;\n\t"
         "}\n"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "l"(limit_ns)
+        : "r"(bar), "r"(parity), "l"(limit_ns)
         : "memory");
     return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns)
+{
+    return mbar_wait(smem_u32(bar), parity, limit_ns);
 }
 
 // ---- TMA ---------------------------------------------------------------------------------------
@@ -125,13 +127,12 @@ __device__ __forceinline__ void prefetch_tmap(const void* tmap)
 
 // 3-D tiled load of one box into shared memory; completion is signalled as transaction bytes on
 // `bar`.  The x coordinate times the element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, uint64_t* bar, int x, int y,
-                                            int z)
+__device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const void* tmap, uint32_t bar, int x, int y, int z)
 {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
-        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_dst),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
 
@@ -156,36 +157,49 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]^T, 16-bit inputs (f16 or bf16 per idesc), fp32 accum.
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                        uint32_t accumulate)
+// One k-block of D[tmem] (+)= A * B^T: four tcgen05.mma along k, issued by one thread.  A descriptor's
+// high word is the same for every tile (sdesc_hi); its low word (sdesc_lo) advances by `a_step` /
+// `b_step` (16-byte units) per k step.  `accumulate` 0 starts the accumulator with the first product.
+// KIND 0: 16-bit inputs (f16 or bf16 per idesc); 1: E4M3.  CG 2: the pair MMA, issued by the leader CTA:
+// A rows and B rows (N) are split between the two CTAs' shared memory at the same offsets; D rows
+// 0-127 land in the leader's TMEM, 128-255 in the peer's.
+// One block for the four, with the descriptors formed by a single add each: the issuing warp's
+// instructions per k-block bound the main loop of tiles narrower than 256 columns (an MMA takes 64
+// clocks at 128 columns and 49 at 64; with 64-bit descriptors built from their fields for every
+// MMA a k-block took 500 clocks whatever its width).
+#define TL_MMA4(GROUP, KINDSTR)                                                                          \
+    asm volatile(                                                                                        \
+        "{\n\t.reg .pred p, q;\n\t.reg .b32 al, bl;\n\t.reg .b64 ad, bd;\n\t"                                 \
+        "setp.ne.b32 p, %5, 0;\n\tsetp.eq.u32 q, 0, 0;\n\t"                                                \
+        "mov.b64 ad, {%1, %3};\n\t"                                                                      \
+        "mov.b64 bd, {%2, %3};\n\t"                                                                      \
+        "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], ad, bd, %4, p;\n\t"                     \
+        "add.u32 al, %1, %6;\n\tadd.u32 bl, %2, %7;\n\t"                                                 \
+        "mov.b64 ad, {al, %3};\n\tmov.b64 bd, {bl, %3};\n\t"                                             \
+        "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], ad, bd, %4, q;\n\t"                     \
+        "add.u32 al, al, %6;\n\tadd.u32 bl, bl, %7;\n\t"                                                 \
+        "mov.b64 ad, {al, %3};\n\tmov.b64 bd, {bl, %3};\n\t"                                             \
+        "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], ad, bd, %4, q;\n\t"                     \
+        "add.u32 al, al, %6;\n\tadd.u32 bl, bl, %7;\n\t"                                                 \
+        "mov.b64 ad, {al, %3};\n\tmov.b64 bd, {bl, %3};\n\t"                                             \
+        "tcgen05.mma.cta_group::" GROUP ".kind::" KINDSTR " [%0], ad, bd, %4, q;\n\t}\n" ::"r"(d_tmem),    \
+        "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(a_step), "r"(b_step)               \
+        : "memory")
+template <int KIND, int CG>
+__device__ __forceinline__ void mma_kblock(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                           uint32_t accumulate, uint32_t a_step, uint32_t b_step)
 {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if constexpr (KIND == 0 && CG == 1) TL_MMA4("1", "f16");
+    else if constexpr (KIND == 0) TL_MMA4("2", "f16");
+    else if constexpr (CG == 1) TL_MMA4("1", "f8f6f4");
+    else TL_MMA4("2", "f8f6f4");
 }
-
-// Same with 8-bit float inputs (E4M3 per idesc), fp32 accumulation.
-__device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
+#undef TL_MMA4
 
 // Arrive once on `bar` when every tcgen05 operation issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* bar)
+__device__ __forceinline__ void mma_commit(uint32_t bar)
 {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // Warp-collective load of 32 consecutive fp32 columns of this warp's 32 TMEM lanes; waits for the
@@ -212,15 +226,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
 // K-major tiles: rows of 128 bytes, 8-row groups 1024 bytes apart (SBO); LBO unused.
 // MN-major tiles: 128-byte rows along MN, one row per k; 8-k groups SBO apart, 64-element MN
 // chunks LBO apart.
-__device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes)
+// The low word (start address, LBO) and the high word (SBO and the fixed fields) separately: a tile
+// address below 256 KB leaves the LBO field alone when a low word is advanced by 16-byte units.
+__device__ __forceinline__ uint32_t sdesc_lo(uint32_t saddr, uint32_t lbo_bytes)
 {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-    d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
-    return d;
+    return ((saddr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
+}
+__device__ __forceinline__ constexpr uint32_t sdesc_hi(uint32_t sbo_bytes)
+{
+    return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (2u << 29);
 }
 
 // ---- clusters and the CTA pair (cta_group::2) ----------------------------------------------------
@@ -265,23 +279,23 @@ __device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_a
 }
 // TMA load into this CTA's shared memory whose completion is signalled on an mbarrier that may live
 // in the peer CTA of the pair (cluster address).
-__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const void* tmap, uint32_t mbar_cluster_addr, int x,
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t smem_dst, const void* tmap, uint32_t mbar_cluster_addr, int x,
                                                  int y, int z)
 {
     asm volatile(
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(smem_dst)),
+        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_dst),
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(mbar_cluster_addr), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
 // The same load multicast to the CTAs in `cta_mask` (same shared-memory offset in each); each
 // destination's completion is counted on the mbarrier at the given offset in its own pair's leader.
-__device__ __forceinline__ void tma_load_3d_pair_mc(void* smem_dst, const void* tmap, uint32_t mbar_cluster_addr,
+__device__ __forceinline__ void tma_load_3d_pair_mc(uint32_t smem_dst, const void* tmap, uint32_t mbar_cluster_addr,
                                                     uint16_t cta_mask, int x, int y, int z)
 {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.multicast::cluster"
-        ".cta_group::2 [%0], [%1, {%4, %5, %6}], [%2], %3;" ::"r"(smem_u32(smem_dst)),
+        ".cta_group::2 [%0], [%1, {%4, %5, %6}], [%2], %3;" ::"r"(smem_dst),
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(mbar_cluster_addr), "h"(cta_mask), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
@@ -299,6 +313,7 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 // Wait until the committed bulk stores of this thread have finished reading shared memory.
 __device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read3() { asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory"); }
 __device__ __forceinline__ void st_shared_u16(uint32_t addr, uint16_t v)
 {
     asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
@@ -353,35 +368,12 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// Pair MMA issued by one thread of the leader CTA: A rows and B rows (N) are split between the two
-// CTAs' shared memory at the same offsets; D rows 0-127 land in the leader's TMEM, 128-255 in the peer's.
-__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void mma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // Arrive once on the mbarrier at this offset in every CTA of `cta_mask` when the pair MMAs issued so
 // far by this thread have completed.
-__device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint16_t cta_mask)
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint16_t cta_mask)
 {
     asm volatile(
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-            smem_u32(bar)),
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
         "h"(cta_mask)
         : "memory");
 }
