@@ -20,9 +20,11 @@ CLI = os.path.join(HERE, "tensilelite")
 
 SOURCES = ["gemm_tc.cu", "gemm_simt.cu", "aux_kernels.cu", "tl_api.cpp", "noalloc.cu"]
 # The tcgen05 kernel template is instantiated in generated units, one per operand kind (0 fp16/bf16,
-# 1 fp8), cluster size and epilogue variant, so they compile in parallel.  Plain kernels write fp32,
-# fp16 or bf16; the fused-epilogue kernels also fp8 (E4M3).
-INSTANCES = [(k, e, cl) for k in (0, 1) for e in (False, True) for cl in (1, 2, 4)]
+# 1 fp8), epilogue variant, cluster size, promotion and grouping, so they compile in parallel.  Plain
+# kernels write fp32, fp16 or bf16; the fused-epilogue kernels also fp8 (E4M3).  Two pairs per cluster
+# (4) have no promotion, grouped kernels neither promotion nor a fused epilogue.
+INSTANCES = [(k, e, cl, pr, g) for k in (0, 1) for e in (False, True) for cl in (1, 2, 4) for pr in (False, True)
+             for g in (False, True) if not (pr and cl == 4) and not (g and (e or pr))]
 OUT_TYPES = ("float", "__half", "__nv_bfloat16")
 EPI_OUT_TYPES = OUT_TYPES + ("__nv_fp8_e4m3",)
 
@@ -31,16 +33,17 @@ def _instance_sources():
     gen = os.path.join(BUILD, "gen")
     os.makedirs(gen, exist_ok=True)
     paths = []
-    for k, e, cl in INSTANCES:
+    flag = {False: "false", True: "true"}
+    for k, e, cl, pr, g in INSTANCES:
         lines = ['#include "tensilelite_gb300/csrc/gemm_tc_kernel.cuh"', "namespace tl {", "namespace tc {"]
         for td in (EPI_OUT_TYPES if e else OUT_TYPES):
-            lines.append(f"template tl_status launch_kernel<{k}, {td}, {cl}, {'true' if e else 'false'}>("
+            lines.append(f"template tl_status launch_kernel<{k}, {td}, {cl}, {flag[e]}, {flag[pr]}, {flag[g]}>("
                          "const TcKernelParams&, int, size_t, cudaStream_t);")
-            if not e:
+            if not e and not pr and not g:
                 lines.append(f"template int max_clusters<{k}, {td}, {cl}>(size_t);")
         lines += ["}  // namespace tc", "}  // namespace tl", ""]
         text = "\n".join(lines)
-        path = os.path.join(gen, f"tc_k{k}_e{int(e)}_c{cl}.cu")
+        path = os.path.join(gen, f"tc_k{k}_e{int(e)}_c{cl}_p{int(pr)}_g{int(g)}.cu")
         if not os.path.exists(path) or open(path).read() != text:
             with open(path, "w") as f:
                 f.write(text)

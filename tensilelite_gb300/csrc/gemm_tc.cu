@@ -10,11 +10,12 @@
 // :1822-1906) becomes four warps draining TMEM with tcgen05.ld while the next tile accumulates into
 // the second TMEM buffer.
 //
-// Roles (192 threads, one CTA per SM, persistent over work units):
-//   warp 0     TMA producer: per k-block one box of B (128 n-rows) and one of A (bm m-rows)
-//   warp 1     TMEM allocator + MMA issuer (lane 0): 4 tcgen05.mma per k-block, commit -> empty
-//   warps 2-5  epilogue: TMEM lane = problem n, TMEM column = problem m, so each thread owns a
+// Roles (320 threads, one CTA per SM, persistent over work units):
+//   warp 0     TMA producer (one lane): per k-block one box of B (128 n-rows) and one of A (bm m-rows)
+//   warp 1     TMEM allocator + MMA issuer (one lane): 4 tcgen05.mma per k-block, commit -> empty
+//   warps 2-9  epilogue: TMEM lane = problem n, TMEM column = problem m, so each thread owns a
 //              contiguous run of m for one n -- column-major D rows are written as 16-byte vectors.
+//              (The promotion kernels have four epilogue warps with 128 running sums per thread.)
 // The problem's B^T is the MMA "A" operand (M = 128 along n) and A is the MMA "B" operand
 // (N = bm along m).  K-major operands (TN, the reference's layout) and MN-major operands (NN/NT)
 // are both read straight from global memory by TMA with 128-byte swizzling; no transpose pass.
@@ -35,13 +36,20 @@ namespace tl {
 namespace tc {
 
 // instantiated in the generated instance units (one per operand kind, cluster size, epilogue)
-#define TL_TC_EXTERN(K, TD, CL, E) extern template tl_status launch_kernel<K, TD, CL, E>(const TcKernelParams&, int, size_t, cudaStream_t);
-#define TL_TC_EXTERN_CL(K, CL)                                                                                 \
-    TL_TC_EXTERN(K, float, CL, false) TL_TC_EXTERN(K, __half, CL, false) TL_TC_EXTERN(K, __nv_bfloat16, CL, false) \
-    TL_TC_EXTERN(K, float, CL, true) TL_TC_EXTERN(K, __half, CL, true) TL_TC_EXTERN(K, __nv_bfloat16, CL, true)    \
-    TL_TC_EXTERN(K, __nv_fp8_e4m3, CL, true)                                                                  \
-    extern template int max_clusters<K, float, CL>(size_t);                                                   \
-    extern template int max_clusters<K, __half, CL>(size_t);                                                  \
+#define TL_TC_EXTERN(K, TD, CL, E, P, G) \
+    extern template tl_status launch_kernel<K, TD, CL, E, P, G>(const TcKernelParams&, int, size_t, cudaStream_t);
+#define TL_TC_EXTERN_EP(K, CL, P)                                                                  \
+    TL_TC_EXTERN(K, float, CL, false, P, false) TL_TC_EXTERN(K, __half, CL, false, P, false)                     \
+    TL_TC_EXTERN(K, __nv_bfloat16, CL, false, P, false) TL_TC_EXTERN(K, float, CL, true, P, false)               \
+    TL_TC_EXTERN(K, __half, CL, true, P, false) TL_TC_EXTERN(K, __nv_bfloat16, CL, true, P, false)               \
+    TL_TC_EXTERN(K, __nv_fp8_e4m3, CL, true, P, false)
+#define TL_TC_EXTERN_CL(K, CL)                                  \
+    TL_TC_EXTERN_EP(K, CL, false)                               \
+    TL_TC_EXTERN(K, float, CL, false, false, true)              \
+    TL_TC_EXTERN(K, __half, CL, false, false, true)             \
+    TL_TC_EXTERN(K, __nv_bfloat16, CL, false, false, true)      \
+    extern template int max_clusters<K, float, CL>(size_t);     \
+    extern template int max_clusters<K, __half, CL>(size_t);    \
     extern template int max_clusters<K, __nv_bfloat16, CL>(size_t);
 TL_TC_EXTERN_CL(0, 1)
 TL_TC_EXTERN_CL(0, 2)
@@ -49,7 +57,12 @@ TL_TC_EXTERN_CL(0, 4)
 TL_TC_EXTERN_CL(1, 1)
 TL_TC_EXTERN_CL(1, 2)
 TL_TC_EXTERN_CL(1, 4)
+TL_TC_EXTERN_EP(0, 1, true)
+TL_TC_EXTERN_EP(0, 2, true)
+TL_TC_EXTERN_EP(1, 1, true)
+TL_TC_EXTERN_EP(1, 2, true)
 #undef TL_TC_EXTERN_CL
+#undef TL_TC_EXTERN_EP
 #undef TL_TC_EXTERN
 
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -81,26 +94,6 @@ bool par_reduce_enabled()
     return on;
 }
 
-// TMA-store epilogue: on unless TL_TMA_STORE=0 in the environment.
-bool tma_store_enabled()
-{
-    static const bool on = [] {
-        const char* e = getenv("TL_TMA_STORE");
-        return !(e && e[0] == '0');
-    }();
-    return on;
-}
-
-// A CTA's last tile is written with direct stores unless TL_LAST_DIRECT=0 in the environment.
-bool last_direct_enabled()
-{
-    static const bool on = [] {
-        const char* e = getenv("TL_LAST_DIRECT");
-        return !(e && e[0] == '0');
-    }();
-    return on;
-}
-
 // Programmatic dependent launch for the tensor-core kernel: on unless TL_PDL=0 in the environment.
 bool pdl_enabled()
 {
@@ -111,35 +104,40 @@ bool pdl_enabled()
     return on;
 }
 
+template <int KIND, int CL, bool PROMO, bool GROUP>
+tl_status dispatch_out(int out_dtype, const TcKernelParams& kp, int grid, size_t smem, cudaStream_t s)
+{
+    if (!GROUP && kp.epi_on) {
+        // the fused-epilogue kernels (they also write every fp8 output)
+        if constexpr (!GROUP) {
+            if (out_dtype == TL_DTYPE_FP32) return launch_kernel<KIND, float, CL, true, PROMO, false>(kp, grid, smem, s);
+            if (out_dtype == TL_DTYPE_FP16) return launch_kernel<KIND, __half, CL, true, PROMO, false>(kp, grid, smem, s);
+            if (out_dtype == TL_DTYPE_BF16) return launch_kernel<KIND, __nv_bfloat16, CL, true, PROMO, false>(kp, grid, smem, s);
+            if (out_dtype == TL_DTYPE_FP8_E4M3)
+                return launch_kernel<KIND, __nv_fp8_e4m3, CL, true, PROMO, false>(kp, grid, smem, s);
+        }
+    } else {
+        if (out_dtype == TL_DTYPE_FP32) return launch_kernel<KIND, float, CL, false, PROMO, GROUP>(kp, grid, smem, s);
+        if (out_dtype == TL_DTYPE_FP16) return launch_kernel<KIND, __half, CL, false, PROMO, GROUP>(kp, grid, smem, s);
+        if (out_dtype == TL_DTYPE_BF16) return launch_kernel<KIND, __nv_bfloat16, CL, false, PROMO, GROUP>(kp, grid, smem, s);
+    }
+    return fail(TL_ERR_UNSUPPORTED, "tcgen05 kernel: unsupported output type");
+}
+
 template <int CL>
 tl_status dispatch_cl(int in_dtype, int out_dtype, const TcKernelParams& kp, int grid, size_t smem, cudaStream_t s)
 {
     const int kind = (in_dtype == TL_DTYPE_FP8_E4M3) ? 1 : 0;
-    if (kp.epi_on) {
-        // the fused-epilogue kernels (they also write every fp8 output)
-        if (kind == 0) {
-            if (out_dtype == TL_DTYPE_FP32) return launch_kernel<0, float, CL, true>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_FP16) return launch_kernel<0, __half, CL, true>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_BF16) return launch_kernel<0, __nv_bfloat16, CL, true>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_FP8_E4M3) return launch_kernel<0, __nv_fp8_e4m3, CL, true>(kp, grid, smem, s);
-        } else {
-            if (out_dtype == TL_DTYPE_FP32) return launch_kernel<1, float, CL, true>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_FP16) return launch_kernel<1, __half, CL, true>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_BF16) return launch_kernel<1, __nv_bfloat16, CL, true>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_FP8_E4M3) return launch_kernel<1, __nv_fp8_e4m3, CL, true>(kp, grid, smem, s);
-        }
-        return fail(TL_ERR_UNSUPPORTED, "tcgen05 kernel: unsupported output type");
+    if (kp.promote_kb > 0) {
+        if constexpr (CL == 4) return fail(TL_ERR_UNSUPPORTED, "tcgen05 kernel: no promotion with two CTA pairs");
+        else return kind == 0 ? dispatch_out<0, CL, true, false>(out_dtype, kp, grid, smem, s)
+                              : dispatch_out<1, CL, true, false>(out_dtype, kp, grid, smem, s);
     }
-    if (kind == 0) {
-        if (out_dtype == TL_DTYPE_FP32) return launch_kernel<0, float, CL>(kp, grid, smem, s);
-        if (out_dtype == TL_DTYPE_FP16) return launch_kernel<0, __half, CL>(kp, grid, smem, s);
-        if (out_dtype == TL_DTYPE_BF16) return launch_kernel<0, __nv_bfloat16, CL>(kp, grid, smem, s);
-    } else {
-        if (out_dtype == TL_DTYPE_FP32) return launch_kernel<1, float, CL>(kp, grid, smem, s);
-        if (out_dtype == TL_DTYPE_FP16) return launch_kernel<1, __half, CL>(kp, grid, smem, s);
-        if (out_dtype == TL_DTYPE_BF16) return launch_kernel<1, __nv_bfloat16, CL>(kp, grid, smem, s);
-    }
-    return fail(TL_ERR_UNSUPPORTED, "tcgen05 kernel: unsupported output type");
+    if (kp.group != nullptr)
+        return kind == 0 ? dispatch_out<0, CL, false, true>(out_dtype, kp, grid, smem, s)
+                         : dispatch_out<1, CL, false, true>(out_dtype, kp, grid, smem, s);
+    return kind == 0 ? dispatch_out<0, CL, false, false>(out_dtype, kp, grid, smem, s)
+                     : dispatch_out<1, CL, false, false>(out_dtype, kp, grid, smem, s);
 }
 
 template <int CL>
@@ -222,8 +220,8 @@ size_t tc_smem_bytes(int bm, int stages)
     return static_cast<size_t>(stages) * (kTcTileN * kTcRowBytes + bm * kTcRowBytes) + kTcEpiStageBytes + 1024 + 512;
 }
 
-// Staging buffers per epilogue warp: two where they fit beside the ring (every tile at up to six
-// 32 KB stages), else one.
+// Output staging in units of kTcEpiStageBytes (4 KB for each of four epilogue warps): two, one for
+// every epilogue warp, where they fit beside the ring (every tile at up to six 32 KB stages), else one.
 static int epi_buffers(size_t smem_one) { return smem_one + kTcEpiStageBytes <= kTcMaxSmem ? 2 : 1; }
 
 int tc_workers(int in_dtype, int out_dtype, int cl, int bm, int stages, int sm_count)
@@ -280,51 +278,19 @@ tl_status tc_encode_operand(CUtensorMap* tm, int in_dtype, const TcOperand& op, 
     return TL_SUCCESS;
 }
 
-// Tensor map of the output for TMA stores: boxes of 128 bytes along m by 32 rows (n), 128-byte
-// swizzle.  False when TMA cannot address D (alignment of the base, ldd or batch stride).
-bool tc_encode_output(CUtensorMap* tm, int out_dtype, void* D, int64_t M, int64_t N, int64_t ldd, int64_t batch,
-                      int64_t stride_d)
+// Columns of whole 16-byte vectors: the base, ld and batch stride are aligned to them and `rows` is a
+// multiple of their elements.
+static bool vec16(const void* ptr, int64_t rows, int64_t ld, int64_t batch, int64_t stride, int es)
 {
-    EncodeTiledFn enc = get_encode_fn();
-    if (!enc || !D) return false;
-    const int es = dtype_bytes(out_dtype);
-    if ((reinterpret_cast<uintptr_t>(D) & 15) || (ldd * es) % 16 || (batch > 1 && (stride_d * es) % 16)) return false;
-    const CUtensorMapDataType dt = out_dtype == TL_DTYPE_FP32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                   : out_dtype == TL_DTYPE_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                   : out_dtype == TL_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
-                                                                : CU_TENSOR_MAP_DATA_TYPE_UINT8;
-    cuuint64_t dims[3] = {static_cast<cuuint64_t>(M), static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(batch)};
-    cuuint64_t strides[2] = {static_cast<cuuint64_t>(ldd) * es,
-                             batch > 1 ? static_cast<cuuint64_t>(stride_d) * es
-                                       : ((static_cast<cuuint64_t>(ldd) * es * N) + 15) & ~cuuint64_t(15)};
-    cuuint32_t box[3] = {static_cast<cuuint32_t>(kTcRowBytes / es), 32, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    return enc(tm, dt, 3, D, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0 && (rows * es) % 16 == 0 && (ld * es) % 16 == 0 &&
+           (batch <= 1 || (stride * es) % 16 == 0);
 }
 
-// The caller's D for a transposed output: the kernel's n runs along D's rows (dimension 0, N of
-// the launch) and its m along D's columns; boxes of 32 x 32 elements, one epilogue warp's rows by
-// one 32-column chunk, unswizzled (a 64- or 128-byte inner extent).
-bool tc_encode_output_t(CUtensorMap* tm, int out_dtype, void* D, int64_t rows, int64_t cols, int64_t ldd,
-                        int64_t batch, int64_t stride_d)
+bool tc_vec_output(int out_dtype, int64_t rows, const void* D, int64_t ldd, const void* C, int64_t ldc, int64_t batch,
+                   int64_t stride_d, int64_t stride_c)
 {
-    EncodeTiledFn enc = get_encode_fn();
-    if (!enc || !D) return false;
-    if (out_dtype != TL_DTYPE_FP32 && out_dtype != TL_DTYPE_FP16 && out_dtype != TL_DTYPE_BF16) return false;
     const int es = dtype_bytes(out_dtype);
-    if ((reinterpret_cast<uintptr_t>(D) & 15) || (ldd * es) % 16 || (batch > 1 && (stride_d * es) % 16)) return false;
-    const CUtensorMapDataType dt = out_dtype == TL_DTYPE_FP32   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                   : out_dtype == TL_DTYPE_FP16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                                                : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    cuuint64_t dims[3] = {static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(batch)};
-    cuuint64_t strides[2] = {static_cast<cuuint64_t>(ldd) * es,
-                             batch > 1 ? static_cast<cuuint64_t>(stride_d) * es
-                                       : ((static_cast<cuuint64_t>(ldd) * es * cols) + 15) & ~cuuint64_t(15)};
-    cuuint32_t box[3] = {32, 32, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    return enc(tm, dt, 3, D, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-               CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return vec16(D, rows, ldd, batch, stride_d, es) && (C == nullptr || vec16(C, rows, ldc, batch, stride_c, es));
 }
 
 tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launches)
@@ -458,21 +424,9 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
         const int workers = persistent_workers(L.in_dtype, L.out_dtype, cg, L.ctas, L.sm_count, smem);
         kp.par_reduce = (kp.split_units > 0 && kp.bal_kb == 0 && kp.split_units <= workers && par_reduce_enabled()) ? 1 : 0;
     }
-    // whole tiles leave through TMA stores (not with promotion, which drains chains into registers)
-    // (an fp8 output's 128-byte box is 128 columns wide: only tiles made of whole boxes)
     kp.out_t = L.out_t;
-    if (L.out_t)
-        kp.tma_store = (L.promote_k == 0 && tma_store_enabled() &&
-                        tc_encode_output_t(&kp.tmD, L.out_dtype, L.D, L.N, L.M, L.ldd, L.batch, L.stride_d))
-                           ? 1
-                           : 0;
-    else
-        kp.tma_store = (L.promote_k == 0 && tma_store_enabled() && (L.out_dtype != TL_DTYPE_FP8_E4M3 || L.bm % 128 == 0) &&
-                        tc_encode_output(&kp.tmD, L.out_dtype, L.D, L.M, L.N, L.ldd, L.batch, L.stride_d))
-                           ? 1
-                           : 0;
-    kp.direct_last = last_direct_enabled() ? 1 : 0;
-    kp.narrow = (kp.total_work < (int64_t(1) << 31) && tiles < (int64_t(1) << 31) &&
+    kp.vec = tc_vec_output(L.out_dtype, L.out_t ? L.N : L.M, L.D, L.ldd, L.C, L.ldc, L.batch, L.stride_d, L.stride_c) ? 1 : 0;
+    kp.narrow = (kp.bal_kb == 0 && kp.total_work < (int64_t(1) << 31) && tiles < (int64_t(1) << 31) &&
                  static_cast<int64_t>(kp.num_kb) * (kp.tail_split + 1) < (int64_t(1) << 31))
                     ? 1
                     : 0;
@@ -493,7 +447,6 @@ tl_status tc_grouped_launch(const TcGroupLaunch& G, cudaStream_t stream, int64_t
     memset(&kp, 0, sizeof(kp));
     kp.group = G.d_entries;
     kp.group_units = G.d_units;
-    kp.direct_last = last_direct_enabled() ? 1 : 0;
     kp.bm = G.bm;
     kp.stages = G.stages;
     kp.split_k = 1;

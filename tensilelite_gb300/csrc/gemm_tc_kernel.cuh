@@ -21,10 +21,9 @@ namespace tc {
 
 struct TcKernelParams {
     CUtensorMap tmN[3], tmM[3];   // split-precision pieces 0..2 (piece 0 = the operand itself)
-    CUtensorMap tmD;              // the output, boxes of 128 bytes x 32 rows (tma_store)
-    int tma_store;                // whole tiles leave through shared memory and TMA stores
-    int epi_bufs;                 // staging buffers of 4 KB per epilogue warp (1 or 2)
-    int direct_last;              // a CTA's last tile (beta == 0) leaves through direct stores
+    int vec;                      // D (and C, with beta) consist of whole aligned 16-byte vectors: whole
+                                  // tiles leave through shared memory in full lines
+    int epi_bufs;                 // output staging in units of kTcEpiStageBytes (1 or 2)
     // fused epilogue (kernels instantiated with EPI): D = act(alpha*acc + beta*C + bias[m]), and
     // max |D| into *epi_amax
     const void* epi_bias;
@@ -49,7 +48,7 @@ struct TcKernelParams {
     int promote_kb;               // >0: the A0*B0 product restarts its TMEM chain every promote_kb
                                   // k-blocks; the epilogue adds each chain into fp32 registers
     int tiles_m, tiles_n;
-    int narrow;                   // work units, tiles and split k-block products fit 32 bits
+    int narrow;                   // work units, tiles and split k-block products fit 32 bits, no balanced split
     int64_t total_work;
     int64_t split_units;          // work units below this are k-slices of the first split_tiles tiles
     int64_t split_tiles;          // tiles split along k; the rest are whole
@@ -99,7 +98,7 @@ __device__ __forceinline__ unsigned long long global_ns()
 struct TileJob {
     const void* tmN;
     const void* tmM;
-    const CUtensorMap* tmD;       // the output for TMA stores, or null
+    int vec;                      // D and C in 16-byte vectors (TcKernelParams::vec)
     void* D;
     const void* C;
     int64_t ldd, ldc;
@@ -109,116 +108,144 @@ struct TileJob {
     int kb0, kb1;
     int split, nsplit;            // this unit's k split and the tile's number of splits
     int out_t;                    // transposed output (TcKernelParams::out_t)
-    int64_t tile;
     int64_t slot;                 // split tiles: index of the tile's workspace slabs and counter
 };
 
 // Grouped launches: the unit-table entry of work unit w (a zero entry past the end or without a group).
+template <bool GROUP>
 __device__ __forceinline__ int4 load_unit(const TcKernelParams& p, int64_t w)
 {
-    if (p.group == nullptr || w >= p.total_work) return make_int4(0, 0, 0, 0);
+    if (!GROUP || w >= p.total_work) return make_int4(0, 0, 0, 0);
     return __ldg(p.group_units + w);
 }
 
+// Where a work unit lies: tile and its coordinates, its k split and k-blocks.
+struct UnitPos {
+    int64_t tile;
+    int b, in, jm, kb0, kb1, split, nsplit;
+};
+
+// The decode of balanced-split units and of launches beyond 32 bits, out of line: 64-bit divisions
+// take hundreds of instructions, and inlined at every use they made the kernel 200 KB of code, whose
+// fetches stalled every role (ncu: 8 of 10 cycles between a warp's instructions).
+static __device__ __noinline__ void unit_pos_wide(const TcKernelParams& p, int64_t w, UnitPos& u)
+{
+    if (p.bal_kb > 0 && w < 2 * static_cast<int64_t>(p.bal_stride)) {
+        // balanced split: worker `wk` owns k-blocks [s0, s1) of the split tiles laid end to end;
+        // piece 0 is the part in its first tile, piece 1 the rest (possibly empty)
+        const int64_t wk = w % p.bal_stride, piece = w / p.bal_stride;
+        const int64_t R = p.bal_kb, Wb = p.bal_workers, nkb = p.num_kb;
+        int64_t a = 0, e = 0;
+        if (wk < Wb) {
+            const int64_t s0 = wk * R / Wb, s1 = (wk + 1) * R / Wb;
+            const int64_t cut = min(s1, (s0 / nkb + 1) * nkb);
+            a = piece == 0 ? s0 : cut;
+            e = piece == 0 ? cut : s1;
+        }
+        if (a >= e) {
+            u.tile = 0;                    // empty unit: every role skips it
+            u.kb0 = u.kb1 = 0;
+            u.split = 0;
+            u.nsplit = 1;
+        } else {
+            u.tile = a / nkb;
+            u.kb0 = static_cast<int>(a - u.tile * nkb);
+            u.kb1 = static_cast<int>(e - u.tile * nkb);
+            // the workers covering this tile: the one holding its first and its last k-block
+            const int64_t first = ((u.tile * nkb + 1) * Wb - 1) / R;
+            const int64_t last = (((u.tile + 1) * nkb) * Wb - 1) / R;
+            u.nsplit = static_cast<int>(last - first + 1);
+            u.split = static_cast<int>(wk - first);
+        }
+    } else if (w < p.split_units) {
+        u.nsplit = p.tail_split;
+        u.tile = w / p.tail_split;
+        u.split = static_cast<int>(w % p.tail_split);
+        u.kb0 = static_cast<int>((static_cast<int64_t>(u.split) * p.num_kb) / u.nsplit);
+        u.kb1 = static_cast<int>((static_cast<int64_t>(u.split + 1) * p.num_kb) / u.nsplit);
+    } else {
+        u.tile = p.split_tiles + (w - p.split_units);
+        u.split = 0;
+        u.nsplit = 1;
+        u.kb0 = 0;
+        u.kb1 = p.num_kb;
+    }
+    const int64_t tpb = static_cast<int64_t>(p.tiles_m) * p.tiles_n;
+    u.b = static_cast<int>(u.tile / tpb);
+    const int64_t t = u.tile % tpb;
+    if (p.raster > 0) {
+        const int64_t group_tiles = static_cast<int64_t>(p.raster) * p.tiles_m;
+        const int64_t g = t / group_tiles;
+        const int first_n = static_cast<int>(g * p.raster);
+        const int gsize = min(p.raster, p.tiles_n - first_n);
+        const int64_t r = t % group_tiles;
+        u.in = first_n + static_cast<int>(r % gsize);
+        u.jm = static_cast<int>(r / gsize);
+    } else {
+        u.in = static_cast<int>(t / p.tiles_m);
+        u.jm = static_cast<int>(t % p.tiles_m);
+    }
+}
+
+// Every index fits 32 bits (host-checked) and no balanced split: 32-bit divisions only, on the path
+// between the launch and the first load.
+__device__ __forceinline__ void unit_pos_narrow(const TcKernelParams& p, uint32_t w, UnitPos& u)
+{
+    const uint32_t nkb = static_cast<uint32_t>(p.num_kb);
+    uint32_t tile;
+    if (w < static_cast<uint32_t>(p.split_units)) {
+        // split tiles come first, so the last arriver's reduction overlaps later whole tiles
+        const uint32_t ts = static_cast<uint32_t>(p.tail_split);
+        tile = w / ts;
+        const uint32_t split = w - tile * ts;
+        u.split = static_cast<int>(split);
+        u.nsplit = static_cast<int>(ts);
+        u.kb0 = static_cast<int>((split * nkb) / ts);
+        u.kb1 = static_cast<int>(((split + 1) * nkb) / ts);
+    } else {
+        tile = static_cast<uint32_t>(p.split_tiles) + (w - static_cast<uint32_t>(p.split_units));
+        u.split = 0;
+        u.nsplit = 1;
+        u.kb0 = 0;
+        u.kb1 = p.num_kb;
+    }
+    u.tile = tile;
+    uint32_t t = tile;
+    u.b = 0;
+    if (p.batch > 1) {
+        const uint32_t tpb = static_cast<uint32_t>(p.tiles_m) * static_cast<uint32_t>(p.tiles_n);
+        const uint32_t ub = tile / tpb;
+        u.b = static_cast<int>(ub);
+        t = tile - ub * tpb;
+    }
+    if (p.raster > 0) {
+        const uint32_t group_tiles = static_cast<uint32_t>(p.raster) * static_cast<uint32_t>(p.tiles_m);
+        const uint32_t g = t / group_tiles;
+        const int first_n = static_cast<int>(g * static_cast<uint32_t>(p.raster));
+        const uint32_t gsize = static_cast<uint32_t>(min(p.raster, p.tiles_n - first_n));
+        const uint32_t r = t - g * group_tiles;
+        const uint32_t rq = r / gsize;
+        u.in = first_n + static_cast<int>(r - rq * gsize);
+        u.jm = static_cast<int>(rq);
+    } else {
+        const uint32_t q = t / static_cast<uint32_t>(p.tiles_m);
+        u.in = static_cast<int>(q);
+        u.jm = static_cast<int>(t - q * static_cast<uint32_t>(p.tiles_m));
+    }
+}
+
+// Without a group the problem's fields stay in the kernel parameters (constant memory): only the
+// unit's position is computed.
+template <bool GROUP>
 __device__ __forceinline__ void get_job(const TcKernelParams& p, int64_t w, const int4& u, TileJob& j)
 {
-    if (p.group == nullptr) {
-        int64_t tile;
-        int split, nsplit;
-        int kb0, kb1;
-        if (p.bal_kb > 0 && w < 2 * static_cast<int64_t>(p.bal_stride)) {
-            // balanced split: worker `wk` owns k-blocks [s0, s1) of the split tiles laid end to end;
-            // piece 0 is the part in its first tile, piece 1 the rest (possibly empty)
-            const int64_t wk = w % p.bal_stride, piece = w / p.bal_stride;
-            const int64_t R = p.bal_kb, Wb = p.bal_workers, nkb = p.num_kb;
-            int64_t a = 0, e = 0;
-            if (wk < Wb) {
-                const int64_t s0 = wk * R / Wb, s1 = (wk + 1) * R / Wb;
-                const int64_t cut = min(s1, (s0 / nkb + 1) * nkb);
-                a = piece == 0 ? s0 : cut;
-                e = piece == 0 ? cut : s1;
-            }
-            if (a >= e) {
-                tile = 0;                    // empty unit: every role skips it
-                kb0 = kb1 = 0;
-                split = 0;
-                nsplit = 1;
-            } else {
-                tile = a / nkb;
-                kb0 = static_cast<int>(a - tile * nkb);
-                kb1 = static_cast<int>(e - tile * nkb);
-                // the workers covering this tile: the one holding its first and its last k-block
-                const int64_t first = ((tile * nkb + 1) * Wb - 1) / R;
-                const int64_t last = (((tile + 1) * nkb) * Wb - 1) / R;
-                nsplit = static_cast<int>(last - first + 1);
-                split = static_cast<int>(wk - first);
-            }
-        } else if (w < p.split_units) {
-            // split tiles come first, so the last arriver's reduction overlaps later whole tiles
-            nsplit = p.tail_split;
-            if (p.narrow) {
-                const uint32_t uw = static_cast<uint32_t>(w), ts = static_cast<uint32_t>(nsplit);
-                const uint32_t q = uw / ts, nkb = static_cast<uint32_t>(p.num_kb);
-                tile = q;
-                split = static_cast<int>(uw - q * ts);
-                kb0 = static_cast<int>((static_cast<uint32_t>(split) * nkb) / ts);
-                kb1 = static_cast<int>((static_cast<uint32_t>(split + 1) * nkb) / ts);
-            } else {
-                tile = w / p.tail_split;
-                split = static_cast<int>(w % p.tail_split);
-                kb0 = static_cast<int>((static_cast<int64_t>(split) * p.num_kb) / nsplit);
-                kb1 = static_cast<int>((static_cast<int64_t>(split + 1) * p.num_kb) / nsplit);
-            }
-        } else {
-            tile = p.split_tiles + (w - p.split_units);
-            split = 0;
-            nsplit = 1;
-            kb0 = 0;
-            kb1 = p.num_kb;
-        }
-        int b, in, jm;
-        if (p.narrow) {
-            // every tile index fits 32 bits (host-checked): 32-bit divisions are several times
-            // shorter than 64-bit ones, and this decode sits between the launch and the first load
-            const uint32_t ut = static_cast<uint32_t>(tile);
-            const uint32_t tpb = static_cast<uint32_t>(p.tiles_m) * static_cast<uint32_t>(p.tiles_n);
-            const uint32_t ub = ut / tpb;
-            const uint32_t t = ut - ub * tpb;
-            b = static_cast<int>(ub);
-            if (p.raster > 0) {
-                const uint32_t group_tiles = static_cast<uint32_t>(p.raster) * static_cast<uint32_t>(p.tiles_m);
-                const uint32_t g = t / group_tiles;
-                const int first_n = static_cast<int>(g * static_cast<uint32_t>(p.raster));
-                const uint32_t gsize = static_cast<uint32_t>(min(p.raster, p.tiles_n - first_n));
-                const uint32_t r = t - g * group_tiles;
-                const uint32_t rq = r / gsize;
-                in = first_n + static_cast<int>(r - rq * gsize);
-                jm = static_cast<int>(rq);
-            } else {
-                const uint32_t q = t / static_cast<uint32_t>(p.tiles_m);
-                in = static_cast<int>(q);
-                jm = static_cast<int>(t - q * static_cast<uint32_t>(p.tiles_m));
-            }
-        } else {
-            const int64_t tpb = static_cast<int64_t>(p.tiles_m) * p.tiles_n;
-            b = static_cast<int>(tile / tpb);
-            const int64_t t = tile % tpb;
-            if (p.raster > 0) {
-                const int64_t group_tiles = static_cast<int64_t>(p.raster) * p.tiles_m;
-                const int64_t g = t / group_tiles;
-                const int first_n = static_cast<int>(g * p.raster);
-                const int gsize = min(p.raster, p.tiles_n - first_n);
-                const int64_t r = t % group_tiles;
-                in = first_n + static_cast<int>(r % gsize);
-                jm = static_cast<int>(r / gsize);
-            } else {
-                in = static_cast<int>(t / p.tiles_m);
-                jm = static_cast<int>(t % p.tiles_m);
-            }
-        }
+    if constexpr (!GROUP) {
+        UnitPos pos;
+        if (p.narrow) unit_pos_narrow(p, static_cast<uint32_t>(w), pos);
+        else unit_pos_wide(p, w, pos);
         j.tmN = &p.tmN[0];
         j.tmM = &p.tmM[0];
-        j.tmD = p.tma_store ? &p.tmD : nullptr;
+        j.vec = p.vec;
         j.D = static_cast<char*>(p.D);
         j.C = p.C;
         j.ldd = p.ldd;
@@ -227,23 +254,22 @@ __device__ __forceinline__ void get_job(const TcKernelParams& p, int64_t w, cons
         j.N = p.N;
         j.alpha = p.alpha;
         j.beta = p.beta;
-        j.b = b;
-        j.n0 = in * p.tile_rows;
-        j.m0 = jm * p.bm;
-        j.kb0 = kb0;
-        j.kb1 = kb1;
-        j.split = split;
-        j.nsplit = nsplit;
+        j.b = pos.b;
+        j.n0 = pos.in * p.tile_rows;
+        j.m0 = pos.jm * p.bm;
+        j.kb0 = pos.kb0;
+        j.kb1 = pos.kb1;
+        j.split = pos.split;
+        j.nsplit = pos.nsplit;
         j.out_t = p.out_t;
-        j.tile = tile;
-        j.slot = tile;                 // split tiles are 0 .. split_tiles-1
+        j.slot = pos.tile;             // split tiles are 0 .. split_tiles-1
     } else {
         // grouped: the unit's problem and tile come from the plan's unit table (loaded ahead by
         // the caller); only the epilogue reads the problem's entry
         const TcGroupEntry& e = p.group[u.x];
         j.tmN = &e.tmN;
         j.tmM = &e.tmM;
-        j.tmD = e.tma_store ? &e.tmD : nullptr;
+        j.vec = e.vec;
         j.D = e.D;
         j.C = e.C;
         j.ldd = e.ldd;
@@ -260,7 +286,6 @@ __device__ __forceinline__ void get_job(const TcKernelParams& p, int64_t w, cons
         j.split = 0;
         j.nsplit = 1;
         j.out_t = 0;
-        j.tile = w;
         j.slot = 0;
     }
 }
@@ -349,193 +374,132 @@ __device__ __forceinline__ void unpack2(uint32_t w, int is_half, float& a, float
     }
 }
 
-// Fused epilogue of one output value at row m: + bias[m], activation (1 relu, 2 gelu with the tanh
-// approximation, 3 silu), and the running max |value| of this thread over the stored values.
-__device__ __forceinline__ float epi_fn(const TcKernelParams& p, int m, bool stored, float o, float& amax)
+// Ragged edges, unaligned matrices and transposed outputs, element by element and out of line (the
+// unrolled code of each use took more instruction memory than everything else).
+template <typename TD>
+__device__ __noinline__ void load_elements(const void* base, int64_t idx, int64_t step, int count, float* out)
 {
-    if (p.epi_bias != nullptr && stored) {
-        if (p.epi_bias_dtype == TL_DTYPE_FP32) o += __ldg(static_cast<const float*>(p.epi_bias) + m);
-        else if (p.epi_bias_dtype == TL_DTYPE_FP16) o += __half2float(static_cast<const __half*>(p.epi_bias)[m]);
-        else o += __bfloat162float(static_cast<const __nv_bfloat16*>(p.epi_bias)[m]);
-    }
-    if (p.epi_act == 1) {
-        o = fmaxf(o, 0.0f);
-    } else if (p.epi_act == 2) {
-        const float u = 0.7978845608028654f * fmaf(0.044715f * o * o, o, o);
-        o = 0.5f * o * (1.0f + tanhf(u));
-    } else if (p.epi_act == 3) {
-        o = o / (1.0f + expf(-o));
-    }
-    if (stored) amax = fmaxf(amax, fabsf(o));
-    return o;
+#pragma unroll 4
+    for (int i = 0; i < count; ++i) out[i] = Out<TD>::load(base, idx + i * step);
+}
+template <typename TD>
+__device__ __noinline__ void store_elements(void* base, int64_t idx, int64_t step, int count, const float* v, float scale,
+                                            int trunc)
+{
+#pragma unroll 4
+    for (int i = 0; i < count; ++i) Out<TD>::store(base, idx + i * step, sizeof(TD) == 1 ? v[i] * scale : v[i], trunc);
 }
 
-// Finish 32 consecutive outputs m..m+31 of column n: v = alpha*acc + beta*C (then the fused
-// epilogue when EPI), convert, store.
-template <typename TD, bool EPI>
-__device__ __forceinline__ void store_chunk(const TcKernelParams& p, float& amax, const TileJob& j, int64_t base_c,
-                                           int64_t base_d, int m, float (&acc)[32], int trunc)
+// The bias of rows m .. m+W-1 (rows past M: 0), every load in flight at once.
+template <int W>
+__device__ __forceinline__ void load_bias(const TcKernelParams& p, int M, int m, float (&b)[W])
 {
-    const bool full = (m + 32 <= j.M);
-    const bool use_c = (j.beta != 0.0f) && (j.C != nullptr);
-    char* dptr = static_cast<char*>(j.D) + (base_d + m) * Out<TD>::kBytes;
-    const char* cptr = use_c ? static_cast<const char*>(j.C) + (base_c + m) * Out<TD>::kBytes : nullptr;
-    const bool vec = full && !j.out_t && ((reinterpret_cast<uintptr_t>(dptr) & 15) == 0) &&
-                     (!use_c || (reinterpret_cast<uintptr_t>(cptr) & 15) == 0);
-    if (vec) {
-        if constexpr (sizeof(TD) == 4) {
+    const int es = p.epi_bias_dtype == TL_DTYPE_FP32 ? 4 : 2;
+    const char* src = static_cast<const char*>(p.epi_bias) + static_cast<int64_t>(m) * es;
+    if (m + W <= M && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+        if (es == 4) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                float4 c4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (use_c) c4 = __ldg(reinterpret_cast<const float4*>(cptr) + q);
-                float4 o;
-                if (use_c) {
-                    o.x = fmaf(j.alpha, acc[4 * q + 0], j.beta * c4.x);
-                    o.y = fmaf(j.alpha, acc[4 * q + 1], j.beta * c4.y);
-                    o.z = fmaf(j.alpha, acc[4 * q + 2], j.beta * c4.z);
-                    o.w = fmaf(j.alpha, acc[4 * q + 3], j.beta * c4.w);
-                } else {
-                    o.x = j.alpha * acc[4 * q + 0];
-                    o.y = j.alpha * acc[4 * q + 1];
-                    o.z = j.alpha * acc[4 * q + 2];
-                    o.w = j.alpha * acc[4 * q + 3];
-                }
-                if constexpr (EPI) {
-                    o.x = epi_fn(p, m + 4 * q + 0, true, o.x, amax);
-                    o.y = epi_fn(p, m + 4 * q + 1, true, o.y, amax);
-                    o.z = epi_fn(p, m + 4 * q + 2, true, o.z, amax);
-                    o.w = epi_fn(p, m + 4 * q + 3, true, o.w, amax);
-                }
-                reinterpret_cast<float4*>(dptr)[q] = o;
+            for (int q = 0; q < W / 4; ++q) {
+                const float4 f = __ldg(reinterpret_cast<const float4*>(src) + q);
+                b[4 * q] = f.x;
+                b[4 * q + 1] = f.y;
+                b[4 * q + 2] = f.z;
+                b[4 * q + 3] = f.w;
             }
-        } else if constexpr (sizeof(TD) == 1) {
-            // E4M3: 32 outputs in two 16-byte stores (no C: fp8 outputs take beta == 0)
-            uint32_t ow[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                float o[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    o[t] = j.alpha * acc[4 * q + t];
-                    if constexpr (EPI) o[t] = epi_fn(p, m + 4 * q + t, true, o[t], amax);
-                    o[t] = out_scale<TD>(p, o[t]);
-                }
-                ow[q] = pack4_e4m3(o[0], o[1], o[2], o[3]);
-            }
-            reinterpret_cast<uint4*>(dptr)[0] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-            reinterpret_cast<uint4*>(dptr)[1] = make_uint4(ow[4], ow[5], ow[6], ow[7]);
         } else {
-            constexpr int is_half = std::is_same<TD, __half>::value ? 1 : 0;
+            const int is_half = p.epi_bias_dtype == TL_DTYPE_FP16 ? 1 : 0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                uint4 cw = make_uint4(0, 0, 0, 0);
-                if (use_c) cw = __ldg(reinterpret_cast<const uint4*>(cptr) + q);
-                uint32_t cws[4] = {cw.x, cw.y, cw.z, cw.w};
-                uint32_t ow[4];
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    float c0 = 0.f, c1 = 0.f;
-                    if (use_c) unpack2(cws[h], is_half, c0, c1);
-                    const float a0 = acc[8 * q + 2 * h], a1 = acc[8 * q + 2 * h + 1];
-                    float o0 = use_c ? fmaf(j.alpha, a0, j.beta * c0) : j.alpha * a0;
-                    float o1 = use_c ? fmaf(j.alpha, a1, j.beta * c1) : j.alpha * a1;
-                    if constexpr (EPI) {
-                        o0 = epi_fn(p, m + 8 * q + 2 * h, true, o0, amax);
-                        o1 = epi_fn(p, m + 8 * q + 2 * h + 1, true, o1, amax);
-                    }
-                    ow[h] = pack2(o0, o1, is_half, trunc);
-                }
-                reinterpret_cast<uint4*>(dptr)[q] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+            for (int q = 0; q < W / 8; ++q) {
+                const uint4 w = __ldg(reinterpret_cast<const uint4*>(src) + q);
+                unpack2(w.x, is_half, b[8 * q], b[8 * q + 1]);
+                unpack2(w.y, is_half, b[8 * q + 2], b[8 * q + 3]);
+                unpack2(w.z, is_half, b[8 * q + 4], b[8 * q + 5]);
+                unpack2(w.w, is_half, b[8 * q + 6], b[8 * q + 7]);
             }
         }
     } else {
-        // element m + i at (m + i) * step: 1, or ld for a transposed output (a warp's 32 rows then
-        // make one coalesced access per element)
-        // C in groups of sixteen, each group read before its D is written: the loads of a group
-        // overlap (a store may alias a later load, so none is moved above one), and D may be C itself
-        const int64_t dstep = j.out_t ? j.ldd : 1, cstep = j.out_t ? j.ldc : 1;
 #pragma unroll
-        for (int i0 = 0; i0 < 32; i0 += 16) {
-            float cv[16];
-#pragma unroll
-            for (int t = 0; t < 16; ++t)
-                cv[t] = (use_c && m + i0 + t < j.M) ? Out<TD>::load(j.C, base_c + (m + i0 + t) * cstep) : 0.f;
-#pragma unroll
-            for (int t = 0; t < 16; ++t) {
-                const int i = i0 + t;
-                if (m + i < j.M) {
-                    float o = use_c ? fmaf(j.alpha, acc[i], j.beta * cv[t]) : j.alpha * acc[i];
-                    if constexpr (EPI) o = epi_fn(p, m + i, true, o, amax);
-                    Out<TD>::store(j.D, base_d + (m + i) * dstep, out_scale<TD>(p, o), trunc);
-                }
+        for (int i = 0; i < W; ++i) {
+            b[i] = 0.f;
+            if (m + i < M) {
+                if (es == 4) b[i] = __ldg(reinterpret_cast<const float*>(src) + i);
+                else if (p.epi_bias_dtype == TL_DTYPE_FP16) b[i] = __half2float(reinterpret_cast<const __half*>(src)[i]);
+                else b[i] = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(src)[i]);
             }
         }
     }
 }
 
-// Split-k completion, run by the four epilogue warps after this split parked its partial tile in
-// the workspace (layout [32-column chunk][column][row], so every warp access is one 128-byte line): the last split of a tile to arrive (per-tile counter) sums every split's partial
-// in split order -- so the result does not depend on which CTA finished last -- and runs the
-// epilogue.  The counter is reset for the next launch.  Every thread passes the same three named
-// barriers whether or not it has work, so a warp that gave up on a wait cannot strand the others.
-template <typename TD, bool EPI>
-__device__ __forceinline__ void split_finish(const TcKernelParams& p, float& amax, const TileJob& j, bool ok, int et,
-                                             int row, bool row_ok, int64_t base_c, int64_t base_d,
-                                             volatile int* last_flag)
+// The bias of rows m, m + 32, ... (one per lane of a warp and chunk; rows past M: 0).
+template <int N>
+__device__ __forceinline__ void lane_bias(const TcKernelParams& p, int M, int m, float (&b)[N])
 {
-    __threadfence();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (et == 0) {
-        int last = 0;
-        if (ok) last = (atomicAdd(p.counters + j.slot, 1) == j.nsplit - 1) ? 1 : 0;
-        *last_flag = last;
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    const int is_last = *last_flag;
-    if (is_last && ok) {
-        __threadfence();
-        const int chunks = p.bm / 32;
-        for (int c = 0; c < chunks; ++c) {
-            float v[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.f;
-            const size_t slab_elems = static_cast<size_t>(kTcTileN) * p.bm;
-            const float* src0 = p.ws + static_cast<size_t>(j.slot) * p.tail_split * slab_elems +
-                                static_cast<size_t>(c) * 32 * kTcTileN + row;
-            for (int s = 0; s < j.nsplit; s += 2) {       // two slabs' loads in flight per step
-                float a[32], b[32];
-                const float* sa = src0 + static_cast<size_t>(s) * slab_elems;
-                const bool two = s + 1 < j.nsplit;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    a[i] = __ldcg(sa + i * kTcTileN);
-                    b[i] = two ? __ldcg(sa + slab_elems + i * kTcTileN) : 0.f;
-                }
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] += a[i];
-                if (two) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] += b[i];
-                }
-            }
-            const int m = j.m0 + c * 32;
-            if (row_ok && m < j.M) store_chunk<TD, EPI>(p, amax, j, base_c, base_d, m, v, p.out_trunc);
+    for (int t = 0; t < N; ++t) {
+        const int r = m + 32 * t;
+        b[t] = 0.f;
+        if (p.epi_bias != nullptr && r < M) {
+            if (p.epi_bias_dtype == TL_DTYPE_FP32) b[t] = __ldg(static_cast<const float*>(p.epi_bias) + r);
+            else if (p.epi_bias_dtype == TL_DTYPE_FP16) b[t] = __half2float(static_cast<const __half*>(p.epi_bias)[r]);
+            else b[t] = __bfloat162float(static_cast<const __nv_bfloat16*>(p.epi_bias)[r]);
         }
-        if (et == 0) p.counters[j.slot] = 0;   // ready for the next launch
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");   // last_flag is reused by the next tile
 }
 
-// C for one 32-output chunk, loaded ahead of its use (the epilogue keeps the next chunk's loads in
-// flight while it finishes the current one).  16-bit outputs occupy cw[0..15] as packed pairs.
-template <typename TD>
-__device__ __forceinline__ void load_c_chunk(const TileJob& j, int64_t base_c, int m, uint32_t (&cw)[32])
+// Fused epilogue of W output values at rows m..: + bias b, activation (1 relu, 2 gelu with the tanh
+// approximation, 3 silu), and this thread's running max |value| over the stored ones (`row_ok`: the
+// column n is stored).  The tests on the kind sit outside the element loops, the bias comes in
+// registers, and the activation's code is there once: a launch that does not follow another at once
+// fetches its instructions anew, ~500 clocks per 128 bytes of straight-line code, and with a bias load, three
+// type tests and both activations unrolled over 32 elements the two chunks of a 32-row linear layer
+// took 23000 clocks (11 us).  gelu(x) = x (1 + tanh u) / 2 = x / (1 + exp(-2u)): the form of silu,
+// without the cancellation of 1 + tanh at negative x.
+template <int W>
+__device__ __forceinline__ void epi_apply(const TcKernelParams& p, int M, int m, bool row_ok, const float (&b)[W],
+                                          float (&o)[W], float& amax)
+{
+    if (p.epi_bias != nullptr) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) o[i] += b[i];
+    }
+    if (p.epi_act == 1) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) o[i] = fmaxf(o[i], 0.0f);
+    } else if (p.epi_act >= 2) {
+        const bool gelu = p.epi_act == 2;
+        // two elements at a time, the values rotated through the registers: one copy of the code
+#pragma unroll 1
+        for (int i = 0; i < W; i += 2) {
+            float r[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float x = o[e];
+                const float t = gelu ? 1.5957691216057308f * fmaf(0.044715f * x * x, x, x) : x;
+                r[e] = __fdividef(x, 1.0f + expf(-t));   // 2 ulp; an infinite divisor gives 0 without a slow path
+            }
+#pragma unroll
+            for (int k = 0; k < W - 2; ++k) o[k] = o[k + 2];
+            o[W - 2] = r[0];
+            o[W - 1] = r[1];
+        }
+    }
+    if (p.epi_amax != nullptr) {
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+            if (row_ok && m + i < M) amax = fmaxf(amax, fabsf(o[i]));
+    }
+}
+
+// C for one chunk of W outputs, loaded ahead of its use (the epilogue keeps the next chunk's loads in
+// flight while it finishes the current one).  16-bit outputs occupy cw[0..W/2-1] as packed pairs.
+template <typename TD, int W>
+__device__ __forceinline__ void load_c_chunk(const TileJob& j, int64_t base_c, int m, uint32_t (&cw)[W])
 {
     if constexpr (sizeof(TD) == 1) return;        // fp8 outputs take beta == 0: no C
     if (!(j.beta != 0.0f && j.C != nullptr) || m >= j.M) return;
     const char* cptr = static_cast<const char*>(j.C) + (base_c + m) * Out<TD>::kBytes;
-    if (!j.out_t && m + 32 <= j.M && (reinterpret_cast<uintptr_t>(cptr) & 15) == 0) {
-        constexpr int nvec = sizeof(TD) == 4 ? 8 : 4;
+    if (!j.out_t && m + W <= j.M && (reinterpret_cast<uintptr_t>(cptr) & 15) == 0) {
+        constexpr int nvec = W * static_cast<int>(sizeof(TD)) / 16;
 #pragma unroll
         for (int q = 0; q < nvec; ++q) {
             const uint4 w = __ldg(reinterpret_cast<const uint4*>(cptr) + q);
@@ -545,17 +509,17 @@ __device__ __forceinline__ void load_c_chunk(const TileJob& j, int64_t base_c, i
             cw[4 * q + 3] = w.w;
         }
     } else {
+        float c[W];
+        load_elements<TD>(j.C, base_c + m * (j.out_t ? j.ldc : 1), j.out_t ? j.ldc : 1, min(W, j.M - m), c);
 #pragma unroll
-        const int64_t cstep = j.out_t ? j.ldc : 1;
-        for (int i = 0; i < 32; ++i) {
-            const float c = (m + i < j.M) ? Out<TD>::load(j.C, base_c + (m + i) * cstep) : 0.f;
+        for (int i = 0; i < W; ++i) {
             if constexpr (sizeof(TD) == 4) {
-                cw[i] = __float_as_uint(c);
+                cw[i] = __float_as_uint(c[i]);
             } else {
                 // repack as the vector path does: element i in the low (even) / high (odd) half
-                const uint32_t bits = (sizeof(TD) == 2 && std::is_same<TD, __half>::value)
-                                          ? static_cast<uint32_t>(__half_as_ushort(__float2half_rn(c)))
-                                          : (__float_as_uint(c) >> 16);
+                const uint32_t bits = std::is_same<TD, __half>::value
+                                          ? static_cast<uint32_t>(__half_as_ushort(__float2half_rn(c[i])))
+                                          : (__float_as_uint(c[i]) >> 16);
                 if (i & 1) cw[i >> 1] |= bits << 16;
                 else cw[i >> 1] = bits;
             }
@@ -563,101 +527,141 @@ __device__ __forceinline__ void load_c_chunk(const TileJob& j, int64_t base_c, i
     }
 }
 
-// alpha*acc + beta*C for 32 outputs (C in registers from load_c_chunk), converted and packed into
-// the output's bytes: 32 words for fp32, 16 for 16-bit types.
-template <typename TD, bool EPI>
-__device__ __forceinline__ void finish_pack(const TcKernelParams& p, float& amax, const TileJob& j, int m, bool row_ok,
-                                            const uint32_t (&r)[32], const uint32_t (&cw)[32], int trunc, uint32_t* out)
+// alpha*acc + beta*C for W outputs (C in registers from load_c_chunk), then the fused epilogue when
+// EPI.  Rows past N and columns past M are computed but never stored: they stay out of the amax.
+template <typename TD, bool EPI, int W>
+__device__ __forceinline__ void finish_values(const TcKernelParams& p, float& amax, const TileJob& j, int m, bool row_ok,
+                                              const uint32_t (&cw)[W], const float (&bias)[W], float (&o)[W])
 {
-    // rows past N and columns past M are computed but never stored: they stay out of the amax
-    const bool use_c = (j.beta != 0.0f) && (j.C != nullptr);
-    if constexpr (sizeof(TD) == 4) {
+    if constexpr (sizeof(TD) != 1) {
+        if (j.beta != 0.0f && j.C != nullptr) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const float a = __uint_as_float(r[i]);
-            float o = use_c ? fmaf(j.alpha, a, j.beta * __uint_as_float(cw[i])) : j.alpha * a;
-            if constexpr (EPI) o = epi_fn(p, m + i, row_ok && m + i < j.M, o, amax);
-            out[i] = __float_as_uint(o);
-        }
-    } else if constexpr (sizeof(TD) == 1) {
-        // E4M3: 32 outputs in 8 words (no C: fp8 outputs take beta == 0)
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            float o[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                o[t] = j.alpha * __uint_as_float(r[4 * q + t]);
-                if constexpr (EPI) o[t] = epi_fn(p, m + 4 * q + t, row_ok && m + 4 * q + t < j.M, o[t], amax);
-                o[t] = out_scale<TD>(p, o[t]);
+            for (int i = 0; i < W; ++i) {
+                float c;
+                if constexpr (sizeof(TD) == 4) {
+                    c = __uint_as_float(cw[i]);
+                } else {
+                    float lo, hi;
+                    unpack2(cw[i >> 1], std::is_same<TD, __half>::value ? 1 : 0, lo, hi);
+                    c = (i & 1) ? hi : lo;
+                }
+                o[i] = fmaf(j.alpha, o[i], j.beta * c);
             }
-            out[q] = pack4_e4m3(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i) o[i] *= j.alpha;
         }
     } else {
-        constexpr int is_half = std::is_same<TD, __half>::value ? 1 : 0;
 #pragma unroll
-        for (int h = 0; h < 16; ++h) {
-            float c0 = 0.f, c1 = 0.f;
-            if (use_c) unpack2(cw[h], is_half, c0, c1);
-            const float a0 = __uint_as_float(r[2 * h]), a1 = __uint_as_float(r[2 * h + 1]);
-            float o0 = use_c ? fmaf(j.alpha, a0, j.beta * c0) : j.alpha * a0;
-            float o1 = use_c ? fmaf(j.alpha, a1, j.beta * c1) : j.alpha * a1;
-            if constexpr (EPI) {
-                o0 = epi_fn(p, m + 2 * h, row_ok && m + 2 * h < j.M, o0, amax);
-                o1 = epi_fn(p, m + 2 * h + 1, row_ok && m + 2 * h + 1 < j.M, o1, amax);
-            }
-            out[h] = pack2(o0, o1, is_half, trunc);
+        for (int i = 0; i < W; ++i) o[i] *= j.alpha;      // no C: fp8 outputs take beta == 0
+    }
+    if constexpr (EPI) epi_apply<W>(p, j.M, m, row_ok, bias, o, amax);
+}
+
+// W finished values as the output's bytes: W words for fp32, W/2 for 16-bit types, W/4 for fp8.
+template <typename TD, int W>
+__device__ __forceinline__ void pack_values(const TcKernelParams& p, const float (&o)[W], uint32_t* out)
+{
+    if constexpr (sizeof(TD) == 4) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) out[i] = __float_as_uint(o[i]);
+    } else if constexpr (sizeof(TD) == 1) {
+#pragma unroll
+        for (int q = 0; q < W / 4; ++q)
+            out[q] = pack4_e4m3(out_scale<TD>(p, o[4 * q]), out_scale<TD>(p, o[4 * q + 1]), out_scale<TD>(p, o[4 * q + 2]),
+                                out_scale<TD>(p, o[4 * q + 3]));
+    } else {
+        constexpr int is_half = std::is_same<TD, __half>::value ? 1 : 0;
+        if (!is_half && p.out_trunc) {
+#pragma unroll
+            for (int h = 0; h < W / 2; ++h) out[h] = pack2(o[2 * h], o[2 * h + 1], 0, 1);
+        } else {
+#pragma unroll
+            for (int h = 0; h < W / 2; ++h) out[h] = pack2(o[2 * h], o[2 * h + 1], is_half, 0);
         }
     }
 }
 
-// Finish a chunk with C already in registers (from load_c_chunk): v = alpha*acc + beta*C, store.
-template <typename TD, bool EPI>
+// Finish a chunk of W consecutive outputs m.. of row n with C already in registers (load_c_chunk):
+// v = alpha*acc + beta*C, the fused epilogue when EPI, convert, store (16-byte vectors, or element
+// by element at ragged edges, unaligned D and for a transposed output, where element m + i lies at
+// (m + i) * ld and a warp's 32 rows make one coalesced access per element).
+template <typename TD, bool EPI, int W>
 __device__ __forceinline__ void store_chunk_pre(const TcKernelParams& p, float& amax, const TileJob& j,
-                                                int64_t base_d, int m, float (&acc)[32], const uint32_t (&cw)[32],
-                                                int trunc)
+                                                int64_t base_d, int m, float (&o)[W], const uint32_t (&cw)[W])
 {
-    const bool use_c = (j.beta != 0.0f) && (j.C != nullptr);
-    float c[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) {
-        if constexpr (sizeof(TD) == 4) {
-            c[i] = __uint_as_float(cw[i]);
-        } else {
-            const uint32_t w = cw[i >> 1];
-            float lo, hi;
-            unpack2(w, std::is_same<TD, __half>::value ? 1 : 0, lo, hi);
-            c[i] = (i & 1) ? hi : lo;
-        }
-    }
-    float o[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) o[i] = use_c ? fmaf(j.alpha, acc[i], j.beta * c[i]) : j.alpha * acc[i];
+    float bias[W];
     if constexpr (EPI) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = epi_fn(p, m + i, m + i < j.M, o[i], amax);
+        if (p.epi_bias != nullptr) load_bias<W>(p, j.M, m, bias);
     }
+    finish_values<TD, EPI, W>(p, amax, j, m, true, cw, bias, o);
     char* dptr = static_cast<char*>(j.D) + (base_d + m) * Out<TD>::kBytes;
-    if (!j.out_t && m + 32 <= j.M && (reinterpret_cast<uintptr_t>(dptr) & 15) == 0) {
-        if constexpr (sizeof(TD) == 4) {
+    if (!j.out_t && m + W <= j.M && (reinterpret_cast<uintptr_t>(dptr) & 15) == 0) {
+        constexpr int words = W * static_cast<int>(sizeof(TD)) / 4;
+        uint32_t w[words];
+        pack_values<TD, W>(p, o, w);
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                reinterpret_cast<float4*>(dptr)[q] = make_float4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
-        } else {
-            constexpr int is_half = std::is_same<TD, __half>::value ? 1 : 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                reinterpret_cast<uint4*>(dptr)[q] =
-                    make_uint4(pack2(o[8 * q], o[8 * q + 1], is_half, trunc), pack2(o[8 * q + 2], o[8 * q + 3], is_half, trunc),
-                               pack2(o[8 * q + 4], o[8 * q + 5], is_half, trunc),
-                               pack2(o[8 * q + 6], o[8 * q + 7], is_half, trunc));
-        }
+        for (int q = 0; q < words / 4; ++q)
+            reinterpret_cast<uint4*>(dptr)[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
     } else {
-        const int64_t dstep = j.out_t ? j.ldd : 1;
+        float v[W];
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-            if (m + i < j.M) Out<TD>::store(j.D, base_d + (m + i) * dstep, o[i], trunc);
+        for (int i = 0; i < W; ++i) v[i] = o[i];
+        const int64_t step = j.out_t ? j.ldd : 1;
+        store_elements<TD>(j.D, base_d + m * step, step, min(W, j.M - m), v, p.epi_dscale, p.out_trunc);
     }
 }
+
+// The same with C read here: all of the chunk's C before any of its D is written (D may be C itself).
+template <typename TD, bool EPI, int W>
+__device__ __forceinline__ void store_chunk(const TcKernelParams& p, float& amax, const TileJob& j, int64_t base_c,
+                                           int64_t base_d, int m, float (&acc)[W])
+{
+    uint32_t cw[W];
+    load_c_chunk<TD, W>(j, base_c, m, cw);
+    store_chunk_pre<TD, EPI, W>(p, amax, j, base_d, m, acc, cw);
+}
+
+// A warp's access to 32 rows x 128 bytes of C or D, whole lines at a time: in step i lane L holds
+// 16-byte unit L % 8 of row 4 i + L / 8 (eight lanes to a row's 128 bytes).  In shared memory unit u of
+// row r sits at u ^ (r & 7).  Rows past `rows` and units past M are neither read nor written (M is a
+// whole number of units).
+template <typename TD>
+struct LineAccess {
+    static constexpr int EPU = 16 / static_cast<int>(sizeof(TD));
+    int u, r0, rows, M;
+    __device__ __forceinline__ LineAccess(int lane, int rows_, int M_) : u(lane & 7), r0(lane >> 3), rows(rows_), M(M_) {}
+    __device__ __forceinline__ uint32_t at(int i) const
+    {
+        const int r = 4 * i + r0;
+        return static_cast<uint32_t>(r * 128 + ((u ^ (r & 7)) * 16));
+    }
+    // `base`: element (m = 0, first row); `ld`: elements between rows
+    __device__ __forceinline__ void load(const void* C, int64_t base, int64_t ld, int m, uint4 (&v)[8]) const
+    {
+        const int col = m + u * EPU;
+        const TD* src = static_cast<const TD*>(C) + base + static_cast<int64_t>(r0) * ld + col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            v[i] = (4 * i + r0 < rows && col < M) ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<int64_t>(4 * i) * ld))
+                                                  : make_uint4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ void stage(uint32_t buf, const uint4 (&v)[8]) const
+    {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ptx::st_shared_v4(buf + at(i), v[i].x, v[i].y, v[i].z, v[i].w);
+    }
+    __device__ __forceinline__ void store(void* D, int64_t base, int64_t ld, int m, uint32_t buf) const
+    {
+        const int col = m + u * EPU;
+        TD* dst = static_cast<TD*>(D) + base + static_cast<int64_t>(r0) * ld + col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint4 v = ptx::ld_shared_v4(buf + at(i));
+            if (4 * i + r0 < rows && col < M) *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(4 * i) * ld) = v;
+        }
+    }
+};
 
 // Hand a drained TMEM buffer back to the MMA issuer: one arrival per epilogue warp, on the leader
 // CTA's barrier (a remote arrival when this CTA is the peer of a pair).
@@ -673,80 +677,6 @@ __device__ __forceinline__ void release_tmem(uint64_t* bar, int lane)
     }
 }
 
-// Split-k completion that keeps this split's own partial in TMEM: the partial was parked in the
-// workspace for the other splits; if this CTA is the last of the tile to arrive it sums the
-// partials in split order -- its own read back from TMEM, the others from the workspace with all of
-// a chunk's loads in flight -- and runs the epilogue.  The TMEM buffer is released afterwards.
-template <typename TD, int CG, bool EPI>
-__device__ __forceinline__ void split_finish_tmem(const TcKernelParams& p, float& amax, const TileJob& j, bool ok,
-                                                  int et, int lane,
-                                                  int row, bool row_ok, int64_t base_c, int64_t base_d,
-                                                  volatile int* last_flag, uint32_t tbase, uint64_t* tempty_bar)
-{
-    __threadfence();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (et == 0) {
-        int last = 0;
-        if (ok) last = (atomicAdd(p.counters + j.slot, 1) == j.nsplit - 1) ? 1 : 0;
-        *last_flag = last;
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    const int is_last = *last_flag;
-    if (is_last && ok) {
-        __threadfence();
-        // CPS 32-column chunks per step (two for 16-bit outputs, one for fp32, whose C takes twice
-        // the registers): their C values and every other split's partials are in flight together
-        // (the reduction is latency-bound), summed in split order
-        constexpr int CPS = sizeof(TD) == 2 ? 2 : 1;
-        const int chunks = p.bm / 32;     // even: bm is 64, 128, 192 or 256
-        const size_t slab_elems = static_cast<size_t>(kTcTileN) * p.bm;
-        const float* base = p.ws + static_cast<size_t>(j.slot) * p.tail_split * slab_elems + row;
-        for (int c = 0; c < chunks; c += CPS) {
-            const int m0 = j.m0 + c * 32;
-            uint32_t cw[CPS][32];
-            if (CPS > 1 && row_ok) {
-#pragma unroll
-                for (int q = 0; q < CPS; ++q) load_c_chunk<TD>(j, base_c, m0 + 32 * q, cw[q]);
-            }
-            float v[CPS * 32];
-#pragma unroll
-            for (int i = 0; i < CPS * 32; ++i) v[i] = 0.f;
-            for (int s = 0; s < j.nsplit; ++s) {
-                if (s == j.split) {
-#pragma unroll
-                    for (int q = 0; q < CPS; ++q) {
-                        uint32_t r[32];
-                        __syncwarp();
-                        ptx::tmem_ld32(tbase + (c + q) * 32, r);
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) v[32 * q + i] += __uint_as_float(r[i]);
-                    }
-                } else {
-                    float a[CPS * 32];
-                    const float* src = base + static_cast<size_t>(s) * slab_elems + static_cast<size_t>(c) * 32 * kTcTileN;
-#pragma unroll
-                    for (int i = 0; i < CPS * 32; ++i) a[i] = __ldcg(src + i * kTcTileN);
-#pragma unroll
-                    for (int i = 0; i < CPS * 32; ++i) v[i] += a[i];
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < CPS; ++q) {
-                if (row_ok && m0 + 32 * q < j.M) {
-                    float o[32];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) o[i] = v[32 * q + i];
-                    if constexpr (CPS > 1) store_chunk_pre<TD, EPI>(p, amax, j, base_d, m0 + 32 * q, o, cw[q], p.out_trunc);
-                    else store_chunk<TD, EPI>(p, amax, j, base_c, base_d, m0 + 32 * q, o, p.out_trunc);
-                }
-            }
-        }
-        if (et == 0) p.counters[j.slot] = 0;   // ready for the next launch
-    }
-    if (ok) release_tmem<CG>(tempty_bar, lane);
-    asm volatile("bar.sync 1, 128;" ::: "memory");   // last_flag is reused by the next tile
-}
-
 // Bounded wait until *ctr >= target (acquire at GPU scope); false once limit_ns has passed.
 __device__ __forceinline__ bool wait_counter_ge(const int* ctr, int target, uint64_t limit_ns)
 {
@@ -760,69 +690,80 @@ __device__ __forceinline__ bool wait_counter_ge(const int* ctr, int target, uint
     }
 }
 
-// Split-k completion when every split unit of the launch is resident at once (all of them in the
-// first round of the persistent schedule): each split has parked its partial tile, waits until the
-// tile's other splits have too, then reduces its share of the tile -- 32-column chunks split,
-// split + nsplit, ... -- summing the partials in split order (the same sums, bit for bit, as the
-// last-arriver path) and runs their epilogue.  The tile counter counts arrivals up to nsplit, then
-// finished shares up to 2 * nsplit, when the last one resets it for the next launch.
-template <typename TD, int CG, bool EPI>
-__device__ __forceinline__ void split_finish_parallel(const TcKernelParams& p, float& amax, const TileJob& j, bool& ok,
-                                                      int et,
-                                                      int lane, int row, bool row_ok, int64_t base_c, int64_t base_d,
-                                                      volatile int* last_flag, uint64_t* tempty_bar,
-                                                      volatile int* abort_flag, bool c_staged, uint32_t c_row)
+// Split-k completion, run by the epilogue warps after this split parked its partial tile in the
+// workspace (layout [32-column chunk][column][row], so every warp access is one 128-byte line; the
+// TMEM buffer is free again).  The partials are summed in split order, so the result does not depend on
+// which CTA finishes when, and the epilogue runs on the sums.  A warp of each TMEM quarter takes W of
+// a chunk's 32 columns.
+//   p.par_reduce   every split unit of the launch is resident at once (all in the first round of the
+//                  persistent schedule): each split waits until the tile's other splits have parked
+//                  theirs, then reduces its share of the tile -- chunks split, split + nsplit, ...
+//                  The tile counter counts arrivals up to nsplit, then finished shares up to
+//                  2 * nsplit, when the last one resets it for the next launch.
+//   otherwise      the last split to arrive (tile counter) reduces the whole tile and resets it.
+// Every thread passes the same named barriers whether or not it has work, so a warp that gave up on
+// a wait cannot strand the others.
+template <typename TD, bool EPI, int NH>
+__device__ __forceinline__ void split_finish(const TcKernelParams& p, float& amax, const TileJob& j, bool& ok, int et,
+                                             int lane, int half, int row, bool row_ok, int64_t base_c, int64_t base_d,
+                                             volatile int* last_flag, volatile int* abort_flag, bool c_staged,
+                                             uint32_t c_row)
 {
-    if (ok) release_tmem<CG>(tempty_bar, lane);     // this split's partial is in the workspace
+    constexpr int W = 32 / NH;                      // columns of a chunk per warp
+    const bool par = p.par_reduce != 0;
     __threadfence();
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    ptx::named_sync<NH * 128>();
     if (et == 0) {
         int go = 0;
         if (ok) {
-            atomicAdd(p.counters + j.slot, 1);
-            go = wait_counter_ge(p.counters + j.slot, j.nsplit, p.timeout_ns) ? 1 : 0;
-            if (!go) record_error(p, abort_flag, 16);
+            const int before = atomicAdd(p.counters + j.slot, 1);
+            if (par) {
+                go = wait_counter_ge(p.counters + j.slot, j.nsplit, p.timeout_ns) ? 1 : 0;
+                if (!go) record_error(p, abort_flag, 16);
+            } else {
+                go = before == j.nsplit - 1 ? 1 : 0;
+            }
         }
         *last_flag = go;
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    ptx::named_sync<NH * 128>();
     const int go = *last_flag;
     if (go) {
         __threadfence();
-        const int chunks = p.bm / 32;
+        const int chunks = p.bm / 32, step = par ? j.nsplit : 1;
         const size_t slab_elems = static_cast<size_t>(kTcTileN) * p.bm;
-        const float* base = p.ws + static_cast<size_t>(j.slot) * p.tail_split * slab_elems + row;
-        for (int c = j.split; c < chunks; c += j.nsplit) {
-            const int m = j.m0 + c * 32;
-            const bool live = row_ok && m < j.M;
+        const float* base = p.ws + static_cast<size_t>(j.slot) * p.tail_split * slab_elems +
+                            static_cast<size_t>(half) * W * kTcTileN + row;
+        for (int c = par ? j.split : 0; c < chunks; c += step) {
+            const int m = j.m0 + c * 32 + half * W;
             // two splits' partials at a time are in flight together (the reduction is
             // latency-bound), summed in split order
-            float v[32];
+            float v[W];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = 0.f;
-            for (int s = 0; s < j.nsplit; s += 2) {
-                float a[32], b[32];
-                const float* sa = base + static_cast<size_t>(s) * slab_elems + static_cast<size_t>(c) * 32 * kTcTileN;
+            for (int i = 0; i < W; ++i) v[i] = 0.f;
+            const float* sa = base + static_cast<size_t>(c) * 32 * kTcTileN;
+            for (int s = 0; s < j.nsplit; s += 2, sa += 2 * slab_elems) {
+                float a[W], b[W];
                 const bool two = s + 1 < j.nsplit;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
+                for (int i = 0; i < W; ++i) {
                     a[i] = __ldcg(sa + i * kTcTileN);
                     b[i] = two ? __ldcg(sa + slab_elems + i * kTcTileN) : 0.f;
                 }
 #pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] += a[i];
+                for (int i = 0; i < W; ++i) v[i] += a[i];
                 if (two) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) v[i] += b[i];
+                    for (int i = 0; i < W; ++i) v[i] += b[i];
                 }
             }
-            if (live) {
+            if (row_ok && m < j.M) {
+                uint32_t cw[W];
                 if (c == j.split && c_staged) {
                     // this chunk's C row was copied into shared memory while the tile accumulated
                     // (16-byte unit u at u ^ (lane & 7))
-                    uint32_t cw[32];
                     ptx::cp_async_wait0();
-                    constexpr int NU = 32 * static_cast<int>(sizeof(TD)) / 16;
+                    constexpr int NU = W * static_cast<int>(sizeof(TD)) / 16;
 #pragma unroll
                     for (int u = 0; u < NU; ++u) {
                         const uint4 w4 = ptx::ld_shared_v4(c_row + static_cast<uint32_t>((u ^ (lane & 7)) * 16));
@@ -831,28 +772,32 @@ __device__ __forceinline__ void split_finish_parallel(const TcKernelParams& p, f
                         cw[4 * u + 2] = w4.z;
                         cw[4 * u + 3] = w4.w;
                     }
-                    store_chunk_pre<TD, EPI>(p, amax, j, base_d, m, v, cw, p.out_trunc);
                 } else {
-                    store_chunk<TD, EPI>(p, amax, j, base_c, base_d, m, v, p.out_trunc);
+                    load_c_chunk<TD, W>(j, base_c, m, cw);
                 }
+                store_chunk_pre<TD, EPI, W>(p, amax, j, base_d, m, v, cw);
             }
         }
-    } else {
+    } else if (par) {
         ok = false;
     }
     if (c_staged) ptx::cp_async_wait0();   // the staging buffer is free again (also on the error path)
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    ptx::named_sync<NH * 128>();           // last_flag is reused by the next tile
     if (et == 0 && go) {
+        if (!par) p.counters[j.slot] = 0;  // ready for the next launch
         // counts this split out of the tile: the last one resets the counter for the next launch.
         // No fence: the counter only orders the splits' waits (same-address atomics), and the next
         // launch's use of the workspace is ordered by the kernel boundary.
-        if (atomicAdd(p.counters + j.slot, 1) == 2 * j.nsplit - 1) atomicExch(p.counters + j.slot, 0);
+        else if (atomicAdd(p.counters + j.slot, 1) == 2 * j.nsplit - 1) atomicExch(p.counters + j.slot, 0);
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");   // last_flag is reused by the next tile
 }
 
-template <int KIND, typename TD, int CL, bool EPI>
-__global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_constant__ TcKernelParams p)
+// PROMO: the kernels with promoted accumulation (promote_k > 0), whose four epilogue warps hold 128
+// running sums per thread; the others have eight epilogue warps, two per quarter of the TMEM lanes,
+// which take alternate column groups of a tile (half the drain time of a CTA's last tile, and of every
+// tile whose k is too short to hide it).  GROUP: the work units and problems come from a plan's tables.
+template <int KIND, typename TD, int CL, bool EPI, bool PROMO, bool GROUP>
+__global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __grid_constant__ TcKernelParams p)
 {
     // CL CTAs per cluster.  CL == 2: a CTA pair on two SMs works on one 256-row tile.  Each CTA
     // stages its own 128 rows of the n-side operand and its half of the m-side operand; the leader
@@ -866,6 +811,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
     // have released it (each slot's empty barrier expects one commit from each pair's leader).
     constexpr int CG = CL >= 2 ? 2 : 1;         // CTAs per MMA (cta_group)
     constexpr int MC = CL / CG;                 // pairs sharing the m-side operand
+    constexpr int NH = PROMO ? 1 : 2;           // epilogue warps per TMEM lane quarter
     if (threadIdx.x == 0 && p.trace != nullptr) {
         trace_mark(p, TL_TRACE_ENTRY);
         trace_put(p, TL_TRACE_ENTRY_NS, global_ns());
@@ -878,7 +824,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
     const uint32_t bmc = static_cast<uint32_t>(p.bm) / CG;            // m-side rows staged by this CTA
     const uint32_t tileN_bytes = kTcTileN * kTcRowBytes;
     const uint32_t stage_bytes = tileN_bytes + bmc * kTcRowBytes;
-    // output staging for TMA stores: 4 epilogue warps x epi_bufs x 32 rows x 128 bytes, 1024-byte aligned
+    // output staging for TMA stores: epi_bufs x 4 epilogue warps x 32 rows x 128 bytes, 1024-byte aligned
     uint8_t* epi_stage = smem + static_cast<size_t>(p.stages) * stage_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + static_cast<size_t>(p.epi_bufs) * kTcEpiStageBytes);
     uint64_t* empty = full + kTcMaxStages;
@@ -900,12 +846,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
     const bool leader = (pair_rank == 0);
     const int64_t unit0 = (CL > 1) ? static_cast<int64_t>(ptx::cluster_id_x()) : static_cast<int64_t>(blockIdx.x);
     const int64_t units = (CL > 1) ? static_cast<int64_t>(ptx::ncluster_x()) : static_cast<int64_t>(gridDim.x);
-    const bool promo = p.promote_kb > 0;
-    const bool sep_small = promo && p.nterms > 1;
+    const bool sep_small = PROMO && p.nterms > 1;
     // TMEM columns: main accumulator x2 (+ small-term accumulator x2 when they are kept apart)
     const uint32_t need_cols = static_cast<uint32_t>(p.bm) * (sep_small ? 4u : 2u);
     const uint32_t tmem_cols = need_cols <= 128 ? 128u : (need_cols <= 256 ? 256u : 512u);
-    const uint32_t epi_arrivals = 4u * CG;     // one per epilogue warp of each CTA
+    const uint32_t epi_arrivals = 4u * NH * CG;     // one per epilogue warp of each CTA
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
@@ -932,7 +877,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
             ptx::tmem_relinquish();
         }
     }
-    if (warp == 0 && lane == 0 && p.group == nullptr) {
+    if (!GROUP && warp == 0 && lane == 0) {
         for (int v = 0; v < p.nterms; ++v) {
             ptx::prefetch_tmap(&p.tmN[p.term_n[v]]);
             ptx::prefetch_tmap(&p.tmM[p.term_m[v]]);
@@ -946,11 +891,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
     if (threadIdx.x == 0) trace_mark(p, TL_TRACE_SETUP);
     // Launched as a programmatic dependent: everything above (barrier set-up, TMEM allocation,
     // descriptor prefetch) may have run while the previous kernel in the stream was finishing.
-    // Wait for that grid to complete (its writes visible) before touching global memory, then let
-    // the next dependent grid start its own set-up as soon as SMs free up.
-    ptx::grid_dep_wait();
-    ptx::grid_dep_launch_dependents();
-    if (threadIdx.x == 0) trace_mark(p, TL_TRACE_DEP);
+    // Every role that touches global memory first decodes its first work unit (from the kernel
+    // parameters and, for a group, the plan's tables, which no kernel writes), then waits for that
+    // grid to complete (its writes visible); the producer then lets the next dependent grid start
+    // its own set-up as soon as SMs free up.  Decoding after the wait put ~2000 clocks, most of it
+    // instruction fetch, between the previous grid's end and the first copy.
     const int nvirt = p.nterms;
     const uint64_t tlim = p.timeout_ns;
 
@@ -1042,45 +987,58 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                 }
                 return true;
             };
-            auto produce = [&](auto n_mn, auto m_mn) {
-                int4 u_next = load_unit(p, unit0);
-                for (int64_t w = unit0; w < p.total_work && ok; w += units) {
-                    const int4 u = u_next;
-                    u_next = load_unit(p, w + units);      // in flight during this tile
-                    TileJob j;
-                    get_job(p, w, u, j);
-                    const int n0 = j.n0 + static_cast<int>(rank) * kTcTileN;
-                    const int m0 = j.m0 + static_cast<int>(pair_rank * bmc);
-                    // timeline stamps stay outside the k-block loops (a branch there slows the issue)
-                    if (w == unit0) trace_mark(p, TL_TRACE_LOAD_FIRST);
-                    int k0 = j.kb0 * W;
-                    if (nvirt == 1) {
-                        const void* mapN = j.tmN;
-                        const void* mapM = j.tmM;
-                        for (int i = j.kb1 - j.kb0; i > 0; --i) {
-                            if (!(ok = fill(n_mn, m_mn, mapN, mapM, k0, n0, m0, j.b))) break;
-                            k0 += W;
-                        }
-                    } else {
-                        // split-precision products, smallest first (term table set by the host)
-                        for (int i = j.kb1 - j.kb0; i > 0 && ok; --i) {
-                            for (int v = 0; v < nvirt; ++v)
-                                if (!(ok = fill(n_mn, m_mn, &p.tmN[p.term_n[v]], &p.tmM[p.term_m[v]], k0, n0, m0, j.b)))
-                                    break;
+            // a tile's stages; the layouts are compile-time inside
+            auto produce = [&](auto n_mn, auto m_mn, const TileJob& j, int n0, int m0) {
+                int k0 = j.kb0 * W;
+                if (nvirt == 1) {
+                    for (int i = j.kb1 - j.kb0; i > 0; --i) {
+                        if (!(ok = fill(n_mn, m_mn, j.tmN, j.tmM, k0, n0, m0, j.b))) break;
+                        k0 += W;
+                    }
+                } else {
+                    // split-precision products, smallest first (term table set by the host)
+                    int v = 0;
+                    for (int i = (j.kb1 - j.kb0) * nvirt; i > 0; --i) {
+                        if (!(ok = fill(n_mn, m_mn, &p.tmN[p.term_n[v]], &p.tmM[p.term_m[v]], k0, n0, m0, j.b))) break;
+                        if (++v == nvirt) {
+                            v = 0;
                             k0 += W;
                         }
                     }
-                    if (w == unit0) trace_mark(p, TL_TRACE_LOAD_LAST);
                 }
             };
             using Yes = std::true_type;
             using No = std::false_type;
-            if (p.n_mn_major) {
-                if (p.m_mn_major) produce(Yes{}, Yes{});
-                else produce(Yes{}, No{});
-            } else {
-                if (p.m_mn_major) produce(No{}, Yes{});
-                else produce(No{}, No{});
+            int64_t w = unit0;                         // < total_work: the grid is never larger
+            int4 u = load_unit<GROUP>(p, w);
+            int4 u_next = load_unit<GROUP>(p, w + units);     // in flight during this tile
+            bool first = true;
+#pragma unroll 1
+            while (true) {
+                TileJob j;
+                get_job<GROUP>(p, w, u, j);
+                const int n0 = j.n0 + static_cast<int>(rank) * kTcTileN;
+                const int m0 = j.m0 + static_cast<int>(pair_rank * bmc);
+                // timeline stamps stay outside the k-block loops (a branch there slows the issue)
+                if (first) {
+                    ptx::grid_dep_wait();
+                    ptx::grid_dep_launch_dependents();
+                    trace_mark(p, TL_TRACE_DEP);
+                    trace_mark(p, TL_TRACE_LOAD_FIRST);
+                }
+                if (p.n_mn_major) {
+                    if (p.m_mn_major) produce(Yes{}, Yes{}, j, n0, m0);
+                    else produce(Yes{}, No{}, j, n0, m0);
+                } else {
+                    if (p.m_mn_major) produce(No{}, Yes{}, j, n0, m0);
+                    else produce(No{}, No{}, j, n0, m0);
+                }
+                if (first) trace_mark(p, TL_TRACE_LOAD_LAST);
+                first = false;
+                w += units;
+                if (!ok || w >= p.total_work) break;
+                u = u_next;
+                u_next = load_unit<GROUP>(p, w + units);
             }
         }
         __syncwarp();
@@ -1127,12 +1085,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                 return true;
             };
             bool ok = true;
-            int4 u_next = load_unit(p, unit0);
+            // (touches no global memory but the error word and the timeline)
+            if (p.trace != nullptr) ptx::grid_dep_wait();
+            int4 u_next = load_unit<GROUP>(p, unit0);
             for (int64_t w = unit0; w < p.total_work && ok; w += units) {
                 const int4 u = u_next;
-                u_next = load_unit(p, w + units);      // in flight during this tile
+                u_next = load_unit<GROUP>(p, w + units);      // in flight during this tile
                 TileJob j;
-                get_job(p, w, u, j);
+                get_job<GROUP>(p, w, u, j);
                 const int nkb = j.kb1 - j.kb0;
                 if (nkb <= 0) continue;                 // an empty unit of a balanced split
                 if (sep_small) {
@@ -1153,7 +1113,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                     ptx::mbar_wait(bar, phase, tlim);
                     trace_mark(p, TL_TRACE_MMA_FIRST);
                 }
-                if (!promo) {
+                if constexpr (!PROMO) {
                     // every product of the tile into one accumulator
                     const uint32_t d_tmem = tmem_base + mbuf * bmu;
                     uint32_t accumulate = 0;
@@ -1208,26 +1168,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
         }
         __syncwarp();
     } else {
-        // ------------------------------------------------------------------ epilogue (4 warps, each CTA)
-        // All four warps run the same loop and, in split-k mode, the same named barriers: after a
+        // ------------------------------------------------------------------ epilogue (4 * NH warps, each CTA)
+        // All of them run the same loop and, in split-k mode, the same named barriers: after a
         // timed-out wait a warp keeps the control flow and only skips the work, so no warp can be
         // left waiting at bar.sync 1 for one that gave up.
         const int quarter = warp & 3;             // TMEM lanes 32*quarter .. +31
         const int row = quarter * 32 + lane;      // tile row = problem n offset within this CTA
-        const int et = threadIdx.x - 64;          // 0..127
-        uint8_t* const my_stage = epi_stage + static_cast<size_t>(quarter) * p.epi_bufs * 4096u;   // this warp's staging
-        const uint32_t my_stage_a = ptx::smem_u32(my_stage);
-        uint32_t stage_off = 0;                   // buffer the next staged store fills
+        const int half = (warp - 2) >> 2;         // which of the quarter's NH warps
+        const int et = threadIdx.x - 64;          // 0 .. 128 * NH - 1
+        // staging: 4 KB per warp; where shared memory holds only 16 KB of it, the second warp of a quarter
+        // takes no part in staged stores.  The one warp of a promotion kernel stages nothing.
+        const int nst = min(NH, p.epi_bufs);      // staging warps per quarter
+        const uint32_t my_stage_a = ptx::smem_u32(epi_stage) + static_cast<uint32_t>(min(half, nst - 1) * 4 + quarter) * 4096u;
         const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
         uint32_t mbuf = 0, mph = 0, sbuf = 0, sph = 0;
         const int chunks = p.bm / 32;
         bool ok = true;
         float amax = 0.0f;                        // fused epilogue: this thread's max |output|
         unsigned long long units_done = 0;
+#pragma unroll 1
         for (int64_t w = unit0; w < p.total_work; w += units) {
-            const int4 u = load_unit(p, w);      // the epilogue trails the MMAs: no need to load ahead
+            // the epilogue trails the MMAs: no need to load the unit ahead
             TileJob j;
-            get_job(p, w, u, j);
+            get_job<GROUP>(p, w, load_unit<GROUP>(p, w), j);
+            if (w == unit0) ptx::grid_dep_wait();
             if (j.kb1 <= j.kb0) continue;             // an empty unit of a balanced split
             ++units_done;
             const bool tr = (et == 0 && w == unit0);  // timeline stamps: the first tile, one thread
@@ -1244,27 +1208,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                 // while the tile is still accumulating
                 const char* cp = static_cast<const char*>(j.C) + (base_c + j.m0) * static_cast<int64_t>(sizeof(TD));
                 const int cbytes = (min(p.bm, j.M - j.m0)) * static_cast<int>(sizeof(TD));
-                for (int off = 0; off < cbytes; off += 128)
+                for (int off = 128 * half; off < cbytes; off += 128 * NH)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(cp + off));
             }
-            if (ok && j.out_t && j.beta != 0.0f && j.C != nullptr) {
-                // transposed output: the warp's C is a 64- or 128-byte run of each column; lane L
-                // pulls column L of every 32-column chunk into L2 (both lines a run may touch)
-                const int nrow0 = j.n0 + quarter * 32;
-                if (nrow0 < j.N) {
-                    for (int c = 0; c < chunks; ++c) {
-                        const int ccol = j.m0 + c * 32 + lane;
-                        if (ccol >= j.M) break;
-                        const char* cp = static_cast<const char*>(j.C) +
-                                         (static_cast<int64_t>(j.b) * p.stride_c + static_cast<int64_t>(ccol) * j.ldc + nrow0) *
-                                             static_cast<int64_t>(sizeof(TD));
-                        const int last = (min(32, j.N - nrow0) * static_cast<int>(sizeof(TD))) - 1;
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cp));
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(cp + last));
-                    }
-                }
-            }
-            if (promo) {
+            if constexpr (PROMO) {
                 // ---- promotion: sum the A0*B0 chains (and the small terms) in fp32 registers; bm == 128
                 float run[128];
 #pragma unroll
@@ -1326,7 +1273,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                             float v[32];
 #pragma unroll
                             for (int i = 0; i < 32; ++i) v[i] = run[q * 32 + i];
-                            store_chunk<TD, EPI>(p, amax, j, base_c, base_d, m, v, p.out_trunc);
+                            store_chunk<TD, EPI, 32>(p, amax, j, base_c, base_d, m, v);
                         }
                     }
                     if (tr) trace_mark(p, TL_TRACE_STORED);
@@ -1342,26 +1289,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                         }
                     }
                     if (tr) trace_mark(p, TL_TRACE_STORED);
-                    split_finish<TD, EPI>(p, amax, j, ok, et, row, row_ok, base_c, base_d, last_flag);
+                    split_finish<TD, EPI, 1>(p, amax, j, ok, et, lane, 0, row, row_ok, base_c, base_d, last_flag, abort_flag,
+                                             false, 0u);
                     if (tr) trace_mark(p, TL_TRACE_REDUCED);
                 }
-                continue;
-            }
+            } else {
             // ---- one TMEM accumulator per tile
             // parallel split-k: this split finishes 32-column chunk `split` of the tile.  Its C does
             // not depend on the accumulator: each thread copies its row of it into the warp's
-            // output staging buffer (free in this mode: no TMA store is in flight from it) while the
-            // tile accumulates.
+            // output staging buffer (free in this mode) while the tile accumulates.
             bool c_staged = false;
             const uint32_t c_row = my_stage_a + static_cast<uint32_t>(lane) * 128u;
             if constexpr (sizeof(TD) >= 2) {
-                const int mc = j.m0 + j.split * 32;
-                if (p.par_reduce && !j.out_t && j.nsplit > 1 && j.beta != 0.0f && j.C != nullptr && j.split * 32 < p.bm) {
-                    if (lane == 0) ptx::bulk_wait_read0();
-                    __syncwarp();
+                constexpr int WC = 32 / NH;           // this warp's columns of the chunk
+                const int mc = j.m0 + j.split * 32 + half * WC;
+                if (p.par_reduce && half < nst && !j.out_t && j.nsplit > 1 && j.beta != 0.0f && j.C != nullptr &&
+                    j.split * 32 < p.bm) {
                     const char* cptr = static_cast<const char*>(j.C) + (base_c + mc) * static_cast<int64_t>(sizeof(TD));
-                    if (row_ok && mc + 32 <= j.M && (reinterpret_cast<uintptr_t>(cptr) & 15) == 0) {
-                        constexpr int NU = 32 * static_cast<int>(sizeof(TD)) / 16;
+                    if (row_ok && mc + WC <= j.M && (reinterpret_cast<uintptr_t>(cptr) & 15) == 0) {
+                        constexpr int NU = WC * static_cast<int>(sizeof(TD)) / 16;
 #pragma unroll
                         for (int u = 0; u < NU; ++u)
                             ptx::cp_async16(c_row + static_cast<uint32_t>((u ^ (lane & 7)) * 16), cptr + 16 * u);
@@ -1370,112 +1316,75 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                     ptx::cp_async_commit();
                 }
             }
-            // (D may be C itself: a chunk's C is read before any of its columns is stored)
-            uint32_t cw[32];
-            if (row_ok && j.nsplit == 1 && !j.out_t && j.tmD != nullptr) load_c_chunk<TD>(j, base_c, j.m0, cw);
+            // whole tiles with 16-byte accessible D and C leave through this warp's staging buffer, a
+            // group of CPS 32-column chunks (128 bytes of output per row) at a time.  C comes in
+            // through it too, whole lines at a time like the stores; the first group's C is in flight
+            // before the accumulator is ready (D may be C itself: a group's C is read before any of
+            // its columns is stored).
+            constexpr int CPS = static_cast<int>(4 / sizeof(TD));
+            const int nrow0 = j.n0 + quarter * 32;
+            const bool staged = j.vec && j.nsplit == 1 && !j.out_t && chunks >= CPS;
+            const bool use_c = j.beta != 0.0f && j.C != nullptr;
+            const int groups = half < nst ? chunks / CPS : 0;
+            constexpr int WQ = EPI && sizeof(TD) != 1 ? 8 : 16;      // columns finished at a time
+            LineAccess<TD> la(lane, j.N - nrow0, j.M);
+            uint4 cl[8];
+            float bl[CPS];
+            if constexpr (EPI) {
+                if (staged && half < groups) lane_bias<CPS>(p, j.M, j.m0 + half * CPS * 32 + lane, bl);
+            }
+            if constexpr (sizeof(TD) >= 2) {
+                if (staged && use_c && half < groups)
+                    la.load(j.C, static_cast<int64_t>(j.b) * p.stride_c + static_cast<int64_t>(nrow0) * j.ldc, j.ldc,
+                            j.m0 + half * CPS * 32, cl);
+            }
+            const uint32_t tbase = tmem_base + lane_off + mbuf * static_cast<uint32_t>(p.bm);
             bool got = ok && ptx::mbar_wait(&tfull[mbuf], mph, tlim);
             got = __all_sync(0xffffffffu, got);
             if (ok && !got) {
                 if (lane == 0) record_error(p, abort_flag, 8);
                 ok = false;
             }
-            const uint32_t tbase = tmem_base + lane_off + mbuf * static_cast<uint32_t>(p.bm);
             if (ok) ptx::tc_fence_after();
             if (tr) trace_mark(p, TL_TRACE_ACC_READY);
-            // A staged TMA store costs a round trip per 32 rows (the one 4 KB buffer per warp is
-            // refilled only after the previous store has read it): hidden behind the next tile's
-            // main loop, but exposed on a CTA's last tile, which uses the direct stores instead
-            // when beta == 0 (with a C operand to read, the staged path measured faster).
-            const bool direct = p.direct_last && !j.out_t && j.beta == 0.0f && w + units >= p.total_work;
             if constexpr (sizeof(TD) >= 2 && !EPI) {
-                if (j.out_t && j.nsplit == 1 && j.tmD != nullptr) {
-                    // transposed output: a warp's 32 rows are 32 consecutive elements of D's columns,
-                    // so each 32-column chunk is one 32 x 32 box of D, staged [column][row] (two boxes
-                    // per 4 KB buffer for 16-bit outputs, one for fp32) and written by one TMA store.
-                    // The boxes are filled in turn, one per committed store; a box is refilled once
-                    // the store that last used it has read it.  With beta, lane L first brings column L of the chunk's C (contiguous
-                    // in memory) into the box, and every lane then replaces its row of C by D.
-                    constexpr int CB = 32 * 32 * static_cast<int>(sizeof(TD));   // bytes per box
-                    const uint32_t stage_bytes_all = static_cast<uint32_t>(p.epi_bufs) * 4096u;
-                    constexpr int COLB = CB / 32;                                  // bytes per box column
-                    const int nrow0 = j.n0 + quarter * 32;
-                    const bool use_c = j.beta != 0.0f && j.C != nullptr;
-                    for (int c = 0; c < chunks && ok; ++c) {
+                if (j.out_t && j.nsplit == 1 && j.vec) {
+                    // transposed output (beta == 0): a warp's 32 rows are 32 consecutive elements of D's
+                    // columns, so each 32-column chunk is staged [column][row] and written in runs of
+                    // a column's 64 (16-bit) or 128 bytes
+                    constexpr int COLB = 32 * static_cast<int>(sizeof(TD));      // bytes per column
+                    constexpr int UPC = COLB / 16, EPU = 16 / static_cast<int>(sizeof(TD));
+                    const int u = lane % UPC, col0 = lane / UPC;
+                    const bool in_n = nrow0 + u * EPU < j.N;      // N (D's rows here) is whole units
+                    if (half >= nst && ok) release_tmem<CG>(&tempty[mbuf], lane);
+                    for (int c = half; c < chunks && half < nst && ok; c += nst) {
                         const int m = j.m0 + c * 32;
-                        if (lane == 0) {
-                            if (stage_bytes_all == 4 * CB) ptx::bulk_wait_read3();
-                            else if (stage_bytes_all == 2 * CB) ptx::bulk_wait_read1();
-                            else ptx::bulk_wait_read0();
-                        }
-                        __syncwarp();
-                        uint8_t* box = my_stage + stage_off;
-                        const uint32_t ba = ptx::smem_u32(box);
-                        if (use_c) {
-                            const int ccol = m + lane;
-                            if (ccol < j.M) {
-                                const int64_t cbase = static_cast<int64_t>(j.b) * p.stride_c +
-                                                      static_cast<int64_t>(ccol) * j.ldc + nrow0;
-                                const char* src = static_cast<const char*>(j.C) + cbase * static_cast<int64_t>(sizeof(TD));
-                                if (nrow0 + 32 <= j.N && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-                                    // every load of the column is in flight before the first store
-                                    uint4 v4[COLB / 16];
-#pragma unroll
-                                    for (int q = 0; q < COLB / 16; ++q) v4[q] = __ldg(reinterpret_cast<const uint4*>(src) + q);
-#pragma unroll
-                                    for (int q = 0; q < COLB / 16; ++q)
-                                        ptx::st_shared_v4(ba + static_cast<uint32_t>(lane * COLB + q * 16), v4[q].x, v4[q].y,
-                                                          v4[q].z, v4[q].w);
-                                } else {
-#pragma unroll 1
-                                    for (int rr = 0; rr < 32; ++rr) {
-                                        const float cv = (nrow0 + rr < j.N) ? Out<TD>::load(j.C, cbase + rr) : 0.f;
-                                        const uint32_t a = ba + static_cast<uint32_t>(lane * COLB + rr * static_cast<int>(sizeof(TD)));
-                                        if constexpr (sizeof(TD) == 4) ptx::st_shared_u32(a, __float_as_uint(cv));
-                                        else if constexpr (std::is_same<TD, __half>::value)
-                                            ptx::st_shared_u16(a, __half_as_ushort(__float2half_rn(cv)));
-                                        else ptx::st_shared_u16(a, static_cast<uint16_t>(__float_as_uint(cv) >> 16));
-                                    }
-                                }
-                            }
-                            __syncwarp();
-                        }
                         uint32_t r[32];
                         __syncwarp();
                         ptx::tmem_ld32(tbase + c * 32, r);
-                        if (c == chunks - 1) release_tmem<CG>(&tempty[mbuf], lane);
+                        if (c + nst >= chunks) release_tmem<CG>(&tempty[mbuf], lane);
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            const uint32_t a = ba + static_cast<uint32_t>((i * 32 + lane) * static_cast<int>(sizeof(TD)));
-                            const float acc = __uint_as_float(r[i]);
+                            const uint32_t a = my_stage_a + static_cast<uint32_t>((i * 32 + lane) * static_cast<int>(sizeof(TD)));
+                            const float o = j.alpha * __uint_as_float(r[i]);
                             if constexpr (sizeof(TD) == 4) {
-                                const float o = use_c ? fmaf(j.alpha, acc, j.beta * __uint_as_float(ptx::ld_shared_u32(a)))
-                                                      : j.alpha * acc;
                                 ptx::st_shared_u32(a, __float_as_uint(o));
                             } else {
-                                constexpr bool half = std::is_same<TD, __half>::value;
-                                float cf = 0.f;
-                                if (use_c) {
-                                    const uint32_t bits = ptx::ld_shared_u16(a);
-                                    cf = half ? __half2float(__ushort_as_half(static_cast<unsigned short>(bits)))
-                                              : __uint_as_float(bits << 16);
-                                }
-                                const float o = use_c ? fmaf(j.alpha, acc, j.beta * cf) : j.alpha * acc;
                                 uint16_t ob;
-                                if constexpr (half) ob = __half_as_ushort(__float2half_rn(o));
+                                if constexpr (std::is_same<TD, __half>::value) ob = __half_as_ushort(__float2half_rn(o));
                                 else ob = p.out_trunc ? static_cast<uint16_t>(__float_as_uint(o) >> 16)
                                                       : __bfloat16_as_ushort(__float2bfloat16_rn(o));
                                 ptx::st_shared_u16(a, ob);
                             }
                         }
-                        ptx::fence_proxy_async_smem();
                         __syncwarp();
-                        if (m < j.M && nrow0 < j.N) {
-                            if (lane == 0) {
-                                ptx::tma_store_3d(j.tmD, box, nrow0, m, j.b);
-                                ptx::bulk_commit();
-                            }
-                            stage_off += CB;
-                            if (stage_off == stage_bytes_all) stage_off = 0;
+#pragma unroll
+                        for (int it = 0; it < UPC; ++it) {
+                            const int col = it * (32 / UPC) + col0;
+                            const uint4 v = ptx::ld_shared_v4(my_stage_a + static_cast<uint32_t>(col * COLB + u * 16));
+                            if (m + col < j.M && in_n)
+                                *reinterpret_cast<uint4*>(static_cast<TD*>(j.D) + static_cast<int64_t>(j.b) * p.stride_d +
+                                                          static_cast<int64_t>(m + col) * j.ldd + nrow0 + u * EPU) = v;
                         }
                     }
                     if (tr) trace_mark(p, TL_TRACE_STORED);
@@ -1484,64 +1393,92 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                     continue;
                 }
             }
-            if (j.nsplit == 1 && j.tmD != nullptr && !direct) {
-                // each warp stages its 32 rows x 128 bytes of output (128-byte swizzle: 16-byte unit
-                // u of row r sits at u ^ (r & 7)) and writes them with one TMA store; the tensor
-                // map clips the ragged edges.  With two buffers per warp a store is read out of one
-                // while the other fills (the issuing lane waits until the store before the last has
-                // been read); with one, every 128 bytes of columns wait ~1 us for the store before.
-                // C of the next 32 columns is in flight while the current ones are finished.
-                constexpr int CPS = static_cast<int>(4 / sizeof(TD));    // 32-column chunks per 128 bytes
-                const int nrow0 = j.n0 + quarter * 32;
-                for (int c0 = 0; c0 < chunks && ok; c0 += CPS) {
-                    const int m = j.m0 + c0 * 32;
-                    if (lane == 0) {
-                        if (p.epi_bufs == 2) ptx::bulk_wait_read1();
-                        else ptx::bulk_wait_read0();
+            if (staged) {
+                // 16-byte unit u of row r sits at u ^ (r & 7): rows are written and lines read without
+                // bank conflicts.  The columns are finished WQ at a time in a loop that is not unrolled: a
+                // tile passes through this code a few times only, and straight-line code for 64 columns
+                // ran at the rate of instruction fetch (~580 clocks per 32 columns).
+                constexpr int GC = CPS * 32;                     // columns of a group
+                constexpr int UPQ = WQ * static_cast<int>(sizeof(TD)) / 16;
+                constexpr int CWN = WQ * static_cast<int>(sizeof(TD)) / 4;
+                const bool warp_ok = nrow0 < j.N;                // this warp has rows to store
+                if (half >= groups && ok) release_tmem<CG>(&tempty[mbuf], lane);
+                const uint32_t rowaddr = my_stage_a + static_cast<uint32_t>(lane) * 128u;
+                for (int g = half; g < groups && ok; g += nst) {
+                    const int m = j.m0 + g * GC;
+                    const uint32_t tcol = tbase + static_cast<uint32_t>(g * GC);
+                    if (!warp_ok) {
+                        if (g + nst >= groups) release_tmem<CG>(&tempty[mbuf], lane);
+                        continue;
                     }
-                    __syncwarp();
-                    const uint32_t rowaddr = my_stage_a + stage_off + static_cast<uint32_t>(lane) * 128u;
+                    float bcur[CPS];
+                    if constexpr (EPI) {
 #pragma unroll
-                    for (int q = 0; q < CPS; ++q) {
-                        uint32_t r[32];
-                        __syncwarp();
-                        ptx::tmem_ld32(tbase + (c0 + q) * 32, r);
-                        uint32_t w[32 / CPS];
-                        finish_pack<TD, EPI>(p, amax, j, m + 32 * q, row_ok, r, cw, p.out_trunc, w);
-                        if (row_ok && c0 + q + 1 < chunks) load_c_chunk<TD>(j, base_c, m + 32 * (q + 1), cw);
-#pragma unroll
-                        for (int uu = 0; uu < 8 / CPS; ++uu) {
-                            const int u = q * (8 / CPS) + uu;
-                            ptx::st_shared_v4(rowaddr + static_cast<uint32_t>((u ^ (lane & 7)) * 16), w[4 * uu],
-                                              w[4 * uu + 1], w[4 * uu + 2], w[4 * uu + 3]);
+                        for (int t = 0; t < CPS; ++t) bcur[t] = bl[t];
+                        if (g + nst < groups) lane_bias<CPS>(p, j.M, m + nst * GC + lane, bl);
+                    }
+                    if constexpr (sizeof(TD) >= 2) {
+                        if (use_c) {
+                            la.stage(my_stage_a, cl);
+                            __syncwarp();
+                            if (g + nst < groups)
+                                la.load(j.C, static_cast<int64_t>(j.b) * p.stride_c + static_cast<int64_t>(nrow0) * j.ldc,
+                                        j.ldc, m + nst * GC, cl);
                         }
                     }
-                    if (c0 + CPS >= chunks) release_tmem<CG>(&tempty[mbuf], lane);
-                    ptx::fence_proxy_async_smem();
-                    __syncwarp();
-                    if (m < j.M && nrow0 < j.N) {
-                        if (lane == 0) {
-                            ptx::tma_store_3d(j.tmD, my_stage + stage_off, m, nrow0, j.b);
-                            ptx::bulk_commit();
+#pragma unroll 1
+                    for (int q = 0; q < GC / WQ; ++q) {
+                        float o[WQ];
+                        ptx::tmem_ld<WQ>(tcol + static_cast<uint32_t>(q * WQ), o);
+                        if (q == GC / WQ - 1 && g + nst >= groups) release_tmem<CG>(&tempty[mbuf], lane);
+                        const uint32_t u0 = static_cast<uint32_t>(q * UPQ);
+                        const uint32_t sw = static_cast<uint32_t>(lane & 7);
+                        uint32_t cw[WQ];
+                        if (use_c) {
+#pragma unroll
+                            for (int uu = 0; uu < UPQ; ++uu) {
+                                const uint4 v = ptx::ld_shared_v4(rowaddr + ((u0 + uu) ^ sw) * 16u);
+                                cw[4 * uu] = v.x;
+                                cw[4 * uu + 1] = v.y;
+                                cw[4 * uu + 2] = v.z;
+                                cw[4 * uu + 3] = v.w;
+                            }
                         }
-                        // the buffers alternate with the committed stores, which the wait counts
-                        if (p.epi_bufs == 2) stage_off ^= 4096u;
+                        float bias[WQ];
+                        if constexpr (EPI) {
+                            float bsel = bcur[0];
+#pragma unroll
+                            for (int t = 1; t < CPS; ++t) bsel = q * WQ >= 32 * t ? bcur[t] : bsel;
+#pragma unroll
+                            for (int i = 0; i < WQ; ++i) bias[i] = __shfl_sync(0xffffffffu, bsel, (q * WQ + i) & 31);
+                        }
+                        finish_values<TD, EPI, WQ>(p, amax, j, m + q * WQ, row_ok, cw, bias, o);
+                        uint32_t w[CWN];
+                        pack_values<TD, WQ>(p, o, w);
+#pragma unroll
+                        for (int uu = 0; uu < UPQ; ++uu)
+                            ptx::st_shared_v4(rowaddr + ((u0 + uu) ^ sw) * 16u, w[4 * uu], w[4 * uu + 1], w[4 * uu + 2],
+                                              w[4 * uu + 3]);
                     }
+                    __syncwarp();
+                    la.store(j.D, static_cast<int64_t>(j.b) * p.stride_d + static_cast<int64_t>(nrow0) * j.ldd, j.ldd, m,
+                             my_stage_a);
+                    __syncwarp();
                 }
                 if (tr) trace_mark(p, TL_TRACE_STORED);
             } else if (j.nsplit == 1) {
-                // output TMA cannot address (unaligned D): 16-byte vector stores per thread
-                for (int c = 0; c < chunks && ok; ++c) {
+                // D or C not made of whole 16-byte vectors (and fp8 tiles narrower than a line)
+                for (int c = half; c < chunks && ok; c += NH) {       // at least two chunks: one per warp
                     const int m = j.m0 + c * 32;
                     uint32_t r[32];
                     __syncwarp();
                     ptx::tmem_ld32(tbase + c * 32, r);
-                    if (c == chunks - 1) release_tmem<CG>(&tempty[mbuf], lane);
+                    if (c + NH >= chunks) release_tmem<CG>(&tempty[mbuf], lane);
                     if (row_ok && m < j.M) {
                         float v[32];
 #pragma unroll
                         for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-                        store_chunk<TD, EPI>(p, amax, j, base_c, base_d, m, v, p.out_trunc);
+                        store_chunk<TD, EPI, 32>(p, amax, j, base_c, base_d, m, v);
                     }
                 }
                 if (tr) trace_mark(p, TL_TRACE_STORED);
@@ -1549,7 +1486,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                 // split-k: park this split's partial tile, layout [chunk][column][row] (coalesced)
                 float* slab = p.ws + (static_cast<size_t>(j.slot) * p.tail_split + j.split) *
                                          (static_cast<size_t>(kTcTileN) * p.bm);
-                for (int c = 0; c < chunks && ok; ++c) {
+                for (int c = half; c < chunks && ok; c += NH) {
                     uint32_t r[32];
                     __syncwarp();
                     ptx::tmem_ld32(tbase + c * 32, r);
@@ -1558,16 +1495,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
                     for (int i = 0; i < 32; ++i) __stcg(dst + i * kTcTileN, __uint_as_float(r[i]));
                 }
                 if (tr) trace_mark(p, TL_TRACE_STORED);
-                if (p.par_reduce)
-                    split_finish_parallel<TD, CG, EPI>(p, amax, j, ok, et, lane, row, row_ok, base_c, base_d, last_flag,
-                                                  &tempty[mbuf], abort_flag, c_staged, c_row);
-                else
-                    split_finish_tmem<TD, CG, EPI>(p, amax, j, ok, et, lane, row, row_ok, base_c, base_d, last_flag, tbase,
-                                              &tempty[mbuf]);
+                if (ok) release_tmem<CG>(&tempty[mbuf], lane);
+                split_finish<TD, EPI, NH>(p, amax, j, ok, et, lane, half, row, row_ok, base_c, base_d, last_flag,
+                                          abort_flag, c_staged, c_row);
                 if (tr) trace_mark(p, TL_TRACE_REDUCED);
             }
             mbuf ^= 1u;
             if (mbuf == 0) mph ^= 1u;
+            }
         }
         if (et == 0) {
             trace_mark(p, TL_TRACE_EPI_END);
@@ -1583,7 +1518,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
         }
     }
 
-    if (warp >= 2 && lane == 0) ptx::bulk_wait0();   // the epilogue's TMA stores have completed
     ptx::tc_fence_before();
     __syncthreads();
     if constexpr (CL > 1) ptx::cluster_sync();     // no remote arrival, multicast or pair MMA still targets us
@@ -1602,10 +1536,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemm_kernel(const __grid_con
 // ---- launch (templates; instantiated in the generated instance units) ---------------------------
 bool pdl_enabled();
 
-template <int KIND, typename TD, int CL, bool EPI = false>
+template <int KIND, typename TD, int CL, bool EPI, bool PROMO, bool GROUP>
 tl_status launch_kernel(const TcKernelParams& kp, int grid, size_t smem, cudaStream_t stream)
 {
-    auto kern = tc_gemm_kernel<KIND, TD, CL, EPI>;
+    auto kern = tc_gemm_kernel<KIND, TD, CL, EPI, PROMO, GROUP>;
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [&] {
@@ -1615,7 +1549,7 @@ tl_status launch_kernel(const TcKernelParams& kp, int grid, size_t smem, cudaStr
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-    cfg.blockDim = dim3(kTcThreads, 1, 1);
+    cfg.blockDim = dim3(tc_threads(PROMO), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -1653,12 +1587,12 @@ int max_clusters(size_t smem)
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(smem);
     if (it != cache.end()) return it->second;
-    auto kern = tc_gemm_kernel<KIND, TD, CL, false>;
+    auto kern = tc_gemm_kernel<KIND, TD, CL, false, false, false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTcMaxSmem));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(CL, 1, 1);
-    cfg.blockDim = dim3(kTcThreads, 1, 1);
+    cfg.blockDim = dim3(tc_threads(false), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

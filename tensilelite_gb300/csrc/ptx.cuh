@@ -119,6 +119,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64
     return mbar_wait(smem_u32(bar), parity, limit_ns);
 }
 
+// Barrier 1 over the N threads of the epilogue warps.
+template <int N>
+__device__ __forceinline__ void named_sync()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(N) : "memory");
+}
+
 // ---- TMA ---------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const void* tmap)
 {
@@ -219,6 +226,29 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
         : "memory");
 }
 
+// The same for 8 or 16 columns, as floats.
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&r)[N])
+{
+    static_assert(N == 8 || N == 16, "8 or 16 columns");
+    if constexpr (N == 16)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+            "tcgen05.wait::ld.sync.aligned;\n"
+            : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]),
+              "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+            : "r"(taddr)
+            : "memory");
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+            "tcgen05.wait::ld.sync.aligned;\n"
+            : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
+            : "r"(taddr)
+            : "memory");
+}
+
 // Shared-memory matrix descriptor for tcgen05.mma with 128-byte swizzling:
 //   bits  0-13 start address >> 4, 16-29 leading-dimension byte offset >> 4,
 //   bits 32-45 stride-dimension byte offset >> 4, bits 46-48 fixed 0b001,
@@ -299,21 +329,6 @@ __device__ __forceinline__ void tma_load_3d_pair_mc(uint32_t smem_dst, const voi
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(mbar_cluster_addr), "h"(cta_mask), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
-// TMA store of one box from this CTA's shared memory (bulk async-group completion); elements
-// outside the tensor are not written.  Coordinates are non-negative; x * element size is a
-// multiple of 16 bytes.
-__device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_src, int x, int y, int z)
-{
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-                     reinterpret_cast<uint64_t>(tmap)),
-                 "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Wait until the committed bulk stores of this thread have finished reading shared memory.
-__device__ __forceinline__ void bulk_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read3() { asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory"); }
 __device__ __forceinline__ void st_shared_u16(uint32_t addr, uint16_t v)
 {
     asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
@@ -334,8 +349,6 @@ __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr)
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
-// Wait until the committed bulk stores of this thread are complete.
-__device__ __forceinline__ void bulk_wait0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // 16-byte global -> shared copy without a register round trip (completion per thread, by group)
 __device__ __forceinline__ void cp_async16(uint32_t smem_addr, const void* gptr)
 {

@@ -1541,8 +1541,7 @@ TL_API tl_status tl_grouped_plan_create(tl_handle* h, const tl_gemm_problem* pro
         e.tiles_n = static_cast<int32_t>((p.n + s.macro_tile1 - 1) / s.macro_tile1);
         e.alpha = p.alpha * scale_of(p.scale_a) * scale_of(p.scale_b);
         e.beta = p.beta;
-        e.tma_store = (p.m > 0 && p.n > 0 &&
-                       tc_encode_output(&e.tmD, p.dtype_d, D[i], p.m, p.n, p.ldd, 1, p.stride_d)) ? 1 : 0;
+        e.vec = tc_vec_output(p.dtype_d, p.m, D[i], p.ldd, e.C, p.ldc, 1, 0, 0) ? 1 : 0;
         prefix[i + 1] = prefix[i] + static_cast<int64_t>(e.tiles_m) * e.tiles_n;
         flops += 2.0 * static_cast<double>(p.m) * p.n * p.k;
     }

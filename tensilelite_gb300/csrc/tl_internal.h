@@ -38,9 +38,10 @@ inline int dtype_bytes(int dt)
 constexpr int kTcMaxStages = 8;
 constexpr int kTcTileN = 128;          // tcgen05 M extent: problem n rows on TMEM lanes
 constexpr int kTcRowBytes = 128;       // one swizzle row: depth_u * element size
-constexpr int kTcEpiStageBytes = 4 * 32 * 128;   // output staging of the 4 epilogue warps (TMA stores)
+constexpr int kTcEpiStageBytes = 4 * 32 * 128;   // output staging of 4 epilogue warps
 constexpr size_t kTcMaxSmem = 227 * 1024;        // dynamic shared memory a CTA may ask for
-constexpr int kTcThreads = 192;        // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
+// warp 0 TMA, warp 1 MMA, then eight epilogue warps (four in the promotion kernels)
+constexpr int tc_threads(bool promo) { return promo ? 192 : 320; }
 
 // One operand's TMA view: K-major (rows x k, k contiguous) or MN-major (k rows of contiguous rows).
 struct TcOperand {
@@ -61,8 +62,7 @@ struct TcGroupEntry {   // aligned like CUtensorMap
     int32_t M, N, K;
     int32_t tiles_m, tiles_n;
     float alpha, beta;
-    int32_t tma_store;   // tmD describes D: whole tiles leave through TMA stores
-    CUtensorMap tmD;     // problem D, boxes of 128 bytes x 32 rows
+    int32_t vec;         // D and C consist of whole aligned 16-byte vectors
 };
 
 struct TcLaunch {
@@ -109,9 +109,10 @@ struct TcLaunch {
 
 // Dynamic shared memory of one CTA staging bm_cta m-rows per stage (bm / 2 for a CTA pair).
 size_t tc_smem_bytes(int bm_cta, int stages);
-// Tensor map of an output for TMA stores (false when TMA cannot address it).
-bool tc_encode_output(CUtensorMap* tm, int out_dtype, void* D, int64_t M, int64_t N, int64_t ldd, int64_t batch,
-                      int64_t stride_d);
+// Whether the columns (of `rows` elements) of D, and of C where there is one, are whole aligned 16-byte
+// vectors.
+bool tc_vec_output(int out_dtype, int64_t rows, const void* D, int64_t ldd, const void* C, int64_t ldc, int64_t batch,
+                   int64_t stride_d, int64_t stride_c);
 // Persistent workers (CTAs, or co-resident clusters of `cl` CTAs) a tensor-core launch gets.
 int tc_workers(int in_dtype, int out_dtype, int cl, int bm, int stages, int sm_count);
 int tc_tmem_cols(int bm);
