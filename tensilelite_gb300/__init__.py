@@ -235,10 +235,28 @@ def _ptr(x) -> Optional[int]:
     return x.data_ptr()
 
 
+_RAW_STREAM = None
+
+
+def _current_stream() -> int:
+    """The calling thread's current CUDA stream on its current device (3 us through the Stream object,
+    0.2 us raw)."""
+    global _RAW_STREAM
+    if _RAW_STREAM is None:
+        import torch
+        torch.cuda.current_stream()          # initialises CUDA
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        device = getattr(torch._C, "_cuda_getDevice", None)
+        if raw is not None and device is not None:
+            _RAW_STREAM = lambda: raw(device())
+        else:
+            _RAW_STREAM = lambda: torch.cuda.current_stream().cuda_stream
+    return _RAW_STREAM()
+
+
 def _stream_ptr(stream) -> Optional[int]:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return _current_stream()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
@@ -291,8 +309,10 @@ class Handle:
         check(lib().tl_check_solution(self._h, ctypes.byref(p), ctypes.byref(s)))
 
     def gemm(self, p: Problem, D, C, A, B, solution: Optional[Solution] = None, stream=None):
-        check(lib().tl_gemm(self._h, ctypes.byref(p), ctypes.byref(solution) if solution is not None else None,
-                            _ptr(D), _ptr(C), _ptr(A), _ptr(B), _stream_ptr(stream)))
+        st = lib().tl_gemm(self._h, ctypes.byref(p), ctypes.byref(solution) if solution is not None else None,
+                           _ptr(D), _ptr(C), _ptr(A), _ptr(B), _stream_ptr(stream))
+        if st:
+            check(st)
 
     def tune(self, p: Problem, D, C, A, B, max_candidates=16, reps=10, cache_path=None):
         s, ms = Solution(), ctypes.c_float()
@@ -327,17 +347,15 @@ class Handle:
                 d_scale=0.0, solution: Optional[Solution] = None, stream=None):
         """tl_gemm_ex: tl_gemm with a fused bias / activation / amax epilogue (and, for an fp8 output,
         the quantisation scale d_scale)."""
-        e = Epilogue()
-        e.d_scale = d_scale
-        e.bias = _ptr(bias)
         if bias is not None and bias_dtype is None:
             bias_dtype = torch_dtype_code(bias.dtype)
-        e.bias_dtype = (DTYPE_NAMES[bias_dtype] if isinstance(bias_dtype, str) else bias_dtype) or FP32
-        e.activation = ACTIVATIONS[activation] if isinstance(activation, str) else int(activation)
-        e.amax = _ptr(amax)
-        check(lib().tl_gemm_ex(self._h, ctypes.byref(p), ctypes.byref(e),
-                               ctypes.byref(solution) if solution is not None else None,
-                               _ptr(D), _ptr(C), _ptr(A), _ptr(B), _stream_ptr(stream)))
+        e = Epilogue(_ptr(bias), (DTYPE_NAMES[bias_dtype] if isinstance(bias_dtype, str) else bias_dtype) or FP32,
+                     ACTIVATIONS[activation] if isinstance(activation, str) else int(activation), _ptr(amax), d_scale)
+        st = lib().tl_gemm_ex(self._h, ctypes.byref(p), ctypes.byref(e),
+                              ctypes.byref(solution) if solution is not None else None,
+                              _ptr(D), _ptr(C), _ptr(A), _ptr(B), _stream_ptr(stream))
+        if st:
+            check(st)
 
     def tensile_launch(self, kernel_name: str, kernarg: bytes, stream=None):
         """tl_tensile_launch: the GEMM a Tensile-layout (Cijk_Alik_Bljk) argument buffer describes."""
@@ -481,10 +499,15 @@ def default_handle() -> Handle:
     return h
 
 
+_TORCH_CODES = {}
+
+
 def torch_dtype_code(t) -> int:
-    import torch
-    return {torch.float32: FP32, torch.float16: FP16, torch.bfloat16: BF16,
-            torch.float8_e4m3fn: FP8, torch.uint8: FP8}[t]
+    if not _TORCH_CODES:
+        import torch
+        _TORCH_CODES.update({torch.float32: FP32, torch.float16: FP16, torch.bfloat16: BF16,
+                             torch.float8_e4m3fn: FP8, torch.uint8: FP8})
+    return _TORCH_CODES[t]
 
 
 def gemm_colmajor(A, B, m, n, k, *, C=None, D=None, alpha=1.0, beta=0.0, trans_a=False, trans_b=False,
@@ -506,27 +529,41 @@ def gemm_colmajor(A, B, m, n, k, *, C=None, D=None, alpha=1.0, beta=0.0, trans_a
     return D
 
 
-_MM_PROBLEMS = {}
+_PROBLEMS = {}
+_MAX_PROBLEMS = 4096
+
+
+def _problem(key, m, n, k, **kw):
+    """The problem descriptor of `key`, built once per (dtype, layout, shape) and reused (2.4 us each)."""
+    p = _PROBLEMS.get(key)
+    if p is None:
+        p = Problem.make(m, n, k, **kw)
+        if len(_PROBLEMS) >= _MAX_PROBLEMS:
+            _PROBLEMS.clear()
+        _PROBLEMS[key] = p
+    return p
 
 
 def _mm_rowmajor(X, W, trans_x=False, trans_w=False):
     """Row-major X(M,K) @ W(K,N) through the column-major kernels (op flags on the stored tensors).
-    The problem descriptor is built once per (dtype, layout, shape) and reused: the per-call host cost
-    is then the two tensor-map encodings and the launch."""
+    The per-call host cost is the output tensor, the two tensor-map encodings and the launch."""
     import torch
     Xs, Ws = X.contiguous(), W.contiguous()
-    M = Xs.shape[1] if trans_x else Xs.shape[0]
-    K = Xs.shape[0] if trans_x else Xs.shape[1]
-    N = Ws.shape[0] if trans_w else Ws.shape[1]
-    key = (X.dtype, trans_x, trans_w, M, N, K)
-    p = _MM_PROBLEMS.get(key)
+    dt = X.dtype
+    xs, ws = Xs.shape, Ws.shape
+    x1, w1 = xs[1], ws[1]
+    M, K = (x1, xs[0]) if trans_x else (xs[0], x1)
+    N = ws[0] if trans_w else w1
+    key = (dt, trans_x, trans_w, M, N, K)
+    p = _PROBLEMS.get(key)
     if p is None:
         # Y (row-major M x N) == column-major N x M:  Y^T = op(W)^T op(X)^T
-        p = Problem.make(N, M, K, dtype=torch_dtype_code(X.dtype), trans_a=trans_w, trans_b=trans_x,
-                         lda=Ws.shape[1], ldb=Xs.shape[1], ldd=N)
-        _MM_PROBLEMS[key] = p
-    Y = torch.empty((M, N), dtype=X.dtype, device=X.device)
-    default_handle().gemm(p, Y, None, Ws, Xs)
+        p = _problem(key, N, M, K, dtype=torch_dtype_code(dt), trans_a=trans_w, trans_b=trans_x, lda=w1, ldb=x1, ldd=N)
+    Y = torch.empty((M, N), dtype=dt, device=X.device)
+    st = lib().tl_gemm(default_handle()._h, ctypes.byref(p), None, Y.data_ptr(), None, Ws.data_ptr(), Xs.data_ptr(),
+                       _current_stream())
+    if st:
+        check(st)
     return Y
 
 
@@ -576,7 +613,7 @@ def linear(X, W, bias=None, activation="none", amax=None):
     N = Ws.shape[1]
     Y = torch.empty((M, N), dtype=X.dtype, device=X.device)
     # Y^T = W^T X^T column-major: m = N (bias index), n = M
-    p = Problem.make(N, M, K, dtype=torch_dtype_code(X.dtype), lda=N, ldb=K, ldd=N)
+    p = _problem((X.dtype, "linear", M, N, K), N, M, K, dtype=torch_dtype_code(X.dtype), lda=N, ldb=K, ldd=N)
     default_handle().gemm_ex(p, Y, None, Ws, Xs, bias=bias, activation=activation, amax=amax)
     return Y
 

@@ -17,9 +17,34 @@
 #include <fstream>
 #include <sstream>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "tl_internal.h"
+
+namespace tl {
+// What a heuristic pick depends on besides the handle.
+struct PlanKey {
+    int64_t m, n, k, batch;
+    int32_t dtype_a, dtype_d, trans_a, trans_b, kernel, beta, allow_view, pad;
+    bool operator==(const PlanKey& o) const { return memcmp(this, &o, sizeof(*this)) == 0; }
+};
+struct PlanKeyHash {
+    size_t operator()(const PlanKey& q) const
+    {
+        uint64_t h = 1469598103934665603ull;      // FNV-1a over the words
+        const uint64_t* w = reinterpret_cast<const uint64_t*>(&q);
+        for (size_t i = 0; i < sizeof(q) / sizeof(uint64_t); ++i) h = (h ^ w[i]) * 1099511628211ull;
+        return static_cast<size_t>(h ^ (h >> 32));
+    }
+};
+static_assert(sizeof(PlanKey) == 64, "no padding: compared and hashed as bytes");
+struct Plan {
+    tl_gemm_solution s;
+    bool view;
+};
+constexpr size_t kMaxPlans = 4096;
+}  // namespace tl
 
 struct tl_handle {
     int device = 0;
@@ -39,7 +64,9 @@ struct tl_handle {
     unsigned long long* trace = nullptr;   // device timeline buffer (tl_set_trace), or null
     int64_t trace_bytes = 0;
     std::map<std::string, tl_gemm_solution> tuned;
-    std::mutex mu;
+    // heuristic picks by problem shape (the cost model takes 1.5 to 7 us a problem); at most kMaxPlans
+    std::unordered_map<tl::PlanKey, tl::Plan, tl::PlanKeyHash> plans;
+    std::mutex mu;                 // tuned, plans
     // Once a stream capture has recorded this handle's workspace address, a grown workspace retires
     // the old buffer here (freed by tl_destroy) instead of freeing it under a live graph.
     bool captured = false;
@@ -613,7 +640,7 @@ tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solut
         view = !epilogue && tc_nn_view(p, kernel) && view_solution_ok(P.s);
     } else {
         std::lock_guard<std::mutex> g(h->mu);
-        auto it = h->tuned.find(problem_key(h, p));
+        auto it = h->tuned.empty() ? h->tuned.end() : h->tuned.find(problem_key(h, p));
         if (it != h->tuned.end()) {
             P.s = it->second;
             kernel = P.s.kernel;
@@ -621,7 +648,17 @@ tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solut
         } else if (kernel == TL_KERNEL_SIMT) {
             simt_solution(&P.s);
         } else {
-            tc_heuristic_viewed(h, p, kernel, !epilogue, &P.s, &view);
+            const PlanKey key{p.m, p.n, p.k, p.batch, p.dtype_a, p.dtype_d, p.trans_a, p.trans_b, kernel,
+                              p.beta != 0.0f ? 1 : 0, epilogue ? 0 : 1, 0};
+            auto pl = h->plans.find(key);
+            if (pl == h->plans.end()) {
+                Plan n;
+                tc_heuristic_viewed(h, p, kernel, !epilogue, &n.s, &n.view);
+                if (h->plans.size() >= kMaxPlans) h->plans.clear();
+                pl = h->plans.emplace(key, n).first;
+            }
+            P.s = pl->second.s;
+            view = pl->second.view;
         }
     }
     // an NN problem runs as its transposed view from here on (solutions are for the view)
