@@ -1808,9 +1808,7 @@ TL_API tl_status tl_quantize_fp8(tl_handle* h, tl_dtype src_dtype, const void* s
     if (src_dtype != TL_DTYPE_FP32 && src_dtype != TL_DTYPE_FP16 && src_dtype != TL_DTYPE_BF16)
         return fail(TL_ERR_UNSUPPORTED, "quantize: source must be fp32, fp16 or bf16");
     float* amax = amax_out ? amax_out : h->d_amax;
-    tl_status st = aux_amax(src_dtype, src, n, amax, S(stream), &h->launches);
-    if (st != TL_SUCCESS) return st;
-    return aux_quant_e4m3(src_dtype, src, n, amax, static_cast<uint8_t*>(dst), scale_out, S(stream), &h->launches);
+    return aux_quantize_e4m3(src_dtype, src, n, amax, static_cast<uint8_t*>(dst), scale_out, S(stream), &h->launches);
 }
 
 TL_API tl_status tl_split_bf16x2(tl_handle* h, const float* src, int64_t n, void* hi, void* lo, void* stream)

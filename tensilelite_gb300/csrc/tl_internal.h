@@ -157,9 +157,9 @@ tl_status simt_gemm_launch(const SimtLaunch& L, cudaStream_t stream, int64_t* la
 tl_status aux_split_bf16(const float* src, int64_t rows, int64_t cols, int64_t ld, int64_t batch,
                          int64_t batch_stride, uint16_t* p0, uint16_t* p1, uint16_t* p2, cudaStream_t s,
                          int64_t* launches);
-tl_status aux_amax(int src_dtype, const void* src, int64_t n, float* amax_dev, cudaStream_t s, int64_t* launches);
-tl_status aux_quant_e4m3(int src_dtype, const void* src, int64_t n, const float* amax_dev, uint8_t* dst,
-                         float* scale_out_dev, cudaStream_t s, int64_t* launches);
+// Per-tensor E4M3 quantisation: *amax_dev = max |x|, dst = e4m3(x * 448 / amax), *scale_out_dev = amax / 448.
+tl_status aux_quantize_e4m3(int src_dtype, const void* src, int64_t n, float* amax_dev, uint8_t* dst,
+                            float* scale_out_dev, cudaStream_t s, int64_t* launches);
 tl_status aux_error_norms(int dtype_d, const void* D, int64_t ldd, const double* R, const double* W, int64_t ldr,
                           int64_t m, int64_t n, double* out_dev, cudaStream_t s, int64_t* launches);
 tl_status aux_fill_pattern(int dtype, void* dst, int64_t count, float code, cudaStream_t s, int64_t* launches);
