@@ -20,11 +20,13 @@ CLI = os.path.join(HERE, "tensilelite")
 
 SOURCES = ["gemm_tc.cu", "gemm_simt.cu", "aux_kernels.cu", "tl_api.cpp", "noalloc.cu"]
 # The tcgen05 kernel template is instantiated in generated units, one per operand kind (0 fp16/bf16,
-# 1 fp8), epilogue variant, cluster size, promotion and grouping, so they compile in parallel.  Plain
+# 1 fp8), epilogue variant, cluster size, mode and grouping, so they compile in parallel.  Plain
 # kernels write fp32, fp16 or bf16; the fused-epilogue kernels also fp8 (E4M3).  Two pairs per cluster
 # (4) have no promotion, grouped kernels neither promotion nor a fused epilogue.
-INSTANCES = [(k, e, cl, pr, g) for k in (0, 1) for e in (False, True) for cl in (1, 2, 4) for pr in (False, True)
-             for g in (False, True) if not (pr and cl == 4) and not (g and (e or pr))]
+MODES = {0: "kModePlain", 1: "kModePromo", 2: "kModePieces"}
+INSTANCES = [(k, e, cl, md, g) for k in (0, 1) for e in (False, True) for cl in (1, 2, 4) for md in (0, 1)
+             for g in (False, True) if not (md and cl == 4) and not (g and (e or md))]
+INSTANCES += [(0, e, 2, 2, False) for e in (False, True)]      # shared pieces of the fp32 split: fp32 output only
 OUT_TYPES = ("float", "__half", "__nv_bfloat16")
 EPI_OUT_TYPES = OUT_TYPES + ("__nv_fp8_e4m3",)
 
@@ -34,16 +36,16 @@ def _instance_sources():
     os.makedirs(gen, exist_ok=True)
     paths = []
     flag = {False: "false", True: "true"}
-    for k, e, cl, pr, g in INSTANCES:
+    for k, e, cl, md, g in INSTANCES:
         lines = ['#include "tensilelite_gb300/csrc/gemm_tc_kernel.cuh"', "namespace tl {", "namespace tc {"]
-        for td in (EPI_OUT_TYPES if e else OUT_TYPES):
-            lines.append(f"template tl_status launch_kernel<{k}, {td}, {cl}, {flag[e]}, {flag[pr]}, {flag[g]}>("
+        for td in (("float",) if md == 2 else EPI_OUT_TYPES if e else OUT_TYPES):
+            lines.append(f"template tl_status launch_kernel<{k}, {td}, {cl}, {flag[e]}, {MODES[md]}, {flag[g]}>("
                          "const TcKernelParams&, int, size_t, cudaStream_t);")
-            if not e and not pr and not g:
+            if not e and not md and not g:
                 lines.append(f"template int max_clusters<{k}, {td}, {cl}>(size_t);")
         lines += ["}  // namespace tc", "}  // namespace tl", ""]
         text = "\n".join(lines)
-        path = os.path.join(gen, f"tc_k{k}_e{int(e)}_c{cl}_p{int(pr)}_g{int(g)}.cu")
+        path = os.path.join(gen, f"tc_k{k}_e{int(e)}_c{cl}_m{md}_g{int(g)}.cu")
         if not os.path.exists(path) or open(path).read() != text:
             with open(path, "w") as f:
                 f.write(text)

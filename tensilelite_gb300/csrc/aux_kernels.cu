@@ -76,23 +76,66 @@ __device__ __forceinline__ void split_pieces(float x, uint16_t (&o)[3])
     }
 }
 
-template <int NP>
-__global__ void split_kernel(const float* __restrict__ src, int64_t rows, int64_t cols, int64_t ld, int64_t batch,
-                             int64_t bs, uint16_t* __restrict__ p0, uint16_t* __restrict__ p1,
-                             uint16_t* __restrict__ p2)
+// Bound by HBM: 4 bytes read and 2 NP written per element.  Four consecutive elements of a column per
+// thread and step, by flat index, so that neither few long columns nor many short ones leave threads
+// idle.  The operands of a GEMM are split by two launches that overlap: the second is a programmatic
+// dependent of the first and waits for it only before it ends (so what depends on the second
+// has both).  RANGE: the operand's magnitudes go to args.range, one pair of atomics per block.
+struct SplitArgs {
+    SplitOperand op;
+    uint32_t* range;
+};
+template <int NP, bool RANGE>
+__global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ SplitArgs args)
 {
-    // element e of the logical rows x cols x batch block lives at b*bs + c*ld + r
-    const int64_t total = rows * cols * batch;
-    const bool dense = (ld == rows) && (batch == 1 || bs == rows * cols);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    uint32_t most = 0, least = 0xffffffffu;                  // bits of the largest and smallest nonzero |x|
+    auto seen = [&](float x) {
+        if constexpr (RANGE) {
+            const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+            most = max(most, u);
+            least = min(least, u - 1u);                       // zero wraps to the largest value
+        }
+    };
+    const SplitOperand& o = args.op;
+    const int64_t g = (o.rows + 3) / 4;                       // groups of four per column
+    const int64_t total = g * o.cols * o.batch;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    uint16_t* out[3] = {p0, p1, p2};
-    bool vec = dense && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+    // without gaps in either layout the groups follow each other
+    const bool flat = o.rows % 4 == 0 && o.ld == o.rows && o.pld == o.rows &&
+                      (o.batch == 1 || (o.batch_stride == o.rows * o.cols && o.p_batch_stride == o.batch_stride));
+    const bool small = total < (int64_t(1) << 31);
+    bool vec = (reinterpret_cast<uintptr_t>(o.src) & 15) == 0 && o.ld % 4 == 0 && o.pld % 4 == 0 &&
+               (o.batch == 1 || (o.batch_stride % 4 == 0 && o.p_batch_stride % 4 == 0));
 #pragma unroll
-    for (int i = 0; i < NP; ++i) vec = vec && (reinterpret_cast<uintptr_t>(out[i]) & 7) == 0;
-    if (vec) {
-        const int64_t n4 = total / 4;
-        for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n4; i += stride) {
-            const float4 v = reinterpret_cast<const float4*>(src)[i];
+    for (int i = 0; i < NP; ++i) vec = vec && (reinterpret_cast<uintptr_t>(o.p[i]) & 7) == 0;
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += stride) {
+        int64_t src, dst;
+        int left = 4;
+        if (flat) {
+            src = dst = 4 * i;
+        } else {
+            int64_t col, r, b = 0;
+            if (small) {
+                col = static_cast<uint32_t>(i) / static_cast<uint32_t>(g);
+            } else {
+                col = i / g;
+            }
+            r = 4 * (i - col * g);
+            if (o.batch > 1) {
+                b = col / o.cols;
+                col -= b * o.cols;
+            }
+            src = b * o.batch_stride + col * o.ld + r;
+            dst = b * o.p_batch_stride + col * o.pld + r;
+            left = static_cast<int>(o.rows - r < 4 ? o.rows - r : 4);
+        }
+        if (vec && left == 4) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(o.src + src));
+            seen(v.x);
+            seen(v.y);
+            seen(v.z);
+            seen(v.w);
             uint16_t q[4][3];
             split_pieces<NP>(v.x, q[0]);
             split_pieces<NP>(v.y, q[1]);
@@ -100,27 +143,39 @@ __global__ void split_kernel(const float* __restrict__ src, int64_t rows, int64_
             split_pieces<NP>(v.w, q[3]);
 #pragma unroll
             for (int pc = 0; pc < NP; ++pc)
-                reinterpret_cast<uint2*>(out[pc])[i] = make_uint2(q[0][pc] | (uint32_t(q[1][pc]) << 16),
-                                                                  q[2][pc] | (uint32_t(q[3][pc]) << 16));
-        }
-        for (int64_t i = n4 * 4 + blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += stride) {
-            uint16_t q[3];
-            split_pieces<NP>(src[i], q);
+                *reinterpret_cast<uint2*>(o.p[pc] + dst) = make_uint2(q[0][pc] | (uint32_t(q[1][pc]) << 16),
+                                                                     q[2][pc] | (uint32_t(q[3][pc]) << 16));
+        } else {
+            for (int t = 0; t < left; ++t) {
+                uint16_t q[3];
+                const float x = o.src[src + t];
+                seen(x);
+                split_pieces<NP>(x, q);
 #pragma unroll
-            for (int pc = 0; pc < NP; ++pc) out[pc][i] = q[pc];
+                for (int pc = 0; pc < NP; ++pc) o.p[pc][dst + t] = q[pc];
+            }
         }
-        return;
     }
-    for (int64_t e = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; e < total; e += stride) {
-        const int64_t r = e % rows;
-        const int64_t c = (e / rows) % cols;
-        const int64_t b = e / (rows * cols);
-        const int64_t off = b * bs + c * ld + r;
-        uint16_t q[3];
-        split_pieces<NP>(src[off], q);
+    if constexpr (RANGE) {
+        __shared__ uint32_t sm[2][8];
+        most = __reduce_max_sync(0xffffffffu, most);
+        least = __reduce_min_sync(0xffffffffu, least);
+        if ((threadIdx.x & 31) == 0) {
+            sm[0][threadIdx.x >> 5] = most;
+            sm[1][threadIdx.x >> 5] = least;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
 #pragma unroll
-        for (int pc = 0; pc < NP; ++pc) out[pc][off] = q[pc];
+            for (int w = 1; w < 8; ++w) {
+                most = max(most, sm[0][w]);
+                least = min(least, sm[1][w]);
+            }
+            atomicMax(args.range, most);
+            if (least != 0xffffffffu) atomicMax(args.range + 1, ~(least + 1u));
+        }
     }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // ---- fp8 ----------------------------------------------------------------------------------------------
@@ -365,18 +420,6 @@ tl_status check_launch(const char* what, int64_t* launches)
 
 }  // namespace
 
-tl_status aux_split_bf16(const float* src, int64_t rows, int64_t cols, int64_t ld, int64_t batch,
-                         int64_t batch_stride, uint16_t* p0, uint16_t* p1, uint16_t* p2, cudaStream_t s,
-                         int64_t* launches)
-{
-    const int64_t total = rows * cols * batch;
-    if (total == 0) return TL_SUCCESS;
-    const int grid = grid_for(total, 8, 256);
-    if (p2) split_kernel<3><<<grid, 256, 0, s>>>(src, rows, cols, ld, batch, batch_stride, p0, p1, p2);
-    else split_kernel<2><<<grid, 256, 0, s>>>(src, rows, cols, ld, batch, batch_stride, p0, p1, nullptr);
-    return check_launch("split_kernel", launches);
-}
-
 // Launch as a programmatic dependent of the kernel before it in the stream.
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_dependent(void (*kern)(KArgs...), int grid, int threads, cudaStream_t s, Args... args)
@@ -393,6 +436,31 @@ static cudaError_t launch_dependent(void (*kern)(KArgs...), int grid, int thread
         cfg.numAttrs = 1;
     }
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+tl_status aux_split_bf16(const SplitOperand* ops, int count, int pieces, SplitRange* range, cudaStream_t s,
+                         int64_t* launches)
+{
+    bool first = true;
+    for (int i = 0; i < count; ++i) {
+        const int64_t total = ops[i].rows * ops[i].cols * ops[i].batch;
+        if (total == 0) continue;
+        const SplitArgs args = {ops[i], range ? reinterpret_cast<uint32_t*>(range) + 2 * i : nullptr};
+        const int grid = grid_for(total, 8, 256);
+        void (*kern)(SplitArgs) = pieces == 3 ? (range ? split_kernel<3, true> : split_kernel<3, false>) : split_kernel<2, false>;
+        if (first) {
+            // an ordinary launch: it starts after whatever wrote the operands, or still reads the pieces
+            kern<<<grid, 256, 0, s>>>(args);
+            const tl_status st = check_launch("split_kernel", launches);
+            if (st != TL_SUCCESS) return st;
+        } else {
+            const cudaError_t e = launch_dependent(kern, grid, 256, s, args);
+            if (e != cudaSuccess) return cuda_fail(e, "split_kernel");
+            if (launches) ++*launches;
+        }
+        first = false;
+    }
+    return TL_SUCCESS;
 }
 
 template <typename T>

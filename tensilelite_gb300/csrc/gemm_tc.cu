@@ -44,10 +44,10 @@ namespace tc {
     TL_TC_EXTERN(K, __half, CL, true, P, false) TL_TC_EXTERN(K, __nv_bfloat16, CL, true, P, false)               \
     TL_TC_EXTERN(K, __nv_fp8_e4m3, CL, true, P, false)
 #define TL_TC_EXTERN_CL(K, CL)                                  \
-    TL_TC_EXTERN_EP(K, CL, false)                               \
-    TL_TC_EXTERN(K, float, CL, false, false, true)              \
-    TL_TC_EXTERN(K, __half, CL, false, false, true)             \
-    TL_TC_EXTERN(K, __nv_bfloat16, CL, false, false, true)      \
+    TL_TC_EXTERN_EP(K, CL, kModePlain)                          \
+    TL_TC_EXTERN(K, float, CL, false, kModePlain, true) \
+    TL_TC_EXTERN(K, __half, CL, false, kModePlain, true) \
+    TL_TC_EXTERN(K, __nv_bfloat16, CL, false, kModePlain, true) \
     extern template int max_clusters<K, float, CL>(size_t);     \
     extern template int max_clusters<K, __half, CL>(size_t);    \
     extern template int max_clusters<K, __nv_bfloat16, CL>(size_t);
@@ -57,10 +57,12 @@ TL_TC_EXTERN_CL(0, 4)
 TL_TC_EXTERN_CL(1, 1)
 TL_TC_EXTERN_CL(1, 2)
 TL_TC_EXTERN_CL(1, 4)
-TL_TC_EXTERN_EP(0, 1, true)
-TL_TC_EXTERN_EP(0, 2, true)
-TL_TC_EXTERN_EP(1, 1, true)
-TL_TC_EXTERN_EP(1, 2, true)
+TL_TC_EXTERN_EP(0, 1, kModePromo)
+TL_TC_EXTERN_EP(0, 2, kModePromo)
+TL_TC_EXTERN_EP(1, 1, kModePromo)
+TL_TC_EXTERN_EP(1, 2, kModePromo)
+TL_TC_EXTERN(0, float, 2, false, kModePieces, false)
+TL_TC_EXTERN(0, float, 2, true, kModePieces, false)
 #undef TL_TC_EXTERN_CL
 #undef TL_TC_EXTERN_EP
 #undef TL_TC_EXTERN
@@ -104,22 +106,22 @@ bool pdl_enabled()
     return on;
 }
 
-template <int KIND, int CL, bool PROMO, bool GROUP>
+template <int KIND, int CL, int MODE, bool GROUP>
 tl_status dispatch_out(int out_dtype, const TcKernelParams& kp, int grid, size_t smem, cudaStream_t s)
 {
     if (!GROUP && kp.epi_on) {
         // the fused-epilogue kernels (they also write every fp8 output)
         if constexpr (!GROUP) {
-            if (out_dtype == TL_DTYPE_FP32) return launch_kernel<KIND, float, CL, true, PROMO, false>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_FP16) return launch_kernel<KIND, __half, CL, true, PROMO, false>(kp, grid, smem, s);
-            if (out_dtype == TL_DTYPE_BF16) return launch_kernel<KIND, __nv_bfloat16, CL, true, PROMO, false>(kp, grid, smem, s);
+            if (out_dtype == TL_DTYPE_FP32) return launch_kernel<KIND, float, CL, true, MODE, false>(kp, grid, smem, s);
+            if (out_dtype == TL_DTYPE_FP16) return launch_kernel<KIND, __half, CL, true, MODE, false>(kp, grid, smem, s);
+            if (out_dtype == TL_DTYPE_BF16) return launch_kernel<KIND, __nv_bfloat16, CL, true, MODE, false>(kp, grid, smem, s);
             if (out_dtype == TL_DTYPE_FP8_E4M3)
-                return launch_kernel<KIND, __nv_fp8_e4m3, CL, true, PROMO, false>(kp, grid, smem, s);
+                return launch_kernel<KIND, __nv_fp8_e4m3, CL, true, MODE, false>(kp, grid, smem, s);
         }
     } else {
-        if (out_dtype == TL_DTYPE_FP32) return launch_kernel<KIND, float, CL, false, PROMO, GROUP>(kp, grid, smem, s);
-        if (out_dtype == TL_DTYPE_FP16) return launch_kernel<KIND, __half, CL, false, PROMO, GROUP>(kp, grid, smem, s);
-        if (out_dtype == TL_DTYPE_BF16) return launch_kernel<KIND, __nv_bfloat16, CL, false, PROMO, GROUP>(kp, grid, smem, s);
+        if (out_dtype == TL_DTYPE_FP32) return launch_kernel<KIND, float, CL, false, MODE, GROUP>(kp, grid, smem, s);
+        if (out_dtype == TL_DTYPE_FP16) return launch_kernel<KIND, __half, CL, false, MODE, GROUP>(kp, grid, smem, s);
+        if (out_dtype == TL_DTYPE_BF16) return launch_kernel<KIND, __nv_bfloat16, CL, false, MODE, GROUP>(kp, grid, smem, s);
     }
     return fail(TL_ERR_UNSUPPORTED, "tcgen05 kernel: unsupported output type");
 }
@@ -128,16 +130,21 @@ template <int CL>
 tl_status dispatch_cl(int in_dtype, int out_dtype, const TcKernelParams& kp, int grid, size_t smem, cudaStream_t s)
 {
     const int kind = (in_dtype == TL_DTYPE_FP8_E4M3) ? 1 : 0;
+    if constexpr (CL == 2) {
+        if (kp.pieces_mode)
+            return kp.epi_on ? launch_kernel<0, float, 2, true, kModePieces, false>(kp, grid, smem, s)
+                             : launch_kernel<0, float, 2, false, kModePieces, false>(kp, grid, smem, s);
+    }
     if (kp.promote_kb > 0) {
         if constexpr (CL == 4) return fail(TL_ERR_UNSUPPORTED, "tcgen05 kernel: no promotion with two CTA pairs");
-        else return kind == 0 ? dispatch_out<0, CL, true, false>(out_dtype, kp, grid, smem, s)
-                              : dispatch_out<1, CL, true, false>(out_dtype, kp, grid, smem, s);
+        else return kind == 0 ? dispatch_out<0, CL, kModePromo, false>(out_dtype, kp, grid, smem, s)
+                              : dispatch_out<1, CL, kModePromo, false>(out_dtype, kp, grid, smem, s);
     }
     if (kp.group != nullptr)
-        return kind == 0 ? dispatch_out<0, CL, false, true>(out_dtype, kp, grid, smem, s)
-                         : dispatch_out<1, CL, false, true>(out_dtype, kp, grid, smem, s);
-    return kind == 0 ? dispatch_out<0, CL, false, false>(out_dtype, kp, grid, smem, s)
-                     : dispatch_out<1, CL, false, false>(out_dtype, kp, grid, smem, s);
+        return kind == 0 ? dispatch_out<0, CL, kModePlain, true>(out_dtype, kp, grid, smem, s)
+                         : dispatch_out<1, CL, kModePlain, true>(out_dtype, kp, grid, smem, s);
+    return kind == 0 ? dispatch_out<0, CL, kModePlain, false>(out_dtype, kp, grid, smem, s)
+                     : dispatch_out<1, CL, kModePlain, false>(out_dtype, kp, grid, smem, s);
 }
 
 template <int CL>
@@ -301,15 +308,23 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     const int pieces = L.pieces < 1 ? 1 : L.pieces;
     const int cg = (L.cg == 2 || L.cg == 4) ? L.cg : 1;     // CTAs per cluster
     const int cta_group = cg >= 2 ? 2 : 1;
+    const bool shared = tc_shared_pieces(pieces, cg, L.bm, L.promote_k, L.split_k, L.stages, L.M, L.N, L.batch,
+                                         L.sm_count);
+    const int bm = shared ? 2 * L.bm : L.bm;
+    kp.pieces_mode = shared ? 1 : 0;
     for (int i = 0; i < pieces; ++i) {
         if ((st = tc_encode_operand(&kp.tmN[i], L.in_dtype, L.opN[i], L.K, L.batch, kTcTileN)) != TL_SUCCESS) return st;
-        if ((st = tc_encode_operand(&kp.tmM[i], L.in_dtype, L.opM[i], L.K, L.batch, L.bm / cg)) != TL_SUCCESS) return st;
+        if ((st = tc_encode_operand(&kp.tmM[i], L.in_dtype, L.opM[i], L.K, L.batch, bm / cg)) != TL_SUCCESS) return st;
     }
     // products per k-block, smallest first: 2-piece split -> A1B0, A0B1, A0B0;
     // 3-piece split -> A2B0, A1B1, A0B2, A1B0, A0B1, A0B0
     static const uint8_t t3m[3] = {1, 0, 0}, t3n[3] = {0, 1, 0};
     static const uint8_t t6m[6] = {2, 1, 0, 1, 0, 0}, t6n[6] = {0, 1, 2, 0, 1, 0};
     if (pieces == 1) { kp.nterms = 1; kp.term_m[0] = kp.term_n[0] = 0; }
+    else if (shared) {                       // one stage per piece, smallest first
+        kp.nterms = pieces == 2 ? 2 : 3;
+        for (int i = 0; i < 3; ++i) kp.term_m[i] = kp.term_n[i] = static_cast<uint8_t>(std::max(0, kp.nterms - 1 - i));
+    }
     else if (pieces == 2) { kp.nterms = 3; for (int i = 0; i < 3; ++i) { kp.term_m[i] = t3m[i]; kp.term_n[i] = t3n[i]; } }
     else { kp.nterms = 6; for (int i = 0; i < 6; ++i) { kp.term_m[i] = t6m[i]; kp.term_n[i] = t6n[i]; } }
     const int W = kTcRowBytes / dtype_bytes(L.in_dtype);
@@ -326,17 +341,22 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.batch = static_cast<int>(L.batch);
     kp.alpha = L.alpha;
     kp.beta = L.beta;
-    kp.bm = L.bm;
+    kp.bm = bm;
     kp.stages = L.stages;
     kp.split_k = L.split_k;
     kp.raster = L.raster;
-    kp.tiles_m = static_cast<int>((L.M + L.bm - 1) / L.bm);
+    kp.tiles_m = static_cast<int>((L.M + bm - 1) / bm);
     kp.tile_rows = kTcTileN * cg;
     kp.tiles_n = static_cast<int>((L.N + kp.tile_rows - 1) / kp.tile_rows);
     kp.num_kb = static_cast<int>((L.K + W - 1) / W);
     kp.kb_elems = W;
     kp.promote_kb = L.promote_k > 0 ? static_cast<int>((L.promote_k + W - 1) / W) : 0;
-    size_t smem = tc_smem_bytes(L.bm / cta_group, L.stages);
+    // shared pieces: all products of a chain share its accumulator, so chains are short (the error of the
+    // tensor core's accumulation grows with the products added at full magnitude: 4 of 24 with one k-block
+    // of bf16x6, 16 of 24 with two of bf16x3, 16 with four of A0*B0 alone), as the epilogue has time for
+    if (shared) kp.promote_kb = std::min(kp.promote_kb, pieces == 3 ? 1 : 2);
+    const int64_t kb_work = shared ? (pieces == 3 ? 6 : 3) : 1;      // products per k-block, for the split rules
+    size_t smem = tc_smem_bytes(bm / cta_group, L.stages);
     kp.epi_bufs = epi_buffers(smem);
     smem += static_cast<size_t>(kp.epi_bufs - 1) * kTcEpiStageBytes;
     const int64_t tiles = static_cast<int64_t>(kp.tiles_m) * kp.tiles_n * L.batch;
@@ -355,7 +375,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
         kp.total_work = tiles;
         const int workers = persistent_workers(L.in_dtype, L.out_dtype, cg, L.ctas, L.sm_count, smem);
         const int64_t rem = tiles % workers, full = tiles / workers;
-        const size_t slab = static_cast<size_t>(kTcTileN) * L.bm * sizeof(float);
+        const size_t slab = static_cast<size_t>(kTcTileN) * bm * sizeof(float);
         // measured on GB300: a piece needs about 48 k-blocks (balanced) or 16 (uniform slices) to
         // amortise its partial-tile round trip; shorter pieces lose more than the idle workers
         const int64_t R = rem * kp.num_kb;
@@ -363,8 +383,8 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
         // tail_split -1 asks for the balanced split whatever the piece length
         // (the piece length R / Wmax is only formed once Wmax > 1: no whole last wave, or a single
         // tile of one k-block, leaves Wmax at 0)
-        const bool balanced = rem > 0 && Wmax > 1 && Wmax >= rem && L.promote_k == 0 &&
-                              (L.tail_split == -1 || (L.tail_split == 0 && R / Wmax >= 48));
+        const bool balanced = rem > 0 && Wmax > 1 && Wmax >= rem && (L.promote_k == 0 || shared) &&
+                              (L.tail_split == -1 || (L.tail_split == 0 && R * kb_work / Wmax >= 48));
         if (balanced && L.workspace) {
             // balanced split (automatic, long k): the k-blocks of the last partial wave's tiles
             // are cut into equal contiguous ranges, one per worker (at most 8 pieces per tile); a
@@ -381,7 +401,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
             }
             const int64_t saved = Wb >= rem ? kp.num_kb - (R + Wb - 1) / Wb : 0;
             if (Wb >= rem && Wb > 1 &&
-                (L.tail_split == -1 || saved >= (full >= 1 ? 2 : std::max<int64_t>(8, kp.num_kb / 3)))) {
+                (L.tail_split == -1 || saved * kb_work >= (full >= 1 ? 2 : std::max<int64_t>(8, kb_work * kp.num_kb / 3)))) {
                 const int64_t per = R / Wb;
                 kp.bal_kb = R;
                 kp.bal_workers = static_cast<int>(Wb);
@@ -395,7 +415,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
                    2 * rem <= workers) {
             // uniform tail split (explicit S, or automatic): the last partial wave's tiles are cut
             // into S equal k-slices, scheduled first
-            int S = L.tail_split > 1 ? L.tail_split : static_cast<int>(std::min<int64_t>(workers / rem, kp.num_kb / 16));
+            int S = L.tail_split > 1 ? L.tail_split : static_cast<int>(std::min<int64_t>(workers / rem, kp.num_kb * kb_work / 16));
             if (S > kp.num_kb) S = kp.num_kb;
             if (S > 8) S = 8;
             const size_t need = static_cast<size_t>(rem) * cg * S * slab;
@@ -409,7 +429,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     }
     kp.n_mn_major = L.opN[0].mn_major;
     kp.m_mn_major = L.opM[0].mn_major;
-    kp.idesc = make_idesc(L.in_dtype, kp.n_mn_major, kp.m_mn_major, L.bm, cta_group);
+    kp.idesc = make_idesc(L.in_dtype, kp.n_mn_major, kp.m_mn_major, bm, cta_group);
     desc_params(L.in_dtype, kp.n_mn_major, kp.n_lbo, kp.n_kstep);
     desc_params(L.in_dtype, kp.m_mn_major, kp.m_lbo, kp.m_kstep);
     kp.out_trunc = L.out_trunc;
@@ -430,6 +450,8 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
                  static_cast<int64_t>(kp.num_kb) * (kp.tail_split + 1) < (int64_t(1) << 31))
                     ? 1
                     : 0;
+    kp.range = L.range;
+    kp.range_klog2 = log2_ceil(L.K);
     kp.ws = L.workspace;
     kp.counters = L.counters;
     kp.err = L.err;

@@ -43,8 +43,10 @@ struct TcKernelParams {
     float alpha, beta;
     int bm, stages, split_k, raster;
     int tile_rows;                // n rows per tile: 128 (one CTA) or 256 (CTA pair)
-    int nterms;                   // tensor-core products per k-block (1, or 3 / 6 for the fp32 split)
-    uint8_t term_n[8], term_m[8]; // piece of B / of A used by each product (the last is A0*B0)
+    int nterms;                   // stages per k-block: 1, the 3 / 6 products of the fp32 split, or its 2 / 3
+                                  // pieces (kModePieces)
+    uint8_t term_n[8], term_m[8]; // piece of B / of A in each stage (the last is piece 0 of both)
+    int pieces_mode;              // kModePieces
     int promote_kb;               // >0: the A0*B0 product restarts its TMEM chain every promote_kb
                                   // k-blocks; the epilogue adds each chain into fp32 registers
     int tiles_m, tiles_n;
@@ -71,6 +73,8 @@ struct TcKernelParams {
     unsigned long long timeout_ns;
     int debug_skip_loads;         // TL_DEBUG_SKIP_LOADS: the producer issues no copies (timeout-path test)
     unsigned long long* trace;    // device timeline, TL_TRACE_SLOTS words per CTA, or null
+    const SplitRange* range;      // promoted kernels: run only if split_range_ok(*range, range_klog2), or null
+    int range_klog2;
     int out_t;                    // D and C are the transpose of the kernel's output: element (m, n)
                                   // at n + m * ld (an NN problem run as its transposed TT product)
 };
@@ -290,6 +294,15 @@ __device__ __forceinline__ void get_job(const TcKernelParams& p, int64_t w, cons
     }
 }
 
+// Whether a promoted launch runs at all: its operands' magnitudes, known once the split pass before it has
+// completed, are within what the pieces can stand for.
+template <int MODE>
+__device__ __forceinline__ bool launch_live(const TcKernelParams& p)
+{
+    if constexpr (MODE == kModePlain) return true;
+    else return p.range == nullptr || split_range_ok(*p.range, p.range_klog2);
+}
+
 __device__ __forceinline__ void record_error(const TcKernelParams& p, volatile int* abort_flag, int code)
 {
     *abort_flag = 1;
@@ -396,7 +409,7 @@ __device__ __forceinline__ void load_bias(const TcKernelParams& p, int M, int m,
 {
     const int es = p.epi_bias_dtype == TL_DTYPE_FP32 ? 4 : 2;
     const char* src = static_cast<const char*>(p.epi_bias) + static_cast<int64_t>(m) * es;
-    if (m + W <= M && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    if ((W % 8 == 0 || es == 4) && m + W <= M && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
         if (es == 4) {
 #pragma unroll
             for (int q = 0; q < W / 4; ++q) {
@@ -792,12 +805,17 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
     }
 }
 
-// PROMO: the kernels with promoted accumulation (promote_k > 0), whose four epilogue warps hold 128
-// running sums per thread; the others have eight epilogue warps, two per quarter of the TMEM lanes,
+// MODE
+//   kModePromo   promoted accumulation (promote_k > 0): four epilogue warps hold 128 running sums per
+//                thread.
+//   kModePieces  promoted accumulation of the split-precision products, each piece of an operand staged
+//                once per k-block for all the products that use it; 256-column tiles, sixteen epilogue
+//                warps with 64 running sums per thread.
+//   kModePlain   the others: eight epilogue warps, two per quarter of the TMEM lanes,
 // which take alternate column groups of a tile (half the drain time of a CTA's last tile, and of every
 // tile whose k is too short to hide it).  GROUP: the work units and problems come from a plan's tables.
-template <int KIND, typename TD, int CL, bool EPI, bool PROMO, bool GROUP>
-__global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __grid_constant__ TcKernelParams p)
+template <int KIND, typename TD, int CL, bool EPI, int MODE, bool GROUP>
+__global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __grid_constant__ TcKernelParams p)
 {
     // CL CTAs per cluster.  CL == 2: a CTA pair on two SMs works on one 256-row tile.  Each CTA
     // stages its own 128 rows of the n-side operand and its half of the m-side operand; the leader
@@ -811,7 +829,9 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
     // have released it (each slot's empty barrier expects one commit from each pair's leader).
     constexpr int CG = CL >= 2 ? 2 : 1;         // CTAs per MMA (cta_group)
     constexpr int MC = CL / CG;                 // pairs sharing the m-side operand
-    constexpr int NH = PROMO ? 1 : 2;           // epilogue warps per TMEM lane quarter
+    constexpr bool PROMO = MODE == kModePromo, PIECES = MODE == kModePieces;
+    constexpr int NH = PROMO ? 1 : (PIECES ? 4 : 2);      // epilogue warps per TMEM lane quarter
+    constexpr int EW0 = 2;                      // first epilogue warp
     if (threadIdx.x == 0 && p.trace != nullptr) {
         trace_mark(p, TL_TRACE_ENTRY);
         trace_put(p, TL_TRACE_ENTRY_NS, global_ns());
@@ -846,7 +866,7 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
     const bool leader = (pair_rank == 0);
     const int64_t unit0 = (CL > 1) ? static_cast<int64_t>(ptx::cluster_id_x()) : static_cast<int64_t>(blockIdx.x);
     const int64_t units = (CL > 1) ? static_cast<int64_t>(ptx::ncluster_x()) : static_cast<int64_t>(gridDim.x);
-    const bool sep_small = PROMO && p.nterms > 1;
+    const bool sep_small = PROMO && p.nterms > 1;      // (the pieces' products share one accumulator)
     // TMEM columns: main accumulator x2 (+ small-term accumulator x2 when they are kept apart)
     const uint32_t need_cols = static_cast<uint32_t>(p.bm) * (sep_small ? 4u : 2u);
     const uint32_t tmem_cols = need_cols <= 128 ? 128u : (need_cols <= 256 ? 256u : 512u);
@@ -1023,6 +1043,7 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
                 if (first) {
                     ptx::grid_dep_wait();
                     ptx::grid_dep_launch_dependents();
+                    if (!launch_live<MODE>(p)) break;
                     trace_mark(p, TL_TRACE_DEP);
                     trace_mark(p, TL_TRACE_LOAD_FIRST);
                 }
@@ -1086,7 +1107,8 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
             };
             bool ok = true;
             // (touches no global memory but the error word and the timeline)
-            if (p.trace != nullptr) ptx::grid_dep_wait();
+            if (p.trace != nullptr || (MODE != kModePlain && p.range != nullptr)) ptx::grid_dep_wait();
+            ok = launch_live<MODE>(p);
             int4 u_next = load_unit<GROUP>(p, unit0);
             for (int64_t w = unit0; w < p.total_work && ok; w += units) {
                 const int4 u = u_next;
@@ -1113,7 +1135,74 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
                     ptx::mbar_wait(bar, phase, tlim);
                     trace_mark(p, TL_TRACE_MMA_FIRST);
                 }
-                if constexpr (!PROMO) {
+                if constexpr (PIECES) {
+                    // A k-block's pieces arrive smallest first in nvirt consecutive slots; every product
+                    // of them is formed from there, those of one order with each other (smallest
+                    // first, so that only the last runs at the accumulator's full magnitude), and a
+                    // slot is released by its last product.  The accumulator restarts every
+                    // promote_kb k-blocks in the alternate buffer.
+                    uint32_t acc = 0;
+                    int in_chain = 0;
+                    for (int kb = 0; kb < nkb; ++kb) {
+                        if (in_chain == p.promote_kb) {
+                            ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
+                            mbuf ^= 1u;
+                            if (mbuf == 0) mph ^= 1u;
+                            in_chain = 0;
+                            acc = 0;
+                            if (!ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
+                                record_error(p, abort_flag, 2);
+                                ok = false;
+                                break;
+                            }
+                            ptx::tc_fence_after();
+                        }
+                        const uint32_t d_tmem = tmem_base + mbuf * bmu;
+                        uint32_t sl[3], dn[3];
+#pragma unroll
+                        for (int v = 0; v < 3; ++v) {
+                            if (v < nvirt) {
+                                if (ok && !ptx::mbar_wait(bar, phase, tlim)) {
+                                    record_error(p, abort_flag, 4);
+                                    ok = false;
+                                }
+                                sl[v] = bar + (empty_a - full_a);
+                                dn[v] = dN;
+                                bar += 8u;
+                                dN += dstep;
+                                if (bar == bar_end) {
+                                    bar = full_a;
+                                    dN = dN0;
+                                    phase ^= 1u;
+                                }
+                            }
+                        }
+                        if (!ok) break;
+                        ptx::tc_fence_after();
+                        auto mma = [&](uint32_t n, uint32_t m) {
+                            ptx::mma_kblock<KIND, CG>(d_tmem, n, m + dNM, dhi, idesc, acc, n_kstep, m_kstep);
+                            acc = 1;
+                        };
+                        if (nvirt == 3) {                       // dn: pieces 2, 1, 0
+                            mma(dn[0], dn[2]);
+                            mma(dn[2], dn[0]);
+                            ptx::mma_commit_pair(sl[0], 0x3);
+                            mma(dn[1], dn[1]);
+                            mma(dn[1], dn[2]);
+                            mma(dn[2], dn[1]);
+                            ptx::mma_commit_pair(sl[1], 0x3);
+                            mma(dn[2], dn[2]);
+                            ptx::mma_commit_pair(sl[2], 0x3);
+                        } else {                                // dn: pieces 1, 0
+                            mma(dn[0], dn[1]);
+                            mma(dn[1], dn[0]);
+                            ptx::mma_commit_pair(sl[0], 0x3);
+                            mma(dn[1], dn[1]);
+                            ptx::mma_commit_pair(sl[1], 0x3);
+                        }
+                        ++in_chain;
+                    }
+                } else if constexpr (!PROMO) {
                     // every product of the tile into one accumulator
                     const uint32_t d_tmem = tmem_base + mbuf * bmu;
                     uint32_t accumulate = 0;
@@ -1174,11 +1263,11 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
         // left waiting at bar.sync 1 for one that gave up.
         const int quarter = warp & 3;             // TMEM lanes 32*quarter .. +31
         const int row = quarter * 32 + lane;      // tile row = problem n offset within this CTA
-        const int half = (warp - 2) >> 2;         // which of the quarter's NH warps
-        const int et = threadIdx.x - 64;          // 0 .. 128 * NH - 1
+        const int half = (warp - EW0) >> 2;         // which of the quarter's NH warps
+        const int et = threadIdx.x - 32 * EW0;    // 0 .. 128 * NH - 1
         // staging: 4 KB per warp; where shared memory holds only 16 KB of it, the second warp of a quarter
-        // takes no part in staged stores.  The one warp of a promotion kernel stages nothing.
-        const int nst = min(NH, p.epi_bufs);      // staging warps per quarter
+        // takes no part in staged stores.  The promotion kernels stage nothing.
+        const int nst = MODE == kModePlain ? min(NH, p.epi_bufs) : 1;      // staging warps per quarter
         const uint32_t my_stage_a = ptx::smem_u32(epi_stage) + static_cast<uint32_t>(min(half, nst - 1) * 4 + quarter) * 4096u;
         const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
         uint32_t mbuf = 0, mph = 0, sbuf = 0, sph = 0;
@@ -1191,7 +1280,10 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
             // the epilogue trails the MMAs: no need to load the unit ahead
             TileJob j;
             get_job<GROUP>(p, w, load_unit<GROUP>(p, w), j);
-            if (w == unit0) ptx::grid_dep_wait();
+            if (w == unit0) {
+                ptx::grid_dep_wait();
+                if (!launch_live<MODE>(p)) break;
+            }
             if (j.kb1 <= j.kb0) continue;             // an empty unit of a balanced split
             ++units_done;
             const bool tr = (et == 0 && w == unit0);  // timeline stamps: the first tile, one thread
@@ -1211,11 +1303,15 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
                 for (int off = 128 * half; off < cbytes; off += 128 * NH)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(cp + off));
             }
-            if constexpr (PROMO) {
-                // ---- promotion: sum the A0*B0 chains (and the small terms) in fp32 registers; bm == 128
-                float run[128];
+            if constexpr (MODE != kModePlain) {
+                // ---- promotion: sum the chains (and the separate small terms) in fp32 registers: all 128
+                // columns of the tile, or this warp's 64 of 256
+                constexpr int RC = PROMO ? 128 : 64;                  // columns of this thread
+                constexpr int QW = PROMO ? 16 : 8, NQ = RC / QW;
+                const int col0 = PROMO ? 0 : RC * half;
+                float run[RC];
 #pragma unroll
-                for (int i = 0; i < 128; ++i) run[i] = 0.f;
+                for (int i = 0; i < RC; ++i) run[i] = 0.f;
                 const int nkb = j.kb1 - j.kb0;
                 const int nchain = (nkb + p.promote_kb - 1) / p.promote_kb;
                 for (int c = 0; c < nchain; ++c) {
@@ -1227,14 +1323,14 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
                     }
                     if (ok) {
                         ptx::tc_fence_after();
-                        const uint32_t tb = tmem_base + lane_off + mbuf * static_cast<uint32_t>(p.bm);
+                        const uint32_t tb = tmem_base + lane_off + mbuf * static_cast<uint32_t>(p.bm) + static_cast<uint32_t>(col0);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint32_t r[32];
+                        for (int q = 0; q < NQ; ++q) {
+                            float r[QW];
                             __syncwarp();
-                            ptx::tmem_ld32(tb + q * 32, r);
+                            ptx::tmem_ld<QW>(tb + q * QW, r);
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) run[q * 32 + i] += __uint_as_float(r[i]);
+                            for (int i = 0; i < QW; ++i) run[q * QW + i] += r[i];
                         }
                         release_tmem<CG>(&tempty[mbuf], lane);
                     }
@@ -1252,12 +1348,12 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
                         ptx::tc_fence_after();
                         const uint32_t tb = tmem_base + lane_off + (2u + sbuf) * static_cast<uint32_t>(p.bm);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint32_t r[32];
+                        for (int q = 0; q < NQ; ++q) {
+                            float r[QW];
                             __syncwarp();
-                            ptx::tmem_ld32(tb + q * 32, r);
+                            ptx::tmem_ld<QW>(tb + q * QW, r);
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) run[q * 32 + i] += __uint_as_float(r[i]);
+                            for (int i = 0; i < QW; ++i) run[q * QW + i] += r[i];
                         }
                         release_tmem<CG>(&sempty[sbuf], lane);
                     }
@@ -1265,32 +1361,106 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
                     if (sbuf == 0) sph ^= 1u;
                 }
                 if (tr) trace_mark(p, TL_TRACE_ACC_READY);
+                // With 96 registers of which 64 hold sums, the unit is decoded again here instead of
+                // being held through the loop above (`w` is laundered so that it is): kept, its fields
+                // lived in local memory, which no L1 is left for, and parking a tile took 30000 clocks.
+                if constexpr (PIECES) {
+                    int64_t w2 = w;
+                    asm volatile("" : "+l"(w2));
+                    get_job<GROUP>(p, w2, make_int4(0, 0, 0, 0), j);
+                    j.n0 += static_cast<int>(rank) * kTcTileN;
+                    j.slot = j.slot * CL + rank;
+                }
+                const int n2 = j.n0 + row;
+                const bool row_ok2 = n2 < j.N;
+                const int64_t d2 = static_cast<int64_t>(j.b) * p.stride_d + static_cast<int64_t>(n2) * j.ldd;
+                const int64_t c2 = static_cast<int64_t>(j.b) * p.stride_c + static_cast<int64_t>(n2) * j.ldc;
+                // QW columns at a time, the sums rotated through the registers: one copy of the code (and
+                // no C loads hoisted into registers the sums occupy)
                 if (j.nsplit == 1) {
+                    if constexpr (PIECES) {
+                        // 16 columns at a time through 2 KB of staging per warp (32 rows x 64 bytes, unit u of
+                        // row r at u ^ (r / 2 % 4)): written by row as they are, read and finished in
+                        // 64-byte runs, so that few registers are needed beside the sums and the stores
+                        // cover whole sectors (a lane's own 16-byte stores along its row took 48000
+                        // clocks a tile)
+                        constexpr int SW = 16;
+                        const uint32_t st = ptx::smem_u32(epi_stage) + static_cast<uint32_t>(warp - EW0) * 2048u;
+                        const uint32_t sr = st + static_cast<uint32_t>(lane * 64);
+                        const bool use_c = j.beta != 0.0f && j.C != nullptr;
+                        const int nr = j.n0 + quarter * 32 + (lane >> 2);
+#pragma unroll 1
+                        for (int q = 0; q < RC / SW && ok; ++q) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int m = j.m0 + q * 32;
-                        if (ok && row_ok && m < j.M) {
-                            float v[32];
+                            for (int u = 0; u < 4; ++u)
+                                ptx::st_shared_v4(sr + static_cast<uint32_t>((u ^ ((lane >> 1) & 3)) * 16),
+                                                  __float_as_uint(run[4 * u]), __float_as_uint(run[4 * u + 1]),
+                                                  __float_as_uint(run[4 * u + 2]), __float_as_uint(run[4 * u + 3]));
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) v[i] = run[q * 32 + i];
-                            store_chunk<TD, EPI, 32>(p, amax, j, base_c, base_d, m, v);
+                            for (int i = 0; i < RC - SW; ++i) run[i] = run[i + SW];
+                            __syncwarp();
+                            const int m = j.m0 + col0 + q * SW + 4 * (lane & 3);
+#pragma unroll 1
+                            for (int it = 0; it < 4; ++it) {
+                                const int r = it * 8 + (lane >> 2), n = nr + it * 8;
+                                const uint4 w = ptx::ld_shared_v4(st + static_cast<uint32_t>(r * 64 + (((lane & 3) ^ ((r >> 1) & 3)) * 16)));
+                                if (n < j.N && m < j.M) {
+                                    float o[4] = {__uint_as_float(w.x), __uint_as_float(w.y), __uint_as_float(w.z), __uint_as_float(w.w)};
+                                    uint32_t cw[4];
+                                    float bias[4];
+                                    const int left = j.M - m;
+                                    float* d = static_cast<float*>(j.D) + static_cast<int64_t>(j.b) * p.stride_d +
+                                               static_cast<int64_t>(n) * j.ldd + m;
+                                    if (use_c) {
+                                        const float* c = static_cast<const float*>(j.C) + static_cast<int64_t>(j.b) * p.stride_c +
+                                                         static_cast<int64_t>(n) * j.ldc + m;
+                                        if (j.vec) {
+                                            const uint4 c4 = __ldg(reinterpret_cast<const uint4*>(c));
+                                            cw[0] = c4.x; cw[1] = c4.y; cw[2] = c4.z; cw[3] = c4.w;
+                                        } else {
+#pragma unroll
+                                            for (int e = 0; e < 4; ++e) cw[e] = e < left ? __float_as_uint(c[e]) : 0u;
+                                        }
+                                    }
+                                    if constexpr (EPI) {
+                                        if (p.epi_bias != nullptr) load_bias<4>(p, j.M, m, bias);
+                                    }
+                                    finish_values<TD, EPI, 4>(p, amax, j, m, true, cw, bias, o);
+                                    if (j.vec) {
+                                        *reinterpret_cast<float4*>(d) = make_float4(o[0], o[1], o[2], o[3]);
+                                    } else {
+#pragma unroll
+                                        for (int e = 0; e < 4; ++e)
+                                            if (e < left) d[e] = o[e];
+                                    }
+                                }
+                            }
+                            __syncwarp();
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int q = 0; q < NQ; ++q) {
+                            const int m = j.m0 + col0 + q * QW;
+                            float v[QW];
+#pragma unroll
+                            for (int i = 0; i < QW; ++i) v[i] = run[i];
+#pragma unroll
+                            for (int i = 0; i < RC - QW; ++i) run[i] = run[i + QW];
+                            if (ok && row_ok2 && m < j.M) store_chunk<TD, EPI, QW>(p, amax, j, c2, d2, m, v);
                         }
                     }
                     if (tr) trace_mark(p, TL_TRACE_STORED);
                 } else {
-                    float* slab = p.ws + (static_cast<size_t>(j.slot) * p.tail_split + j.split) *
-                                             (static_cast<size_t>(kTcTileN) * p.bm);
+                    float* dst = p.ws + (static_cast<size_t>(j.slot) * p.tail_split + j.split) *
+                                            (static_cast<size_t>(kTcTileN) * p.bm) +
+                                 static_cast<size_t>(col0) * kTcTileN + row;
                     if (ok) {
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            float* dst = slab + static_cast<size_t>(q) * 32 * kTcTileN + row;
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) __stcg(dst + i * kTcTileN, run[q * 32 + i]);
-                        }
+                        for (int i = 0; i < RC; ++i) __stcg(dst + i * kTcTileN, run[i]);
                     }
                     if (tr) trace_mark(p, TL_TRACE_STORED);
-                    split_finish<TD, EPI, 1>(p, amax, j, ok, et, lane, 0, row, row_ok, base_c, base_d, last_flag, abort_flag,
-                                             false, 0u);
+                    split_finish<TD, EPI, NH>(p, amax, j, ok, et, lane, half, row, row_ok2, c2, d2, last_flag, abort_flag,
+                                              false, 0u);
                     if (tr) trace_mark(p, TL_TRACE_REDUCED);
                 }
             } else {
@@ -1536,10 +1706,10 @@ __global__ void __launch_bounds__(tc_threads(PROMO), 1) tc_gemm_kernel(const __g
 // ---- launch (templates; instantiated in the generated instance units) ---------------------------
 bool pdl_enabled();
 
-template <int KIND, typename TD, int CL, bool EPI, bool PROMO, bool GROUP>
+template <int KIND, typename TD, int CL, bool EPI, int MODE, bool GROUP>
 tl_status launch_kernel(const TcKernelParams& kp, int grid, size_t smem, cudaStream_t stream)
 {
-    auto kern = tc_gemm_kernel<KIND, TD, CL, EPI, PROMO, GROUP>;
+    auto kern = tc_gemm_kernel<KIND, TD, CL, EPI, MODE, GROUP>;
     static std::once_flag once;
     static cudaError_t attr_err = cudaSuccess;
     std::call_once(once, [&] {
@@ -1549,7 +1719,7 @@ tl_status launch_kernel(const TcKernelParams& kp, int grid, size_t smem, cudaStr
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(static_cast<unsigned>(grid), 1, 1);
-    cfg.blockDim = dim3(tc_threads(PROMO), 1, 1);
+    cfg.blockDim = dim3(tc_threads(MODE), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -1587,12 +1757,12 @@ int max_clusters(size_t smem)
     std::lock_guard<std::mutex> g(mu);
     auto it = cache.find(smem);
     if (it != cache.end()) return it->second;
-    auto kern = tc_gemm_kernel<KIND, TD, CL, false, false, false>;
+    auto kern = tc_gemm_kernel<KIND, TD, CL, false, kModePlain, false>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTcMaxSmem));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3(CL, 1, 1);
-    cfg.blockDim = dim3(tc_threads(false), 1, 1);
+    cfg.blockDim = dim3(tc_threads(kModePlain), 1, 1);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;

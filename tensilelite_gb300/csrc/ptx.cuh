@@ -297,15 +297,13 @@ __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Arrive on a barrier that may live in another CTA of the cluster.  Release at CTA scope (the default): it
+// hands over TMEM (ordered by tcgen05.fence), not memory; at cluster scope it waits for every global
+// store and register spill the thread has outstanding (ncu: 8 warps stalled on it per issued
+// instruction of the shared-piece kernel).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)
 {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.release.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr),
-                 "r"(bytes)
-                 : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load into this CTA's shared memory whose completion is signalled on an mbarrier that may live
 // in the peer CTA of the pair (cluster address).

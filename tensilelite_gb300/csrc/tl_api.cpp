@@ -600,7 +600,7 @@ struct Prepared {
     // split-precision operand pieces in the workspace (bf16x3: 2 per operand, bf16x6: 3)
     uint16_t* a_pc[3] = {nullptr, nullptr, nullptr};
     uint16_t* b_pc[3] = {nullptr, nullptr, nullptr};
-    int64_t a_span = 0, b_span = 0;
+    int64_t a_ld = 0, b_ld = 0, a_bs = 0, b_bs = 0;      // the pieces' leading dimensions and batch strides
     float* ws_partials = nullptr;
     size_t part_bytes = 0;
     tl_epilogue epi{};
@@ -714,16 +714,24 @@ tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solut
     if (is_split(kernel)) {
         const int64_t a_rows = p.trans_a ? p.k : p.m, a_cols = p.trans_a ? p.m : p.k;
         const int64_t b_rows = p.trans_b ? p.n : p.k, b_cols = p.trans_b ? p.k : p.n;
-        P.a_span = operand_span(p.lda, a_cols, p.batch, p.stride_a, a_rows);
-        P.b_span = operand_span(p.ldb, b_cols, p.batch, p.stride_b, b_rows);
-        for (int i = 0; i < npc; ++i) { off_a[i] = need; need = align_up(need + P.a_span * 2, 256); }
-        for (int i = 0; i < npc; ++i) { off_b[i] = need; need = align_up(need + P.b_span * 2, 256); }
+        // the pieces' columns start on 128-byte lines whatever the caller's leading dimension: a box row
+        // of a TMA copy that straddles two lines costs two L2 requests (lda 2600: 530 clocks per stage
+        // against 340)
+        P.a_ld = static_cast<int64_t>(align_up(static_cast<size_t>(a_rows), 64));
+        P.b_ld = static_cast<int64_t>(align_up(static_cast<size_t>(b_rows), 64));
+        P.a_bs = P.a_ld * a_cols;
+        P.b_bs = P.b_ld * b_cols;
+        for (int i = 0; i < npc; ++i) { off_a[i] = need; need = align_up(need + P.a_bs * p.batch * 2, 256); }
+        for (int i = 0; i < npc; ++i) { off_b[i] = need; need = align_up(need + P.b_bs * p.batch * 2, 256); }
     }
     const int W = row_elems(tc_in_dtype(p));
     (void)W;
     const int cgp = P.s.macro_tile1 / kTcTileN;
     const int64_t tiles = ((p.n + kTcTileN * cgp - 1) / (kTcTileN * cgp)) * cgp *
                           ((p.m + P.s.macro_tile0 - 1) / P.s.macro_tile0) * p.batch;
+    const int slab_m = tc_shared_pieces(npc, cgp, P.s.macro_tile0, P.s.promote_k, P.s.split_k, P.s.stages, p.m, p.n, p.batch,
+                                        h->sm_count)
+                           ? 2 * P.s.macro_tile0 : P.s.macro_tile0;
     if (P.s.split_k > 1) {
         off_part = need;
         P.part_bytes = static_cast<size_t>(tiles) * P.s.split_k * kTcTileN * P.s.macro_tile0 * sizeof(float);
@@ -734,7 +742,7 @@ tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solut
         // partial slabs per tile, the automatic balanced split up to three (fewer, longer pieces
         // are chosen at launch when a tile would need more)
         off_part = need;
-        P.part_bytes = static_cast<size_t>(h->sm_count) * kTcTileN * P.s.macro_tile0 * sizeof(float) *
+        P.part_bytes = static_cast<size_t>(h->sm_count) * kTcTileN * slab_m * sizeof(float) *
                        static_cast<size_t>(P.s.tail_split > 1 ? P.s.tail_split : (P.s.tail_split == -1 ? 9 : 3));
         need = off_part + P.part_bytes;
         if ((st = ensure_counters(h, static_cast<size_t>(h->sm_count))) != TL_SUCCESS) return st;
@@ -831,11 +839,12 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
     if (L.pieces > 1) {
         const int64_t a_rows = p.trans_a ? p.k : p.m, a_cols = p.trans_a ? p.m : p.k;
         const int64_t b_rows = p.trans_b ? p.n : p.k, b_cols = p.trans_b ? p.k : p.n;
-        tl_status st = aux_split_bf16(static_cast<const float*>(P.A), a_rows, a_cols, p.lda, p.batch, p.stride_a,
-                                      P.a_pc[0], P.a_pc[1], P.a_pc[2], s, &h->launches);
-        if (st != TL_SUCCESS) return st;
-        st = aux_split_bf16(static_cast<const float*>(P.B), b_rows, b_cols, p.ldb, p.batch, p.stride_b, P.b_pc[0],
-                            P.b_pc[1], P.b_pc[2], s, &h->launches);
+        const SplitOperand ops[2] = {
+            {static_cast<const float*>(P.A), a_rows, a_cols, p.lda, p.batch, p.stride_a, {P.a_pc[0], P.a_pc[1], P.a_pc[2]},
+             P.a_ld, P.a_bs},
+            {static_cast<const float*>(P.B), b_rows, b_cols, p.ldb, p.batch, p.stride_b, {P.b_pc[0], P.b_pc[1], P.b_pc[2]},
+             P.b_ld, P.b_bs}};
+        const tl_status st = aux_split_bf16(ops, 2, L.pieces, nullptr, s, &h->launches);
         if (st != TL_SUCCESS) return st;
         for (int i = 0; i < L.pieces; ++i) {
             Apc[i] = P.a_pc[i];
@@ -843,8 +852,9 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
         }
     }
     for (int i = 0; i < L.pieces; ++i) {
-        L.opM[i] = {Apc[i], p.m, p.lda, p.stride_a, m_mn_major(p) ? 1 : 0};
-        L.opN[i] = {Bpc[i], p.n, p.ldb, p.stride_b, n_mn_major(p) ? 1 : 0};
+        const bool split = L.pieces > 1;
+        L.opM[i] = {Apc[i], p.m, split ? P.a_ld : p.lda, split ? P.a_bs : p.stride_a, m_mn_major(p) ? 1 : 0};
+        L.opN[i] = {Bpc[i], p.n, split ? P.b_ld : p.ldb, split ? P.b_bs : p.stride_b, n_mn_major(p) ? 1 : 0};
     }
     L.M = p.m; L.N = p.n; L.K = p.k; L.batch = p.batch;
     L.D = P.D; L.C = (p.beta != 0.0f) ? P.C : nullptr;
@@ -1815,8 +1825,8 @@ TL_API tl_status tl_split_bf16x2(tl_handle* h, const float* src, int64_t n, void
 {
     if (h && h->host_only) return host_only_refused();
     if (!h || n < 0 || (n && (!src || !hi || !lo))) return fail(TL_ERR_INVALID_ARG, "bad argument");
-    return aux_split_bf16(src, n, 1, n, 1, n, static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo), nullptr,
-                          S(stream), &h->launches);
+    const SplitOperand op = {src, n, 1, n, 1, n, {static_cast<uint16_t*>(hi), static_cast<uint16_t*>(lo), nullptr}, n, n};
+    return aux_split_bf16(&op, 1, 2, nullptr, S(stream), &h->launches);
 }
 
 // ---- verification ------------------------------------------------------------------------------------

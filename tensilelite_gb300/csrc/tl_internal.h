@@ -23,6 +23,14 @@ tl_status cuda_fail(cudaError_t e, const char* what);
         if (e_ != cudaSuccess) return ::tl::cuda_fail(e_, #call); \
     } while (0)
 
+// ceil(log2 k)
+inline int log2_ceil(int64_t k)
+{
+    int l = 0;
+    while ((int64_t(1) << l) < k) ++l;
+    return l;
+}
+
 inline int dtype_bytes(int dt)
 {
     switch (dt) {
@@ -40,8 +48,44 @@ constexpr int kTcTileN = 128;          // tcgen05 M extent: problem n rows on TM
 constexpr int kTcRowBytes = 128;       // one swizzle row: depth_u * element size
 constexpr int kTcEpiStageBytes = 4 * 32 * 128;   // output staging of 4 epilogue warps
 constexpr size_t kTcMaxSmem = 227 * 1024;        // dynamic shared memory a CTA may ask for
-// warp 0 TMA, warp 1 MMA, then eight epilogue warps (four in the promotion kernels)
-constexpr int tc_threads(bool promo) { return promo ? 192 : 320; }
+// kernel variants: plain accumulation, promoted accumulation, promoted products of shared pieces
+constexpr int kModePlain = 0, kModePromo = 1, kModePieces = 2;
+// warp 0 TMA, warp 1 MMA, then eight, four or sixteen epilogue warps
+constexpr int tc_threads(int mode) { return mode == kModePromo ? 192 : (mode == kModePieces ? 576 : 320); }
+// The fp32-split products run with shared pieces (kModePieces) on the default solution's tile, a
+// promoted CTA pair with its six-slot ring: two of its 128-column tiles side by side, each piece of A
+// and B loaded once per k-block instead of once per product (bf16x3 needs 2 loads for 3 products,
+// bf16x6 3 for 6) and 256-column MMAs, 1536 / 3072 clocks per k-block against 2 x 1035 / 2070.  Only
+// where the 128-column tiles are more than one wave of pairs: below that the wide tile leaves pairs
+// idle (512 x 4096 x 1024: bf16x3 41 us against 36).  Not for an explicit split-k or another ring,
+// which ask for the tile as it stands.
+inline bool tc_shared_pieces(int pieces, int cg, int bm, int promote_k, int split_k, int stages, int64_t M, int64_t N,
+                             int64_t batch, int sm_count)
+{
+    const int64_t tiles = ((M + 127) / 128) * ((N + 255) / 256) * batch;
+    return pieces > 1 && cg == 2 && bm == 128 && promote_k > 0 && split_k == 1 && stages == 6 && M > 128 &&
+           2 * tiles > sm_count;
+}
+
+// Magnitudes of the two operands of a split-precision product, gathered by the split pass: the bits of
+// the largest |x| and the complement of the bits of the smallest nonzero |x| (0: none), of A then of B.
+struct SplitRange {
+    uint32_t max_a, inv_min_a, max_b, inv_min_b;
+};
+// Whether three bf16 pieces stand for these operands as exactly as fp32 does in a sum of 2^klog2
+// products: everything finite, no piece below bf16's normal range, no product of pieces (down to
+// 2^-16 of its operands' product) below fp32's, and no sum beyond its largest value.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline bool split_range_ok(const SplitRange& r, int klog2)
+{
+    const int ea = static_cast<int>(r.max_a >> 23), eb = static_cast<int>(r.max_b >> 23);
+    if (ea == 255 || eb == 255) return false;
+    const int ma = r.inv_min_a ? static_cast<int>((~r.inv_min_a) >> 23) : 127;
+    const int mb = r.inv_min_b ? static_cast<int>((~r.inv_min_b) >> 23) : 127;
+    return ea + eb - 254 + 2 + klog2 <= 126 && ma >= 27 && mb >= 27 && ma + mb - 254 >= -100;
+}
 
 // One operand's TMA view: K-major (rows x k, k contiguous) or MN-major (k rows of contiguous rows).
 struct TcOperand {
@@ -105,6 +149,7 @@ struct TcLaunch {
     unsigned long long* trace;   // device timeline (tl_set_trace) or null
     int64_t trace_bytes;
     int out_t;               // D and C hold the transpose of this launch's output (NN run as TT)
+    const SplitRange* range; // split products: run only if split_range_ok (device memory), or null
 };
 
 // Dynamic shared memory of one CTA staging bm_cta m-rows per stage (bm / 2 for a CTA pair).
@@ -149,13 +194,21 @@ struct SimtLaunch {
     const void* A; const void* B; const void* C; void* D;
     int64_t lda, ldb, ldc, ldd, sa, sb, sc, sd;
     float alpha, beta;   // alpha already multiplied by fp8 scales
+    const SplitRange* unless = nullptr;   // run only if split_range_ok fails (device memory), or null
 };
 tl_status simt_gemm_launch(const SimtLaunch& L, cudaStream_t stream, int64_t* launches);
 
 // ---- auxiliary kernels ------------------------------------------------------------------------------
 // x = p0 + p1 (+ p2): each piece the bf16 rounding (RNE) of what the previous pieces leave; p2 may be null.
-tl_status aux_split_bf16(const float* src, int64_t rows, int64_t cols, int64_t ld, int64_t batch,
-                         int64_t batch_stride, uint16_t* p0, uint16_t* p1, uint16_t* p2, cudaStream_t s,
+// The pieces have their own leading dimension and batch stride.  One launch per matrix.
+struct SplitOperand {
+    const float* src;
+    int64_t rows, cols, ld, batch, batch_stride;
+    uint16_t* p[3];
+    int64_t pld, p_batch_stride;
+};
+// `range`, if given, receives the operands' magnitudes (zeroed by the caller).
+tl_status aux_split_bf16(const SplitOperand* ops, int count, int pieces, SplitRange* range, cudaStream_t s,
                          int64_t* launches);
 // Per-tensor E4M3 quantisation: *amax_dev = max |x|, dst = e4m3(x * 448 / amax), *scale_out_dev = amax / 448.
 tl_status aux_quantize_e4m3(int src_dtype, const void* src, int64_t n, float* amax_dev, uint8_t* dst,
