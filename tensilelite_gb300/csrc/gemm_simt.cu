@@ -89,6 +89,8 @@ struct SimtParams {
     float alpha, beta;
     int out_trunc;
     int vec_a, vec_b;      // 4-element vector loads are aligned along the contiguous dimension
+    const SplitRange* unless;   // nothing to do if split_range_ok (the tensor cores have done it)
+    int klog2;
 };
 
 // Tile shape: BM x BN outputs, TM x TN per thread and k-group, KG k-groups, BKG k per group and slab,
@@ -145,6 +147,7 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB) simt_gemm_kernel(const Si
     // (its writes visible) before the first global access, then let the next grid get scheduled.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (p.unless != nullptr && split_range_ok(*p.unless, p.klog2)) return;
     const TA* A = static_cast<const TA*>(p.A) + static_cast<int64_t>(b) * p.sa;
     const TA* B = static_cast<const TA*>(p.B) + static_cast<int64_t>(b) * p.sb;
 
@@ -404,6 +407,8 @@ tl_status launch(const SimtLaunch& L, cudaStream_t s)
     p.trans_a = L.trans_a; p.trans_b = L.trans_b;
     p.alpha = L.alpha; p.beta = L.beta;
     p.out_trunc = L.out_trunc;
+    p.unless = L.unless;
+    p.klog2 = log2_ceil(L.K);
     // vector loads need the 4-element groups aligned: base, leading dimension and batch stride
     const uintptr_t vb = 4 * sizeof(TA);
     p.vec_a = ((reinterpret_cast<uintptr_t>(L.A) % vb) == 0 && L.lda % 4 == 0 && (L.batch == 1 || L.sa % 4 == 0)) ? 1 : 0;

@@ -44,6 +44,7 @@ struct Plan {
     bool view;
 };
 constexpr size_t kMaxPlans = 4096;
+constexpr uint64_t kPoolKeep = uint64_t(4) << 30;
 }  // namespace tl
 
 struct tl_handle {
@@ -66,7 +67,12 @@ struct tl_handle {
     std::map<std::string, tl_gemm_solution> tuned;
     // heuristic picks by problem shape (the cost model takes 1.5 to 7 us a problem); at most kMaxPlans
     std::unordered_map<tl::PlanKey, tl::Plan, tl::PlanKeyHash> plans;
-    std::mutex mu;                 // tuned, plans
+    std::mutex mu;                 // tuned, plans, pool
+    // stream-ordered scratch of fp32 GEMMs that run on the tensor cores (gemm_fp32_tc): each call has its
+    // own, so that calls on different streams and threads stay independent.  At most kPoolKeep bytes
+    // stay with the pool between synchronisations.
+    cudaMemPool_t pool = nullptr;
+    bool pool_failed = false;
     // Once a stream capture has recorded this handle's workspace address, a grown workspace retires
     // the old buffer here (freed by tl_destroy) instead of freeing it under a live graph.
     bool captured = false;
@@ -603,8 +609,12 @@ struct Prepared {
     int64_t a_ld = 0, b_ld = 0, a_bs = 0, b_bs = 0;      // the pieces' leading dimensions and batch strides
     float* ws_partials = nullptr;
     size_t part_bytes = 0;
+    int* counters = nullptr;             // split tile counters
+    size_t counters_len = 0;
+    SplitRange* range = nullptr;         // the split pass reports magnitudes; the GEMM depends on them
     tl_epilogue epi{};
     bool epi_on = false;
+    bool tuned = false;      // the solution was tuned or loaded
     bool tview = false;      // p is the transposed view of the caller's NN problem (tc_nn_view)
 };
 
@@ -612,6 +622,61 @@ int64_t operand_span(int64_t ld, int64_t cols, int64_t batch, int64_t bstride, i
 {
     if (rows == 0 || cols == 0) return 0;
     return (batch - 1) * bstride + (cols - 1) * ld + rows;
+}
+
+// Scratch of a tensor-core launch: [split pieces of A][split pieces of B][split-k partials].
+struct Scratch {
+    size_t bytes = 0, off_a[3] = {0, 0, 0}, off_b[3] = {0, 0, 0}, off_part = 0, part_bytes = 0, counters = 0;
+};
+Scratch scratch_of(const tl_handle* h, Prepared& P)
+{
+    Scratch w;
+    const tl_gemm_problem& p = P.p;
+    const int npc = split_pieces(P.kernel);
+    if (is_split(P.kernel)) {
+        const int64_t a_rows = p.trans_a ? p.k : p.m, a_cols = p.trans_a ? p.m : p.k;
+        const int64_t b_rows = p.trans_b ? p.n : p.k, b_cols = p.trans_b ? p.k : p.n;
+        // the pieces' columns start on 128-byte lines whatever the caller's leading dimension: a box row
+        // of a TMA copy that straddles two lines costs two L2 requests (lda 2600: 530 clocks per stage
+        // against 340)
+        P.a_ld = static_cast<int64_t>(align_up(static_cast<size_t>(a_rows), 64));
+        P.b_ld = static_cast<int64_t>(align_up(static_cast<size_t>(b_rows), 64));
+        P.a_bs = P.a_ld * a_cols;
+        P.b_bs = P.b_ld * b_cols;
+        for (int i = 0; i < npc; ++i) { w.off_a[i] = w.bytes; w.bytes = align_up(w.bytes + P.a_bs * p.batch * 2, 256); }
+        for (int i = 0; i < npc; ++i) { w.off_b[i] = w.bytes; w.bytes = align_up(w.bytes + P.b_bs * p.batch * 2, 256); }
+    }
+    const int cgp = P.s.macro_tile1 / kTcTileN;
+    const int64_t tiles = ((p.n + kTcTileN * cgp - 1) / (kTcTileN * cgp)) * cgp *
+                          ((p.m + P.s.macro_tile0 - 1) / P.s.macro_tile0) * p.batch;
+    const int slab_m = tc_shared_pieces(npc, cgp, P.s.macro_tile0, P.s.promote_k, P.s.split_k, P.s.stages, p.m, p.n, p.batch,
+                                        h->sm_count)
+                           ? 2 * P.s.macro_tile0 : P.s.macro_tile0;
+    w.off_part = w.bytes;
+    if (P.s.split_k > 1) {
+        w.part_bytes = static_cast<size_t>(tiles) * P.s.split_k * kTcTileN * P.s.macro_tile0 * sizeof(float);
+        w.counters = static_cast<size_t>(tiles);
+    } else if (P.s.tail_split != 1) {
+        // a split last wave: at most one tile per SM is split; an explicit tail split S keeps S
+        // partial slabs per tile, the automatic balanced split up to three (fewer, longer pieces
+        // are chosen at launch when a tile would need more)
+        w.part_bytes = static_cast<size_t>(h->sm_count) * kTcTileN * slab_m * sizeof(float) *
+                       static_cast<size_t>(P.s.tail_split > 1 ? P.s.tail_split : (P.s.tail_split == -1 ? 9 : 3));
+        w.counters = static_cast<size_t>(h->sm_count);
+    }
+    w.bytes += w.part_bytes;
+    return w;
+}
+void place(Prepared& P, const Scratch& w, char* base)
+{
+    if (is_split(P.kernel)) {
+        for (int i = 0; i < split_pieces(P.kernel); ++i) {
+            P.a_pc[i] = reinterpret_cast<uint16_t*>(base + w.off_a[i]);
+            P.b_pc[i] = reinterpret_cast<uint16_t*>(base + w.off_b[i]);
+        }
+    }
+    P.part_bytes = w.part_bytes;
+    if (w.part_bytes) P.ws_partials = reinterpret_cast<float*>(base + w.off_part);
 }
 
 tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solution* sol, void* D, const void* C,
@@ -643,6 +708,7 @@ tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solut
         auto it = h->tuned.empty() ? h->tuned.end() : h->tuned.find(problem_key(h, p));
         if (it != h->tuned.end()) {
             P.s = it->second;
+            P.tuned = true;
             kernel = P.s.kernel;
             view = !epilogue && tc_nn_view(p, kernel) && view_solution_ok(P.s);
         } else if (kernel == TL_KERNEL_SIMT) {
@@ -707,59 +773,16 @@ tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solut
     if ((st = check_tc_solution(h, p, P.s)) != TL_SUCCESS) return st;
     if (p.m == 0 || p.n == 0 || p.k == 0) return TL_SUCCESS;
 
-    // workspace: [split pieces of A][split pieces of B][split-k partials]
-    size_t need = 0;
-    size_t off_a[3] = {0, 0, 0}, off_b[3] = {0, 0, 0}, off_part = 0;
-    const int npc = split_pieces(kernel);
+    const Scratch w = scratch_of(h, P);
+    if (w.counters && (st = ensure_counters(h, w.counters)) != TL_SUCCESS) return st;
+    if (w.bytes) {
+        if ((st = ensure_ws(h, w.bytes)) != TL_SUCCESS) return st;
+        place(P, w, static_cast<char*>(h->ws));
+    }
+    P.counters = h->counters;
+    P.counters_len = h->counters_len;
     if (is_split(kernel)) {
-        const int64_t a_rows = p.trans_a ? p.k : p.m, a_cols = p.trans_a ? p.m : p.k;
-        const int64_t b_rows = p.trans_b ? p.n : p.k, b_cols = p.trans_b ? p.k : p.n;
-        // the pieces' columns start on 128-byte lines whatever the caller's leading dimension: a box row
-        // of a TMA copy that straddles two lines costs two L2 requests (lda 2600: 530 clocks per stage
-        // against 340)
-        P.a_ld = static_cast<int64_t>(align_up(static_cast<size_t>(a_rows), 64));
-        P.b_ld = static_cast<int64_t>(align_up(static_cast<size_t>(b_rows), 64));
-        P.a_bs = P.a_ld * a_cols;
-        P.b_bs = P.b_ld * b_cols;
-        for (int i = 0; i < npc; ++i) { off_a[i] = need; need = align_up(need + P.a_bs * p.batch * 2, 256); }
-        for (int i = 0; i < npc; ++i) { off_b[i] = need; need = align_up(need + P.b_bs * p.batch * 2, 256); }
-    }
-    const int W = row_elems(tc_in_dtype(p));
-    (void)W;
-    const int cgp = P.s.macro_tile1 / kTcTileN;
-    const int64_t tiles = ((p.n + kTcTileN * cgp - 1) / (kTcTileN * cgp)) * cgp *
-                          ((p.m + P.s.macro_tile0 - 1) / P.s.macro_tile0) * p.batch;
-    const int slab_m = tc_shared_pieces(npc, cgp, P.s.macro_tile0, P.s.promote_k, P.s.split_k, P.s.stages, p.m, p.n, p.batch,
-                                        h->sm_count)
-                           ? 2 * P.s.macro_tile0 : P.s.macro_tile0;
-    if (P.s.split_k > 1) {
-        off_part = need;
-        P.part_bytes = static_cast<size_t>(tiles) * P.s.split_k * kTcTileN * P.s.macro_tile0 * sizeof(float);
-        need = off_part + P.part_bytes;
-        if ((st = ensure_counters(h, static_cast<size_t>(tiles))) != TL_SUCCESS) return st;
-    } else if (P.s.tail_split != 1) {
-        // a split last wave: at most one tile per SM is split; an explicit tail split S keeps S
-        // partial slabs per tile, the automatic balanced split up to three (fewer, longer pieces
-        // are chosen at launch when a tile would need more)
-        off_part = need;
-        P.part_bytes = static_cast<size_t>(h->sm_count) * kTcTileN * slab_m * sizeof(float) *
-                       static_cast<size_t>(P.s.tail_split > 1 ? P.s.tail_split : (P.s.tail_split == -1 ? 9 : 3));
-        need = off_part + P.part_bytes;
-        if ((st = ensure_counters(h, static_cast<size_t>(h->sm_count))) != TL_SUCCESS) return st;
-    }
-    if (need) {
-        if ((st = ensure_ws(h, need)) != TL_SUCCESS) return st;
-        char* base = static_cast<char*>(h->ws);
-        if (is_split(kernel)) {
-            for (int i = 0; i < npc; ++i) {
-                P.a_pc[i] = reinterpret_cast<uint16_t*>(base + off_a[i]);
-                P.b_pc[i] = reinterpret_cast<uint16_t*>(base + off_b[i]);
-            }
-        }
-        if (P.part_bytes) P.ws_partials = reinterpret_cast<float*>(base + off_part);
-    }
-    if (is_split(kernel)) {
-        // the split copies keep the caller's leading dimensions; TMA needs them 16-byte aligned in bf16
+        // the leading dimensions that the split products have always taken
         if ((p.lda * 2) % 16 || (p.ldb * 2) % 16 || (p.batch > 1 && ((p.stride_a * 2) % 16 || (p.stride_b * 2) % 16)))
             return fail(TL_ERR_UNSUPPORTED, "bf16x3/bf16x6: lda/ldb (and batch strides) must be multiples of 8 elements");
     }
@@ -805,6 +828,20 @@ void timing_end(tl_handle* h, cudaStream_t s, bool started, tl_status launch_sta
         h->tev_used += 2;
 }
 
+SimtLaunch simt_launch_of(const Prepared& P, float alpha)
+{
+    const tl_gemm_problem& p = P.p;
+    SimtLaunch L;
+    L.a_dtype = p.dtype_a; L.out_dtype = p.dtype_d; L.out_trunc = p.out_rounding;
+    L.trans_a = p.trans_a; L.trans_b = p.trans_b;
+    L.M = p.m; L.N = p.n; L.K = p.k; L.batch = p.batch;
+    L.A = P.A; L.B = P.B; L.C = P.C; L.D = P.D;
+    L.lda = p.lda; L.ldb = p.ldb; L.ldc = p.ldc; L.ldd = p.ldd;
+    L.sa = p.stride_a; L.sb = p.stride_b; L.sc = p.stride_c; L.sd = p.stride_d;
+    L.alpha = alpha; L.beta = p.beta;
+    return L;
+}
+
 tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
 {
     const tl_gemm_problem& p = P.p;
@@ -815,14 +852,7 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
                            p.batch, p.beta, s, &h->launches);
     }
     if (P.kernel == TL_KERNEL_SIMT) {
-        SimtLaunch L;
-        L.a_dtype = p.dtype_a; L.out_dtype = p.dtype_d; L.out_trunc = p.out_rounding;
-        L.trans_a = p.trans_a; L.trans_b = p.trans_b;
-        L.M = p.m; L.N = p.n; L.K = p.k; L.batch = p.batch;
-        L.A = P.A; L.B = P.B; L.C = P.C; L.D = P.D;
-        L.lda = p.lda; L.ldb = p.ldb; L.ldc = p.ldc; L.ldd = p.ldd;
-        L.sa = p.stride_a; L.sb = p.stride_b; L.sc = p.stride_c; L.sd = p.stride_d;
-        L.alpha = alpha; L.beta = p.beta;
+        const SimtLaunch L = simt_launch_of(P, alpha);
         const bool timed = timing_begin(h, s);
         const tl_status st = simt_gemm_launch(L, s, &h->launches);
         timing_end(h, s, timed, st);
@@ -844,7 +874,7 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
              P.a_ld, P.a_bs},
             {static_cast<const float*>(P.B), b_rows, b_cols, p.ldb, p.batch, p.stride_b, {P.b_pc[0], P.b_pc[1], P.b_pc[2]},
              P.b_ld, P.b_bs}};
-        const tl_status st = aux_split_bf16(ops, 2, L.pieces, nullptr, s, &h->launches);
+        const tl_status st = aux_split_bf16(ops, 2, L.pieces, P.range, s, &h->launches);
         if (st != TL_SUCCESS) return st;
         for (int i = 0; i < L.pieces; ++i) {
             Apc[i] = P.a_pc[i];
@@ -873,8 +903,9 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
     L.trace_bytes = h->trace_bytes;
     L.workspace = P.ws_partials;
     L.workspace_bytes = P.part_bytes;
-    L.counters = h->counters;
-    L.counters_len = h->counters_len;
+    L.counters = P.counters;
+    L.counters_len = P.counters_len;
+    L.range = P.range;
     L.tail_split = P.s.tail_split;
     L.sm_count = h->sm_count;
     // fp8 outputs are written by the fused-epilogue kernels (no bias or activation unless asked for)
@@ -889,6 +920,92 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
     const bool timed = timing_begin(h, s);
     const tl_status st = tc_gemm_launch(L, s, &h->launches);
     timing_end(h, s, timed, st);
+    return st;
+}
+
+// ---- plain fp32 on the tensor cores ---------------------------------------------------------------
+// A large fp32 GEMM left to the library (kernel AUTO, no solution, none tuned) runs as the six products
+// of three bf16 pieces per operand, whose error against 64 bits is below the CUDA-core kernel's at every
+// size and layout measured (relative 2-norm, 4096^3: 1.6e-7 against 1.15e-6; 512 x 4096 x 1024: 1.9e-7
+// against 2.1e-7) and which takes a fifth of its time (4096^3 TN: 490 us against 2770; 1024^3: 28 against
+// 104).  Below kFp32TcWork multiply-adds the split pass and the extra launches cost more than that
+// gives (480 x 512 x 512: 13 us on the CUDA cores).
+//
+// The pieces stand for the operands only within a range of magnitudes (split_range_ok), which is known
+// on the device once the split passes have run: infinities, NaN, numbers near fp32's limits.  So the
+// launches follow each other: the split passes report the magnitudes, the tensor-core launch returns at once
+// if they are out of range, and the CUDA-core launch returns at once if they are not.  What is out of
+// range therefore gets the CUDA-core kernel's results, bit for bit.
+//
+// Each call has its own scratch, allocated and freed in stream order.  While a stream is being
+// captured, or where the scratch cannot be had, the CUDA-core kernel runs as before.
+constexpr double kFp32TcWork = 3.0e8;
+
+bool fp32_tc_wanted(const tl_gemm_problem& p)
+{
+    return p.kernel == TL_KERNEL_AUTO && p.dtype_a == TL_DTYPE_FP32 && p.dtype_d == TL_DTYPE_FP32 && p.m > 0 && p.n > 0 &&
+           p.k > 0 && static_cast<double>(p.m) * static_cast<double>(p.n) * static_cast<double>(p.k) *
+           static_cast<double>(p.batch) >= kFp32TcWork && p.m >= 64 && p.n >= 64 && p.k >= 64 &&
+           p.alpha * scale_of(p.scale_a) * scale_of(p.scale_b) != 0.0f;
+}
+
+cudaMemPool_t fp32_pool(tl_handle* h)
+{
+    std::lock_guard<std::mutex> g(h->mu);
+    if (!h->pool && !h->pool_failed) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = h->device;
+        uint64_t keep = kPoolKeep;
+        if (cudaMemPoolCreate(&h->pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            if (h->pool) cudaMemPoolDestroy(h->pool);
+            h->pool = nullptr;
+            h->pool_failed = true;
+        }
+    }
+    return h->pool;
+}
+
+// P is prepared for the CUDA-core kernel.  *done reports whether the GEMM was enqueued here.
+tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done)
+{
+    *done = false;
+    cudaMemPool_t pool = fp32_pool(h);
+    if (!pool) return TL_SUCCESS;
+    Prepared T = P;
+    T.kernel = TL_KERNEL_BF16X6;
+    T.p.kernel = TL_KERNEL_BF16X6;
+    tc_heuristic(h, T.p, TL_KERNEL_BF16X6, &T.s);
+    if (check_tc_solution(h, T.p, T.s) != TL_SUCCESS) return TL_SUCCESS;
+    const Scratch w = scratch_of(h, T);
+    const size_t head = align_up(sizeof(SplitRange) + w.counters * sizeof(int), 256);
+    void* mem = nullptr;
+    if (cudaMallocFromPoolAsync(&mem, head + w.bytes, pool, s) != cudaSuccess) {
+        cudaGetLastError();
+        return TL_SUCCESS;
+    }
+    *done = true;
+    char* base = static_cast<char*>(mem);
+    T.range = reinterpret_cast<SplitRange*>(base);
+    T.counters = reinterpret_cast<int*>(base + sizeof(SplitRange));
+    T.counters_len = w.counters;
+    place(T, w, base + head);
+    tl_status st = TL_SUCCESS;
+    cudaError_t e = cudaMemsetAsync(base, 0, head, s);
+    if (e != cudaSuccess) st = cuda_fail(e, "cudaMemsetAsync(fp32 scratch)");
+    if (st == TL_SUCCESS) st = enqueue(h, T, s);
+    if (st == TL_SUCCESS) {
+        SimtLaunch L = simt_launch_of(P, P.p.alpha * scale_of(P.p.scale_a) * scale_of(P.p.scale_b));
+        L.unless = T.range;
+        st = simt_gemm_launch(L, s, &h->launches);
+    }
+    e = cudaFreeAsync(mem, s);
+    if (st == TL_SUCCESS && e != cudaSuccess) st = cuda_fail(e, "cudaFreeAsync(fp32 scratch)");
     return st;
 }
 
@@ -1144,6 +1261,7 @@ TL_API tl_status tl_destroy(tl_handle* h)
     cudaDeviceSynchronize();
     if (h->ws) cudaFree(h->ws);
     if (h->counters) cudaFree(h->counters);
+    if (h->pool) cudaMemPoolDestroy(h->pool);
     for (void* r : h->retired) cudaFree(r);
     for (cudaEvent_t e : h->tev) cudaEventDestroy(e);
     if (h->d_err) cudaFree(h->d_err);
@@ -1226,8 +1344,14 @@ TL_API tl_status tl_gemm(tl_handle* h, const tl_gemm_problem* p, const tl_gemm_s
     t_capturing = stream_capturing(S(stream));
     if (t_capturing) h->captured = true;
     tl_status st = prepare(h, p, s, D, C, A, B, &P);
+    const bool capturing = t_capturing;
     t_capturing = false;
     if (st != TL_SUCCESS) return st;
+    if (!s && !capturing && P.kernel == TL_KERNEL_SIMT && !P.tuned && fp32_tc_wanted(*p)) {
+        bool done = false;
+        st = gemm_fp32_tc(h, P, S(stream), &done);
+        if (done) return st;
+    }
     return enqueue(h, P, S(stream));
 }
 

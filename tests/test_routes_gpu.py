@@ -1,0 +1,209 @@
+"""Launch routes chosen by size, alignment and magnitude, at the edges where each begins.
+
+References: the float64 product on the device, and for values that a route must not change the
+CUDA-core kernel's own result, bit for bit.  Tolerances are the bounds of fp32 accumulation
+(k 2^-24 sum |a||b|, the factor 3 of the other parity tests) plus one rounding of the output."""
+import threading
+
+import numpy as np
+import pytest
+
+import tensilelite_gb300 as tl
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+LAYOUTS = ["NN", "NT", "TN", "TT"]
+MANT = {torch.float32: 23, torch.float16: 10, torch.bfloat16: 7}
+
+
+@pytest.fixture(scope="module")
+def h():
+    handle = tl.Handle()
+    yield handle
+    handle.close()
+
+
+def _mat(g, rows, cols, ld, batch, dtype, dist="normal"):
+    n = batch * ld * cols
+    x = torch.randn(n, device="cuda", generator=g) if dist == "normal" else torch.rand(n, device="cuda", generator=g) * 2 - 1
+    x = x.to(dtype)
+    return x, x.view(batch, cols, ld)[:, :, :rows].transpose(1, 2).double()
+
+
+class Case:
+    def __init__(self, dtype, layout, m, n, k, *, beta=0.0, batch=1, pad=0, seed=0, dist="normal"):
+        self.ta, self.tb = layout[0] == "T", layout[1] == "T"
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        ra, ca = (k, m) if self.ta else (m, k)
+        rb, cb = (n, k) if self.tb else (k, n)
+        self.m, self.n, self.k, self.batch, self.beta = m, n, k, batch, beta
+        self.lda, self.ldb, self.ldc = ra + pad, rb + pad, m + pad
+        self.A, a = _mat(g, ra, ca, self.lda, batch, dtype, dist)
+        self.B, b = _mat(g, rb, cb, self.ldb, batch, dtype, dist)
+        self.C, c = _mat(g, m, n, self.ldc, batch, dtype)
+        self.a, self.b = (a.transpose(1, 2) if self.ta else a), (b.transpose(1, 2) if self.tb else b)
+        self.c, self.dtype = c, dtype
+
+    def run(self, h, kernel="auto", in_place=False, stream=None):
+        D = self.C.clone() if in_place else torch.full_like(self.C, float("nan"))
+        p = tl.Problem.make(self.m, self.n, self.k, dtype=tl.torch_dtype_code(self.dtype), trans_a=self.ta,
+                            trans_b=self.tb, beta=self.beta, lda=self.lda, ldb=self.ldb, ldc=self.ldc, ldd=self.ldc,
+                            batch=self.batch, kernel=kernel)
+        h.gemm(p, D, D if in_place else self.C, self.A, self.B, stream=stream)
+        return D
+
+    def view(self, D):
+        return D.view(self.batch, self.n, self.ldc)[:, :, :self.m].transpose(1, 2)
+
+    def check(self, D):
+        ref = self.a @ self.b + self.beta * self.c
+        bound = 3.0 * self.k * 2.0 ** -24 * (self.a.abs() @ self.b.abs()) + 2.0 ** -MANT[self.dtype] * ref.abs() + \
+            2.0 ** -23 * (self.beta * self.c).abs() + 1e-30
+        got = self.view(D).double()
+        assert torch.isfinite(got).all()
+        assert bool(((got - ref).abs() <= bound).all())
+        return float((got - ref).norm() / ref.norm())
+
+
+# ---- shared pieces of the fp32 split: more than one wave of 256 x 128 tiles (here by batch), sizes at the
+# edges of the 256 x 256 tile and of a k-block ----
+@pytest.mark.parametrize("kernel,most", [("bf16x3", 6e-6), ("bf16x6", 4e-7)])
+@pytest.mark.parametrize("layout,m,n,k,beta", [("NN", 136, 256, 64, 0.0), ("TN", 256, 264, 72, 0.5),
+                                               ("NT", 264, 200, 256, 0.0), ("TT", 520, 520, 200, 0.5)])
+def test_shared_pieces_edges(h, kernel, most, layout, m, n, k, beta):
+    c = Case(torch.float32, layout, m, n, k, beta=beta, batch=40, dist="uniform")
+    D = c.run(h, kernel)
+    h.device_status()
+    ref = c.a @ c.b + beta * c.c
+    err = float((c.view(D).double() - ref).norm() / ref.norm())
+    assert err < most      # 2^-18 class for two pieces, fp32 accumulation for three
+
+
+@pytest.mark.parametrize("m,n,k", [(3000, 2000, 1096), (4096, 2560, 64)])
+def test_shared_pieces_last_wave(h, m, n, k):
+    c = Case(torch.float32, "TN", m, n, k, dist="uniform")
+    assert c.check(c.run(h, "bf16x6")) < 4e-7
+    h.device_status()
+
+
+# ---- plain fp32 left to the library: the tensor cores from 3e8 multiply-adds on ----
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("m,n,k,beta,batch,pad", [(1024, 1024, 320, 0.0, 1, 0), (711, 653, 701, 0.5, 1, 3),
+                                                  (64, 5000, 1003, 0.0, 1, 0), (333, 257, 129, 0.5, 40, 1),
+                                                  (2048, 1000, 64, 0.0, 3, 64)])
+def test_fp32_auto_matches_fp64_as_the_cuda_cores(h, layout, m, n, k, beta, batch, pad):
+    c = Case(torch.float32, layout, m, n, k, beta=beta, batch=batch, pad=pad)
+    l0 = h.launch_count()
+    D = c.run(h)
+    assert h.launch_count() - l0 == 4          # two splits, tensor cores, CUDA cores (returning at once)
+    err = c.check(D)
+    h.device_status()
+    assert err <= max(1.5 * c.check(c.run(h, "simt")), 3e-7)
+    if pad:                                     # the gap between columns is not written
+        assert torch.isnan(D.view(batch, n, c.ldc)[:, :, m:]).all()
+    if beta:
+        assert torch.equal(c.run(h, in_place=True).view(torch.int32).view(batch, n, c.ldc)[:, :, :m],
+                           D.view(torch.int32).view(batch, n, c.ldc)[:, :, :m])
+
+
+@pytest.mark.parametrize("where,value", [("A", float("inf")), ("B", float("-inf")), ("A", float("nan")), ("B", 3e38),
+                                         ("A", 1e-40), ("B", 1e-33), ("A", 1e25)])
+def test_fp32_auto_out_of_range_is_the_cuda_core_result(h, where, value):
+    c = Case(torch.float32, "TN", 720, 700, 640, beta=0.5)
+    (c.A if where == "A" else c.B)[12345] = value
+    if value == 1e25:
+        c.B.mul_(1e13)
+    got, want = c.run(h), c.run(h, "simt")
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    # in place, where a first launch that wrote anything would be seen by the second
+    got, want = c.run(h, in_place=True), c.run(h, "simt", in_place=True)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    h.device_status()
+
+
+def test_fp32_auto_zero_operands(h):
+    c = Case(torch.float32, "NN", 700, 700, 700, beta=0.5)
+    c.A.zero_()
+    assert torch.equal(c.run(h).view(torch.int32), c.run(h, "simt").view(torch.int32))
+
+
+def test_fp32_auto_streams_and_threads_are_independent(h):
+    cases = [Case(torch.float32, "TN", 900 + 64 * i, 1100, 512, seed=i) for i in range(4)]
+    want = [c.run(h) for c in cases]
+    torch.cuda.synchronize()
+    got = [None] * 4
+
+    def work(i):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            for _ in range(6):
+                got[i] = cases[i].run(h, stream=s)
+        s.synchronize()
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    for g, w in zip(got, want):
+        assert torch.equal(g.view(torch.int32), w.view(torch.int32))
+    h.device_status()
+
+
+def test_fp32_auto_under_capture_runs_the_cuda_cores():
+    h = tl.Handle()
+    c = Case(torch.float32, "NN", 800, 800, 800)
+    want = c.run(h, "simt")
+    s = torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        with torch.cuda.graph(g, stream=s):
+            D = c.run(h, stream=s)
+        g.replay()
+    s.synchronize()
+    assert torch.equal(D.view(torch.int32), want.view(torch.int32))
+    h.close()
+
+
+# ---- output path: whole lines through shared memory, or element by element ----
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("layout", ["TN", "NT"])
+@pytest.mark.parametrize("m,n,k,beta,pad", [(256, 256, 64, 0.0, 0), (264, 129, 128, 0.5, 0), (257, 300, 136, 0.5, 7),
+                                            (1000, 600, 520, 0.5, 0), (8, 1, 64, 0.0, 8), (72, 513, 64, 0.5, 8)])
+def test_output_lines_and_elements(h, dtype, layout, m, n, k, beta, pad):
+    c = Case(dtype, layout, m, n, k, beta=beta, batch=2)
+    # padded leading dimensions of C and D only: operands stay 16-byte aligned
+    if c.ta is False and m % 8:
+        c = Case(dtype, "TN", m, n, k, beta=beta, batch=2)
+    D = c.run(h)
+    c.check(D)
+    if beta:
+        assert torch.equal(c.run(h, in_place=True).view(torch.int16), D.view(torch.int16))
+    if pad:
+        ld = m + pad
+        W = torch.full((2 * n * ld,), float("nan"), dtype=dtype, device="cuda")
+        Cp = torch.zeros(2, n, ld, dtype=dtype, device="cuda")
+        Cp[:, :, :m] = c.C.view(2, n, m)
+        p = tl.Problem.make(m, n, k, dtype=tl.torch_dtype_code(dtype), trans_a=c.ta, trans_b=c.tb, beta=beta, lda=c.lda,
+                            ldb=c.ldb, ldc=ld, ldd=ld, batch=2)
+        h.gemm(p, W, Cp, c.A, c.B)
+        W = W.view(2, n, ld)
+        assert torch.equal(W[:, :, :m].contiguous().view(torch.int16), D.view(2, n, m).view(torch.int16))
+        assert torch.isnan(W[:, :, m:]).all()
+    h.device_status()
+
+
+# ---- quantisation: vector and element paths, sources and destinations off the 16-byte grid ----
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,so,do", [(1, 0, 0), (15, 1, 0), (16, 0, 0), (17, 0, 1), (4097, 3, 3), (100003, 1, 1),
+                                     (1 << 20, 0, 0), ((1 << 20) + 5, 0, 8)])
+def test_quantize_alignments(h, dtype, n, so, do):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    src = (torch.randn(n + so, device="cuda", generator=g) * 3).to(dtype)[so:]
+    buf = torch.full((n + do + 32,), 0xAA, dtype=torch.uint8, device="cuda")
+    scale, amax = torch.zeros(1, device="cuda"), torch.full((1,), 7e9, device="cuda")
+    h.quantize_fp8(src, n, buf[do:], scale, amax, src_dtype=tl.torch_dtype_code(dtype))
+    a = src.float().abs().max()
+    want = (src.float() * (torch.tensor(448.0, device="cuda") / a)).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+    assert float(amax) == float(a) and np.float32(float(scale)) == np.float32(float(a)) / np.float32(448.0)
+    assert torch.equal(buf[do:do + n], want)
+    assert bool((buf[do + n:] == 0xAA).all()) and bool((buf[:do] == 0xAA).all())
