@@ -1373,8 +1373,8 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 }
                 const int n2 = j.n0 + row;
                 const bool row_ok2 = n2 < j.N;
-                const int64_t d2 = static_cast<int64_t>(j.b) * p.stride_d + static_cast<int64_t>(n2) * j.ldd;
-                const int64_t c2 = static_cast<int64_t>(j.b) * p.stride_c + static_cast<int64_t>(n2) * j.ldc;
+                const int64_t d2 = static_cast<int64_t>(j.b) * p.stride_d + static_cast<int64_t>(n2) * (j.out_t ? 1 : j.ldd);
+                const int64_t c2 = static_cast<int64_t>(j.b) * p.stride_c + static_cast<int64_t>(n2) * (j.out_t ? 1 : j.ldc);
                 // QW columns at a time, the sums rotated through the registers: one copy of the code (and
                 // no C loads hoisted into registers the sums occupy)
                 if (j.nsplit == 1) {

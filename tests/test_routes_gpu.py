@@ -87,6 +87,19 @@ def test_shared_pieces_last_wave(h, m, n, k):
     h.device_status()
 
 
+# ---- promoted chains of an NN problem that runs as its transposed view ----
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k,mt1", [(136, 72, 2048, 128), (520, 392, 2056, 256), (256, 512, 2112, 256)])
+def test_promoted_chains_of_the_transposed_view(h, dtype, m, n, k, mt1):
+    c = Case(dtype, "NN", m, n, k)
+    p = tl.Problem.make(m, n, k, dtype=tl.torch_dtype_code(dtype), lda=c.lda, ldb=c.ldb, ldc=c.ldc, ldd=c.ldc)
+    s = tl.Solution(kernel=tl.KERNEL_TCGEN05, macro_tile0=128, macro_tile1=mt1, stages=4, split_k=1, promote_k=256)
+    D = torch.full_like(c.C, float("nan"))
+    h.gemm(p, D, None, c.A, c.B, solution=s)
+    c.check(D)
+    h.device_status()
+
+
 # ---- plain fp32 left to the library: the tensor cores from 3e8 multiply-adds on ----
 @pytest.mark.parametrize("layout", LAYOUTS)
 @pytest.mark.parametrize("m,n,k,beta,batch,pad", [(1024, 1024, 320, 0.0, 1, 0), (711, 653, 701, 0.5, 1, 3),
