@@ -925,11 +925,12 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
 
 // ---- plain fp32 on the tensor cores ---------------------------------------------------------------
 // A large fp32 GEMM left to the library (kernel AUTO, no solution, none tuned) runs as the six products
-// of three bf16 pieces per operand, whose error against 64 bits is below the CUDA-core kernel's at every
-// size and layout measured (relative 2-norm, 4096^3: 1.6e-7 against 1.15e-6; 512 x 4096 x 1024: 1.9e-7
-// against 2.1e-7) and which takes a fifth of its time (4096^3 TN: 490 us against 2770; 1024^3: 28 against
-// 104).  Below kFp32TcWork multiply-adds the split pass and the extra launches cost more than that
-// gives (480 x 512 x 512: 13 us on the CUDA cores).
+// of three bf16 pieces per operand, whose error against 64 bits is below the CUDA-core kernel's (normal
+// values, relative 2-norm, 4096^3: 1.6e-7 against 1.15e-6; 1024^3: 0.9e-7 against 2.1e-7; 672^3: 0.9e-7
+// against 1.75e-7) and which takes a fifth of its time (4096^3 TN: 490 us against 2770; 1024^3: 33 against
+// 103).  Below kFp32TcWork multiply-adds, twice that where k is one or two k-blocks, the split pass and the
+// extra launches cost more than that gives (672^3: 29 us against 38; 512 x 1024 x 600: 28.6 either way;
+// 2048 x 2048 x 80: 24 against 22; 480 x 512 x 512: 13 on the CUDA cores).
 //
 // The pieces stand for the operands only within a range of magnitudes (split_range_ok), which is known
 // on the device once the split passes have run: infinities, NaN, numbers near fp32's limits.  So the
@@ -940,12 +941,16 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
 // Each call has its own scratch, allocated and freed in stream order.  While a stream is being
 // captured, or where the scratch cannot be had, the CUDA-core kernel runs as before.
 constexpr double kFp32TcWork = 3.0e8;
+// The tensor core drops bits below its accumulator's last one, so a sum of many terms of one sign comes
+// out low: 700^3 of uniform [0, 1), chains of 256: 2.6e-7, CUDA cores 0.7e-7.  Chains of one k-block
+// keep fp32 results at or below the CUDA cores' error.
+constexpr int kFp32Chain = 64;
 
 bool fp32_tc_wanted(const tl_gemm_problem& p)
 {
     return p.kernel == TL_KERNEL_AUTO && p.dtype_a == TL_DTYPE_FP32 && p.dtype_d == TL_DTYPE_FP32 && p.m > 0 && p.n > 0 &&
            p.k > 0 && static_cast<double>(p.m) * static_cast<double>(p.n) * static_cast<double>(p.k) *
-           static_cast<double>(p.batch) >= kFp32TcWork && p.m >= 64 && p.n >= 64 && p.k >= 64 &&
+           static_cast<double>(p.batch) >= (p.k <= 128 ? 2.0 : 1.0) * kFp32TcWork && p.m >= 64 && p.n >= 64 && p.k >= 64 &&
            p.alpha * scale_of(p.scale_a) * scale_of(p.scale_b) != 0.0f;
 }
 
@@ -981,6 +986,7 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
     T.kernel = TL_KERNEL_BF16X6;
     T.p.kernel = TL_KERNEL_BF16X6;
     tc_heuristic(h, T.p, TL_KERNEL_BF16X6, &T.s);
+    T.s.promote_k = kFp32Chain;
     if (check_tc_solution(h, T.p, T.s) != TL_SUCCESS) return TL_SUCCESS;
     const Scratch w = scratch_of(h, T);
     const size_t head = align_up(sizeof(SplitRange) + w.counters * sizeof(int), 256);

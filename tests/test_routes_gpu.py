@@ -104,7 +104,7 @@ def test_promoted_chains_of_the_transposed_view(h, dtype, m, n, k, mt1):
 @pytest.mark.parametrize("layout", LAYOUTS)
 @pytest.mark.parametrize("m,n,k,beta,batch,pad", [(1024, 1024, 320, 0.0, 1, 0), (711, 653, 701, 0.5, 1, 3),
                                                   (64, 5000, 1003, 0.0, 1, 0), (333, 257, 129, 0.5, 40, 1),
-                                                  (2048, 1000, 64, 0.0, 3, 64)])
+                                                  (2048, 1000, 64, 0.0, 5, 64)])
 def test_fp32_auto_matches_fp64_as_the_cuda_cores(h, layout, m, n, k, beta, batch, pad):
     c = Case(torch.float32, layout, m, n, k, beta=beta, batch=batch, pad=pad)
     l0 = h.launch_count()
