@@ -438,6 +438,58 @@ static cudaError_t launch_dependent(void (*kern)(KArgs...), int grid, int thread
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// ---- padded copies --------------------------------------------------------------------------------
+// Bound by memory: 2 B read and 2 B written per element.  The source's columns start on any even
+// address, so a lane reads the aligned words that hold its eight elements, shifts them into place if
+// they start in the middle of a word, and writes one 16-byte vector.  A warp takes 256 rows of a column
+// at a time: one index division per warp and 512 bytes.
+struct PadArgs {
+    PadOperand op[2];
+    int64_t chunks[2], tasks[2];          // 256-row chunks per column; chunks of the operand (0: not there)
+};
+
+__global__ void __launch_bounds__(256) pad_kernel(const __grid_constant__ PadArgs args)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
+    const int64_t total = args.tasks[0] + args.tasks[1];
+    for (int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; t < total; t += warps) {
+        const int w = t >= args.tasks[0];
+        const PadOperand& o = args.op[w];
+        const int64_t i = w ? t - args.tasks[0] : t;
+        int64_t col, b = 0;
+        if (i < (int64_t(1) << 31)) col = static_cast<uint32_t>(i) / static_cast<uint32_t>(args.chunks[w]);
+        else col = i / args.chunks[w];
+        const int64_t r = (i - col * args.chunks[w]) * 256 + lane * 8;
+        if (o.batch > 1) {
+            b = col / o.cols;
+            col -= b * o.cols;
+        }
+        if (r >= o.rows) continue;
+        const uint16_t* src = o.src + b * o.batch_stride + col * o.ld + r;
+        uint32_t v[4];
+        if (o.rows - r >= 8) {
+            const bool odd = (reinterpret_cast<uintptr_t>(src) & 2) != 0;
+            const uint32_t* words = reinterpret_cast<const uint32_t*>(src - (odd ? 1 : 0));
+            uint32_t q[5];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) q[e] = __ldg(words + e);
+            q[4] = odd ? __ldg(words + 4) : 0u;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = odd ? __funnelshift_r(q[e], q[e + 1], 16) : q[e];
+        } else {
+            const int left = static_cast<int>(o.rows - r);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t lo = 2 * e < left ? src[2 * e] : 0u;
+                const uint32_t hi = 2 * e + 1 < left ? src[2 * e + 1] : 0u;
+                v[e] = lo | (hi << 16);
+            }
+        }
+        *reinterpret_cast<uint4*>(o.dst + b * o.p_batch_stride + col * o.pld + r) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+}
+
 tl_status aux_split_bf16(const SplitOperand* ops, int count, int pieces, SplitRange* range, cudaStream_t s,
                          int64_t* launches)
 {
@@ -461,6 +513,21 @@ tl_status aux_split_bf16(const SplitOperand* ops, int count, int pieces, SplitRa
         first = false;
     }
     return TL_SUCCESS;
+}
+
+tl_status aux_pad16(const PadOperand* ops, int count, cudaStream_t s, int64_t* launches)
+{
+    PadArgs args;
+    memset(&args, 0, sizeof(args));
+    for (int i = 0; i < count; ++i) {
+        args.op[i] = ops[i];
+        args.chunks[i] = (ops[i].rows + 255) / 256;
+        args.tasks[i] = args.chunks[i] * ops[i].cols * ops[i].batch;
+    }
+    const int64_t total = args.tasks[0] + args.tasks[1];
+    if (total == 0) return TL_SUCCESS;
+    pad_kernel<<<grid_for(total * 32, 1, 256), 256, 0, s>>>(args);
+    return check_launch("pad_kernel", launches);
 }
 
 template <typename T>

@@ -68,7 +68,7 @@ struct tl_handle {
     // heuristic picks by problem shape (the cost model takes 1.5 to 7 us a problem); at most kMaxPlans
     std::unordered_map<tl::PlanKey, tl::Plan, tl::PlanKeyHash> plans;
     std::mutex mu;                 // tuned, plans, pool
-    // stream-ordered scratch of fp32 GEMMs that run on the tensor cores (gemm_fp32_tc): each call has its
+    // stream-ordered scratch of the GEMMs that re-lay their operands (gemm_fp32_tc, gemm_pad16): each call has its
     // own, so that calls on different streams and threads stay independent.  At most kPoolKeep bytes
     // stay with the pool between synchronisations.
     cudaMemPool_t pool = nullptr;
@@ -954,7 +954,7 @@ bool fp32_tc_wanted(const tl_gemm_problem& p)
            p.alpha * scale_of(p.scale_a) * scale_of(p.scale_b) != 0.0f;
 }
 
-cudaMemPool_t fp32_pool(tl_handle* h)
+cudaMemPool_t call_pool(tl_handle* h)
 {
     std::lock_guard<std::mutex> g(h->mu);
     if (!h->pool && !h->pool_failed) {
@@ -980,7 +980,7 @@ cudaMemPool_t fp32_pool(tl_handle* h)
 tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done)
 {
     *done = false;
-    cudaMemPool_t pool = fp32_pool(h);
+    cudaMemPool_t pool = call_pool(h);
     if (!pool) return TL_SUCCESS;
     Prepared T = P;
     T.kernel = TL_KERNEL_BF16X6;
@@ -1012,6 +1012,88 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
     }
     e = cudaFreeAsync(mem, s);
     if (st == TL_SUCCESS && e != cudaSuccess) st = cuda_fail(e, "cudaFreeAsync(fp32 scratch)");
+    return st;
+}
+
+// ---- 16-bit operands that TMA cannot address --------------------------------------------------------
+// A large fp16 or bf16 GEMM (16-bit output) whose operands start or stride off 16-byte boundaries, left
+// to the library (kernel AUTO, no solution, none tuned), runs on aligned copies of those operands: one
+// pass over memory instead of a CUDA-core kernel at a thirtieth of the tensor cores' rate (2047^3: 556
+// -> 70 us, 65 x 1025 x 3001: 122 -> 26).  Its chains are promoted every 256 k into fp32 registers: the
+// error against 64 bits stays that of the output's rounding (1.6566e-3 for bf16 by either kernel; an
+// fp32 output would show the chains, and keeps the CUDA cores).  Below kPad16Work multiply-adds the
+// copies and the scratch cost more than that gives (501 x 601 x 501: 25 us against 23.5).  Scratch,
+// captures and a scratch that cannot be had: as for fp32 above.
+constexpr double kPad16Work = 2.0e8;
+
+bool pad16_wanted(const tl_gemm_problem& p, const void* A, const void* B)
+{
+    const bool half = p.dtype_a == TL_DTYPE_FP16 || p.dtype_a == TL_DTYPE_BF16;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B);
+    return p.kernel == TL_KERNEL_AUTO && half && (p.dtype_d == TL_DTYPE_FP16 || p.dtype_d == TL_DTYPE_BF16) && at % 2 == 0 && p.m >= 64 && p.n >= 64 && p.k >= 64 &&
+           static_cast<double>(p.m) * static_cast<double>(p.n) * static_cast<double>(p.k) *
+           static_cast<double>(p.batch) >= kPad16Work && p.alpha * scale_of(p.scale_a) * scale_of(p.scale_b) != 0.0f;
+}
+
+// P is prepared for the CUDA-core kernel.  *done reports whether the GEMM was enqueued here.
+tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done)
+{
+    *done = false;
+    cudaMemPool_t pool = call_pool(h);
+    if (!pool) return TL_SUCCESS;
+    Prepared T = P;
+    tl_gemm_problem& p = T.p;
+    p.kernel = TL_KERNEL_TCGEN05;
+    PadOperand ops[2];
+    size_t bytes[2] = {0, 0};
+    int count = 0;
+    const auto copy = [&](const void* X, int64_t rows, int64_t cols, int64_t* ld, int64_t* stride) {
+        if (aligned16(X) && *ld % 8 == 0 && (p.batch == 1 || *stride % 8 == 0)) return -1;
+        PadOperand& o = ops[count];
+        o = {static_cast<const uint16_t*>(X), rows, cols, *ld, p.batch, *stride, nullptr, 0, 0};
+        o.pld = *ld = static_cast<int64_t>(align_up(static_cast<size_t>(rows), 64));
+        o.p_batch_stride = *stride = o.pld * cols;
+        bytes[count] = align_up(static_cast<size_t>(o.p_batch_stride) * p.batch * 2, 256);
+        return count++;
+    };
+    const int ia = copy(P.A, p.trans_a ? p.k : p.m, p.trans_a ? p.m : p.k, &p.lda, &p.stride_a);
+    const int ib = copy(P.B, p.trans_b ? p.n : p.k, p.trans_b ? p.k : p.n, &p.ldb, &p.stride_b);
+    if (count == 0) return TL_SUCCESS;
+    // the tile of the promoted products (tc_heuristic's), for the problem as the launch views it
+    T.kernel = TL_KERNEL_TCGEN05;
+    T.tview = tc_nn_view(p, T.kernel);
+    tc_heuristic(h, T.tview ? nn_view(p) : p, TL_KERNEL_BF16X6, &T.s);
+    if (T.tview && !view_solution_ok(T.s)) {
+        T.tview = false;
+        tc_heuristic(h, p, TL_KERNEL_BF16X6, &T.s);
+    }
+    T.s.kernel = T.kernel;
+    if (T.tview) p = nn_view(p);
+    if (check_tc_solution(h, p, T.s) != TL_SUCCESS) return TL_SUCCESS;
+    const Scratch w = scratch_of(h, T);
+    const size_t head = align_up(w.counters * sizeof(int), 256);
+    void* mem = nullptr;
+    if (cudaMallocFromPoolAsync(&mem, head + align_up(w.bytes, 256) + bytes[0] + bytes[1], pool, s) != cudaSuccess) {
+        cudaGetLastError();
+        return TL_SUCCESS;
+    }
+    *done = true;
+    char* base = static_cast<char*>(mem);
+    T.counters = reinterpret_cast<int*>(base);
+    T.counters_len = w.counters;
+    place(T, w, base + head);
+    base += head + align_up(w.bytes, 256);
+    for (int i = 0; i < count; ++i) ops[i].dst = reinterpret_cast<uint16_t*>(base + (i ? bytes[0] : 0));
+    if (ia >= 0) T.A = ops[ia].dst;
+    if (ib >= 0) T.B = ops[ib].dst;
+    if (T.tview) std::swap(T.A, T.B);
+    tl_status st = TL_SUCCESS;
+    cudaError_t e = cudaSuccess;
+    if (w.counters && (e = cudaMemsetAsync(mem, 0, head, s)) != cudaSuccess) st = cuda_fail(e, "cudaMemsetAsync(tile counters)");
+    if (st == TL_SUCCESS) st = aux_pad16(ops, count, s, &h->launches);
+    if (st == TL_SUCCESS) st = enqueue(h, T, s);
+    e = cudaFreeAsync(mem, s);
+    if (st == TL_SUCCESS && e != cudaSuccess) st = cuda_fail(e, "cudaFreeAsync(padded operands)");
     return st;
 }
 
@@ -1356,6 +1438,11 @@ TL_API tl_status tl_gemm(tl_handle* h, const tl_gemm_problem* p, const tl_gemm_s
     if (!s && !capturing && P.kernel == TL_KERNEL_SIMT && !P.tuned && fp32_tc_wanted(*p)) {
         bool done = false;
         st = gemm_fp32_tc(h, P, S(stream), &done);
+        if (done) return st;
+    }
+    if (!s && !capturing && P.kernel == TL_KERNEL_SIMT && !P.tuned && pad16_wanted(*p, A, B)) {
+        bool done = false;
+        st = gemm_pad16(h, P, S(stream), &done);
         if (done) return st;
     }
     return enqueue(h, P, S(stream));

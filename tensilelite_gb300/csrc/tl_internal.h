@@ -210,6 +210,15 @@ struct SplitOperand {
 // `range`, if given, receives the operands' magnitudes (zeroed by the caller).
 tl_status aux_split_bf16(const SplitOperand* ops, int count, int pieces, SplitRange* range, cudaStream_t s,
                          int64_t* launches);
+// 16-bit matrices copied to columns that start on 128-byte lines (pld a multiple of 64 elements; the
+// elements between rows and the next multiple of eight are zeroed).  One launch for all of them.
+struct PadOperand {
+    const uint16_t* src;
+    int64_t rows, cols, ld, batch, batch_stride;
+    uint16_t* dst;
+    int64_t pld, p_batch_stride;
+};
+tl_status aux_pad16(const PadOperand* ops, int count, cudaStream_t s, int64_t* launches);
 // Per-tensor E4M3 quantisation: *amax_dev = max |x|, dst = e4m3(x * 448 / amax), *scale_out_dev = amax / 448.
 tl_status aux_quantize_e4m3(int src_dtype, const void* src, int64_t n, float* amax_dev, uint8_t* dst,
                             float* scale_out_dev, cudaStream_t s, int64_t* launches);

@@ -177,6 +177,71 @@ def test_fp32_auto_under_capture_runs_the_cuda_cores():
     h.close()
 
 
+# ---- 16-bit operands off 16-byte boundaries: aligned copies and the tensor cores from 2e8 on ----
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,n,k,beta,batch,pad", [(1001, 515, 433, 0.5, 1, 0), (520, 640, 678, 0.0, 1, 3),
+                                                  (64, 1601, 2051, 0.0, 1, 0), (130, 129, 337, 0.5, 40, 1),
+                                                  (777, 65, 4099, 0.0, 1, 0), (2040, 1999, 2049, 0.0, 1, 1)])
+def test_unaligned_half_matches_fp64_as_the_cuda_cores(h, dtype, layout, m, n, k, beta, batch, pad):
+    c = Case(dtype, layout, m, n, k, beta=beta, batch=batch, pad=pad)
+    assert any(ld % 8 for ld in (c.lda, c.ldb))
+    l0 = h.launch_count()
+    D = c.run(h)
+    assert h.launch_count() - l0 == 2          # copies, tensor cores
+    err = c.check(D)
+    h.device_status()
+    assert err <= 1.02 * c.check(c.run(h, "simt"))      # both are one output rounding away
+    if pad:
+        assert torch.isnan(D.view(batch, n, c.ldc)[:, :, m:]).all()
+    if beta:
+        assert torch.equal(c.run(h, in_place=True).view(torch.int16).view(batch, n, c.ldc)[:, :, :m],
+                           D.view(torch.int16).view(batch, n, c.ldc)[:, :, :m])
+
+
+@pytest.mark.parametrize("off_a,off_b", [(1, 0), (0, 3), (2, 5), (7, 4)])
+def test_unaligned_half_bases(h, off_a, off_b):
+    c = Case(torch.float16, "TN", 640, 768, 512)
+    want = c.run(h, "tcgen05")
+    for name, off in (("A", off_a), ("B", off_b)):
+        x = getattr(c, name)
+        y = torch.full((x.numel() + off,), float("nan"), device="cuda", dtype=x.dtype)[off:]
+        y.copy_(x)
+        setattr(c, name, y)
+    D = c.run(h)
+    c.check(D)
+    assert float((D.double() - want.double()).norm() / want.double().norm()) < 2e-4
+    h.device_status()
+
+
+def test_unaligned_half_capture_and_streams():
+    h = tl.Handle()
+    c = Case(torch.bfloat16, "TN", 801, 700, 515, beta=0.5)
+    want = c.run(h, "simt")
+    D = torch.empty_like(want)
+    p = tl.Problem.make(c.m, c.n, c.k, dtype="bf16", trans_a=True, beta=0.5, lda=c.lda, ldb=c.ldb, ldc=c.ldc, ldd=c.ldc)
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=s):
+        h.gemm(p, D, c.C, c.A, c.B, stream=s)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(D.view(torch.int16), want.view(torch.int16))      # captured: the CUDA-core kernel
+    cases = [Case(torch.bfloat16, "NN", 301 + 64 * i, 1100, 1011, seed=i) for i in range(4)]      # split k
+    alone = [x.run(h) for x in cases]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in cases]
+    for _ in range(5):
+        got = []
+        for x, st in zip(cases, streams):
+            with torch.cuda.stream(st):
+                got.append(x.run(h, stream=st))
+        torch.cuda.synchronize()
+        for a, b in zip(got, alone):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+    h.device_status()
+    h.close()
+
+
 # ---- output path: whole lines through shared memory, or element by element ----
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("layout", ["TN", "NT"])
