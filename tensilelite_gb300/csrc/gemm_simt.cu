@@ -23,7 +23,7 @@
 //          k-slab (8 x 8 outputs per thread and group); the groups' partial tiles are summed in
 //          group order through shared memory at the end.  For problems whose 128 x 128 tiles would
 //          leave SMs idle (the reference's 480 x 512 x 512 case: 16 large tiles, 128 small ones),
-//          one CTA per SM, slabs loaded two ahead.
+//          one CTA per SM, slabs loaded two ahead, k-contiguous operands read by whole lines.
 // k-slabs are double-buffered in shared memory and prefetched into registers, with 4-element vector
 // loads along whichever dimension is contiguous in memory; edge tiles are zero-filled on load and
 // masked on store.  Results are deterministic (fixed summation order).
@@ -95,7 +95,7 @@ struct SimtParams {
 
 // Tile shape: BM x BN outputs, TM x TN per thread and k-group, KG k-groups, BKG k per group and slab,
 // PD slabs loaded ahead into registers (1: the next slab's loads overlap one slab of FMAs; 2: two).
-template <int BM_, int BN_, int TM_, int TN_, int KG_, int BKG_, int MINB_, int PD_>
+template <int BM_, int BN_, int TM_, int TN_, int KG_, int BKG_, int MINB_, int PD_, bool LINES_>
 struct Cfg {
     static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_, KG = KG_, BKG = BKG_, MINB = MINB_, PD = PD_;
     static constexpr int TX = BM / TM;           // threads along m in a group
@@ -108,15 +108,27 @@ struct Cfg {
     static constexpr int A_CHUNKS = BK * BM / 4 / THREADS;   // 4-element loads per thread and slab
     static constexpr int B_CHUNKS = BK * BN / 4 / THREADS;
     static constexpr int SMEM_FLOATS = 2 * BK * BM + 2 * BK * BN;
+    // LINES: a k-contiguous operand is read by eight lanes to a 128-byte line, and float4 i of row k sits
+    // at i ^ (k / 4 % 8) in shared memory, so that those lanes' transposed stores hit different banks.
+    // With a lane per row the loads touched a line each and took the shared-memory pipe's time
+    // (480 x 512 x 512 NN 13.3 -> 12.5 us, TN 14.7 -> 12.1; 65 x 1000 x 333 TN 13.0 -> 9.9).  Where neither operand is
+    // k-contiguous (NT) the swizzle only costs (12.1 -> 12.5).
+    static constexpr bool LINES = LINES_;
+    static_assert(!LINES || (BK % 32 == 0 && BM % 32 == 0 && BN % 32 == 0), "eight lanes of 4 k, eight float4 of a row");
+    __device__ static constexpr int swz(int k) { return LINES ? (k >> 2) & 7 : 0; }
+    // 4 consecutive k of row r of a k-contiguous operand with R rows: chunk idx of the slab
+    __device__ static constexpr int chunk_row(int idx, int R) { return LINES ? (idx >> 3) % R : idx % R; }
+    __device__ static constexpr int chunk_k(int idx, int R) { return LINES ? ((idx & 7) + 8 * ((idx >> 3) / R)) * 4 : (idx / R) * 4; }
     static constexpr int RED_FLOATS = KG > 1 ? KG * BM * BN : 0;
     static constexpr size_t SMEM_BYTES = sizeof(float) * (SMEM_FLOATS > RED_FLOATS ? SMEM_FLOATS : RED_FLOATS);
     static_assert(TM % 4 == 0 && TN % 4 == 0, "per-thread tiles are strips of 4");
     static_assert(A_CHUNKS * THREADS * 4 == BK * BM && B_CHUNKS * THREADS * 4 == BK * BN, "whole slabs");
 };
-using CfgLarge = Cfg<128, 128, 16, 8, 1, 8, 2, 1>;
+using CfgLarge = Cfg<128, 128, 16, 8, 1, 8, 2, 1, false>;
 // one CTA per SM (it is used when tiles are fewer than SMs): up to 255 registers, 64-deep k-slabs,
 // loads two slabs ahead (eight warps per SM cannot hide a DRAM round trip behind one slab)
-using CfgSmall = Cfg<64, 32, 8, 8, 8, 8, 1, 2>;
+using CfgSmall = Cfg<64, 32, 8, 8, 8, 8, 1, 2, true>;
+using CfgSmallRows = Cfg<64, 32, 8, 8, 8, 8, 1, 2, false>;
 
 constexpr int kRasterGroup = 16;   // m-tiles per raster group (tiles running together share B columns)
 
@@ -173,7 +185,7 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB) simt_gemm_kernel(const Si
                     }
                 }
             } else {                         // A[k + m*lda]: 4 consecutive k of one m
-                const int m = m_blk + idx % BM, k = k0 + (idx / BM) * 4;
+                const int m = m_blk + G::chunk_row(idx, BM), k = k0 + G::chunk_k(idx, BM);
                 const TA* src = A + k + static_cast<int64_t>(m) * p.lda;
                 if (m < p.M) {
                     if (p.vec_a && k + 3 < p.K) v = load4<TA>(src);
@@ -204,7 +216,7 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB) simt_gemm_kernel(const Si
                     }
                 }
             } else {                         // B[k + n*ldb]: 4 consecutive k of one n
-                const int n = n_blk + idx % BN, k = k0 + (idx / BN) * 4;
+                const int n = n_blk + G::chunk_row(idx, BN), k = k0 + G::chunk_k(idx, BN);
                 const TA* src = B + k + static_cast<int64_t>(n) * p.ldb;
                 if (n < p.N) {
                     if (p.vec_b && k + 3 < p.K) v = load4<TA>(src);
@@ -228,9 +240,9 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB) simt_gemm_kernel(const Si
             const int idx = tid + c * G::THREADS;
             if (!p.trans_a) {
                 const int m = (idx % (BM / 4)) * 4, k = idx / (BM / 4);
-                *reinterpret_cast<float4*>(as + k * BM + m) = ra[r][c];
+                *reinterpret_cast<float4*>(as + k * BM + (m ^ (4 * G::swz(k)))) = ra[r][c];
             } else {
-                const int m = idx % BM, k = (idx / BM) * 4;
+                const int k = G::chunk_k(idx, BM), m = G::chunk_row(idx, BM) ^ (4 * G::swz(k));
                 as[(k + 0) * BM + m] = ra[r][c].x;
                 as[(k + 1) * BM + m] = ra[r][c].y;
                 as[(k + 2) * BM + m] = ra[r][c].z;
@@ -242,9 +254,9 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB) simt_gemm_kernel(const Si
             const int idx = tid + c * G::THREADS;
             if (p.trans_b) {
                 const int n = (idx % (BN / 4)) * 4, k = idx / (BN / 4);
-                *reinterpret_cast<float4*>(bs + k * BN + n) = rb[r][c];
+                *reinterpret_cast<float4*>(bs + k * BN + (n ^ (4 * G::swz(k)))) = rb[r][c];
             } else {
-                const int n = idx % BN, k = (idx / BN) * 4;
+                const int k = G::chunk_k(idx, BN), n = G::chunk_row(idx, BN) ^ (4 * G::swz(k));
                 const float4 q = rb[r][c];
                 bs[(k + 0) * BN + n] = q.x;
                 bs[(k + 1) * BN + n] = q.y;
@@ -268,15 +280,16 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB) simt_gemm_kernel(const Si
 #pragma unroll
         for (int kk = 0; kk < G::BKG; ++kk) {
             float2 a[TM / 2], bd[TN];
+            const int sw = 4 * G::swz(grp * G::BKG + kk);
 #pragma unroll
             for (int st = 0; st < TM / 4; ++st) {
-                const float4 v = *reinterpret_cast<const float4*>(as + kk * BM + st * G::SWM + tx * 4);
+                const float4 v = *reinterpret_cast<const float4*>(as + kk * BM + ((st * G::SWM + tx * 4) ^ sw));
                 a[2 * st] = make_float2(v.x, v.y);
                 a[2 * st + 1] = make_float2(v.z, v.w);
             }
 #pragma unroll
             for (int st = 0; st < TN / 4; ++st) {
-                const float4 v = *reinterpret_cast<const float4*>(bs + kk * BN + st * G::SWN + ty * 4);
+                const float4 v = *reinterpret_cast<const float4*>(bs + kk * BN + ((st * G::SWN + ty * 4) ^ sw));
                 bd[4 * st + 0] = make_float2(v.x, v.x);
                 bd[4 * st + 1] = make_float2(v.y, v.y);
                 bd[4 * st + 2] = make_float2(v.z, v.z);
@@ -421,7 +434,13 @@ tl_status launch(const SimtLaunch& L, cudaStream_t s)
     }();
     // 128 x 128 tiles, or the k-grouped 64 x 32 tiles when the large ones would leave SMs idle
     const int64_t big_tiles = ((L.M + 127) / 128) * ((L.N + 127) / 128) * L.batch;
-    if (big_tiles < sms) return launch_cfg<TA, TD, CfgSmall>(p, L.M, L.N, L.batch, s);
+    if (big_tiles < sms) {
+        // by lines where an operand is k-contiguous; 16-bit A^T comes here mostly off 16-byte boundaries, read
+        // element by element, and is no faster for it (301 x 501 x 401 TN 19.7 us by rows, 19.8 by lines)
+        const bool lines = L.trans_a ? sizeof(TA) == 4 : !L.trans_b;
+        return lines ? launch_cfg<TA, TD, CfgSmall>(p, L.M, L.N, L.batch, s)
+                     : launch_cfg<TA, TD, CfgSmallRows>(p, L.M, L.N, L.batch, s);
+    }
     return launch_cfg<TA, TD, CfgLarge>(p, L.M, L.N, L.batch, s);
 }
 

@@ -242,6 +242,19 @@ def test_unaligned_half_capture_and_streams():
     h.close()
 
 
+# ---- CUDA-core kernel, small tiles: slabs read by lines, at the edges of the 64 x 32 tile and the slab ----
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("m,n,k,beta,pad", [(64, 32, 64, 0.0, 0), (65, 33, 67, 0.5, 0), (63, 31, 1, 0.0, 4), (1, 100, 130, 0.5, 3),
+                                            (200, 96, 316, 0.0, 4)])
+def test_cuda_core_small_tiles(h, dtype, layout, m, n, k, beta, pad):
+    c = Case(dtype, layout, m, n, k, beta=beta, batch=2, pad=pad)
+    D = c.run(h, "simt")
+    c.check(D)
+    if pad:
+        assert torch.isnan(D.view(2, n, c.ldc)[:, :, m:]).all()
+
+
 # ---- output path: whole lines through shared memory, or element by element ----
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("layout", ["TN", "NT"])
