@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
     const uint32_t bmc = static_cast<uint32_t>(p.bm) / CG;            // m-side rows staged by this CTA
     const uint32_t tileN_bytes = kTcTileN * kTcRowBytes;
     const uint32_t stage_bytes = tileN_bytes + bmc * kTcRowBytes;
-    // output staging for TMA stores: epi_bufs x 4 epilogue warps x 32 rows x 128 bytes, 1024-byte aligned
+    // output staging: per epilogue warp 32 rows x 128 bytes (C in, D out), 1024-byte aligned
     uint8_t* epi_stage = smem + static_cast<size_t>(p.stages) * stage_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(epi_stage + static_cast<size_t>(p.epi_bufs) * kTcEpiStageBytes);
     uint64_t* empty = full + kTcMaxStages;

@@ -353,10 +353,12 @@ double tc_cost(const tl_handle* h, const tl_gemm_problem& p, const tl_gemm_solut
                     : (cg == 4 && h->host_clusters4 > 0 ? h->host_clusters4 : h->sm_count / cg));
     const int64_t split = std::max<int64_t>(1, s.split_k);
     const int64_t units = tiles * split;
-    // per k-block and CTA: the MMA issue time (4 MMAs; about 500 clocks for any width up to 128
-    // columns, 716 for 256) plus a cost per staged operand byte that grows with the number of SMs
-    // loading at once -- fitted to the per-k-block times measured on GB300 for one SM / a pair,
-    // 128 / 256 columns (690-1000 clocks with every SM busy)
+    // per k-block and CTA: an issue time (500 clocks for any width up to 128 columns, 716 for 256) plus
+    // a cost per staged operand byte that grows with the number of SMs loading at once.  The constants were
+    // fitted when the issue loop bounded every width; since it issues from one lane the tensor pipe's own
+    // times are 196 / 256 / 384 / 512 clocks for 64 / 128 / 192 / 256 columns.  They still rank the tiles
+    // as sweeps do (bf16 480 x 1024 x 4096: the pick, 128 x 128 at split-k 4, 12.1 us, is the best of 40
+    // tiles; fp16 1000 x 600 x 520 x 24: 256 x 256 24.7, the others 27.9 to 42.7).
     const double mma_kb = std::max(716.0 * bm / 256.0, 500.0);
     const double bytes_kb = static_cast<double>(kTcTileN) * kTcRowBytes + static_cast<double>(bm) / cg * kTcRowBytes;
     auto per_kb = [&](double active_ctas) {
