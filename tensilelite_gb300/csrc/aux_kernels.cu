@@ -442,19 +442,20 @@ static cudaError_t launch_dependent(void (*kern)(KArgs...), int grid, int thread
 // they start in the middle of a word, and writes one 16-byte vector.  A warp takes 256 rows of a column
 // at a time: one index division per warp and 512 bytes.
 struct PadArgs {
-    PadOperand op[2];
-    int64_t chunks[2], tasks[2];          // 256-row chunks per column; chunks of the operand (0: not there)
+    PadOperand op[3];
+    int64_t chunks[3], tasks[3];          // 256-row chunks per column; chunks of the operand (0: not there)
 };
 
 __global__ void __launch_bounds__(256) pad_kernel(const __grid_constant__ PadArgs args)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
-    const int64_t total = args.tasks[0] + args.tasks[1];
+    const int64_t total = args.tasks[0] + args.tasks[1] + args.tasks[2];
     for (int64_t t = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; t < total; t += warps) {
-        const int w = t >= args.tasks[0];
+        int w = 0;
+        int64_t i = t;
+        while (i >= args.tasks[w]) i -= args.tasks[w++];
         const PadOperand& o = args.op[w];
-        const int64_t i = w ? t - args.tasks[0] : t;
         int64_t col, b = 0;
         if (i < (int64_t(1) << 31)) col = static_cast<uint32_t>(i) / static_cast<uint32_t>(args.chunks[w]);
         else col = i / args.chunks[w];
@@ -485,6 +486,46 @@ __global__ void __launch_bounds__(256) pad_kernel(const __grid_constant__ PadArg
             }
         }
         *reinterpret_cast<uint4*>(o.dst + b * o.p_batch_stride + col * o.pld + r) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// The way back: an aligned 16-byte load per lane, stored to any even address as the words that lie whole
+// in the lane's eight elements and a half word at either end.
+__global__ void __launch_bounds__(256) unpad_kernel(const __grid_constant__ PadArgs args)
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x / 32);
+    const PadOperand& o = args.op[0];
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32; i < args.tasks[0]; i += warps) {
+        int64_t col, b = 0;
+        if (i < (int64_t(1) << 31)) col = static_cast<uint32_t>(i) / static_cast<uint32_t>(args.chunks[0]);
+        else col = i / args.chunks[0];
+        const int64_t r = (i - col * args.chunks[0]) * 256 + lane * 8;
+        if (o.batch > 1) {
+            b = col / o.cols;
+            col -= b * o.cols;
+        }
+        if (r >= o.rows) continue;
+        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(o.dst + b * o.p_batch_stride + col * o.pld + r));
+        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+        uint16_t* out = const_cast<uint16_t*>(o.src) + b * o.batch_stride + col * o.ld + r;
+        if (o.rows - r >= 8) {
+            if ((reinterpret_cast<uintptr_t>(out) & 2) == 0) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) reinterpret_cast<uint32_t*>(out)[e] = q[e];
+            } else {
+                out[0] = static_cast<uint16_t>(q[0]);
+#pragma unroll
+                for (int e = 0; e < 3; ++e) reinterpret_cast<uint32_t*>(out + 1)[e] = __funnelshift_r(q[e], q[e + 1], 16);
+                out[7] = static_cast<uint16_t>(q[3] >> 16);
+            }
+        } else {
+            const int left = static_cast<int>(o.rows - r);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (e < left) out[e] = static_cast<uint16_t>(e & 1 ? q[e / 2] >> 16 : q[e / 2]);
+        }
     }
 }
 
@@ -522,10 +563,23 @@ tl_status aux_pad16(const PadOperand* ops, int count, cudaStream_t s, int64_t* l
         args.chunks[i] = (ops[i].rows + 255) / 256;
         args.tasks[i] = args.chunks[i] * ops[i].cols * ops[i].batch;
     }
-    const int64_t total = args.tasks[0] + args.tasks[1];
+    const int64_t total = args.tasks[0] + args.tasks[1] + args.tasks[2];
     if (total == 0) return TL_SUCCESS;
     pad_kernel<<<grid_for(total * 32, 1, 256), 256, 0, s>>>(args);
     return check_launch("pad_kernel", launches);
+}
+
+tl_status aux_unpad16(const PadOperand& op, cudaStream_t s, int64_t* launches)
+{
+    PadArgs args;
+    memset(&args, 0, sizeof(args));
+    args.op[0] = op;
+    args.chunks[0] = (op.rows + 255) / 256;
+    args.tasks[0] = args.chunks[0] * op.cols * op.batch;
+    const cudaError_t e = launch_dependent(unpad_kernel, grid_for(args.tasks[0] * 32, 1, 256), 256, s, args);
+    if (e != cudaSuccess) return cuda_fail(e, "unpad_kernel");
+    if (launches) ++*launches;
+    return TL_SUCCESS;
 }
 
 // Blocks of a quantisation pass over `bytes` of source: at most the resident grid, whose threads stay a

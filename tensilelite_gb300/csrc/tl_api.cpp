@@ -1021,17 +1021,22 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
 // A large fp16 or bf16 GEMM (16-bit output) whose operands start or stride off 16-byte boundaries, left
 // to the library (kernel AUTO, no solution, none tuned), runs on aligned copies of those operands: one
 // pass over memory instead of a CUDA-core kernel at a thirtieth of the tensor cores' rate (2047^3: 556
-// -> 70 us, 65 x 1025 x 3001: 122 -> 26).  Its chains are promoted every 256 k into fp32 registers: the
+// -> 43 us, 129 x 257 x 8191: 294 -> 26).  Its chains are promoted every 256 k into fp32 registers: the
 // error against 64 bits stays that of the output's rounding (1.6566e-3 for bf16 by either kernel; an
 // fp32 output would show the chains, and keeps the CUDA cores).  Below kPad16Work multiply-adds the
 // copies and the scratch cost more than that gives (501 x 601 x 501: 25 us against 23.5).  Scratch,
 // captures and a scratch that cannot be had: as for fp32 above.
 constexpr double kPad16Work = 2.0e8;
+// Outputs from which on a D that is not whole vectors goes through a copy of its own instead of being
+// stored element by element (2047^3: 67 -> 43 us, 4097 x 4095 x 511: 154 -> 59, 601 x 701 x 601: 25.9 ->
+// 20.6; 129 x 257 x 8191 would go 26.2 -> 26.6).
+constexpr double kPad16Out = 2.0e5;
 
-bool pad16_wanted(const tl_gemm_problem& p, const void* A, const void* B)
+bool pad16_wanted(const tl_gemm_problem& p, const void* D, const void* C, const void* A, const void* B)
 {
     const bool half = p.dtype_a == TL_DTYPE_FP16 || p.dtype_a == TL_DTYPE_BF16;
-    const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B);
+    const uintptr_t at = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) |
+                         reinterpret_cast<uintptr_t>(D) | (p.beta != 0.0f ? reinterpret_cast<uintptr_t>(C) : 0);
     return p.kernel == TL_KERNEL_AUTO && half && (p.dtype_d == TL_DTYPE_FP16 || p.dtype_d == TL_DTYPE_BF16) && at % 2 == 0 && p.m >= 64 && p.n >= 64 && p.k >= 64 &&
            static_cast<double>(p.m) * static_cast<double>(p.n) * static_cast<double>(p.k) *
            static_cast<double>(p.batch) >= kPad16Work && p.alpha * scale_of(p.scale_a) * scale_of(p.scale_b) != 0.0f;
@@ -1046,24 +1051,45 @@ tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done
     Prepared T = P;
     tl_gemm_problem& p = T.p;
     p.kernel = TL_KERNEL_TCGEN05;
-    PadOperand ops[2];
-    size_t bytes[2] = {0, 0};
+    T.kernel = TL_KERNEL_TCGEN05;
+    const int64_t m = p.m, m8 = (m + 7) / 8 * 8;
+    const auto lines = [&](const void* X, int64_t ld, int64_t stride) {
+        return aligned16(X) && ld % 8 == 0 && (p.batch == 1 || stride % 8 == 0);
+    };
+    // An output that is not whole vectors is stored element by element, or, from kPad16Out elements on, as
+    // whole lines into a copy of its own (C comes from one too), m rounded up to eight.
+    const bool out = static_cast<double>(m) * static_cast<double>(p.n) * static_cast<double>(p.batch) >= kPad16Out &&
+                     (m8 != m || !lines(P.D, p.ldd, p.stride_d) || (p.beta != 0.0f && !lines(P.C, p.ldc, p.stride_c)));
+    PadOperand ops[3], back = {};
+    size_t at[3] = {0, 0, 0}, bytes = 0;
     int count = 0;
-    const auto copy = [&](const void* X, int64_t rows, int64_t cols, int64_t* ld, int64_t* stride) {
-        if (aligned16(X) && *ld % 8 == 0 && (p.batch == 1 || *stride % 8 == 0)) return -1;
+    // an aligned copy of `cols` columns (room for `room`) of X; returns its index, or -1 if X does as it is
+    const auto copy = [&](bool always, const void* X, int64_t rows, int64_t cols, int64_t room, int64_t* ld, int64_t* stride) {
+        if (!always && lines(X, *ld, *stride)) return -1;
         PadOperand& o = ops[count];
         o = {static_cast<const uint16_t*>(X), rows, cols, *ld, p.batch, *stride, nullptr, 0, 0};
         o.pld = *ld = static_cast<int64_t>(align_up(static_cast<size_t>(rows), 64));
         o.p_batch_stride = *stride = o.pld * cols;
-        bytes[count] = align_up(static_cast<size_t>(o.p_batch_stride) * p.batch * 2, 256);
+        at[count] = bytes;
+        bytes += align_up(static_cast<size_t>(o.p_batch_stride * p.batch + o.pld * (room - cols)) * 2, 256);
         return count++;
     };
-    const int ia = copy(P.A, p.trans_a ? p.k : p.m, p.trans_a ? p.m : p.k, &p.lda, &p.stride_a);
-    const int ib = copy(P.B, p.trans_b ? p.n : p.k, p.trans_b ? p.k : p.n, &p.ldb, &p.stride_b);
-    if (count == 0) return TL_SUCCESS;
+    const int ia = copy(out && m8 != m, P.A, p.trans_a ? p.k : m, p.trans_a ? m : p.k, p.trans_a ? m8 : p.k, &p.lda, &p.stride_a);
+    const int ib = copy(false, P.B, p.trans_b ? p.n : p.k, p.trans_b ? p.k : p.n, p.trans_b ? p.k : p.n, &p.ldb, &p.stride_b);
+    if (ia < 0 && ib < 0) return TL_SUCCESS;
+    int ic = -1;
+    size_t back_at = 0;
+    if (out) {
+        if (p.beta != 0.0f) ic = copy(true, P.C, m, p.n, p.n, &p.ldc, &p.stride_c);
+        back = {static_cast<const uint16_t*>(P.D), m, p.n, p.ldd, p.batch, p.stride_d, nullptr, 0, 0};
+        back.pld = p.ldd = static_cast<int64_t>(align_up(static_cast<size_t>(m), 64));
+        back.p_batch_stride = p.stride_d = back.pld * p.n;
+        back_at = bytes;
+        bytes += align_up(static_cast<size_t>(back.p_batch_stride) * p.batch * 2, 256);
+        p.m = m8;            // rows m .. m8 - 1 of the copy are not copied back
+    }
     // the tile of the promoted products (tc_heuristic's), for the problem as the launch views it
-    T.kernel = TL_KERNEL_TCGEN05;
-    T.tview = tc_nn_view(p, T.kernel);
+    T.tview = !out && tc_nn_view(p, T.kernel);
     tc_heuristic(h, T.tview ? nn_view(p) : p, TL_KERNEL_BF16X6, &T.s);
     if (T.tview && !view_solution_ok(T.s)) {
         T.tview = false;
@@ -1073,9 +1099,9 @@ tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done
     if (T.tview) p = nn_view(p);
     if (check_tc_solution(h, p, T.s) != TL_SUCCESS) return TL_SUCCESS;
     const Scratch w = scratch_of(h, T);
-    const size_t head = align_up(w.counters * sizeof(int), 256);
+    const size_t head = align_up(w.counters * sizeof(int), 256), tail = head + align_up(w.bytes, 256);
     void* mem = nullptr;
-    if (cudaMallocFromPoolAsync(&mem, head + align_up(w.bytes, 256) + bytes[0] + bytes[1], pool, s) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(&mem, tail + bytes, pool, s) != cudaSuccess) {
         cudaGetLastError();
         return TL_SUCCESS;
     }
@@ -1084,16 +1110,18 @@ tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done
     T.counters = reinterpret_cast<int*>(base);
     T.counters_len = w.counters;
     place(T, w, base + head);
-    base += head + align_up(w.bytes, 256);
-    for (int i = 0; i < count; ++i) ops[i].dst = reinterpret_cast<uint16_t*>(base + (i ? bytes[0] : 0));
+    for (int i = 0; i < count; ++i) ops[i].dst = reinterpret_cast<uint16_t*>(base + tail + at[i]);
     if (ia >= 0) T.A = ops[ia].dst;
     if (ib >= 0) T.B = ops[ib].dst;
+    if (ic >= 0) T.C = ops[ic].dst;
+    if (out) T.D = back.dst = reinterpret_cast<uint16_t*>(base + tail + back_at);
     if (T.tview) std::swap(T.A, T.B);
     tl_status st = TL_SUCCESS;
     cudaError_t e = cudaSuccess;
     if (w.counters && (e = cudaMemsetAsync(mem, 0, head, s)) != cudaSuccess) st = cuda_fail(e, "cudaMemsetAsync(tile counters)");
     if (st == TL_SUCCESS) st = aux_pad16(ops, count, s, &h->launches);
     if (st == TL_SUCCESS) st = enqueue(h, T, s);
+    if (st == TL_SUCCESS && out) st = aux_unpad16(back, s, &h->launches);
     e = cudaFreeAsync(mem, s);
     if (st == TL_SUCCESS && e != cudaSuccess) st = cuda_fail(e, "cudaFreeAsync(padded operands)");
     return st;
@@ -1442,7 +1470,7 @@ TL_API tl_status tl_gemm(tl_handle* h, const tl_gemm_problem* p, const tl_gemm_s
         st = gemm_fp32_tc(h, P, S(stream), &done);
         if (done) return st;
     }
-    if (!s && !capturing && P.kernel == TL_KERNEL_SIMT && !P.tuned && pad16_wanted(*p, A, B)) {
+    if (!s && !capturing && P.kernel == TL_KERNEL_SIMT && !P.tuned && pad16_wanted(*p, D, C, A, B)) {
         bool done = false;
         st = gemm_pad16(h, P, S(stream), &done);
         if (done) return st;

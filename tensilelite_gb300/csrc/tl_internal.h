@@ -219,6 +219,8 @@ struct PadOperand {
     int64_t pld, p_batch_stride;
 };
 tl_status aux_pad16(const PadOperand* ops, int count, cudaStream_t s, int64_t* launches);
+// The way back: rows x cols of `dst` (pld, p_batch_stride) to `src`'s place; the gaps stay as they are.
+tl_status aux_unpad16(const PadOperand& op, cudaStream_t s, int64_t* launches);
 // Per-tensor E4M3 quantisation: *amax_dev = max |x|, dst = e4m3(x * 448 / amax), *scale_out_dev = amax / 448.
 tl_status aux_quantize_e4m3(int src_dtype, const void* src, int64_t n, float* amax_dev, uint8_t* dst,
                             float* scale_out_dev, cudaStream_t s, int64_t* launches);

@@ -188,7 +188,8 @@ def test_unaligned_half_matches_fp64_as_the_cuda_cores(h, dtype, layout, m, n, k
     assert any(ld % 8 for ld in (c.lda, c.ldb))
     l0 = h.launch_count()
     D = c.run(h)
-    assert h.launch_count() - l0 == 2          # copies, tensor cores
+    # copies, tensor cores, and from 2e5 outputs that are not whole vectors a copy back
+    assert h.launch_count() - l0 == 2 + (m * n * batch >= 2e5 and (m % 8 or c.ldc % 8) != 0)
     err = c.check(D)
     h.device_status()
     assert err <= 1.02 * c.check(c.run(h, "simt"))      # both are one output rounding away
