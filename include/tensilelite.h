@@ -69,7 +69,7 @@ typedef enum tl_kernel {
     TL_KERNEL_AUTO = 0,     /* fp16/bf16/fp8 -> TCGEN05; fp32 -> SIMT, and from 3e8 multiply-adds on the
                                products of BF16X6 where the operands' magnitudes allow it (checked on
                                the device; otherwise the SIMT kernel's results); fp16/bf16 operands off
-                               16-byte boundaries -> SIMT, and from 2e8 multiply-adds with a 16-bit
+                               16-byte boundaries -> SIMT, and from 1.5e8 multiply-adds with a 16-bit
                                output TCGEN05 on aligned copies */
     TL_KERNEL_SIMT = 1,     /* CUDA-core FMA kernel, any input type, fp32 accumulation */
     TL_KERNEL_TCGEN05 = 2,  /* TMA -> smem ring -> tcgen05.mma (TMEM accumulator) -> epilogue */

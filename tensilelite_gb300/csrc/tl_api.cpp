@@ -251,12 +251,12 @@ bool n_mn_major(const tl_gemm_problem& p) { return p.trans_b == TL_OP_T; }   // 
 
 // NN problems on the tensor cores run as their transposed product D^T = B^T A^T (a TT problem:
 // m and n, A and B exchanged) whose output the epilogue stores transposed, i.e. straight into the
-// caller's column-major D.  An MN-major operand on the MMA's N side (the problem's m side: A of an
-// NN problem) costs ~9 % at 4096^3 (NN and NT 1557 TFLOP/s against TN and TT 1700); on the M side
-// it costs nothing, and the exchange puts it there.  Only for one GEMM (batch 1, the measured
-// case), with beta == 0, k >= 2048 and without explicit split-k: the transposed epilogue reads C and finishes split tiles element by element
-// across a warp, which measured slower than the exchange gains, and with short k its epilogue
-// weighs more (4096 x 4096 x 1024: 31.4 against 30.5 us).  Not with a fused epilogue (its bias and amax
+// caller's column-major D.  With the issue loop that the rule was measured on, an MN-major operand on
+// the MMA's N side (the problem's m side: A of an NN problem) cost ~9 % at 4096^3 and nothing on the M side.
+// With the present loop the layouts take the same time, viewed or not (4096^3, beta 0: 76.8 and 76.3 us;
+// 2048^3 16.6 both); the view stays because tuned solutions of these problems tile it.  Only for one GEMM
+// (batch 1) with beta == 0, k >= 2048 and without explicit split-k: the transposed epilogue reads C and
+// finishes split tiles element by element across a warp.  Not with a fused epilogue (its bias and amax
 // follow the problem's m) nor fp8 (no MN-major fp8 operands).  TL_NN_TRANSPOSE=0 turns it off.
 bool nn_view_enabled()
 {
@@ -1024,9 +1024,10 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
 // -> 43 us, 129 x 257 x 8191: 294 -> 26).  Its chains are promoted every 256 k into fp32 registers: the
 // error against 64 bits stays that of the output's rounding (1.6566e-3 for bf16 by either kernel; an
 // fp32 output would show the chains, and keeps the CUDA cores).  Below kPad16Work multiply-adds the
-// copies and the scratch cost more than that gives (501 x 601 x 501: 25 us against 23.5).  Scratch,
+// copies and the scratch cost more than that gives (401 x 501 x 511: 23.2 us against 21.0; 501 x 601 x
+// 501: 22.7 against 23.6).  Scratch,
 // captures and a scratch that cannot be had: as for fp32 above.
-constexpr double kPad16Work = 2.0e8;
+constexpr double kPad16Work = 1.5e8;
 // Outputs from which on a D that is not whole vectors goes through a copy of its own instead of being
 // stored element by element (2047^3: 67 -> 43 us, 4097 x 4095 x 511: 154 -> 59, 601 x 701 x 601: 25.9 ->
 // 20.6; 129 x 257 x 8191 would go 26.2 -> 26.6).
