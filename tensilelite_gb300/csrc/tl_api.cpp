@@ -67,12 +67,11 @@ struct tl_handle {
     std::map<std::string, tl_gemm_solution> tuned;
     // heuristic picks by problem shape (the cost model takes 1.5 to 7 us a problem); at most kMaxPlans
     std::unordered_map<tl::PlanKey, tl::Plan, tl::PlanKeyHash> plans;
-    std::mutex mu;                 // tuned, plans, pool
+    std::mutex mu;                 // tuned, plans
     // stream-ordered scratch of the GEMMs that re-lay their operands (gemm_fp32_tc, gemm_pad16): each call has its
     // own, so that calls on different streams and threads stay independent.  At most kPoolKeep bytes
     // stay with the pool between synchronisations.
     cudaMemPool_t pool = nullptr;
-    bool pool_failed = false;
     // Once a stream capture has recorded this handle's workspace address, a grown workspace retires
     // the old buffer here (freed by tl_destroy) instead of freeing it under a live graph.
     bool captured = false;
@@ -930,9 +929,9 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
 // of three bf16 pieces per operand, whose error against 64 bits is below the CUDA-core kernel's (normal
 // values, relative 2-norm, 4096^3: 1.6e-7 against 1.15e-6; 1024^3: 0.9e-7 against 2.1e-7; 672^3: 0.9e-7
 // against 1.75e-7) and which takes a fifth of its time (4096^3 TN: 490 us against 2770; 1024^3: 33 against
-// 103).  Below kFp32TcWork multiply-adds, twice that where k is one or two k-blocks, the split pass and the
-// extra launches cost more than that gives (672^3: 29 us against 38; 512 x 1024 x 600: 28.6 either way;
-// 2048 x 2048 x 80: 24 against 22; 480 x 512 x 512: 13 on the CUDA cores).
+// 80).  Below kFp32TcWork multiply-adds, twice that where k is one or two k-blocks, the split pass and the
+// extra launches cost more than that gives (672^3: 29 us against 30; 512 x 1024 x 600: 28.6 either way;
+// 2048 x 2048 x 80: 24 against 22; 480 x 512 x 512: 12.5 on the CUDA cores).
 //
 // The pieces stand for the operands only within a range of magnitudes (split_range_ok), which is known
 // on the device once the split passes have run: infinities, NaN, numbers near fp32's limits.  So the
@@ -956,34 +955,36 @@ bool fp32_tc_wanted(const tl_gemm_problem& p)
            p.alpha * scale_of(p.scale_a) * scale_of(p.scale_b) != 0.0f;
 }
 
-cudaMemPool_t call_pool(tl_handle* h)
+// The pool of a new handle; null where there is none (the calls that want it then run as before).  Made
+// with the handle, not on first use: a GEMM on one stream must not make a call that another thread's
+// capture forbids.
+cudaMemPool_t make_call_pool(int device)
 {
-    std::lock_guard<std::mutex> g(h->mu);
-    if (!h->pool && !h->pool_failed) {
-        cudaMemPoolProps props;
-        memset(&props, 0, sizeof(props));
-        props.allocType = cudaMemAllocationTypePinned;
-        props.handleTypes = cudaMemHandleTypeNone;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = h->device;
-        uint64_t keep = kPoolKeep;
-        if (cudaMemPoolCreate(&h->pool, &props) != cudaSuccess ||
-            cudaMemPoolSetAttribute(h->pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            cudaGetLastError();
-            if (h->pool) cudaMemPoolDestroy(h->pool);
-            h->pool = nullptr;
-            h->pool_failed = true;
-        }
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.handleTypes = cudaMemHandleTypeNone;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = kPoolKeep;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
     }
-    return h->pool;
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        cudaMemPoolDestroy(pool);
+        return nullptr;
+    }
+    return pool;
 }
 
 // P is prepared for the CUDA-core kernel.  *done reports whether the GEMM was enqueued here.
 tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done)
 {
     *done = false;
-    cudaMemPool_t pool = call_pool(h);
-    if (!pool) return TL_SUCCESS;
+    if (!h->pool) return TL_SUCCESS;
     Prepared T = P;
     T.kernel = TL_KERNEL_BF16X6;
     T.p.kernel = TL_KERNEL_BF16X6;
@@ -993,7 +994,7 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
     const Scratch w = scratch_of(h, T);
     const size_t head = align_up(sizeof(SplitRange) + w.counters * sizeof(int), 256);
     void* mem = nullptr;
-    if (cudaMallocFromPoolAsync(&mem, head + w.bytes, pool, s) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(&mem, head + w.bytes, h->pool, s) != cudaSuccess) {
         cudaGetLastError();
         return TL_SUCCESS;
     }
@@ -1047,8 +1048,7 @@ bool pad16_wanted(const tl_gemm_problem& p, const void* D, const void* C, const 
 tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done)
 {
     *done = false;
-    cudaMemPool_t pool = call_pool(h);
-    if (!pool) return TL_SUCCESS;
+    if (!h->pool) return TL_SUCCESS;
     Prepared T = P;
     tl_gemm_problem& p = T.p;
     p.kernel = TL_KERNEL_TCGEN05;
@@ -1102,7 +1102,7 @@ tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done
     const Scratch w = scratch_of(h, T);
     const size_t head = align_up(w.counters * sizeof(int), 256), tail = head + align_up(w.bytes, 256);
     void* mem = nullptr;
-    if (cudaMallocFromPoolAsync(&mem, tail + bytes, pool, s) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(&mem, tail + bytes, h->pool, s) != cudaSuccess) {
         cudaGetLastError();
         return TL_SUCCESS;
     }
@@ -1340,6 +1340,7 @@ TL_API tl_status tl_init(tl_handle** handle)
     h->d_norms = reinterpret_cast<double*>(reinterpret_cast<char*>(h->d_err) + 64);
     h->d_amax = reinterpret_cast<float*>(reinterpret_cast<char*>(h->d_err) + 128);
     if ((e = cudaMemset(h->d_err, 0, 256)) != cudaSuccess) { cudaFree(h->d_err); delete h; return cuda_fail(e, "cudaMemset"); }
+    h->pool = make_call_pool(h->device);
     // the tuned-solution database of this device, when TL_SOLUTIONS names one (a missing file is no error)
     if (const char* path = getenv("TL_SOLUTIONS")) {
         std::ifstream probe(path);
