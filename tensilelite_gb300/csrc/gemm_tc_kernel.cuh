@@ -1490,14 +1490,15 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
             // group of CPS 32-column chunks (128 bytes of output per row) at a time.  C comes in
             // through it too, whole lines at a time like the stores; the first group's C is in flight
             // before the accumulator is ready (D may be C itself: a group's C is read before any of
-            // its columns is stored).
+            // its columns is stored).  A 192-column tile of one-byte outputs ends in half a group: two of
+            // its four chunks.
             constexpr int CPS = static_cast<int>(4 / sizeof(TD));
             const int nrow0 = j.n0 + quarter * 32;
             const bool staged = j.vec && j.nsplit == 1 && !j.out_t && chunks >= CPS;
             const bool use_c = j.beta != 0.0f && j.C != nullptr;
-            const int groups = half < nst ? chunks / CPS : 0;
+            const int groups = half < nst ? (chunks + CPS - 1) / CPS : 0;
             constexpr int WQ = EPI && sizeof(TD) != 1 ? 8 : 16;      // columns finished at a time
-            LineAccess<TD> la(lane, j.N - nrow0, j.M);
+            LineAccess<TD> la(lane, j.N - nrow0, sizeof(TD) == 1 ? min(j.M, j.m0 + p.bm) : j.M);
             uint4 cl[8];
             float bl[CPS];
             if constexpr (EPI) {
@@ -1596,11 +1597,13 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                                         j.ldc, m + nst * GC, cl);
                         }
                     }
+                    // only a group of one-byte outputs can be partial (every tile is whole pairs of chunks)
+                    const int nq = sizeof(TD) == 1 ? min(GC, p.bm - g * GC) / WQ : GC / WQ;
 #pragma unroll 1
-                    for (int q = 0; q < GC / WQ; ++q) {
+                    for (int q = 0; q < nq; ++q) {
                         float o[WQ];
                         ptx::tmem_ld<WQ>(tcol + static_cast<uint32_t>(q * WQ), o);
-                        if (q == GC / WQ - 1 && g + nst >= groups) release_tmem<CG>(&tempty[mbuf], lane);
+                        if (q == nq - 1 && g + nst >= groups) release_tmem<CG>(&tempty[mbuf], lane);
                         const uint32_t u0 = static_cast<uint32_t>(q * UPQ);
                         const uint32_t sw = static_cast<uint32_t>(lane & 7);
                         uint32_t cw[WQ];

@@ -299,3 +299,40 @@ def test_quantize_alignments(h, dtype, n, so, do):
     assert float(amax) == float(a) and np.float32(float(scale)) == np.float32(float(a)) / np.float32(448.0)
     assert torch.equal(buf[do:do + n], want)
     assert bool((buf[do + n:] == 0xAA).all()) and bool((buf[:do] == 0xAA).all())
+
+
+# ---- FP8 outputs: tiles that are no whole number of 128-column groups (192 wide), and the tile that the
+# library picks by itself.  D starts as E4M3's NaN, which a saturating store never writes ----
+@pytest.mark.parametrize("dtype,layout,m,n,k,tile", [
+    ("bf16", "NN", 192, 129, 192, 192), ("fp16", "NT", 400, 128, 64, 192), ("fp8", "TN", 176, 300, 256, 192),
+    ("bf16", "TN", 784, 257, 320, 192), ("bf16", "TN", 1152, 2752, 2624, 0), ("fp8", "TN", 1344, 4608, 1472, 0),
+    ("bf16", "NN", 384, 8192, 1024, 0), ("fp8", "TN", 128, 200, 256, 128), ("bf16", "NT", 320, 200, 128, 64)])
+def test_fp8_output_covers_every_tile(h, dtype, layout, m, n, k, tile):
+    ta, tb = layout[0] == "T", layout[1] == "T"
+    (ra, ca), (rb, cb) = ((k, m) if ta else (m, k)), ((n, k) if tb else (k, n))
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    to = {"bf16": torch.bfloat16, "fp16": torch.float16, "fp8": torch.float8_e4m3fn}[dtype]
+    A, B = (torch.randn(r * c, device="cuda", generator=g).to(to) for r, c in ((ra, ca), (rb, cb)))
+    a, b = (x.double().view(c, r).T for x, r, c in ((A, ra, ca), (B, rb, cb)))
+    ref = (a.T if ta else a) @ (b.T if tb else b)
+    bound = 3.0 * k * 2.0 ** -24 * ((a.T if ta else a).abs() @ (b.T if tb else b).abs())      # fp32 accumulation
+    p = tl.Problem.make(m, n, k, dtype=dtype, out_dtype="fp8", trans_a=ta, trans_b=tb)
+    sol = tl.Solution(kernel=tl.KERNEL_TCGEN05, macro_tile0=tile, macro_tile1=128, stages=4, split_k=1) if tile else None
+    assert tile or h.default_solution(p).macro_tile0 == 192
+    D = torch.full((m * n + 64,), 0x7f, dtype=torch.uint8, device="cuda")
+    amax = torch.zeros(1, device="cuda")
+    scale = 2.0
+    h.gemm_ex(p, D, None, A, B, amax=amax, d_scale=scale, solution=sol)
+    h.device_status()
+    got = D[:m * n].view(torch.float8_e4m3fn).double().view(n, m).T
+    assert torch.isfinite(got).all() and bool((D[m * n:] == 0x7f).all())
+    want = (ref * scale).clamp(-448, 448)
+    # half a step of E4M3 (three bits; 2^-9 below 2^-6) beside the accumulation's error
+    assert bool(((got - want).abs() <= 2.0 ** -4 * want.abs() + 2.0 ** -10 + scale * bound).all())
+    assert abs(float(amax) - float(ref.abs().max())) <= float(bound.max())
+    if not tile:
+        E = torch.full((m * n,), 0x7f, dtype=torch.uint8, device="cuda")
+        h.gemm(p, E, None, A, B)
+        got = E.view(torch.float8_e4m3fn).double().view(n, m).T
+        want = ref.clamp(-448, 448)
+        assert bool(((got - want).abs() <= 2.0 ** -4 * want.abs() + 2.0 ** -10 + bound).all())
