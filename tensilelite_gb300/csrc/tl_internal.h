@@ -73,15 +73,16 @@ struct SplitRange {
     uint32_t max_a, inv_min_a, max_b, inv_min_b;
 };
 // Whether three bf16 pieces stand for these operands as exactly as fp32 does in a sum of 2^klog2
-// products: everything finite, no piece below bf16's normal range, no product of pieces (down to
-// 2^-16 of its operands' product) below fp32's, and no sum beyond its largest value.
+// products: everything finite and still so when rounded to bf16 (from 0x7f7f8000 on a finite value rounds
+// to infinity), no piece below bf16's normal range, no product of pieces (down to 2^-16 of its operands'
+// product) below fp32's, and no sum beyond its largest value.
 #ifdef __CUDACC__
 __host__ __device__
 #endif
 inline bool split_range_ok(const SplitRange& r, int klog2)
 {
+    if (r.max_a >= 0x7f7f8000u || r.max_b >= 0x7f7f8000u) return false;
     const int ea = static_cast<int>(r.max_a >> 23), eb = static_cast<int>(r.max_b >> 23);
-    if (ea == 255 || eb == 255) return false;
     const int ma = r.inv_min_a ? static_cast<int>((~r.inv_min_a) >> 23) : 127;
     const int mb = r.inv_min_b ? static_cast<int>((~r.inv_min_b) >> 23) : 127;
     return ea + eb - 254 + 2 + klog2 <= 126 && ma >= 27 && mb >= 27 && ma + mb - 254 >= -100;

@@ -336,3 +336,23 @@ def test_fp8_output_covers_every_tile(h, dtype, layout, m, n, k, tile):
         got = E.view(torch.float8_e4m3fn).double().view(n, m).T
         want = ref.clamp(-448, 448)
         assert bool(((got - want).abs() <= 2.0 ** -4 * want.abs() + 2.0 ** -10 + bound).all())
+
+
+# ---- magnitudes whose leading bf16 piece is infinite, beside operands small enough for finite sums ----
+@pytest.mark.parametrize("where,bits", [("A", 0x7f7fffff), ("A", 0xff7fffff), ("B", 0x7f7fffff), ("B", 0x7f7f8000),
+                                        ("A", 0x7f7f7fff)])
+def test_fp32_auto_next_to_the_largest_float(h, where, bits):
+    c = Case(torch.float32, "TN", 720, 700, 640)
+    other = c.B if where == "A" else c.A
+    other.mul_(1e-5)
+    x = c.A if where == "A" else c.B
+    x[12345] = float(np.uint32(bits).view(np.float32))
+    got, want = c.run(h), c.run(h, "simt")
+    assert torch.isfinite(want).all() and torch.isfinite(got).all()
+    if bits & 0x7fffffff >= 0x7f7f8000:
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    else:                           # the largest magnitude whose pieces are finite
+        c.a = c.A.view(1, c.m, c.lda)[:, :, :c.k].double()
+        c.b = c.B.view(1, c.n, c.ldb)[:, :, :c.k].transpose(1, 2).double()
+        c.check(got)
+    h.device_status()
