@@ -351,10 +351,6 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.num_kb = static_cast<int>((L.K + W - 1) / W);
     kp.kb_elems = W;
     kp.promote_kb = L.promote_k > 0 ? static_cast<int>((L.promote_k + W - 1) / W) : 0;
-    // shared pieces: all products of a chain share its accumulator, so chains are short (the error of the
-    // tensor core's accumulation grows with the products added at full magnitude: 4 of 24 with one k-block
-    // of bf16x6, 16 of 24 with two of bf16x3, 16 with four of A0*B0 alone), as the epilogue has time for
-    if (shared) kp.promote_kb = std::min(kp.promote_kb, pieces == 3 ? 1 : 2);
     const int64_t kb_work = shared ? (pieces == 3 ? 6 : 3) : 1;      // products per k-block, for the split rules
     size_t smem = tc_smem_bytes(bm / cta_group, L.stages);
     kp.epi_bufs = epi_buffers(smem);

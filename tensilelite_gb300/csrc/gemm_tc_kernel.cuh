@@ -810,7 +810,12 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
 //                thread.
 //   kModePieces  promoted accumulation of the split-precision products, each piece of an operand staged
 //                once per k-block for all the products that use it; 256-column tiles, sixteen epilogue
-//                warps with 64 running sums per thread.
+//                warps with 64 running sums per thread.  The A0*B0 chain and the small products have one
+//                accumulator each, so the errors are those of the tiles that load every product's pieces.
+//                All products in one accumulator, with chains of one or two k-blocks in two buffers, left
+//                larger errors (bf16x6 8192^3, largest error over largest value 4.8e-7 against 3.6e-7) and
+//                were no faster (4096^3: bf16x6 489 us against 476, bf16x3 303 both; 3072 x 3072 x 64, where a
+//                tile waits for the one before it, 24.5 against 25.2).
 //   kModePlain   the others: eight epilogue warps, two per quarter of the TMEM lanes,
 // which take alternate column groups of a tile (half the drain time of a CTA's last tile, and of every
 // tile whose k is too short to hide it).  GROUP: the work units and problems come from a plan's tables.
@@ -866,9 +871,10 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
     const bool leader = (pair_rank == 0);
     const int64_t unit0 = (CL > 1) ? static_cast<int64_t>(ptx::cluster_id_x()) : static_cast<int64_t>(blockIdx.x);
     const int64_t units = (CL > 1) ? static_cast<int64_t>(ptx::ncluster_x()) : static_cast<int64_t>(gridDim.x);
-    const bool sep_small = PROMO && p.nterms > 1;      // (the pieces' products share one accumulator)
-    // TMEM columns: main accumulator x2 (+ small-term accumulator x2 when they are kept apart)
-    const uint32_t need_cols = static_cast<uint32_t>(p.bm) * (sep_small ? 4u : 2u);
+    const bool sep_small = MODE != kModePlain && p.nterms > 1;
+    // TMEM columns: main accumulator x2 (+ small-term accumulator x2 when they are kept apart); with 256
+    // columns one of each
+    const uint32_t need_cols = static_cast<uint32_t>(p.bm) * (sep_small && !PIECES ? 4u : 2u);
     const uint32_t tmem_cols = need_cols <= 128 ? 128u : (need_cols <= 256 ? 256u : 512u);
     const uint32_t epi_arrivals = 4u * NH * CG;     // one per epilogue warp of each CTA
 
@@ -1124,7 +1130,7 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                     }
                     ptx::tc_fence_after();
                 }
-                if (!ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
+                if (!PIECES && !ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
                     record_error(p, abort_flag, 2);
                     break;
                 }
@@ -1137,27 +1143,16 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 }
                 if constexpr (PIECES) {
                     // A k-block's pieces arrive smallest first in nvirt consecutive slots; every product
-                    // of them is formed from there, those of one order with each other (smallest
-                    // first, so that only the last runs at the accumulator's full magnitude), and a
-                    // slot is released by its last product.  The accumulator restarts every
-                    // promote_kb k-blocks in the alternate buffer.
-                    uint32_t acc = 0;
+                    // of them is formed from there and a slot is released by its last product.  The small
+                    // products of the whole tile share one accumulator, the A0*B0 products another that
+                    // starts anew every promote_kb k-blocks.  There is one of each: a chain is drained while
+                    // the next k-block's small products run, and the last chain, whose A0*B0 goes first
+                    // in its last k-block, while the small sums are completed.
+                    const uint32_t d_small = tmem_base + bmu;
+                    uint32_t small_acc = 0, main_acc = 0;
                     int in_chain = 0;
                     for (int kb = 0; kb < nkb; ++kb) {
-                        if (in_chain == p.promote_kb) {
-                            ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
-                            mbuf ^= 1u;
-                            if (mbuf == 0) mph ^= 1u;
-                            in_chain = 0;
-                            acc = 0;
-                            if (!ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
-                                record_error(p, abort_flag, 2);
-                                ok = false;
-                                break;
-                            }
-                            ptx::tc_fence_after();
-                        }
-                        const uint32_t d_tmem = tmem_base + mbuf * bmu;
+                        const bool last = kb == nkb - 1;
                         uint32_t sl[3], dn[3];
 #pragma unroll
                         for (int v = 0; v < 3; ++v) {
@@ -1179,28 +1174,50 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                         }
                         if (!ok) break;
                         ptx::tc_fence_after();
-                        auto mma = [&](uint32_t n, uint32_t m) {
-                            ptx::mma_kblock<KIND, CG>(d_tmem, n, m + dNM, dhi, idesc, acc, n_kstep, m_kstep);
-                            acc = 1;
+                        const uint32_t d0 = nvirt == 3 ? dn[2] : dn[1];          // dn: pieces (2,) 1, 0
+                        auto main_mma = [&] {
+                            if (in_chain == 0) {
+                                if (!ptx::mbar_wait(&tempty[0], mph ^ 1u, tlim)) {
+                                    record_error(p, abort_flag, 2);
+                                    ok = false;
+                                    return;
+                                }
+                                ptx::tc_fence_after();
+                                main_acc = 0;
+                            }
+                            ptx::mma_kblock<KIND, CG>(tmem_base, d0, d0 + dNM, dhi, idesc, main_acc, n_kstep, m_kstep);
+                            main_acc = 1;
+                            if (++in_chain == p.promote_kb || last) {
+                                ptx::mma_commit_pair(ptx::smem_u32(&tfull[0]), pair_mask);
+                                mph ^= 1u;
+                                in_chain = 0;
+                            }
                         };
-                        if (nvirt == 3) {                       // dn: pieces 2, 1, 0
-                            mma(dn[0], dn[2]);
+                        auto mma = [&](uint32_t n, uint32_t m) {
+                            ptx::mma_kblock<KIND, CG>(d_small, n, m + dNM, dhi, idesc, small_acc, n_kstep, m_kstep);
+                            small_acc = 1;
+                        };
+                        // (a chain that starts here would wait for the one before it; a tile's first does not)
+                        const bool main_first = last && (in_chain != 0 || kb == 0);
+                        if (main_first) main_mma();
+                        if (!ok) break;
+                        if (nvirt == 3) {
                             mma(dn[2], dn[0]);
-                            ptx::mma_commit_pair(sl[0], 0x3);
                             mma(dn[1], dn[1]);
-                            mma(dn[1], dn[2]);
+                            mma(dn[0], dn[2]);
+                            ptx::mma_commit_pair(sl[0], 0x3);
                             mma(dn[2], dn[1]);
+                            mma(dn[1], dn[2]);
                             ptx::mma_commit_pair(sl[1], 0x3);
-                            mma(dn[2], dn[2]);
-                            ptx::mma_commit_pair(sl[2], 0x3);
-                        } else {                                // dn: pieces 1, 0
-                            mma(dn[0], dn[1]);
+                        } else {
                             mma(dn[1], dn[0]);
+                            mma(dn[0], dn[1]);
                             ptx::mma_commit_pair(sl[0], 0x3);
-                            mma(dn[1], dn[1]);
-                            ptx::mma_commit_pair(sl[1], 0x3);
                         }
-                        ++in_chain;
+                        if (last) ptx::mma_commit_pair(ptx::smem_u32(&sfull[0]), pair_mask);
+                        if (!main_first) main_mma();
+                        if (!ok) break;
+                        ptx::mma_commit_pair(nvirt == 3 ? sl[2] : sl[1], 0x3);
                     }
                 } else if constexpr (!PROMO) {
                     // every product of the tile into one accumulator
@@ -1240,6 +1257,11 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                     }
                 }
                 if (!ok) break;
+                if constexpr (PIECES) {              // handed over in the loop; one buffer of each kind
+                    if (w == unit0) trace_mark(p, TL_TRACE_MMA_LAST);
+                    sph ^= 1u;
+                    continue;
+                }
                 if constexpr (CG == 2) ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
                 else ptx::mma_commit(ptx::smem_u32(&tfull[mbuf]));
                 if (sep_small) {
@@ -1314,8 +1336,11 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 for (int i = 0; i < RC; ++i) run[i] = 0.f;
                 const int nkb = j.kb1 - j.kb0;
                 const int nchain = (nkb + p.promote_kb - 1) / p.promote_kb;
-                for (int c = 0; c < nchain; ++c) {
-                    bool got = ok && ptx::mbar_wait(&tfull[mbuf], mph, tlim);
+                const int steps = nchain + (sep_small ? 1 : 0);
+                for (int c = 0; c < steps; ++c) {
+                    const bool sm = c == nchain;          // the small terms, after the chains
+                    uint64_t* const full_bar = sm ? &sfull[sbuf] : &tfull[mbuf];
+                    bool got = ok && ptx::mbar_wait(full_bar, sm ? sph : mph, tlim);
                     got = __all_sync(0xffffffffu, got);
                     if (ok && !got) {
                         if (lane == 0) record_error(p, abort_flag, 8);
@@ -1323,7 +1348,8 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                     }
                     if (ok) {
                         ptx::tc_fence_after();
-                        const uint32_t tb = tmem_base + lane_off + mbuf * static_cast<uint32_t>(p.bm) + static_cast<uint32_t>(col0);
+                        const uint32_t buf = sm ? (PIECES ? 1u : 2u + sbuf) : mbuf;
+                        const uint32_t tb = tmem_base + lane_off + buf * static_cast<uint32_t>(p.bm) + static_cast<uint32_t>(col0);
 #pragma unroll
                         for (int q = 0; q < NQ; ++q) {
                             float r[QW];
@@ -1332,33 +1358,15 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
 #pragma unroll
                             for (int i = 0; i < QW; ++i) run[q * QW + i] += r[i];
                         }
-                        release_tmem<CG>(&tempty[mbuf], lane);
+                        release_tmem<CG>(sm ? &sempty[sbuf] : &tempty[mbuf], lane);
                     }
-                    mbuf ^= 1u;
-                    if (mbuf == 0) mph ^= 1u;
-                }
-                if (sep_small) {
-                    bool got = ok && ptx::mbar_wait(&sfull[sbuf], sph, tlim);
-                    got = __all_sync(0xffffffffu, got);
-                    if (ok && !got) {
-                        if (lane == 0) record_error(p, abort_flag, 8);
-                        ok = false;
+                    if (sm) {
+                        if (!PIECES) sbuf ^= 1u;
+                        if (sbuf == 0) sph ^= 1u;
+                    } else {
+                        if (!PIECES) mbuf ^= 1u;
+                        if (mbuf == 0) mph ^= 1u;
                     }
-                    if (ok) {
-                        ptx::tc_fence_after();
-                        const uint32_t tb = tmem_base + lane_off + (2u + sbuf) * static_cast<uint32_t>(p.bm);
-#pragma unroll
-                        for (int q = 0; q < NQ; ++q) {
-                            float r[QW];
-                            __syncwarp();
-                            ptx::tmem_ld<QW>(tb + q * QW, r);
-#pragma unroll
-                            for (int i = 0; i < QW; ++i) run[q * QW + i] += r[i];
-                        }
-                        release_tmem<CG>(&sempty[sbuf], lane);
-                    }
-                    sbuf ^= 1u;
-                    if (sbuf == 0) sph ^= 1u;
                 }
                 if (tr) trace_mark(p, TL_TRACE_ACC_READY);
                 // With 96 registers of which 64 hold sums, the unit is decoded again here instead of
