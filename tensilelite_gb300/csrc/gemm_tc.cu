@@ -96,6 +96,17 @@ bool par_reduce_enabled()
     return on;
 }
 
+// How long a split waits for its tile's others before it leaves its share to the last of them (TcLaunch::shared_gpu):
+// TL_SPLIT_WAIT_NS, 10 us by default.  Splits that start together arrive within a microsecond or two.
+static unsigned long long hand_over_ns()
+{
+    static const unsigned long long ns = [] {
+        const char* e = getenv("TL_SPLIT_WAIT_NS");
+        return e ? strtoull(e, nullptr, 10) : 10000ull;
+    }();
+    return ns;
+}
+
 // Programmatic dependent launch for the tensor-core kernel: on unless TL_PDL=0 in the environment.
 bool pdl_enabled()
 {
@@ -438,7 +449,8 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     // all split units in the first round of the persistent schedule: parallel reduction
     {
         const int workers = persistent_workers(L.in_dtype, L.out_dtype, cg, L.ctas, L.sm_count, smem);
-        kp.par_reduce = (kp.split_units > 0 && kp.bal_kb == 0 && kp.split_units <= workers && par_reduce_enabled()) ? 1 : 0;
+        kp.par_reduce = par_reduce_enabled() ? tc_par_reduce(kp.split_units, kp.bal_kb, workers, L.shared_gpu) : 0;
+        kp.hand_over_ns = hand_over_ns();
     }
     kp.out_t = L.out_t;
     kp.vec = tc_vec_output(L.out_dtype, L.out_t ? L.N : L.M, L.D, L.ldd, L.C, L.ldc, L.batch, L.stride_d, L.stride_c) ? 1 : 0;

@@ -33,7 +33,9 @@ struct TcKernelParams {
     int epi_act;
     int epi_on;
     int par_reduce;               // every split unit runs in the first round: the splits of a tile
-                                  // wait for each other and reduce one share of it each
+                                  // wait for each other and reduce one share of it each; 2: beside other
+                                  // launches (split_finish)
+    unsigned long long hand_over_ns;      // par_reduce 2: how long a split waits for the others
     const TcGroupEntry* group;
     const int4* group_units;       // per work unit: {problem, tile row, tile column, k-blocks}
     void* D;
@@ -703,6 +705,24 @@ __device__ __forceinline__ bool wait_counter_ge(const int* ctr, int target, uint
     }
 }
 
+// A split has arrived and is not its tile's last: the chunks that it reduces itself, `own` once every split has
+// arrived, none if it has no share or leaves it to the last one after limit_ns.
+__device__ __forceinline__ int hand_over(int* ctr, int nsplit, int own, uint64_t limit_ns)
+{
+    if (!own) return 0;
+    const uint64_t t0 = ptx::globaltimer();
+    while (true) {
+        int v;
+        asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+        if ((v & 0xff) >= nsplit) return own;
+        if (ptx::globaltimer() - t0 > limit_ns) {
+            if (atomicCAS(ctr, v, v | (own << 8)) == v) return 0;
+            continue;                               // another split came or left: look again
+        }
+        __nanosleep(64);
+    }
+}
+
 // Split-k completion, run by the epilogue warps after this split parked its partial tile in the
 // workspace (layout [32-column chunk][column][row], so every warp access is one 128-byte line; the
 // TMEM buffer is free again).  The partials are summed in split order, so the result does not depend on
@@ -713,6 +733,10 @@ __device__ __forceinline__ bool wait_counter_ge(const int* ctr, int target, uint
 //                  theirs, then reduces its share of the tile -- chunks split, split + nsplit, ...
 //                  The tile counter counts arrivals up to nsplit, then finished shares up to
 //                  2 * nsplit, when the last one resets it for the next launch.
+//   par_reduce 2   the same where launches on other streams may hold part of the SMs, so that a tile's other
+//                  splits may be unable to start until this CTA leaves: a split waits hand_over_ns at most, then
+//                  leaves its share to the last one to arrive.  The counter's low byte counts arrivals and the
+//                  next holds the chunks left; it is not reset (such a launch has zeroed counters of its own).
 //   otherwise      the last split to arrive (tile counter) reduces the whole tile and resets it.
 // Every thread passes the same named barriers whether or not it has work, so a warp that gave up on
 // a wait cannot strand the others.
@@ -723,18 +747,25 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
                                              uint32_t c_row)
 {
     constexpr int W = 32 / NH;                      // columns of a chunk per warp
-    const bool par = p.par_reduce != 0;
+    const bool par = p.par_reduce == 1;
+    const int chunks = p.bm / 32;
     __threadfence();
     ptx::named_sync<NH * 128>();
     if (et == 0) {
-        int go = 0;
+        int go = 0;                                 // the chunks that this split reduces, a bit each
         if (ok) {
-            const int before = atomicAdd(p.counters + j.slot, 1);
+            int own = 0;
+            for (int c = j.split; c < chunks; c += j.nsplit) own |= 1 << c;
+            int* const ctr = p.counters + j.slot;
+            const int before = atomicAdd(ctr, 1);
             if (par) {
-                go = wait_counter_ge(p.counters + j.slot, j.nsplit, p.timeout_ns) ? 1 : 0;
-                if (!go) record_error(p, abort_flag, 16);
+                // (bit 8: a split without a share counts itself out all the same)
+                if (wait_counter_ge(ctr, j.nsplit, p.timeout_ns)) go = own | 0x100;
+                else record_error(p, abort_flag, 16);
+            } else if (p.par_reduce == 2) {
+                go = (before & 0xff) == j.nsplit - 1 ? own | (before >> 8) : hand_over(ctr, j.nsplit, own, p.hand_over_ns);
             } else {
-                go = before == j.nsplit - 1 ? 1 : 0;
+                go = before == j.nsplit - 1 ? (1 << chunks) - 1 : 0;
             }
         }
         *last_flag = go;
@@ -743,11 +774,11 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
     const int go = *last_flag;
     if (go) {
         __threadfence();
-        const int chunks = p.bm / 32, step = par ? j.nsplit : 1;
         const size_t slab_elems = static_cast<size_t>(kTcTileN) * p.bm;
         const float* base = p.ws + static_cast<size_t>(j.slot) * p.tail_split * slab_elems +
                             static_cast<size_t>(half) * W * kTcTileN + row;
-        for (int c = par ? j.split : 0; c < chunks; c += step) {
+        for (int c = 0; c < chunks; ++c) {
+            if (!((go >> c) & 1)) continue;
             const int m = j.m0 + c * 32 + half * W;
             // two splits' partials at a time are in flight together (the reduction is
             // latency-bound), summed in split order
@@ -796,7 +827,7 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
     }
     if (c_staged) ptx::cp_async_wait0();   // the staging buffer is free again (also on the error path)
     ptx::named_sync<NH * 128>();           // last_flag is reused by the next tile
-    if (et == 0 && go) {
+    if (et == 0 && go && p.par_reduce != 2) {
         if (!par) p.counters[j.slot] = 0;  // ready for the next launch
         // counts this split out of the tile: the last one resets the counter for the next launch.
         // No fence: the counter only orders the splits' waits (same-address atomics), and the next

@@ -613,6 +613,7 @@ struct Prepared {
     int* counters = nullptr;             // split tile counters
     size_t counters_len = 0;
     SplitRange* range = nullptr;         // the split pass reports magnitudes; the GEMM depends on them
+    bool own_scratch = false;            // scratch of this call alone: it may run beside others (TcLaunch::shared_gpu)
     tl_epilogue epi{};
     bool epi_on = false;
     bool tuned = false;      // the solution was tuned or loaded
@@ -907,6 +908,7 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
     L.counters = P.counters;
     L.counters_len = P.counters_len;
     L.range = P.range;
+    L.shared_gpu = P.own_scratch ? 1 : 0;
     L.tail_split = P.s.tail_split;
     L.sm_count = h->sm_count;
     // fp8 outputs are written by the fused-epilogue kernels (no bias or activation unless asked for)
@@ -939,8 +941,9 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
 // if they are out of range, and the CUDA-core launch returns at once if they are not.  What is out of
 // range therefore gets the CUDA-core kernel's results, bit for bit.
 //
-// Each call has its own scratch, allocated and freed in stream order.  While a stream is being
-// captured, or where the scratch cannot be had, the CUDA-core kernel runs as before.
+// Each call has its own scratch, allocated and freed in stream order, and none of its CTAs relies on
+// another's start (tc_par_reduce), so calls on different streams are as independent as with the CUDA-core
+// kernel.  While a stream is being captured, or where the scratch cannot be had, that kernel runs as before.
 constexpr double kFp32TcWork = 3.0e8;
 // The tensor core drops bits below its accumulator's last one, so a sum of many terms of one sign comes
 // out low: 700^3 of uniform [0, 1), chains of 256: 2.6e-7, CUDA cores 0.7e-7.  Chains of one k-block
@@ -1001,6 +1004,7 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
     *done = true;
     char* base = static_cast<char*>(mem);
     T.range = reinterpret_cast<SplitRange*>(base);
+    T.own_scratch = true;
     T.counters = reinterpret_cast<int*>(base + sizeof(SplitRange));
     T.counters_len = w.counters;
     place(T, w, base + head);
@@ -1108,6 +1112,7 @@ tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done
     }
     *done = true;
     char* base = static_cast<char*>(mem);
+    T.own_scratch = true;
     T.counters = reinterpret_cast<int*>(base);
     T.counters_len = w.counters;
     place(T, w, base + head);

@@ -151,7 +151,18 @@ struct TcLaunch {
     int64_t trace_bytes;
     int out_t;               // D and C hold the transpose of this launch's output (NN run as TT)
     const SplitRange* range; // split products: run only if split_range_ok (device memory), or null
+    int shared_gpu;          // launches like this one may run beside it on other streams: no CTA relies on another's
+                             // start (the counters are this launch's own, zeroed)
 };
+
+// How the splits of a tile are summed: 0 by the last one to arrive, 1 by all of them, a share each, once all have
+// arrived, 2 the same without relying on it.  All of a launch's split units have to be resident at
+// once for 1: where launches on other streams may hold part of the SMs, two of them, each partly resident,
+// would wait until the limit for CTAs that cannot start.
+inline int tc_par_reduce(int64_t split_units, int64_t bal_kb, int64_t workers, int shared_gpu)
+{
+    return split_units > 0 && bal_kb == 0 && split_units <= workers ? (shared_gpu ? 2 : 1) : 0;
+}
 
 // Dynamic shared memory of one CTA staging bm_cta m-rows per stage (bm / 2 for a CTA pair).
 size_t tc_smem_bytes(int bm_cta, int stages);

@@ -3,6 +3,10 @@
 References: the float64 product on the device, and for values that a route must not change the
 CUDA-core kernel's own result, bit for bit.  Tolerances are the bounds of fp32 accumulation
 (k 2^-24 sum |a||b|, the factor 3 of the other parity tests) plus one rounding of the output."""
+import hashlib
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -383,3 +387,31 @@ def test_shared_pieces_are_as_exact_as_single_products(h, kernel, k, dist):
     h.device_status()
     for got, want in zip(*errs):
         assert got <= 1.1 * want
+
+
+# ---- splits of a call with scratch of its own: whoever sums a chunk, the same bits.  Waiting as by default, not at
+# all (every share is left to the last split) and by the last split alone ----
+SPLIT_CASES = [(torch.float32, "TN", 300, 400, 4096, 0.5), (torch.float32, "NN", 700, 700, 700, 0.0),
+               (torch.bfloat16, "NN", 129, 257, 8191, 0.0), (torch.float16, "TN", 301, 1100, 1011, 0.5)]
+
+
+def split_digests(h):
+    out = []
+    for dtype, layout, m, n, k, beta in SPLIT_CASES:
+        c = Case(dtype, layout, m, n, k, beta=beta)
+        for _ in range(3):
+            D = c.run(h)
+        h.device_status()
+        c.check(D)
+        out.append(hashlib.sha256(c.view(D).contiguous().view(torch.uint8).cpu().numpy().tobytes()).hexdigest())
+    return out
+
+
+@pytest.mark.parametrize("env", [{"TL_SPLIT_WAIT_NS": "0"}, {"TL_SPLIT_WAIT_NS": "700"}, {"TL_PAR_REDUCE": "0"}])
+def test_split_shares_left_to_the_last(h, env):
+    here = os.path.dirname(os.path.abspath(__file__))
+    code = ("import sys; sys.path[:0] = %r\nimport test_routes_gpu as t\nh = t.tl.Handle()\nprint(' '.join(t.split_digests(h)))"
+            % [os.path.dirname(here), here])
+    r = subprocess.run([sys.executable, "-c", code], env={**os.environ, **env}, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == split_digests(h)
