@@ -362,6 +362,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.num_kb = static_cast<int>((L.K + W - 1) / W);
     kp.kb_elems = W;
     kp.promote_kb = L.promote_k > 0 ? static_cast<int>((L.promote_k + W - 1) / W) : 0;
+    kp.promote_half = pieces > 1 && !shared && L.promote_k > 0 && L.promote_k <= W / 2 ? 1 : 0;
     const int64_t kb_work = shared ? (pieces == 3 ? 6 : 3) : 1;      // products per k-block, for the split rules
     size_t smem = tc_smem_bytes(bm / cta_group, L.stages);
     kp.epi_bufs = epi_buffers(smem);

@@ -51,6 +51,7 @@ struct TcKernelParams {
     int pieces_mode;              // kModePieces
     int promote_kb;               // >0: the A0*B0 product restarts its TMEM chain every promote_kb
                                   // k-blocks; the epilogue adds each chain into fp32 registers
+    int promote_half;             // two A0*B0 chains per k-block (16-bit pieces, promote_kb 1)
     int tiles_m, tiles_n;
     int narrow;                   // work units, tiles and split k-block products fit 32 bits, no balanced split
     int64_t total_work;
@@ -1122,14 +1123,17 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
             const uint32_t dstep = stage_bytes >> 4;
             const uint32_t bar_end = full_a + 8u * static_cast<uint32_t>(p.stages);
             uint32_t dN = dN0, bar = full_a;
-            // one stage into `d_tmem`: wait for its bytes, issue its MMAs, release its slot when they complete
-            auto consume = [&](uint32_t d_tmem, uint32_t accumulate) {
+            // a stage's bytes have arrived
+            auto arrived = [&] {
                 if (!ptx::mbar_wait(bar, phase, tlim)) {
                     record_error(p, abort_flag, 4);
                     return false;
                 }
                 ptx::tc_fence_after();
-                ptx::mma_kblock<KIND, CG>(d_tmem, dN, dN + dNM, dhi, idesc, accumulate, n_kstep, m_kstep);
+                return true;
+            };
+            // its slot is released when the MMAs issued so far complete
+            auto release = [&] {
                 // both pairs' ring slots are released (MC == 2: every CTA of the cluster)
                 if constexpr (CG == 2) ptx::mma_commit_pair(bar + (empty_a - full_a), MC == 2 ? 0xF : 0x3);
                 else ptx::mma_commit(bar + (empty_a - full_a));
@@ -1140,6 +1144,25 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                     dN = dN0;
                     phase ^= 1u;
                 }
+            };
+            // one stage into `d_tmem`
+            auto consume = [&](uint32_t d_tmem, uint32_t accumulate) {
+                if (!arrived()) return false;
+                ptx::mma_kblock<KIND, CG>(d_tmem, dN, dN + dNM, dhi, idesc, accumulate, n_kstep, m_kstep);
+                release();
+                return true;
+            };
+            // hand the main accumulator's chain to the epilogue and continue in the other buffer
+            auto next_chain = [&] {
+                if constexpr (CG == 2) ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
+                else ptx::mma_commit(ptx::smem_u32(&tfull[mbuf]));
+                mbuf ^= 1u;
+                if (mbuf == 0) mph ^= 1u;
+                if (!ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
+                    record_error(p, abort_flag, 2);
+                    return false;
+                }
+                ptx::tc_fence_after();
                 return true;
             };
             bool ok = true;
@@ -1263,24 +1286,28 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                     int in_chain = 0;
                     for (int kb = 0; kb < nkb && ok; ++kb) {
                         if (in_chain == p.promote_kb) {
-                            // end of a chain of the main product: hand it to the epilogue, continue in
-                            // the other buffer (a tile's last chain is handed over after the loop)
-                            if constexpr (CG == 2) ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
-                            else ptx::mma_commit(ptx::smem_u32(&tfull[mbuf]));
-                            mbuf ^= 1u;
-                            if (mbuf == 0) mph ^= 1u;
+                            // (a tile's last chain is handed over after the loop)
+                            if (!(ok = next_chain())) break;
                             in_chain = 0;
                             main_acc = 0;
-                            if (!ptx::mbar_wait(&tempty[mbuf], mph ^ 1u, tlim)) {
-                                record_error(p, abort_flag, 2);
-                                ok = false;
-                                break;
-                            }
-                            ptx::tc_fence_after();
                         }
                         for (int v = 0; v < nvirt - 1 && ok; ++v) {
                             ok = consume(tmem_base + (2u + sbuf) * bmu, small_acc);
                             small_acc = 1;
+                        }
+                        if constexpr (KIND == 0) {
+                            if (ok && p.promote_half) {
+                                if (!(ok = arrived())) break;
+                                for (uint32_t i = 0; i < 4u; ++i) {
+                                    if (i == 2u && !(ok = next_chain())) break;
+                                    ptx::mma_k16<CG>(tmem_base + mbuf * bmu, dN + i * n_kstep, dN + dNM + i * m_kstep, dhi, idesc,
+                                                     i & 1u);
+                                }
+                                if (!ok) break;
+                                release();
+                                ++in_chain;
+                                continue;
+                            }
                         }
                         if (ok) ok = consume(tmem_base + mbuf * bmu, main_acc);
                         main_acc = 1;
@@ -1366,7 +1393,7 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
 #pragma unroll
                 for (int i = 0; i < RC; ++i) run[i] = 0.f;
                 const int nkb = j.kb1 - j.kb0;
-                const int nchain = (nkb + p.promote_kb - 1) / p.promote_kb;
+                const int nchain = PROMO && p.promote_half ? 2 * nkb : (nkb + p.promote_kb - 1) / p.promote_kb;
                 const int steps = nchain + (sep_small ? 1 : 0);
                 for (int c = 0; c < steps; ++c) {
                     const bool sm = c == nchain;          // the small terms, after the chains

@@ -201,6 +201,22 @@ __device__ __forceinline__ void mma_kblock(uint32_t d_tmem, uint32_t a_lo, uint3
     else if constexpr (CG == 1) TL_MMA4("1", "f8f6f4");
     else TL_MMA4("2", "f8f6f4");
 }
+// One of the four (16-bit inputs).
+template <int CG>
+__device__ __forceinline__ void mma_k16(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                        uint32_t accumulate)
+{
+#define TL_MMA1(GROUP)                                                                                       \
+    asm volatile(                                                                                            \
+        "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"                                                        \
+        "setp.ne.b32 p, %5, 0;\n\tmov.b64 ad, {%1, %3};\n\tmov.b64 bd, {%2, %3};\n\t"                         \
+        "tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], ad, bd, %4, p;\n\t}\n" ::"r"(d_tmem),              \
+        "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)                                            \
+        : "memory")
+    if constexpr (CG == 1) TL_MMA1("1");
+    else TL_MMA1("2");
+#undef TL_MMA1
+}
 #undef TL_MMA4
 
 // Arrive once on `bar` when every tcgen05 operation issued so far by this thread has completed.

@@ -945,10 +945,16 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
 // another's start (tc_par_reduce), so calls on different streams are as independent as with the CUDA-core
 // kernel.  While a stream is being captured, or where the scratch cannot be had, that kernel runs as before.
 constexpr double kFp32TcWork = 3.0e8;
-// The tensor core drops bits below its accumulator's last one, so a sum of many terms of one sign comes
-// out low: 700^3 of uniform [0, 1), chains of 256: 2.6e-7, CUDA cores 0.7e-7.  Chains of one k-block
-// keep fp32 results at or below the CUDA cores' error.
-constexpr int kFp32Chain = 64;
+// The tensor core drops bits below its accumulator's last one, so a sum of many terms of one sign comes out
+// low, and every chain that the epilogue adds is a rounding.  Relative 2-norm for uniform [0, 1), chains
+// of 256 / 64 / 32 / 16 against the CUDA cores: 700^3 2.6e-7 / 8.2e-8 / 6.3e-8 / - against 7.1e-8;
+// 1024 x 1024 x 320 - / 8.5e-8 / 6.9e-8 / 7.9e-8 against 6.0e-8; 1024 x 1024 x 2048 - / 8.7e-8 / 7.4e-8 / - against 9.0e-8.
+// Halves of a k-block below k = 2048 therefore (1024^3 32.6 -> 33.2 us), whole ones from there on.  What
+// is left: values of one sign, k below 512 and too few tiles for the shared pieces, up to 1.16 times the CUDA
+// cores' error, whose sums run in eight groups there.  With the rounding errors of the epilogue's sums added back
+// (two-sum) it is 0.8 times, and takes 45 us there: not taken.  Normal and uniform [-1, 1)
+// values are at 0.7 times or below throughout.
+int fp32_chain(int64_t k) { return k < 2048 ? 32 : 64; }
 
 bool fp32_tc_wanted(const tl_gemm_problem& p)
 {
@@ -992,7 +998,7 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
     T.kernel = TL_KERNEL_BF16X6;
     T.p.kernel = TL_KERNEL_BF16X6;
     tc_heuristic(h, T.p, TL_KERNEL_BF16X6, &T.s);
-    T.s.promote_k = kFp32Chain;
+    T.s.promote_k = fp32_chain(T.p.k);
     if (check_tc_solution(h, T.p, T.s) != TL_SUCCESS) return TL_SUCCESS;
     const Scratch w = scratch_of(h, T);
     const size_t head = align_up(sizeof(SplitRange) + w.counters * sizeof(int), 256);

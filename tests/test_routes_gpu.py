@@ -415,3 +415,20 @@ def test_split_shares_left_to_the_last(h, env):
     r = subprocess.run([sys.executable, "-c", code], env={**os.environ, **env}, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
     assert r.stdout.split() == split_digests(h)
+
+
+# ---- plain fp32, the sizes at which the CUDA cores would sum in eight groups of k: the relative 2-norm against
+# float64 is no larger than theirs.  Values of one sign with short k, where a chain's two truncations (3.3e-8
+# together) add up instead of averaging out, may take a fifth more ----
+@pytest.mark.parametrize("dist", ["normal", "uniform", "positive"])
+@pytest.mark.parametrize("m,n,k", [(1024, 1024, 320), (2304, 1024, 256), (2048, 1024, 160), (1024, 600, 512), (700, 700, 700),
+                                   (64, 5000, 1003), (1024, 1024, 2048), (300, 400, 4096)])
+def test_fp32_auto_is_as_exact_as_the_cuda_cores(h, m, n, k, dist):
+    c = Case(torch.float32, "TN", m, n, k, dist="normal" if dist == "normal" else "uniform")
+    if dist == "positive":
+        for x in (c.A, c.B, c.a, c.b):
+            x.abs_()
+    ref = c.a @ c.b
+    errs = [float((c.view(c.run(h, kernel)).double() - ref).norm() / ref.norm()) for kernel in ("auto", "simt")]
+    h.device_status()
+    assert errs[0] <= (1.2 if dist == "positive" and k < 512 else 1.0) * errs[1]
