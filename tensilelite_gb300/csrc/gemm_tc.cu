@@ -451,6 +451,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     {
         const int workers = persistent_workers(L.in_dtype, L.out_dtype, cg, L.ctas, L.sm_count, smem);
         kp.par_reduce = par_reduce_enabled() ? tc_par_reduce(kp.split_units, kp.bal_kb, workers, L.shared_gpu) : 0;
+        if (kp.par_reduce == 2 && kp.promote_kb == 0) kp.par_reduce = 0;      // (split_finish: the promoted kernels)
         kp.hand_over_ns = hand_over_ns();
     }
     kp.out_t = L.out_t;

@@ -741,32 +741,32 @@ __device__ __forceinline__ int hand_over(int* ctr, int nsplit, int own, uint64_t
 //   otherwise      the last split to arrive (tile counter) reduces the whole tile and resets it.
 // Every thread passes the same named barriers whether or not it has work, so a warp that gave up on
 // a wait cannot strand the others.
-template <typename TD, bool EPI, int NH>
+// BESIDE: kernels that par_reduce 2 may be asked of (the promoted ones; the others' code stays as short as it was).
+template <typename TD, bool EPI, int NH, bool BESIDE>
 __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& amax, const TileJob& j, bool& ok, int et,
                                              int lane, int half, int row, bool row_ok, int64_t base_c, int64_t base_d,
                                              volatile int* last_flag, volatile int* abort_flag, bool c_staged,
                                              uint32_t c_row)
 {
     constexpr int W = 32 / NH;                      // columns of a chunk per warp
-    const bool par = p.par_reduce == 1;
-    const int chunks = p.bm / 32;
+    const bool beside = BESIDE && p.par_reduce == 2;
+    const bool par = p.par_reduce != 0 && !beside;
     __threadfence();
     ptx::named_sync<NH * 128>();
     if (et == 0) {
-        int go = 0;                                 // the chunks that this split reduces, a bit each
+        int go = 0;                                 // beside: the chunks that this split reduces, a bit each
         if (ok) {
-            int own = 0;
-            for (int c = j.split; c < chunks; c += j.nsplit) own |= 1 << c;
             int* const ctr = p.counters + j.slot;
             const int before = atomicAdd(ctr, 1);
             if (par) {
-                // (bit 8: a split without a share counts itself out all the same)
-                if (wait_counter_ge(ctr, j.nsplit, p.timeout_ns)) go = own | 0x100;
-                else record_error(p, abort_flag, 16);
-            } else if (p.par_reduce == 2) {
+                go = wait_counter_ge(ctr, j.nsplit, p.timeout_ns) ? 1 : 0;
+                if (!go) record_error(p, abort_flag, 16);
+            } else if (beside) {
+                int own = 0;
+                for (int c = j.split; c < p.bm / 32; c += j.nsplit) own |= 1 << c;
                 go = (before & 0xff) == j.nsplit - 1 ? own | (before >> 8) : hand_over(ctr, j.nsplit, own, p.hand_over_ns);
             } else {
-                go = before == j.nsplit - 1 ? (1 << chunks) - 1 : 0;
+                go = before == j.nsplit - 1 ? 1 : 0;
             }
         }
         *last_flag = go;
@@ -775,11 +775,12 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
     const int go = *last_flag;
     if (go) {
         __threadfence();
+        const int chunks = p.bm / 32, step = par ? j.nsplit : 1;
         const size_t slab_elems = static_cast<size_t>(kTcTileN) * p.bm;
         const float* base = p.ws + static_cast<size_t>(j.slot) * p.tail_split * slab_elems +
                             static_cast<size_t>(half) * W * kTcTileN + row;
-        for (int c = 0; c < chunks; ++c) {
-            if (!((go >> c) & 1)) continue;
+        for (int c = par ? j.split : 0; c < chunks; c += step) {
+            if (beside && !((go >> c) & 1)) continue;
             const int m = j.m0 + c * 32 + half * W;
             // two splits' partials at a time are in flight together (the reduction is
             // latency-bound), summed in split order
@@ -828,7 +829,7 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
     }
     if (c_staged) ptx::cp_async_wait0();   // the staging buffer is free again (also on the error path)
     ptx::named_sync<NH * 128>();           // last_flag is reused by the next tile
-    if (et == 0 && go && p.par_reduce != 2) {
+    if (et == 0 && go && !beside) {
         if (!par) p.counters[j.slot] = 0;  // ready for the next launch
         // counts this split out of the tile: the last one resets the counter for the next launch.
         // No fence: the counter only orders the splits' waits (same-address atomics), and the next
@@ -1525,7 +1526,7 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                         for (int i = 0; i < RC; ++i) __stcg(dst + i * kTcTileN, run[i]);
                     }
                     if (tr) trace_mark(p, TL_TRACE_STORED);
-                    split_finish<TD, EPI, NH>(p, amax, j, ok, et, lane, half, row, row_ok2, c2, d2, last_flag, abort_flag,
+                    split_finish<TD, EPI, NH, true>(p, amax, j, ok, et, lane, half, row, row_ok2, c2, d2, last_flag, abort_flag,
                                               false, 0u);
                     if (tr) trace_mark(p, TL_TRACE_REDUCED);
                 }
@@ -1735,7 +1736,7 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 }
                 if (tr) trace_mark(p, TL_TRACE_STORED);
                 if (ok) release_tmem<CG>(&tempty[mbuf], lane);
-                split_finish<TD, EPI, NH>(p, amax, j, ok, et, lane, half, row, row_ok, base_c, base_d, last_flag,
+                split_finish<TD, EPI, NH, false>(p, amax, j, ok, et, lane, half, row, row_ok, base_c, base_d, last_flag,
                                           abort_flag, c_staged, c_row);
                 if (tr) trace_mark(p, TL_TRACE_REDUCED);
             }
