@@ -319,8 +319,8 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     const int pieces = L.pieces < 1 ? 1 : L.pieces;
     const int cg = (L.cg == 2 || L.cg == 4) ? L.cg : 1;     // CTAs per cluster
     const int cta_group = cg >= 2 ? 2 : 1;
-    const bool shared = tc_shared_pieces(pieces, cg, L.bm, L.promote_k, L.split_k, L.stages, L.M, L.N, L.batch,
-                                         L.sm_count);
+    const bool shared = tc_shared_pieces(pieces, cg, L.bm, L.promote_k, L.split_k, L.M, L.N, L.batch, L.sm_count);
+    const int stages = shared ? kTcSharedStages : L.stages;
     const int bm = shared ? 2 * L.bm : L.bm;
     kp.pieces_mode = shared ? 1 : 0;
     for (int i = 0; i < pieces; ++i) {
@@ -353,7 +353,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.alpha = L.alpha;
     kp.beta = L.beta;
     kp.bm = bm;
-    kp.stages = L.stages;
+    kp.stages = stages;
     kp.split_k = L.split_k;
     kp.raster = L.raster;
     kp.tiles_m = static_cast<int>((L.M + bm - 1) / bm);
@@ -364,7 +364,7 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.promote_kb = L.promote_k > 0 ? static_cast<int>((L.promote_k + W - 1) / W) : 0;
     kp.promote_half = pieces > 1 && !shared && L.promote_k > 0 && L.promote_k <= W / 2 ? 1 : 0;
     const int64_t kb_work = shared ? (pieces == 3 ? 6 : 3) : 1;      // products per k-block, for the split rules
-    size_t smem = tc_smem_bytes(bm / cta_group, L.stages);
+    size_t smem = tc_smem_bytes(bm / cta_group, stages);
     kp.epi_bufs = epi_buffers(smem);
     smem += static_cast<size_t>(kp.epi_bufs - 1) * kTcEpiStageBytes;
     const int64_t tiles = static_cast<int64_t>(kp.tiles_m) * kp.tiles_n * L.batch;

@@ -651,8 +651,7 @@ Scratch scratch_of(const tl_handle* h, Prepared& P)
     const int cgp = P.s.macro_tile1 / kTcTileN;
     const int64_t tiles = ((p.n + kTcTileN * cgp - 1) / (kTcTileN * cgp)) * cgp *
                           ((p.m + P.s.macro_tile0 - 1) / P.s.macro_tile0) * p.batch;
-    const int slab_m = tc_shared_pieces(npc, cgp, P.s.macro_tile0, P.s.promote_k, P.s.split_k, P.s.stages, p.m, p.n, p.batch,
-                                        h->sm_count)
+    const int slab_m = tc_shared_pieces(npc, cgp, P.s.macro_tile0, P.s.promote_k, P.s.split_k, p.m, p.n, p.batch, h->sm_count)
                            ? 2 * P.s.macro_tile0 : P.s.macro_tile0;
     w.off_part = w.bytes;
     if (P.s.split_k > 1) {
@@ -1634,12 +1633,19 @@ TL_API tl_status tl_tune(tl_handle* h, const tl_gemm_problem* p, void* D, const 
         cands.push_back(s);
     } else {
         cands = tc_candidates(h, tc_nn_view(*p, kernel) ? nn_view(*p) : *p, kernel);
+        // first what a call without a solution runs: the pick is never slower than that
+        tl_gemm_solution pick;
+        bool view = false;
+        tc_heuristic_viewed(h, *p, kernel, true, &pick, &view);
+        if (check_tc_solution(h, view ? nn_view(*p) : *p, pick) == TL_SUCCESS) cands.insert(cands.begin(), pick);
     }
     // the multicast variant only where A and B are this GPU's memory
-    if (!multicast_ok(A, B, h->device))
+    if (!multicast_ok(A, B, h->device)) {
+        if (kernel != TL_KERNEL_SIMT && !cands.empty()) drop_cluster4(h, &cands[0]);
         cands.erase(std::remove_if(cands.begin(), cands.end(),
                                    [](const tl_gemm_solution& c) { return c.macro_tile1 == 4 * kTcTileN; }),
                     cands.end());
+    }
     if (cands.empty()) return fail(TL_ERR_UNSUPPORTED, "no legal candidate solution");
     if (max_candidates <= 0) max_candidates = 16;
     if (reps <= 0) reps = 10;

@@ -52,19 +52,20 @@ constexpr size_t kTcMaxSmem = 227 * 1024;        // dynamic shared memory a CTA 
 constexpr int kModePlain = 0, kModePromo = 1, kModePieces = 2;
 // warp 0 TMA, warp 1 MMA, then eight, four or sixteen epilogue warps
 constexpr int tc_threads(int mode) { return mode == kModePromo ? 192 : (mode == kModePieces ? 576 : 320); }
-// The fp32-split products run with shared pieces (kModePieces) on the default solution's tile, a
-// promoted CTA pair with its six-slot ring: two of its 128-column tiles side by side, each piece of A
-// and B loaded once per k-block instead of once per product (bf16x3 needs 2 loads for 3 products,
-// bf16x6 3 for 6) and 256-column MMAs, 1536 / 3072 clocks per k-block against 2 x 1035 / 2070.  Only
-// where the 128-column tiles are more than one wave of pairs: below that the wide tile leaves pairs
-// idle (512 x 4096 x 1024: bf16x3 41 us against 36).  Not for an explicit split-k or another ring,
-// which ask for the tile as it stands.
-inline bool tc_shared_pieces(int pieces, int cg, int bm, int promote_k, int split_k, int stages, int64_t M, int64_t N,
-                             int64_t batch, int sm_count)
+// The fp32-split products run with shared pieces (kModePieces) on a promoted CTA pair of 128-column tiles,
+// the default solution's: two of them side by side, each piece of A and B loaded once per k-block instead
+// of once per product (bf16x3 needs 2 loads for 3 products, bf16x6 3 for 6) and 256-column MMAs, 1536 / 3072
+// clocks per k-block against 2 x 1035 / 2070.  Only where the 128-column tiles are more than one wave of
+// pairs: below that the wide tile leaves pairs idle (512 x 4096 x 1024: bf16x3 41 us against 36).  Not for an
+// explicit split-k, which asks for the tile as it stands.  The ring has kTcSharedStages slots whatever depth
+// the solution names: its depth is for the 24 KB stages of single products, and says nothing about which
+// loads to make.
+constexpr int kTcSharedStages = 6;
+inline bool tc_shared_pieces(int pieces, int cg, int bm, int promote_k, int split_k, int64_t M, int64_t N, int64_t batch,
+                             int sm_count)
 {
     const int64_t tiles = ((M + 127) / 128) * ((N + 255) / 256) * batch;
-    return pieces > 1 && cg == 2 && bm == 128 && promote_k > 0 && split_k == 1 && stages == 6 && M > 128 &&
-           2 * tiles > sm_count;
+    return pieces > 1 && cg == 2 && bm == 128 && promote_k > 0 && split_k == 1 && M > 128 && 2 * tiles > sm_count;
 }
 
 // Magnitudes of the two operands of a split-precision product, gathered by the split pass: the bits of

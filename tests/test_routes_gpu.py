@@ -432,3 +432,49 @@ def test_fp32_auto_is_as_exact_as_the_cuda_cores(h, m, n, k, dist):
     errs = [float((c.view(c.run(h, kernel)).double() - ref).norm() / ref.norm()) for kernel in ("auto", "simt")]
     h.device_status()
     assert errs[0] <= (1.2 if dist == "positive" and k < 512 else 1.0) * errs[1]
+
+
+# ---- tuning: no slower than no solution ----
+def _median_us(run, reps=7):
+    run(), run()
+    times = []
+    for _ in range(reps):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        for _ in range(5):
+            run()
+        e1.record()
+        torch.cuda.synchronize()
+        times.append(e0.elapsed_time(e1) * 200)
+    return sorted(times)[reps // 2]
+
+
+@pytest.mark.parametrize("kernel", ["bf16x3", "bf16x6"])
+def test_tuned_split_products_keep_the_shared_pieces(kernel):
+    h = tl.Handle()
+    c = Case(torch.float32, "TN", 4096, 4096, 2048)
+    p = tl.Problem.make(4096, 4096, 2048, dtype="fp32", trans_a=True, kernel=kernel)
+    D = torch.empty_like(c.C)
+    run = lambda: h.gemm(p, D, None, c.A, c.B)
+    before = _median_us(run)
+    h.tune(p, D, None, c.A, c.B, max_candidates=3, reps=3)
+    assert _median_us(run) <= 1.2 * before
+    # the ring's depth does not choose the algorithm: a deeper ring is no slower
+    s = h.default_solution(p)
+    s.stages = 8
+    assert _median_us(lambda: h.gemm(p, D, None, c.A, c.B, solution=s)) <= 1.2 * before
+    h.close()
+
+
+@pytest.mark.parametrize("dtype,kernel", [("fp32", "bf16x6"), ("bf16", "auto"), ("fp8", "auto")])
+def test_the_first_candidate_is_the_default(dtype, kernel):
+    h = tl.Handle()
+    m, n, k = 1152, 2048, 1024
+    t = {"fp32": torch.float32, "bf16": torch.bfloat16, "fp8": torch.float8_e4m3fn}[dtype]
+    A, B = torch.randn(m * k, device="cuda").to(t), torch.randn(n * k, device="cuda").to(t)
+    D = torch.empty(m * n, device="cuda", dtype=torch.bfloat16 if dtype == "fp8" else t)
+    p = tl.Problem.make(m, n, k, dtype=dtype, out_dtype="bf16" if dtype == "fp8" else dtype, trans_a=True, kernel=kernel)
+    best, ms = h.tune(p, D, None, A, B, max_candidates=1, reps=2)
+    want = h.default_solution(p)
+    assert ms > 0 and best.as_dict() == want.as_dict()
+    h.close()
