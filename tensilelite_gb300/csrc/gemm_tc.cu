@@ -363,6 +363,15 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.kb_elems = W;
     kp.promote_kb = L.promote_k > 0 ? static_cast<int>((L.promote_k + W - 1) / W) : 0;
     kp.promote_half = pieces > 1 && !shared && L.promote_k > 0 && L.promote_k <= W / 2 ? 1 : 0;
+    // Shared pieces of bf16x6 have the time for shorter chains than asked for: every MMA into a chain drops
+    // bits, every chain that the epilogue adds is a rounding, so the longer k the longer the chain that
+    // balances them.  The small products' sum drops bits too and starts anew every 1024 k.  Relative 2-norm of
+    // uniform [-1, 1) values, chains of 256 as asked for and of this rule: k 512 1.9e-7 and 0.8e-7, 2048 2.0e-7
+    // and 1.2e-7, 4096 2.1e-7 and 1.4e-7, 8192 2.3e-7 and 1.9e-7; largest error over largest value 3.5e-7 and
+    // 1.9e-7, 3.3e-7 and 2.8e-7, 3.4e-7 and 3.5e-7, 3.9e-7 and 3.8e-7.  bf16x3's errors are those of the products that
+    // it leaves out (3.8e-6) whatever the chain.
+    if (shared && pieces == 3) kp.promote_kb = std::min(kp.promote_kb, L.K < 3072 ? 1 : (L.K < 6144 ? 2 : 3));
+    kp.small_chains = pieces == 3 ? std::max(1, 16 / std::max(1, kp.promote_kb)) : INT32_MAX;
     const int64_t kb_work = shared ? (pieces == 3 ? 6 : 3) : 1;      // products per k-block, for the split rules
     size_t smem = tc_smem_bytes(bm / cta_group, stages);
     kp.epi_bufs = epi_buffers(smem);

@@ -52,6 +52,7 @@ struct TcKernelParams {
     int promote_kb;               // >0: the A0*B0 product restarts its TMEM chain every promote_kb
                                   // k-blocks; the epilogue adds each chain into fp32 registers
     int promote_half;             // two A0*B0 chains per k-block (16-bit pieces, promote_kb 1)
+    int small_chains;             // kModePieces: the small products' accumulator starts anew every so many chains
     int tiles_m, tiles_n;
     int narrow;                   // work units, tiles and split k-block products fit 32 bits, no balanced split
     int64_t total_work;
@@ -844,11 +845,9 @@ __device__ __forceinline__ void split_finish(const TcKernelParams& p, float& ama
 //   kModePieces  promoted accumulation of the split-precision products, each piece of an operand staged
 //                once per k-block for all the products that use it; 256-column tiles, sixteen epilogue
 //                warps with 64 running sums per thread.  The A0*B0 chain and the small products have one
-//                accumulator each, so the errors are those of the tiles that load every product's pieces.
-//                All products in one accumulator, with chains of one or two k-blocks in two buffers, left
-//                larger errors (bf16x6 8192^3, largest error over largest value 4.8e-7 against 3.6e-7) and
-//                were no faster (4096^3: bf16x6 489 us against 476, bf16x3 303 both; 3072 x 3072 x 64, where a
-//                tile waits for the one before it, 24.5 against 25.2).
+//                accumulator each.  With all products in one accumulator and two of those alternating,
+//                every product but a chain's first dropped the bits of a sum at full magnitude (bf16x6
+//                8192^3, largest error over largest value 5.3e-7).
 //   kModePlain   the others: eight epilogue warps, two per quarter of the TMEM lanes,
 // which take alternate column groups of a tile (half the drain time of a CTA's last tile, and of every
 // tile whose k is too short to hide it).  GROUP: the work units and problems come from a plan's tables.
@@ -1178,7 +1177,7 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 get_job<GROUP>(p, w, u, j);
                 const int nkb = j.kb1 - j.kb0;
                 if (nkb <= 0) continue;                 // an empty unit of a balanced split
-                if (sep_small) {
+                if (sep_small && !PIECES) {
                     if (!ptx::mbar_wait(&sempty[sbuf], sph ^ 1u, tlim)) {
                         record_error(p, abort_flag, 2);
                         break;
@@ -1199,15 +1198,17 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 if constexpr (PIECES) {
                     // A k-block's pieces arrive smallest first in nvirt consecutive slots; every product
                     // of them is formed from there and a slot is released by its last product.  The small
-                    // products of the whole tile share one accumulator, the A0*B0 products another that
-                    // starts anew every promote_kb k-blocks.  There is one of each: a chain is drained while
-                    // the next k-block's small products run, and the last chain, whose A0*B0 goes first
-                    // in its last k-block, while the small sums are completed.
+                    // products share one accumulator, which starts anew every small_chains chains, the
+                    // A0*B0 products another that starts anew every promote_kb k-blocks.  There is one of
+                    // each: a chain is drained while the next k-block's small products run, the small sums
+                    // while the last A0*B0 of the chain that they end with does.
                     const uint32_t d_small = tmem_base + bmu;
                     uint32_t small_acc = 0, main_acc = 0;
-                    int in_chain = 0;
+                    int in_chain = 0, chains = 0;
                     for (int kb = 0; kb < nkb; ++kb) {
                         const bool last = kb == nkb - 1;
+                        const bool chain_ends = in_chain + 1 == p.promote_kb || last;
+                        const bool small_ends = last || (chain_ends && chains + 1 == p.small_chains);
                         uint32_t sl[3], dn[3];
 #pragma unroll
                         for (int v = 0; v < 3; ++v) {
@@ -1230,32 +1231,16 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                         if (!ok) break;
                         ptx::tc_fence_after();
                         const uint32_t d0 = nvirt == 3 ? dn[2] : dn[1];          // dn: pieces (2,) 1, 0
-                        auto main_mma = [&] {
-                            if (in_chain == 0) {
-                                if (!ptx::mbar_wait(&tempty[0], mph ^ 1u, tlim)) {
-                                    record_error(p, abort_flag, 2);
-                                    ok = false;
-                                    return;
-                                }
-                                ptx::tc_fence_after();
-                                main_acc = 0;
-                            }
-                            ptx::mma_kblock<KIND, CG>(tmem_base, d0, d0 + dNM, dhi, idesc, main_acc, n_kstep, m_kstep);
-                            main_acc = 1;
-                            if (++in_chain == p.promote_kb || last) {
-                                ptx::mma_commit_pair(ptx::smem_u32(&tfull[0]), pair_mask);
-                                mph ^= 1u;
-                                in_chain = 0;
-                            }
-                        };
                         auto mma = [&](uint32_t n, uint32_t m) {
                             ptx::mma_kblock<KIND, CG>(d_small, n, m + dNM, dhi, idesc, small_acc, n_kstep, m_kstep);
                             small_acc = 1;
                         };
-                        // (a chain that starts here would wait for the one before it; a tile's first does not)
-                        const bool main_first = last && (in_chain != 0 || kb == 0);
-                        if (main_first) main_mma();
-                        if (!ok) break;
+                        if (small_acc == 0 && !ptx::mbar_wait(&sempty[0], sph ^ 1u, tlim)) {
+                            record_error(p, abort_flag, 2);
+                            ok = false;
+                            break;
+                        }
+                        ptx::tc_fence_after();
                         if (nvirt == 3) {
                             mma(dn[2], dn[0]);
                             mma(dn[1], dn[1]);
@@ -1269,9 +1254,30 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                             mma(dn[0], dn[1]);
                             ptx::mma_commit_pair(sl[0], 0x3);
                         }
-                        if (last) ptx::mma_commit_pair(ptx::smem_u32(&sfull[0]), pair_mask);
-                        if (!main_first) main_mma();
-                        if (!ok) break;
+                        if (small_ends) {
+                            ptx::mma_commit_pair(ptx::smem_u32(&sfull[0]), pair_mask);
+                            sph ^= 1u;
+                            small_acc = 0;
+                        }
+                        if (in_chain == 0) {
+                            if (!ptx::mbar_wait(&tempty[0], mph ^ 1u, tlim)) {
+                                record_error(p, abort_flag, 2);
+                                ok = false;
+                                break;
+                            }
+                            ptx::tc_fence_after();
+                            main_acc = 0;
+                        }
+                        ptx::mma_kblock<KIND, CG>(tmem_base, d0, d0 + dNM, dhi, idesc, main_acc, n_kstep, m_kstep);
+                        main_acc = 1;
+                        ++in_chain;
+                        if (chain_ends) {
+                            ptx::mma_commit_pair(ptx::smem_u32(&tfull[0]), pair_mask);
+                            mph ^= 1u;
+                            in_chain = 0;
+                            ++chains;
+                        }
+                        if (small_ends) chains = 0;
                         ptx::mma_commit_pair(nvirt == 3 ? sl[2] : sl[1], 0x3);
                     }
                 } else if constexpr (!PROMO) {
@@ -1318,7 +1324,6 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 if (!ok) break;
                 if constexpr (PIECES) {              // handed over in the loop; one buffer of each kind
                     if (w == unit0) trace_mark(p, TL_TRACE_MMA_LAST);
-                    sph ^= 1u;
                     continue;
                 }
                 if constexpr (CG == 2) ptx::mma_commit_pair(ptx::smem_u32(&tfull[mbuf]), pair_mask);
@@ -1395,9 +1400,11 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                 for (int i = 0; i < RC; ++i) run[i] = 0.f;
                 const int nkb = j.kb1 - j.kb0;
                 const int nchain = PROMO && p.promote_half ? 2 * nkb : (nkb + p.promote_kb - 1) / p.promote_kb;
-                const int steps = nchain + (sep_small ? 1 : 0);
-                for (int c = 0; c < steps; ++c) {
-                    const bool sm = c == nchain;          // the small terms, after the chains
+                // the small terms: after the chains, or (one buffer of each kind) before the chain that they end
+                // with, the last one and every small_chains'th
+                int left = nchain, chains = 0;
+                bool sm = PIECES && (left == 1 || p.small_chains == 1);
+                while (left > 0 || sm) {
                     uint64_t* const full_bar = sm ? &sfull[sbuf] : &tfull[mbuf];
                     bool got = ok && ptx::mbar_wait(full_bar, sm ? sph : mph, tlim);
                     got = __all_sync(0xffffffffu, got);
@@ -1422,9 +1429,14 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                     if (sm) {
                         if (!PIECES) sbuf ^= 1u;
                         if (sbuf == 0) sph ^= 1u;
+                        sm = false;
+                        chains = -1;
                     } else {
                         if (!PIECES) mbuf ^= 1u;
                         if (mbuf == 0) mph ^= 1u;
+                        --left;
+                        ++chains;
+                        sm = PIECES ? left == 1 || (left > 0 && chains + 1 == p.small_chains) : sep_small && left == 0;
                     }
                 }
                 if (tr) trace_mark(p, TL_TRACE_ACC_READY);

@@ -952,8 +952,10 @@ constexpr double kFp32TcWork = 3.0e8;
 // is left: values of one sign, k below 512 and too few tiles for the shared pieces, up to 1.16 times the CUDA
 // cores' error, whose sums run in eight groups there.  With the rounding errors of the epilogue's sums added back
 // (two-sum) it is 0.8 times, and takes 45 us there: not taken.  Normal and uniform [-1, 1)
-// values are at 0.7 times or below throughout.
-int fp32_chain(int64_t k) { return k < 2048 ? 32 : 64; }
+// values are at 0.7 times or below throughout.  With shared pieces the CUDA cores' sums are serial and their
+// errors larger by far; there two k-blocks balance dropped bits and roundings from k = 5120 on (normal
+// values, k 4096: 1.56e-7, with two 1.58e-7; 8192: 2.2e-7 and 1.9e-7).
+int fp32_chain(int64_t k, bool shared) { return k < 2048 ? 32 : (shared && k >= 5120 ? 128 : 64); }
 
 bool fp32_tc_wanted(const tl_gemm_problem& p)
 {
@@ -997,7 +999,8 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
     T.kernel = TL_KERNEL_BF16X6;
     T.p.kernel = TL_KERNEL_BF16X6;
     tc_heuristic(h, T.p, TL_KERNEL_BF16X6, &T.s);
-    T.s.promote_k = fp32_chain(T.p.k);
+    T.s.promote_k = fp32_chain(T.p.k, tc_shared_pieces(split_pieces(T.kernel), T.s.macro_tile1 / kTcTileN, T.s.macro_tile0,
+                                                       T.s.promote_k, T.s.split_k, T.p.m, T.p.n, T.p.batch, h->sm_count));
     if (check_tc_solution(h, T.p, T.s) != TL_SUCCESS) return TL_SUCCESS;
     const Scratch w = scratch_of(h, T);
     const size_t head = align_up(sizeof(SplitRange) + w.counters * sizeof(int), 256);
