@@ -198,8 +198,10 @@ TL_API tl_status tl_gemm(tl_handle* handle, const tl_gemm_problem* problem,
  * `best`; the result is cached in the handle and, if `cache_path` is non-NULL, merged into that
  * JSON file keyed by device and problem.  A candidate whose launches report a device error (a
  * bounded wait that ran out) is dropped, never returned or cached.  When D == C with beta != 0 the
- * candidates write a scratch output instead, so C is left intact.  Synchronous.  Replaces
- * test/perf_test.py:58-167. */
+ * candidates write a scratch output instead, so C is left intact.  A plain fp32 problem (kernel AUTO)
+ * is timed as tl_gemm runs it without a solution, which may be on the tensor cores: *best then names the
+ * CUDA-core kernel as always, and neither it in the cache nor a loaded entry keeps tl_gemm with solution NULL from
+ * those launches.  Synchronous.  Replaces test/perf_test.py:58-167. */
 TL_API tl_status tl_tune(tl_handle* handle, const tl_gemm_problem* problem, void* D, const void* C,
                          const void* A, const void* B, int max_candidates, int reps,
                          const char* cache_path, tl_gemm_solution* best, float* best_ms);

@@ -616,7 +616,7 @@ struct Prepared {
     bool own_scratch = false;            // scratch of this call alone: it may run beside others (TcLaunch::shared_gpu)
     tl_epilogue epi{};
     bool epi_on = false;
-    bool tuned = false;      // the solution was tuned or loaded
+    bool tuned = false;      // a tuned or loaded solution runs
     bool tview = false;      // p is the transposed view of the caller's NN problem (tc_nn_view)
 };
 
@@ -744,6 +744,7 @@ tl_status prepare(tl_handle* h, const tl_gemm_problem* prob, const tl_gemm_solut
         if (p.kernel == TL_KERNEL_AUTO && !sol && p.dtype_d != TL_DTYPE_FP8_E4M3) {
             kernel = TL_KERNEL_SIMT;
             simt_solution(&P.s);
+            P.tuned = false;          // a solution for aligned operands of these sizes
             if (P.tview) {            // the CUDA-core kernel takes the caller's problem as it is
                 P.p = *prob;
                 P.A = B;
@@ -1480,7 +1481,9 @@ TL_API tl_status tl_gemm(tl_handle* h, const tl_gemm_problem* p, const tl_gemm_s
     const bool capturing = t_capturing;
     t_capturing = false;
     if (st != TL_SUCCESS) return st;
-    if (!s && !capturing && P.kernel == TL_KERNEL_SIMT && !P.tuned && fp32_tc_wanted(*p)) {
+    // (a tuned or loaded entry does not hold a plain fp32 problem on the CUDA cores: their tile is all such an
+    // entry can name, and the tuner times the call as it runs here)
+    if (!s && !capturing && P.kernel == TL_KERNEL_SIMT && fp32_tc_wanted(*p)) {
         bool done = false;
         st = gemm_fp32_tc(h, P, S(stream), &done);
         if (done) return st;
@@ -1698,14 +1701,23 @@ TL_API tl_status tl_tune(tl_handle* h, const tl_gemm_problem* p, void* D, const 
         }
         return true;
     };
+    // a plain fp32 problem that tl_gemm takes to the tensor cores is timed as it runs there
+    auto launch = [&](const Prepared& P) {
+        if (P.kernel == TL_KERNEL_SIMT && fp32_tc_wanted(*p)) {
+            bool done = false;
+            const tl_status r = gemm_fp32_tc(h, P, s, &done);
+            if (done) return r;
+        }
+        return enqueue(h, P, s);
+    };
     for (const auto& c : cands) {
         Prepared P;
         if (prepare(h, p, &c, Dt, C, A, B, &P) != TL_SUCCESS) continue;
-        if (enqueue(h, P, s) != TL_SUCCESS) continue;          // warm-up
+        if (launch(P) != TL_SUCCESS) continue;          // warm-up
         if (!device_clean(c)) continue;
         cudaEventRecord(e0, s);
         bool ok = true;
-        for (int r = 0; r < reps && ok; ++r) ok = enqueue(h, P, s) == TL_SUCCESS;
+        for (int r = 0; r < reps && ok; ++r) ok = launch(P) == TL_SUCCESS;
         cudaEventRecord(e1, s);
         if (!ok || cudaEventSynchronize(e1) != cudaSuccess) { cudaGetLastError(); continue; }
         if (!device_clean(c)) continue;

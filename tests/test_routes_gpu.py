@@ -478,3 +478,45 @@ def test_the_first_candidate_is_the_default(dtype, kernel):
     want = h.default_solution(p)
     assert ms > 0 and best.as_dict() == want.as_dict()
     h.close()
+
+
+def test_tuned_fp32_keeps_the_tensor_cores(tmp_path):
+    h = tl.Handle()
+    c = Case(torch.float32, "TN", 1024, 1024, 1024)
+    p = tl.Problem.make(1024, 1024, 1024, dtype="fp32", trans_a=True)
+    D = torch.empty_like(c.C)
+    run = lambda handle=h, **kw: handle.gemm(p, D, None, c.A, c.B, **kw)
+
+    def launches(handle):
+        l0 = handle.launch_count()
+        run(handle)
+        return handle.launch_count() - l0
+
+    assert launches(h) == 4
+    want = D.clone()
+    path = str(tmp_path / "tuned.json")
+    best, ms = h.tune(p, D, None, c.A, c.B, reps=5, cache_path=path)
+    h.check_solution(p, best)
+    simt = _median_us(lambda: run(solution=best))
+    assert best.kernel == tl.KERNEL_SIMT and ms * 1e3 < 0.75 * simt
+    assert launches(h) == 4 and torch.equal(D.view(torch.int32), want.view(torch.int32))
+    h2 = tl.Handle()
+    assert h2.load_solutions(path) == 1 and launches(h2) == 4
+    h2.close()
+    h.close()
+
+
+def test_tuned_for_aligned_operands_leaves_unaligned_ones_their_route():
+    h = tl.Handle()
+    c = Case(torch.bfloat16, "TN", 640, 768, 512)
+    p = tl.Problem.make(640, 768, 512, dtype="bf16", trans_a=True)
+    D = torch.empty_like(c.C)
+    h.tune(p, D, None, c.A, c.B, max_candidates=2, reps=2)
+    A = torch.empty(c.A.numel() + 1, dtype=c.A.dtype, device="cuda")[1:]
+    A.copy_(c.A)
+    l0 = h.launch_count()
+    h.gemm(p, D, None, A, c.B)
+    assert h.launch_count() - l0 == 2          # aligned copies, tensor cores
+    c.check(D)
+    h.device_status()
+    h.close()
