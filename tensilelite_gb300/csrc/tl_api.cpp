@@ -844,7 +844,9 @@ SimtLaunch simt_launch_of(const Prepared& P, float alpha)
     return L;
 }
 
-tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
+// `behind`: a CUDA-core launch that stands in for the tensor-core one where the operands' magnitudes call for it;
+// the two are timed as one, since either may be the one that does the work.
+tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s, const SimtLaunch* behind = nullptr)
 {
     const tl_gemm_problem& p = P.p;
     if (p.m == 0 || p.n == 0) return TL_SUCCESS;
@@ -921,7 +923,8 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s)
     L.debug_flags = P.s.debug_flags;
     L.out_t = P.tview ? 1 : 0;
     const bool timed = timing_begin(h, s);
-    const tl_status st = tc_gemm_launch(L, s, &h->launches);
+    tl_status st = tc_gemm_launch(L, s, &h->launches);
+    if (st == TL_SUCCESS && behind) st = simt_gemm_launch(*behind, s, &h->launches);
     timing_end(h, s, timed, st);
     return st;
 }
@@ -1020,11 +1023,10 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
     tl_status st = TL_SUCCESS;
     cudaError_t e = cudaMemsetAsync(base, 0, head, s);
     if (e != cudaSuccess) st = cuda_fail(e, "cudaMemsetAsync(fp32 scratch)");
-    if (st == TL_SUCCESS) st = enqueue(h, T, s);
     if (st == TL_SUCCESS) {
         SimtLaunch L = simt_launch_of(P, P.p.alpha * scale_of(P.p.scale_a) * scale_of(P.p.scale_b));
         L.unless = T.range;
-        st = simt_gemm_launch(L, s, &h->launches);
+        st = enqueue(h, T, s, &L);
     }
     e = cudaFreeAsync(mem, s);
     if (st == TL_SUCCESS && e != cudaSuccess) st = cuda_fail(e, "cudaFreeAsync(fp32 scratch)");

@@ -520,3 +520,22 @@ def test_tuned_for_aligned_operands_leaves_unaligned_ones_their_route():
     c.check(D)
     h.device_status()
     h.close()
+
+
+# ---- kernel timing of a plain fp32 GEMM: the launch that did the work, whichever it was ----
+def test_kernel_timing_of_out_of_range_operands():
+    h = tl.Handle()
+    c = Case(torch.float32, "TN", 2048, 2048, 1024)
+    c.A[77] = float("inf")
+    c.run(h), c.run(h, "simt")
+    h.set_kernel_timing(True)
+    h.kernel_timing(reset=True)
+    for _ in range(4):
+        c.run(h)
+    auto, n = h.kernel_timing(reset=True)
+    assert n == 4
+    for _ in range(4):
+        c.run(h, "simt")
+    simt, n = h.kernel_timing(reset=True)
+    assert n == 4 and auto >= 0.9 * simt
+    h.close()
