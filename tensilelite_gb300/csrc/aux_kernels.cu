@@ -438,8 +438,8 @@ static cudaError_t launch_dependent(void (*kern)(KArgs...), int grid, int thread
 
 // ---- padded copies --------------------------------------------------------------------------------
 // Bound by memory: 2 B read and 2 B written per element.  The source's columns start on any even
-// address, so a lane reads the aligned words that hold its eight elements, shifts them into place if
-// they start in the middle of a word, and writes one 16-byte vector.  A warp takes 256 rows of a column
+// address, so a lane reads the aligned words that lie whole in its eight elements and a half word at either
+// end, shifts them into place if they start in the middle of a word, and writes one 16-byte vector.  A warp takes 256 rows of a column
 // at a time: one index division per warp and 512 bytes.
 struct PadArgs {
     PadOperand op[3];
@@ -468,14 +468,8 @@ __global__ void __launch_bounds__(256) pad_kernel(const __grid_constant__ PadArg
         const uint16_t* src = o.src + b * o.batch_stride + col * o.ld + r;
         uint32_t v[4];
         if (o.rows - r >= 8) {
-            const bool odd = (reinterpret_cast<uintptr_t>(src) & 2) != 0;
-            const uint32_t* words = reinterpret_cast<const uint32_t*>(src - (odd ? 1 : 0));
-            uint32_t q[5];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) q[e] = __ldg(words + e);
-            q[4] = odd ? __ldg(words + 4) : 0u;
-#pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = odd ? __funnelshift_r(q[e], q[e + 1], 16) : q[e];
+            load_eight16((reinterpret_cast<uintptr_t>(src) & 2) != 0, [&](int e) { return static_cast<uint32_t>(__ldg(src + e)); },
+                         [&](int e) { return __ldg(reinterpret_cast<const uint32_t*>(src + e)); }, v);
         } else {
             const int left = static_cast<int>(o.rows - r);
 #pragma unroll

@@ -232,6 +232,27 @@ struct PadOperand {
     int64_t pld, p_batch_stride;
 };
 tl_status aux_pad16(const PadOperand* ops, int count, cudaStream_t s, int64_t* launches);
+// Eight 16-bit elements that start on an even address, as four words: half(i) reads element i, word(i) elements
+// i and i + 1 (4-byte aligned).  `odd`: the first starts in the middle of a word.  Nothing outside the eight
+// is read.
+template <class Half, class Word>
+#ifdef __CUDACC__
+__device__ __forceinline__
+#else
+inline
+#endif
+void load_eight16(bool odd, Half half, Word word, uint32_t (&v)[4])
+{
+    if (!odd) {
+        for (int e = 0; e < 4; ++e) v[e] = word(2 * e);
+        return;
+    }
+    const uint32_t first = half(0), w0 = word(1), w1 = word(3), w2 = word(5), last = half(7);
+    v[0] = first | (w0 << 16);
+    v[1] = (w0 >> 16) | (w1 << 16);
+    v[2] = (w1 >> 16) | (w2 << 16);
+    v[3] = (w2 >> 16) | (last << 16);
+}
 // The way back: rows x cols of `dst` (pld, p_batch_stride) to `src`'s place; the gaps stay as they are.
 tl_status aux_unpad16(const PadOperand& op, cudaStream_t s, int64_t* launches);
 // Per-tensor E4M3 quantisation: *amax_dev = max |x|, dst = e4m3(x * 448 / amax), *scale_out_dev = amax / 448.

@@ -26,3 +26,20 @@ def host_program(tmp_path, body):
 def test_splits_rely_on_each_other_only_alone(tmp_path, units, workers, beside_others, mode):
     out = host_program(tmp_path, f'    printf("%d", tc_par_reduce({units}, 0, {workers}, {beside_others}));')
     assert out == [str(mode)]
+
+
+@pytest.mark.parametrize("odd", [0, 1])
+def test_eight_halves_read_nothing_else(tmp_path, odd):
+    """Elements 1 .. 8 of a guarded buffer: the values in order, and no read outside [0, 8)."""
+    body = f"""
+    uint16_t src[8];
+    for (int i = 0; i < 8; ++i) src[i] = static_cast<uint16_t>(0x1100 * (i + 1) + i);
+    int low = 100, high = -100;
+    const auto seen = [&](int a, int b) {{ if (a < low) low = a; if (b > high) high = b; }};
+    uint32_t v[4];
+    load_eight16({odd}, [&](int e) {{ seen(e, e); return static_cast<uint32_t>(src[e & 7]); }},
+                 [&](int e) {{ seen(e, e + 1); return src[e & 7] | (static_cast<uint32_t>(src[(e + 1) & 7]) << 16); }}, v);
+    int bad = 0;
+    for (int i = 0; i < 8; ++i) bad += (v[i / 2] >> (16 * (i & 1)) & 0xffff) != src[i];
+    printf("%d %d %d", low, high, bad);"""
+    assert host_program(tmp_path, body) == ["0", "7", "0"]
