@@ -626,6 +626,9 @@ int64_t operand_span(int64_t ld, int64_t cols, int64_t batch, int64_t bstride, i
     return (batch - 1) * bstride + (cols - 1) * ld + rows;
 }
 
+// Matrices of a batched operand that differ: one where every problem of the batch reads the same.
+int64_t distinct(int64_t batch, int64_t stride) { return stride == 0 ? 1 : batch; }
+
 // Scratch of a tensor-core launch: [split pieces of A][split pieces of B][split-k partials].
 struct Scratch {
     size_t bytes = 0, off_a[3] = {0, 0, 0}, off_b[3] = {0, 0, 0}, off_part = 0, part_bytes = 0, counters = 0;
@@ -643,10 +646,11 @@ Scratch scratch_of(const tl_handle* h, Prepared& P)
         // against 340)
         P.a_ld = static_cast<int64_t>(align_up(static_cast<size_t>(a_rows), 64));
         P.b_ld = static_cast<int64_t>(align_up(static_cast<size_t>(b_rows), 64));
-        P.a_bs = P.a_ld * a_cols;
-        P.b_bs = P.b_ld * b_cols;
-        for (int i = 0; i < npc; ++i) { w.off_a[i] = w.bytes; w.bytes = align_up(w.bytes + P.a_bs * p.batch * 2, 256); }
-        for (int i = 0; i < npc; ++i) { w.off_b[i] = w.bytes; w.bytes = align_up(w.bytes + P.b_bs * p.batch * 2, 256); }
+        const int64_t a_mats = distinct(p.batch, p.stride_a), b_mats = distinct(p.batch, p.stride_b);
+        P.a_bs = a_mats == 1 ? 0 : P.a_ld * a_cols;
+        P.b_bs = b_mats == 1 ? 0 : P.b_ld * b_cols;
+        for (int i = 0; i < npc; ++i) { w.off_a[i] = w.bytes; w.bytes = align_up(w.bytes + P.a_ld * a_cols * a_mats * 2, 256); }
+        for (int i = 0; i < npc; ++i) { w.off_b[i] = w.bytes; w.bytes = align_up(w.bytes + P.b_ld * b_cols * b_mats * 2, 256); }
     }
     const int cgp = P.s.macro_tile1 / kTcTileN;
     const int64_t tiles = ((p.n + kTcTileN * cgp - 1) / (kTcTileN * cgp)) * cgp *
@@ -874,9 +878,9 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s, const SimtLau
         const int64_t a_rows = p.trans_a ? p.k : p.m, a_cols = p.trans_a ? p.m : p.k;
         const int64_t b_rows = p.trans_b ? p.n : p.k, b_cols = p.trans_b ? p.k : p.n;
         const SplitOperand ops[2] = {
-            {static_cast<const float*>(P.A), a_rows, a_cols, p.lda, p.batch, p.stride_a, {P.a_pc[0], P.a_pc[1], P.a_pc[2]},
+            {static_cast<const float*>(P.A), a_rows, a_cols, p.lda, distinct(p.batch, p.stride_a), p.stride_a, {P.a_pc[0], P.a_pc[1], P.a_pc[2]},
              P.a_ld, P.a_bs},
-            {static_cast<const float*>(P.B), b_rows, b_cols, p.ldb, p.batch, p.stride_b, {P.b_pc[0], P.b_pc[1], P.b_pc[2]},
+            {static_cast<const float*>(P.B), b_rows, b_cols, p.ldb, distinct(p.batch, p.stride_b), p.stride_b, {P.b_pc[0], P.b_pc[1], P.b_pc[2]},
              P.b_ld, P.b_bs}};
         const tl_status st = aux_split_bf16(ops, 2, L.pieces, P.range, s, &h->launches);
         if (st != TL_SUCCESS) return st;
@@ -1083,11 +1087,12 @@ tl_status gemm_pad16(tl_handle* h, const Prepared& P, cudaStream_t s, bool* done
     const auto copy = [&](bool always, const void* X, int64_t rows, int64_t cols, int64_t room, int64_t* ld, int64_t* stride) {
         if (!always && lines(X, *ld, *stride)) return -1;
         PadOperand& o = ops[count];
-        o = {static_cast<const uint16_t*>(X), rows, cols, *ld, p.batch, *stride, nullptr, 0, 0};
+        const int64_t mats = p.batch > 1 ? distinct(p.batch, *stride) : 1;
+        o = {static_cast<const uint16_t*>(X), rows, cols, *ld, mats, *stride, nullptr, 0, 0};
         o.pld = *ld = static_cast<int64_t>(align_up(static_cast<size_t>(rows), 64));
-        o.p_batch_stride = *stride = o.pld * cols;
+        o.p_batch_stride = *stride = mats == 1 ? 0 : o.pld * cols;
         at[count] = bytes;
-        bytes += align_up(static_cast<size_t>(o.p_batch_stride * p.batch + o.pld * (room - cols)) * 2, 256);
+        bytes += align_up(static_cast<size_t>(o.pld * (cols * mats + room - cols)) * 2, 256);
         return count++;
     };
     const int ia = copy(out && m8 != m, P.A, p.trans_a ? p.k : m, p.trans_a ? m : p.k, p.trans_a ? m8 : p.k, &p.lda, &p.stride_a);

@@ -539,3 +539,36 @@ def test_kernel_timing_of_out_of_range_operands():
     simt, n = h.kernel_timing(reset=True)
     assert n == 4 and auto >= 0.9 * simt
     h.close()
+
+
+# ---- one matrix for a whole batch (stride 0): its pieces and aligned copies are made once ----
+@pytest.mark.parametrize("which", ["A", "B"])
+@pytest.mark.parametrize("dtype,kernel,k", [(torch.float32, "bf16x3", 1024), (torch.float32, "bf16x6", 1024), (torch.float32, "auto", 1024),
+                                            (torch.bfloat16, "auto", 1023)])
+def test_one_matrix_for_a_whole_batch(dtype, kernel, k, which):
+    h = tl.Handle()
+    batch, big, small = 48, 2048, 64
+    m, n = (big, small) if which == "A" else (small, big)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    one = lambda r: torch.randn(r * k, device="cuda", generator=g).to(dtype)
+    many = lambda r: torch.randn(batch * r * k, device="cuda", generator=g).to(dtype)
+    A, B = (one(m), many(n)) if which == "A" else (many(m), one(n))
+    D = torch.full((batch * m * n,), float("nan"), dtype=dtype, device="cuda")
+    p = tl.Problem.make(m, n, k, dtype=tl.torch_dtype_code(dtype), trans_a=True, kernel=kernel, batch=batch)
+    setattr(p, "stride_a" if which == "A" else "stride_b", 0)
+    h.gemm(tl.Problem.make(64, 64, 64, dtype="bf16", trans_a=True), torch.empty(4096, device="cuda", dtype=torch.bfloat16), None,
+           torch.zeros(4096, device="cuda", dtype=torch.bfloat16), torch.zeros(4096, device="cuda", dtype=torch.bfloat16))
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    h.gemm(p, D, None, A, B)
+    h.device_status()
+    used = free - torch.cuda.mem_get_info()[0]
+    # six bytes an element and pieces or copies of every other operand's matrix, partial sums, allocation granules
+    assert used <= 6 * (A.numel() + B.numel()) + (160 << 20)
+    a = A.view(-1, m, k).double()
+    b = B.view(-1, n, k).double().transpose(1, 2)
+    ref = a @ b
+    bound = (3.0 * k * 2.0 ** -24 if kernel != "bf16x3" else 2.0 ** -15) * (a.abs() @ b.abs()) + 2.0 ** -MANT[dtype] * ref.abs()
+    got = D.view(batch, n, m).transpose(1, 2).double()
+    assert bool(((got - ref).abs() <= bound).all())
+    h.close()
