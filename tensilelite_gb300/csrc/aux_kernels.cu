@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(256) split_kernel(const __grid_constant__ Spli
     const bool flat = o.rows % 4 == 0 && o.ld == o.rows && o.pld == o.rows &&
                       (o.batch == 1 || (o.batch_stride == o.rows * o.cols && o.p_batch_stride == o.batch_stride));
     const bool small = total < (int64_t(1) << 31);
-    bool vec = (reinterpret_cast<uintptr_t>(o.src) & 15) == 0 && o.ld % 4 == 0 && o.pld % 4 == 0 &&
+    bool vec = (reinterpret_cast<uintptr_t>(o.src) & 15) == 0 && (o.cols == 1 || (o.ld % 4 == 0 && o.pld % 4 == 0)) &&
                (o.batch == 1 || (o.batch_stride % 4 == 0 && o.p_batch_stride % 4 == 0));
 #pragma unroll
     for (int i = 0; i < NP; ++i) vec = vec && (reinterpret_cast<uintptr_t>(o.p[i]) & 7) == 0;

@@ -572,3 +572,16 @@ def test_one_matrix_for_a_whole_batch(dtype, kernel, k, which):
     got = D.view(batch, n, m).transpose(1, 2).double()
     assert bool(((got - ref).abs() <= bound).all())
     h.close()
+
+
+# ---- the two-piece split of a vector: counts that are no multiple of four are read by vectors as well ----
+def test_split_of_a_ragged_vector(h):
+    n = (1 << 26) + 3
+    x = torch.randn(n, device="cuda")
+    hi, lo = (torch.empty(n, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    split = lambda count: h.split_bf16x2(x, count, hi, lo)
+    split(n)
+    want = x.bfloat16()
+    assert torch.equal(hi.view(torch.int16), want.view(torch.int16))
+    assert torch.equal(lo.view(torch.int16), (x - want.float()).bfloat16().view(torch.int16))
+    assert _median_us(lambda: split(n)) <= 1.3 * _median_us(lambda: split(n - 3))
