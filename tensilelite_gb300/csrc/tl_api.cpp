@@ -44,7 +44,9 @@ struct Plan {
     bool view;
 };
 constexpr size_t kMaxPlans = 4096;
-constexpr uint64_t kPoolKeep = uint64_t(4) << 30;
+// What the call scratch's pool keeps between synchronisations: the pieces of fp32 operands of up to 1.7e8
+// elements (8192 x 8192 by 8192 x 8192: 0.8 GB).
+constexpr uint64_t kPoolKeep = uint64_t(1) << 30;
 }  // namespace tl
 
 struct tl_handle {
@@ -554,7 +556,18 @@ tl_status ensure_ws(tl_handle* h, size_t bytes)
     }
     size_t want = std::max<size_t>(bytes, 1 << 20);
     cudaError_t e = cudaMalloc(&h->ws, want);
-    if (e != cudaSuccess) return fail(TL_ERR_ALLOC, "workspace allocation failed");
+    if (e != cudaSuccess && h->pool) {
+        // what finished calls left with the pool
+        cudaGetLastError();
+        cudaDeviceSynchronize();
+        cudaMemPoolTrimTo(h->pool, 0);
+        e = cudaMalloc(&h->ws, want);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        h->ws = nullptr;
+        return fail(TL_ERR_ALLOC, "workspace allocation failed");
+    }
     h->ws_bytes = want;
     return TL_SUCCESS;
 }

@@ -585,3 +585,22 @@ def test_split_of_a_ragged_vector(h):
     assert torch.equal(hi.view(torch.int16), want.view(torch.int16))
     assert torch.equal(lo.view(torch.int16), (x - want.float()).bfloat16().view(torch.int16))
     assert _median_us(lambda: split(n)) <= 1.3 * _median_us(lambda: split(n - 3))
+
+
+# ---- the call scratch's pool keeps a bounded amount ----
+def test_call_scratch_is_given_back():
+    h = tl.Handle()
+    m, k = 8192, 24576                        # 2.4 GB of pieces
+    A, B = (torch.ones(m * k, device="cuda") for _ in range(2))
+    D = torch.empty(m * m, device="cuda")
+    p = tl.Problem.make(m, m, k, dtype="fp32", trans_a=True)
+    h.gemm(tl.Problem.make(1024, 1024, 1024, dtype="fp32", trans_a=True), D, None, A, B)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    h.gemm(p, D, None, A, B)
+    torch.cuda.synchronize()
+    h.gemm(tl.Problem.make(1024, 1024, 1024, dtype="fp32", trans_a=True), D, None, A, B)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= (1 << 30) + (64 << 20)
+    h.device_status()
+    h.close()
