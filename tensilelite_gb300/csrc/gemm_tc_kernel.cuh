@@ -471,7 +471,11 @@ __device__ __forceinline__ void lane_bias(const TcKernelParams& p, int M, int m,
 // type tests and both activations unrolled over 32 elements the two chunks of a 32-row linear layer
 // took 23000 clocks (11 us).  gelu(x) = x (1 + tanh u) / 2 = x / (1 + exp(-2u)): the form of silu,
 // without the cancellation of 1 + tanh at negative x.
-template <int W>
+// FULL, for fp32 outputs: the quotient without an overflow and corrected by its residual, as a correctly
+// rounded division's last step is (Markstein 1990).  The quick quotient is half a unit in the last place
+// worse (silu of N(0, 1) products, relative 2-norm 5.3e-8 against 4.2e-8), which narrower outputs round
+// away; there it saves 7 % of a 4096 x 1024 x 4096 layer.  A plain division's slow path costs the 32-row layer 10 us.
+template <int W, bool FULL>
 __device__ __forceinline__ void epi_apply(const TcKernelParams& p, int M, int m, bool row_ok, const float (&b)[W],
                                           float (&o)[W], float& amax)
 {
@@ -492,7 +496,13 @@ __device__ __forceinline__ void epi_apply(const TcKernelParams& p, int M, int m,
             for (int e = 0; e < 2; ++e) {
                 const float x = o[e];
                 const float t = gelu ? 1.5957691216057308f * fmaf(0.044715f * x * x, x, x) : x;
-                r[e] = __fdividef(x, 1.0f + expf(-t));   // 2 ulp; an infinite divisor gives 0 without a slow path
+                if constexpr (FULL) {
+                    const float z = expf(-fabsf(t)), y = 1.0f + z, num = t < 0.0f ? x * z : x;
+                    const float inv = __fdividef(1.0f, y), q = num * inv;
+                    r[e] = fabsf(q) < __int_as_float(0x7f800000) ? fmaf(fmaf(-q, y, num), inv, q) : q;
+                } else {
+                    r[e] = __fdividef(x, 1.0f + expf(-t));   // 2 ulp; an infinite divisor gives 0 without a slow path
+                }
             }
 #pragma unroll
             for (int k = 0; k < W - 2; ++k) o[k] = o[k + 2];
@@ -572,7 +582,7 @@ __device__ __forceinline__ void finish_values(const TcKernelParams& p, float& am
 #pragma unroll
         for (int i = 0; i < W; ++i) o[i] *= j.alpha;      // no C: fp8 outputs take beta == 0
     }
-    if constexpr (EPI) epi_apply<W>(p, j.M, m, row_ok, bias, o, amax);
+    if constexpr (EPI) epi_apply<W, sizeof(TD) == 4>(p, j.M, m, row_ok, bias, o, amax);
 }
 
 // W finished values as the output's bytes: W words for fp32, W/2 for 16-bit types, W/4 for fp8.

@@ -604,3 +604,31 @@ def test_call_scratch_is_given_back():
     assert free - torch.cuda.mem_get_info()[0] <= (1 << 30) + (64 << 20)
     h.device_status()
     h.close()
+
+
+# ---- fused activations with an fp32 output: as exact as plain fp32 arithmetic with a correctly rounded quotient ----
+@pytest.mark.parametrize("scale", [0.1, 1.0, 6.0])
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+def test_activation_of_fp32_outputs(h, act, scale):
+    m, n, k = 1024, 512, 64
+    g = torch.Generator(device="cuda").manual_seed(1)
+    A = (torch.randn(m * k, device="cuda", generator=g) * scale).bfloat16()
+    B = (torch.randn(n * k, device="cuda", generator=g) / 8).bfloat16()
+    x, D = torch.empty(m * n, device="cuda"), torch.empty(m * n, device="cuda")
+    p = tl.Problem.make(m, n, k, dtype="bf16", out_dtype="fp32", trans_a=True)
+    h.gemm(p, x, None, A, B)
+    h.gemm_ex(p, D, None, A, B, activation=act)
+    h.device_status()
+    f = (lambda v: 0.7978845608028654 * 2 * (v + 0.044715 * v * v * v)) if act == "gelu" else (lambda v: v)
+    ref = x.double() / (1 + torch.exp(-f(x.double())))
+    plain = x / (1 + torch.exp(-f(x)))
+    err = lambda v: float((v.double() - ref).norm() / ref.norm())
+    assert err(D) <= 1.05 * err(plain)
+    edge = torch.tensor([float("inf"), float("nan"), -87.9, -1e4, 0.0, -0.0], device="cuda")
+    A1, B1 = torch.zeros(64 * 64, device="cuda").bfloat16(), torch.zeros(64 * 64, device="cuda").bfloat16()
+    E, bias = torch.empty(64 * 64, device="cuda"), torch.zeros(64, device="cuda")
+    bias[:6] = edge
+    h.gemm_ex(tl.Problem.make(64, 64, 64, dtype="bf16", out_dtype="fp32", trans_a=True), E, None, A1, B1, bias=bias,
+              activation=act)
+    e = E[:6]
+    assert float(e[0]) == float("inf") and bool(torch.isnan(e[1])) and abs(float(e[2])) < 1e-35 and not e[3:].any()
