@@ -1686,6 +1686,7 @@ __global__ void __launch_bounds__(tc_threads(MODE), 1) tc_gemm_kernel(const __gr
                                         j.ldc, m + nst * GC, cl);
                         }
                     }
+                    __syncwarp();        // tcgen05.ld is for the whole warp; the loads above are not
                     // only a group of one-byte outputs can be partial (every tile is whole pairs of chunks)
                     const int nq = sizeof(TD) == 1 ? min(GC, p.bm - g * GC) / WQ : GC / WQ;
 #pragma unroll 1
