@@ -567,10 +567,6 @@ def _mm_rowmajor(X, W, trans_x=False, trans_w=False):
     return Y
 
 
-class _Matmul:
-    pass
-
-
 def _make_autograd():
     import torch
 

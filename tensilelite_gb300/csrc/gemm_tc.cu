@@ -7,22 +7,21 @@
 // full/empty mbarriers; its math waves (LDS -> VGPR -> MFMA into AccVGPRs, :433-466/:1403-1547)
 // become one thread issuing tcgen05.mma from shared-memory descriptors into a TMEM accumulator;
 // its fused epilogue (beta*C pre-scaled, fma(alpha, acc, beta*C), convert, store; :1572-1768,
-// :1822-1906) becomes four warps draining TMEM with tcgen05.ld while the next tile accumulates into
-// the second TMEM buffer.
+// :1822-1906) becomes eight warps draining TMEM with tcgen05.ld while the next tile accumulates into
+// the second TMEM buffer (four or sixteen where accumulation is promoted, see MODE in the kernel).
 //
 // Roles (320 threads, one CTA per SM, persistent over work units):
 //   warp 0     TMA producer (one lane): per k-block one box of B (128 n-rows) and one of A (bm m-rows)
 //   warp 1     TMEM allocator + MMA issuer (one lane): 4 tcgen05.mma per k-block, commit -> empty
 //   warps 2-9  epilogue: TMEM lane = problem n, TMEM column = problem m, so each thread owns a
-//              contiguous run of m for one n -- column-major D rows are written as 16-byte vectors.
-//              (The promotion kernels have four epilogue warps with 128 running sums per thread.)
+//              contiguous run of m for one n -- staged in shared memory and written as whole lines.
 // The problem's B^T is the MMA "A" operand (M = 128 along n) and A is the MMA "B" operand
 // (N = bm along m).  K-major operands (TN, the reference's layout) and MN-major operands (NN/NT)
 // are both read straight from global memory by TMA with 128-byte swizzling; no transpose pass.
 //
-// Work unit = (tile, k-split).  Split-k partials go to a workspace; the last CTA to finish a tile
-// (arrival counter) sums the partials in split order and runs the epilogue, so results do not
-// depend on scheduling.  The grouped variant walks a problem table with per-problem TMA maps.
+// Work unit = (tile, k-split).  Split-k partials go to a workspace and are summed in split order, by the
+// last CTA to finish a tile (arrival counter) or by all of the tile's, a share each (split_finish), so
+// results do not depend on scheduling.  The grouped variant walks a problem table with per-problem TMA maps.
 //
 // Every mbarrier wait is bounded (globaltimer); on expiry the kernel sets *err and returns.
 
@@ -248,8 +247,6 @@ int tc_workers(int in_dtype, int out_dtype, int cl, int bm, int stages, int sm_c
     return persistent_workers(in_dtype, out_dtype, cl, 0, sm_count, tc_smem_bytes(bm / cta_group, stages));
 }
 
-int tc_tmem_cols(int bm) { return (2 * bm <= 128) ? 128 : (2 * bm <= 256 ? 256 : 512); }
-
 tl_status tc_encode_operand(CUtensorMap* tm, int in_dtype, const TcOperand& op, int64_t K, int64_t batch,
                             int box_rows)
 {
@@ -360,7 +357,6 @@ tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launch
     kp.tile_rows = kTcTileN * cg;
     kp.tiles_n = static_cast<int>((L.N + kp.tile_rows - 1) / kp.tile_rows);
     kp.num_kb = static_cast<int>((L.K + W - 1) / W);
-    kp.kb_elems = W;
     kp.promote_kb = L.promote_k > 0 ? static_cast<int>((L.promote_k + W - 1) / W) : 0;
     kp.promote_half = pieces > 1 && !shared && L.promote_k > 0 && L.promote_k <= W / 2 ? 1 : 0;
     // Shared pieces of bf16x6 have the time for shorter chains than asked for: every MMA into a chain drops
@@ -496,7 +492,6 @@ tl_status tc_grouped_launch(const TcGroupLaunch& G, cudaStream_t stream, int64_t
     kp.split_units = 0;
     kp.split_tiles = 0;
     kp.tail_split = 1;
-    kp.kb_elems = kTcRowBytes / dtype_bytes(G.in_dtype);
     kp.stride_c = 0;
     kp.stride_d = 0;
     kp.n_mn_major = G.n_mn_major;

@@ -66,7 +66,6 @@ struct TcKernelParams {
     int bal_workers;
     int bal_stride;
     int num_kb;
-    int kb_elems;          // k elements per k-block (one 128-byte row)
     uint32_t idesc;
     uint32_t n_lbo, m_lbo, n_kstep, m_kstep;
     int n_mn_major, m_mn_major;

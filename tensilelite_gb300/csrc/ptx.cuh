@@ -351,18 +351,6 @@ __device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v)
 {
     asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ uint32_t ld_shared_u16(uint32_t addr)
-{
-    uint16_t v;
-    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(v) : "r"(addr));
-    return v;
-}
-__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr)
-{
-    uint32_t v;
-    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
 // 16-byte global -> shared copy without a register round trip (completion per thread, by group)
 __device__ __forceinline__ void cp_async16(uint32_t smem_addr, const void* gptr)
 {

@@ -947,19 +947,22 @@ tl_status enqueue(tl_handle* h, const Prepared& P, cudaStream_t s, const SimtLau
 }
 
 // ---- plain fp32 on the tensor cores ---------------------------------------------------------------
-// A large fp32 GEMM left to the library (kernel AUTO, no solution, none tuned) runs as the six products
-// of three bf16 pieces per operand, whose error against 64 bits is below the CUDA-core kernel's (normal
-// values, relative 2-norm, 4096^3: 1.6e-7 against 1.15e-6; 1024^3: 0.9e-7 against 2.1e-7; 672^3: 0.9e-7
-// against 1.75e-7) and which takes a fifth of its time (4096^3 TN: 490 us against 2770; 1024^3: 33 against
-// 80).  Below kFp32TcWork multiply-adds, twice that where k is one or two k-blocks, the split pass and the
-// extra launches cost more than that gives (672^3: 29 us against 30; 512 x 1024 x 600: 28.6 either way;
-// 2048 x 2048 x 80: 24 against 22; 480 x 512 x 512: 12.5 on the CUDA cores).
+// A large fp32 GEMM left to the library (kernel AUTO, no solution) runs as the six products of three bf16
+// pieces per operand, whose error against 64 bits is below the CUDA-core kernel's but for values of one sign
+// and short k (fp32_chain; normal values, relative 2-norm, 4096^3: 1.6e-7 against 1.15e-6; 1024^3: 0.9e-7
+// against 2.1e-7; 700^3: 0.8e-7 against 1.8e-7) and which takes a fifth of its time (4096^3 TN: 517 us on end, 558 padded
+// as a case of its own, against 2737; 1024^3: 33 against 79).  Below kFp32TcWork multiply-adds, twice that where
+// k is one or two k-blocks, the split pass and the extra launches cost more than that gives (672^3: 28.4 us
+// against 29.4; 512 x 1024 x 600: 28.6 either way; 2048 x 2048 x 80: 24 against 22; 480 x 512 x 512: 12.5 on the
+// CUDA cores).
 //
 // The pieces stand for the operands only within a range of magnitudes (split_range_ok), which is known
-// on the device once the split passes have run: infinities, NaN, numbers near fp32's limits.  So the
+// on the device once the split passes have run: infinities, NaN, numbers near fp32's largest, and numbers so
+// small that a product of the smallest magnitudes of A and of B is below 2^-100.  So the
 // launches follow each other: the split passes report the magnitudes, the tensor-core launch returns at once
 // if they are out of range, and the CUDA-core launch returns at once if they are not.  What is out of
-// range therefore gets the CUDA-core kernel's results, bit for bit.
+// range therefore gets the CUDA-core kernel's results, bit for bit, and pays for the passes before it
+// (700^3 42 us for 30, 1024^3 92 for 79, 4096^3 2848 for 2759).
 //
 // Each call has its own scratch, allocated and freed in stream order, and none of its CTAs relies on
 // another's start (tc_par_reduce), so calls on different streams are as independent as with the CUDA-core
@@ -1055,11 +1058,11 @@ tl_status gemm_fp32_tc(tl_handle* h, const Prepared& P, cudaStream_t s, bool* do
 // to the library (kernel AUTO, no solution, none tuned), runs on aligned copies of those operands: one
 // pass over memory instead of a CUDA-core kernel at a thirtieth of the tensor cores' rate (2047^3: 556
 // -> 43 us, 129 x 257 x 8191: 294 -> 26).  Its chains are promoted every 256 k into fp32 registers: the
-// error against 64 bits stays that of the output's rounding (1.6566e-3 for bf16 by either kernel; an
-// fp32 output would show the chains, and keeps the CUDA cores).  Below kPad16Work multiply-adds the
+// error against 64 bits stays that of the output's rounding (bf16 1.6565e-3 by either kernel; fp16
+// 2.0730e-4, of one sign 2.2050e-4 for 2.2050e-4, where the chains are 3e-7 low; an fp32 output would show
+// them, and keeps the CUDA cores).  Below kPad16Work multiply-adds the
 // copies and the scratch cost more than that gives (401 x 501 x 511: 23.2 us against 21.0; 501 x 601 x
-// 501: 22.7 against 23.6).  Scratch,
-// captures and a scratch that cannot be had: as for fp32 above.
+// 501: 22.7 against 23.6).  Scratch, captures and a scratch that cannot be had: as for fp32 above.
 constexpr double kPad16Work = 1.5e8;
 // Outputs from which on a D that is not whole vectors goes through a copy of its own instead of being
 // stored element by element (2047^3: 67 -> 43 us, 4097 x 4095 x 511: 154 -> 59, 601 x 701 x 601: 25.9 ->

@@ -173,7 +173,6 @@ bool tc_vec_output(int out_dtype, int64_t rows, const void* D, int64_t ldd, cons
                    int64_t stride_d, int64_t stride_c);
 // Persistent workers (CTAs, or co-resident clusters of `cl` CTAs) a tensor-core launch gets.
 int tc_workers(int in_dtype, int out_dtype, int cl, int bm, int stages, int sm_count);
-int tc_tmem_cols(int bm);
 tl_status tc_gemm_launch(const TcLaunch& L, cudaStream_t stream, int64_t* launches);
 // Checks a tcgen05 GEMM and fills its launch description without allocating anything; the caller
 // provides err, workspace and counters (sizes reported in ws_bytes / counter_count).
