@@ -177,7 +177,8 @@ TL_API tl_status tl_device_info(tl_handle* handle, int* sm_count, int* cc_major,
  * column-major leading dimensions, alpha = 1, beta = 0, scales = 1, kernel = AUTO, RNE. */
 TL_API tl_status tl_problem_init(tl_gemm_problem* problem, tl_dtype dtype_ab, tl_dtype dtype_cd,
                                  tl_op trans_a, tl_op trans_b, int64_t m, int64_t n, int64_t k);
-/* Heuristic solution for a problem (no timing).  Replaces GemmMfmaSolver::generateSolver. */
+/* Heuristic solution for a problem (no timing).  Replaces GemmMfmaSolver::generateSolver.  For a plain fp32
+ * problem it names the CUDA-core kernel, also where tl_gemm without a solution runs on the tensor cores. */
 TL_API tl_status tl_default_solution(tl_handle* handle, const tl_gemm_problem* problem,
                                      tl_gemm_solution* solution);
 /* Legality of a solution for a problem (tile shape, smem/TMEM budget, alignment, k split);
